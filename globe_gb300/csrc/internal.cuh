@@ -64,6 +64,7 @@ struct Genetic {
     uint8_t* blk1 = nullptr;   // SNP-major: every genotype kernel (built at load)
     uint8_t* blk2 = nullptr;   // individual-major: tensor-core pass 2, GRM build (first use)
     int nch1 = 0, ntiles1 = 0, nch2 = 0, ntiles2 = 0;
+    int f64_tc = 0;            // FP64 products on the tensor cores: 0 not tried, 1 run, -1 no memory for them
     // dense source
     float* grm = nullptr;    // N(N+1)/2
     // digit planes of the dense GRM for the tensor-core product (first GLOBE_PREC_MIXED use):
@@ -113,6 +114,8 @@ struct globe_ctx {
     globe::Genetic gen;
     double vc[5] = {0, 0, 0, 0, 0};
     bool vc_set = false;
+    int in_solve = 0;             // inside a call that repeats its products (SolveScope)
+    bool tc_used = false;         // a tensor-core product was launched since the error word was last read
     int prec = GLOBE_PREC_FP64;   // precision of operator calls (globe_set_precision / PCG options)
     int model = GLOBE_MODEL_FULL; // GLOBE_MODEL_NO_TIME: components (sig2e, sig2g) only
     int digits = 9;               // base-32 digits per column of the tensor-core product (globe_set_digits)
@@ -229,6 +232,15 @@ struct ProfScope {
     ~ProfScope() { prof_end(c, h); }
 };
 
+// Marks a call that repeats its GRM products (a solve), for the products' choice of kernel
+struct SolveScope {
+    globe_ctx* c;
+    explicit SolveScope(globe_ctx* ctx) : c(ctx) { ++c->in_solve; }
+    ~SolveScope() { --c->in_solve; }
+    SolveScope(const SolveScope&) = delete;
+    SolveScope& operator=(const SolveScope&) = delete;
+};
+
 // ---- bounds-checked debug build -------------------------------------------------
 // Built with -DGLOBE_CHECK_BOUNDS (e.g. GLOBE_BUILD_TAG=bounds GLOBE_NVCC_FLAGS=
 // -DGLOBE_CHECK_BOUNDS), the kernels check the indices they take from data (record
@@ -320,7 +332,7 @@ int pcg_update_df(globe_ctx* ctx, const float2* H, const float2* alpha, float2* 
                   const float2* Vp, float2* z, const int32_t* cols, int kact, double* rr, double* rz);
 
 // k_grm_geno.cu
-int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
+int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
 int geno_diag(globe_ctx* ctx, double* d);
 
 // k_grm_dense.cu
@@ -337,12 +349,13 @@ int ensure_blk1(globe_ctx* ctx);   // SNP-major tile-blocked copy; frees the com
 int ensure_blk2(globe_ctx* ctx);   // individual-major tile-blocked copy (first tensor-core use)
 int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, float min_maf, float max_miss,
                   int64_t* d_alt, int64_t* d_miss, float* d_maf, float* d_mr, uint8_t* d_keep, globe_bed_info* info);
-int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
+int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);    // GLOBE_PREC_MIXED
+int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);   // GLOBE_PREC_FP64
 int tc_err_word(globe_ctx* ctx, unsigned** err);   // the kernels' timeout word (cleared when created)
 int tc_check_error(globe_ctx* ctx);                 // reads and clears it: GLOBE_ERR_CUDA if set
 int tc_counters(globe_ctx* ctx, size_t n, unsigned** cnt);   // >= n zeroed per-column arrival counts
-// rc of a call at `precision`, or the tensor-core timeout behind it (the root cause) if one was set
-int with_tc_check(globe_ctx* ctx, int precision, int rc);
+// rc of a call, or the tensor-core timeout behind it (the root cause) if one was set
+int with_tc_check(globe_ctx* ctx, int rc);
 
 // solver.cu
 int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out);

@@ -417,7 +417,7 @@ extern "C" int globe_grm_build_dev(globe_ctx* ctx, float* d_lt) {
     GLOBE_RET(grm_ready(ctx));
     if (!d_lt) return set_err(ctx, GLOBE_ERR_ARG, "globe_grm_build_dev: null output");
     ProfScope p(ctx, GLOBE_PROF_GRM_BUILD);
-    if (ctx->prec == GLOBE_PREC_MIXED) return with_tc_check(ctx, GLOBE_PREC_MIXED, grm_build_tc(ctx, d_lt));
+    if (ctx->prec == GLOBE_PREC_MIXED) return with_tc_check(ctx, grm_build_tc(ctx, d_lt));
     return grm_build_f64(ctx, d_lt);
 }
 

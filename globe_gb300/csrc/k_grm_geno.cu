@@ -1,4 +1,6 @@
-// k_grm_geno.cu -- on-the-fly genotype GRM product in FP64 (the plain path).
+// k_grm_geno.cu -- on-the-fly genotype GRM product on the FP64 pipe: the small GLOBE_PREC_FP64
+// products, and all of them where the second genotype copy does not fit (geno_apply_f64 in
+// k_tc_geno.cu chooses).
 //
 //   out (N x k) = scale * Zs' (Zs Z),  zs(s,i) = (g - 2 f_s) inv_std_s,
 //   missing -> g = 0, scale = sig2g / M            (PCGsolver.cpp:1130-1201)
@@ -187,7 +189,7 @@ static int geno_chunk(globe_ctx* ctx, const double* Z, int kc, double scale, dou
     return GLOBE_OK;
 }
 
-int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
     if (g.Mk == 0) {

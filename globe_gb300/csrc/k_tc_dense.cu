@@ -362,6 +362,7 @@ static int launch_dense(globe_ctx* ctx, const CUtensorMap& mA, const CUtensorMap
     const int splits = (nchunks + cps - 1) / cps;
     const dim3 grid((unsigned)(rows / DROWS), (unsigned)splits);
     k_tc_dense<NMMA><<<grid, 256, smem, ctx->stream>>>(mA, mB, rows, nchunks, cps, part, ldp, err, stall);
+    ctx->tc_used = true;
     GLOBE_LAUNCHED(ctx, "k_tc_dense");
     return GLOBE_OK;
 }

@@ -496,6 +496,168 @@ __global__ void k_combine2(const float* __restrict__ part, int nsplit, int nmma,
     }
 }
 
+// ---- the FP64 product's statistics and epilogues ------------------------------
+//
+// GLOBE_PREC_FP64 runs the same two passes with ND64 = 12 digits (columns held to 2^-60 of
+// their largest entry).  What the mixed form rounds around the integer products is carried in
+// double-double here: the centring terms 2 f S and sum 2 f u cancel the uncentred products to
+// a few hundredths or less (S is the exact integer column sum of the digits, isum), so they
+// are subtracted before the one rounding.  Pass 1 works on z 2^-e (u stays at that scale, and
+// e enters once, in the last multiplication), so no column's magnitude leaves the range of a
+// double on the way.  The epilogues read 4 bytes x ND64 x splits per value and are bound by
+// those loads.  N = 20k, M = 20k, k = 5: 148 us a product, 14.5 ms on the FP64 pipe
+// (k_geno_p1 / p2, which it replaces from geno_apply_f64's sizes on).
+
+__device__ __forceinline__ double warp_max_bits(double m) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = absmax_bits(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
+// (h, l) += (a, b): two-sum of the high parts, everything else into l
+__device__ __forceinline__ void dd_add(double& h, double& l, double a, double b) {
+    const double s = __dadd_rn(h, a), bp = __dsub_rn(s, h);
+    l = __dadd_rn(l, __dadd_rn(b, __dadd_rn(__dsub_rn(h, __dsub_rn(s, bp)), __dsub_rn(a, bp))));
+    h = s;
+}
+// colinfo = {scale exponent, 0 or NaN} from max |x| (its bits: NaN and infinity win)
+__device__ __forceinline__ void col_info64(double mx, double* __restrict__ colinfo) {
+    const bool bad = !isfinite(mx);
+    int E = 0;
+    if (!bad && mx > 0) frexp(mx, &E);
+    colinfo[0] = bad ? 0.0 : (double)(E - (DBITS - 1));
+    colinfo[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+}
+
+// max |x| of each column; the column's last CTA forms colinfo[c] and clears isum for k_digits
+__global__ void k_col_max64(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
+                            unsigned* __restrict__ cnt, double* __restrict__ colinfo,
+                            unsigned long long* __restrict__ isum) {
+    __shared__ double smx[8];
+    __shared__ bool last;
+    const int c = blockIdx.y, nparts = (int)gridDim.x;
+    double mx = 0;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+        mx = absmax_bits(mx, X[r + c * ld]);
+    mx = warp_max_bits(mx);
+    if ((threadIdx.x & 31) == 0) smx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = absmax_bits(mx, smx[w]);
+        pmax[blockIdx.x + (size_t)c * nparts] = mx;
+        __threadfence();
+        last = atomicAdd(&cnt[c], 1u) == (unsigned)nparts - 1u;
+    }
+    __syncthreads();
+    if (last && threadIdx.x < 32) {
+        __threadfence();
+        mx = 0;
+        for (int j = threadIdx.x; j < nparts; j += 32) mx = absmax_bits(mx, __ldcg(pmax + j + (size_t)c * nparts));
+        mx = warp_max_bits(mx);
+        if (threadIdx.x == 0) {
+            col_info64(mx, colinfo + 2 * c);
+            isum[2 * c] = isum[2 * c + 1] = 0ull;
+            cnt[c] = 0u;
+        }
+    }
+}
+
+// pass-1 epilogue: u = inv^2 (P1 - 2 f S) at the scale 2^-e of column c; per CTA max |u| and
+// sum 2 f u (double-double), and from the column's last CTA colinfo2[c] and the centring term
+// c2[2c], c2[2c+1]
+__global__ void __launch_bounds__(256) k_combine1_64(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                                     int64_t rows, const double* __restrict__ colinfo,
+                                                     const long long* __restrict__ isum, const double* __restrict__ f,
+                                                     const double* __restrict__ inv, double* __restrict__ U,
+                                                     double* __restrict__ pmax, double* __restrict__ psum,
+                                                     unsigned* __restrict__ cnt, double* __restrict__ colinfo2,
+                                                     double* __restrict__ c2) {
+    __shared__ double smx[8], ssh[8], ssl[8];
+    __shared__ bool last;
+    const int c = blockIdx.y, nparts = (int)gridDim.x;
+    const double bad = colinfo[2 * c + 1];   // 0, or NaN
+    const double Sh = ll_times_pow2(isum[2 * c], 0x1p-25), Sl = ll_times_pow2(isum[2 * c + 1], 0x1p-55);
+    double mx = 0, sh = 0, sl = 0;
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
+        long long hi, lo;
+        recombine_int<ND64>(part, nsplit, nmma, ldp, c, s, hi, lo);
+        const double f2 = 2.0 * f[s], iv = inv[s];
+        const double p = __dmul_rn(f2, Sh), pe = __fma_rn(f2, Sh, -p);
+        double d = ll_times_pow2(hi, 0x1p-25), r = 0.0;
+        dd_add(d, r, -p, __dsub_rn(ll_times_pow2(lo, 0x1p-55), __fma_rn(f2, Sl, pe)));
+        const double u = iv * iv * (d + r) + bad;
+        U[s + c * rows] = u;
+        mx = absmax_bits(mx, u);
+        const double t = __dmul_rn(f2, u);
+        dd_add(sh, sl, t, __fma_rn(f2, u, -t));
+    }
+    mx = warp_max_bits(mx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double a = __shfl_xor_sync(0xffffffffu, sh, o), b = __shfl_xor_sync(0xffffffffu, sl, o);
+        dd_add(sh, sl, a, b);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        const int w = threadIdx.x >> 5;
+        smx[w] = mx;
+        ssh[w] = sh;
+        ssl[w] = sl;
+    }
+    __syncthreads();
+    const size_t o0 = (size_t)c * nparts;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+            mx = absmax_bits(mx, smx[w]);
+            dd_add(sh, sl, ssh[w], ssl[w]);
+        }
+        pmax[o0 + blockIdx.x] = mx;
+        psum[2 * (o0 + blockIdx.x)] = sh;
+        psum[2 * (o0 + blockIdx.x) + 1] = sl;
+        __threadfence();
+        last = atomicAdd(&cnt[c], 1u) == (unsigned)nparts - 1u;
+    }
+    __syncthreads();
+    if (last && threadIdx.x < 32) {
+        __threadfence();
+        mx = sh = sl = 0;
+        for (int j = threadIdx.x; j < nparts; j += 32) {
+            mx = absmax_bits(mx, __ldcg(pmax + o0 + j));
+            dd_add(sh, sl, __ldcg(psum + 2 * (o0 + j)), __ldcg(psum + 2 * (o0 + j) + 1));
+        }
+        mx = warp_max_bits(mx);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double a = __shfl_xor_sync(0xffffffffu, sh, o), b = __shfl_xor_sync(0xffffffffu, sl, o);
+            dd_add(sh, sl, a, b);
+        }
+        if (threadIdx.x == 0) {
+            col_info64(mx, colinfo2 + 2 * c);
+            c2[2 * c] = sh;
+            c2[2 * c + 1] = sl;
+            cnt[c] = 0u;
+        }
+    }
+}
+
+// pass-2 epilogue: out[i,c] = scale 2^e (P2 - sum 2 f u), 2^e in two factors
+__global__ void __launch_bounds__(256) k_combine2_64(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                                     int64_t rows, const double* __restrict__ colinfo1,
+                                                     const double* __restrict__ colinfo2, const double* __restrict__ c2,
+                                                     double scale, double* __restrict__ out, int64_t ldo) {
+    const int c = blockIdx.y;
+    double s_hi, s_lo;
+    recombine_scales<ND64>((int)colinfo2[2 * c], s_hi, s_lo);
+    const int e = (int)colinfo1[2 * c];
+    const double ea = ldexp(1.0, e / 2), eb = ldexp(1.0, e - e / 2);
+    const double Ch = c2[2 * c], Cl = c2[2 * c + 1], bad = colinfo2[2 * c + 1];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
+        long long hi, lo;
+        recombine_int<ND64, 4>(part, nsplit, nmma, ldp, c, i, hi, lo);
+        double d = ll_times_pow2(hi, s_hi), r = 0.0;
+        dd_add(d, r, -Ch, __dsub_rn(ll_times_pow2(lo, s_lo), Cl));
+        out[i + c * ldo] = scale * (d + r) * ea * eb + bad;
+    }
+}
+
 // blk2 from blk1 by 2-bit block transposes.  blk1 block (t1, c1) holds SNP rows 128 t1 .. + 127
 // and individuals 128 c1 .. + 127 (32 bytes per row); blk2 block (t2, c2) holds individual rows
 // 128 t2 .. and SNPs 128 c2 .. -- the transpose of blk1 block (c2, t2).  Blocks of blk2 past blk1's
@@ -689,6 +851,7 @@ static int launch_gemm(globe_ctx* ctx, const uint8_t* blk, int ntiles, const CUt
     dim3 grid((unsigned)((rows + G::MT * BM - 1) / (G::MT * BM)), (unsigned)splits, (unsigned)zg.nz);
     k_tc_gemm<NMMA><<<grid, G::NTHREADS, smem, ctx->stream>>>(blk, mB, rows, nchunks, cps, part, ldp, zg.pz,
                                                                zg.skip0, zg.skipz, err, zg.stall);
+    ctx->tc_used = true;
     GLOBE_LAUNCHED(ctx, "k_tc_gemm");
     return GLOBE_OK;
 }
@@ -853,6 +1016,7 @@ static int tune_splits(globe_ctx* ctx, int pass, int nmma, const uint8_t* blk, i
 }
 
 // out (N x k) = scale * Zs'(Zs Z) for one group of <= 256 / ND columns, ND digits per column
+// (ND64: the FP64 product, with its own statistics and epilogues)
 template <int ND>
 static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out) {
     auto& g = ctx->gen;
@@ -883,12 +1047,15 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     GLOBE_RET(ws(ctx, WS_TC_P1, (size_t)(spmax1 + 1) * nmma * ldp1, &P1));
     GLOBE_RET(ws(ctx, WS_TC_P2, (size_t)(spmax2 + 1) * nmma * ldp2, &P2));
     GLOBE_RET(ws(ctx, WS_TC_U, (size_t)g.Mk * kg + 1, &U));
+    constexpr bool F64 = ND == ND64;
     const int nbr = 304;
-    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(4 * kg + 2 * nbr * kg + 8), &cst));
+    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(8 * kg + 3 * nbr * kg + 8), &cst));
     double* col1 = cst;           // 2*kg
     double* col2 = cst + 2 * kg;  // 2*kg
-    pm = cst + 4 * kg;
-    ps = pm + (size_t)nbr * kg;
+    double* c2 = cst + 4 * kg;    // 2*kg, F64: sum 2 f u in double-double
+    unsigned long long* isum = reinterpret_cast<unsigned long long*>(cst + 6 * kg);   // 2*kg, F64: column sums of digits
+    pm = cst + 8 * kg;
+    ps = pm + (size_t)nbr * kg;   // nbr*kg (F64: twice that)
     GLOBE_RET(tc_err_word(ctx, &err));
     CUtensorMap mB1, mB2;
     GLOBE_RET(make_map(ctx, &mB1, D1, (uint64_t)kpad1, (uint64_t)nmma, BK, (uint32_t)nmma, true));
@@ -897,14 +1064,15 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     const int nz = col_parts(N);
     unsigned* cnt;
     GLOBE_RET(tc_counters(ctx, 2 * kg, &cnt));
-    k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col1);
+    if constexpr (F64) k_col_max64<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, cnt, col1, isum);
+    else k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col1);
     GLOBE_LAUNCHED(ctx, "k_col_maxsum");
     // digit rows past the kg columns stay zero
     if (nmma > kg * ND)
         GLOBE_CK(ctx, cudaMemsetAsync(D1 + (size_t)kg * ND * kpad1, 0, (size_t)(nmma - kg * ND) * kpad1,
                                       ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad1 / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, kg, col1, D1, kpad1);
+        Z, N, N, kg, col1, D1, kpad1, F64 ? isum : nullptr);
     GLOBE_LAUNCHED(ctx, "k_digits");
     // ---- pass 1
     int sp1 = 0;
@@ -917,15 +1085,20 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
         GLOBE_RET(gemm_dispatch(ctx, nmma, g.blk1, g.ntiles1, mB1, (int)g.Mk, nch1, sp1, P1, ldp1, err, zg));
     }
     const int sp1e = eff_splits(nch1, sp1);
-    k_combine1<ND><<<dim3(nbr, kg), 256, 0, ctx->stream>>>(P1, sp1e, nmma, ldp1, g.Mk, kg, col1, g.f, g.inv, U, pm, ps,
-                                                           cnt + kg, col2);
+    if constexpr (F64)
+        k_combine1_64<<<dim3(std::min(nbr, div_up(g.Mk, 256)), kg), 256, 0, ctx->stream>>>(
+            P1, sp1e, nmma, ldp1, g.Mk, col1, reinterpret_cast<const long long*>(isum), g.f, g.inv, U, pm, ps, cnt + kg,
+            col2, c2);
+    else
+        k_combine1<ND><<<dim3(nbr, kg), 256, 0, ctx->stream>>>(P1, sp1e, nmma, ldp1, g.Mk, kg, col1, g.f, g.inv, U, pm,
+                                                               ps, cnt + kg, col2);
     GLOBE_LAUNCHED(ctx, "k_combine1");
     // ---- digits of u, pass 2
     if (nmma > kg * ND)
         GLOBE_CK(ctx, cudaMemsetAsync(D2 + (size_t)kg * ND * kpad2, 0, (size_t)(nmma - kg * ND) * kpad2,
                                       ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad2 / 4, 256), 2048), kg), 256, 0, ctx->stream>>>(
-        U, g.Mk, g.Mk, kg, col2, D2, kpad2);
+        U, g.Mk, g.Mk, kg, col2, D2, kpad2, nullptr);
     GLOBE_LAUNCHED(ctx, "k_digits");
     int sp2 = 0;
     GLOBE_RET(tune_splits(ctx, 2, nmma, g.blk2, g.ntiles2, mB2, N, nch2, cand2, P2, ldp2, err, &sp2));
@@ -934,8 +1107,11 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
         GLOBE_RET(gemm_dispatch(ctx, nmma, g.blk2, g.ntiles2, mB2, N, nch2, sp2, P2, ldp2, err, ZGrid()));
     }
     const int sp2e = eff_splits(nch2, sp2);
-    k_combine2<ND><<<dim3(div_up(N, 256) < 1024 ? div_up(N, 256) : 1024, kg), 256, 0, ctx->stream>>>(
-        P2, sp2e, nmma, ldp2, N, kg, col2, scale, out, N);
+    const dim3 g2((unsigned)std::min(div_up(N, 256), 1024), kg);
+    if constexpr (F64)
+        k_combine2_64<<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, col1, col2, c2, scale, out, N);
+    else
+        k_combine2<ND><<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, kg, col2, scale, out, N);
     GLOBE_LAUNCHED(ctx, "k_combine2");
     return GLOBE_OK;
 }
@@ -950,11 +1126,13 @@ static int tc_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double s
         case 7: return tc_group<7>(ctx, Z, kg, scale, out);
         case 8: return tc_group<8>(ctx, Z, kg, scale, out);
         case 9: return tc_group<9>(ctx, Z, kg, scale, out);
+        case ND64: return tc_group<ND64>(ctx, Z, kg, scale, out);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
 
-int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+// out (N x k) = scale * Zs'(Zs Z) with nd digits per column
+static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
     if (g.Mk == 0) {
@@ -962,7 +1140,6 @@ int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* 
         return GLOBE_OK;
     }
     GLOBE_RET(ensure_blk2(ctx));
-    const int nd = ctx->digits;
     // near-equal groups of <= 256 / nd columns (MMA width <= 256).  Groups wider than
     // 192 / nd (MMA width > 192) run one row tile per CTA, which costs more per column than
     // two groups of two tiles once k > 256 / nd: then groups of <= 192 / nd columns
@@ -1003,6 +1180,54 @@ int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* 
     return run(cand[best]);
 }
 
+int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+    return geno_apply_nd(ctx, ctx->digits, Z, k, scale, out);
+}
+
+// The FP64 product.  On the tensor cores (ND64 digits) it needs the individual-major copy and
+// ~7 short launches, ~60 us whatever its size while it is small; on the FP64 pipe
+// (k_grm_geno.cu) it needs neither and takes about N Mk k / 1.4e11 seconds above ~25 us (70 us
+// with more than one column).  So, by its size N Mk k (FP64 pipe / tensor cores, us a product):
+//  - inside a solve, which repeats the product, from where the two cross: 8e6 for one column
+//    (3e6: 40 / 62; 8e6: 66 / 68; 2e7: 136 / 72), 1e6 for more (7.5e5: 73 / 59; 4.5e6: 113 / 66;
+//    1e8: 696 / 82; 2e9: 14474 / 148);
+//  - a single operator call from F64_CALL_MIN on, where the first call, which also lays out the
+//    copy, costs about the same on either (4e7: 351 / 315; 2e7: 166 / 394; 2e8: 1317 / 526).
+// The choice depends on the sizes only.  Where the copy and the workspaces do not fit in free
+// device memory, the FP64 pipe runs (decided once per load of genotypes).
+// Error against 128-bit sums (N = 6000, M = 3000; normal, constant, count, lognormal, unit and
+// wide-range columns): 1.3e-16 to 1.9e-16 of the column, FP64 pipe 3.9e-16 to 1.1e-15.
+#ifndef F64_SOLVE_MIN
+#define F64_SOLVE_MIN (k == 1 ? 8e6 : 1e6)
+#endif
+#ifndef F64_CALL_MIN
+#define F64_CALL_MIN 4e7
+#endif
+int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+    auto& g = ctx->gen;
+    const int32_t N = ctx->coh.N;
+    const double size = (double)N * (double)g.Mk * k;
+    if (g.f64_tc >= 0 && size >= (ctx->in_solve ? F64_SOLVE_MIN : F64_CALL_MIN)) {
+        if (g.f64_tc == 0 && !g.blk2) {
+            // the copy, and at most ~16 split partials of 256 columns beside U, digits and the rest
+            const double need = (double)N * (double)g.Mk / 4 * 1.01 + 256.0 * 4 * 16 * (double)N +
+                                256.0 * (4 * 2 + 2 + 1) * (double)std::max<int64_t>(g.Mk, N) + (double)(1ull << 30);
+            size_t fr = 0, tot = 0;
+            GLOBE_CK(ctx, cudaMemGetInfo(&fr, &tot));
+            if (need > (double)fr) g.f64_tc = -1;
+        }
+        if (g.f64_tc >= 0) {
+            const int rc = geno_apply_nd(ctx, ND64, Z, k, scale, out);
+            if (rc != GLOBE_ERR_NOMEM) {
+                if (rc == GLOBE_OK) g.f64_tc = 1;
+                return rc;
+            }
+            g.f64_tc = -1;
+        }
+    }
+    return geno_apply_fp64_pipe(ctx, Z, k, scale, out);
+}
+
 // The tensor-core kernels' error word: word 0 of the WS_TC_ERR slot (words 1-2 serve
 // k_dense_absmax).  Cleared once, when the slot is created; the kernels only set bits in it
 // and tc_check_error reads and clears it, so a timeout in any product of a solve is still
@@ -1030,13 +1255,14 @@ int tc_check_error(globe_ctx* ctx) {
     if (!p) return GLOBE_OK;
     GLOBE_CK(ctx, cudaMemcpyAsync(&h, p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    ctx->tc_used = false;
     if (!h) return GLOBE_OK;
     GLOBE_CK(ctx, cudaMemsetAsync(p, 0, sizeof(unsigned), ctx->stream));
     return set_err(ctx, GLOBE_ERR_CUDA, "tensor-core GRM kernel timed out waiting (code 0x%x)", h);
 }
 
-int with_tc_check(globe_ctx* ctx, int precision, int rc) {
-    if (precision != GLOBE_PREC_MIXED) return rc;
+int with_tc_check(globe_ctx* ctx, int rc) {
+    if (!ctx->tc_used) return rc;
     const int rt = tc_check_error(ctx);
     return rt != GLOBE_OK ? rt : rc;
 }

@@ -95,9 +95,10 @@ int pcg_dev(globe_ctx* ctx, const double* B, double* X, int k, const globe_pcg_o
         return set_err(ctx, GLOBE_ERR_ARG, "unknown precision mode %d", o->precision);
     const int saved = ctx->prec;
     ctx->prec = o->precision;
+    SolveScope solve(ctx);
     const int rc = pcg_run(ctx, B, X, k, o, info);
     ctx->prec = saved;
-    return with_tc_check(ctx, o->precision, rc);
+    return with_tc_check(ctx, rc);
 }
 
 // Captures `body` (stream work only, nothing run) into a graph and makes ctx->pcg_graph[slot]
@@ -683,7 +684,7 @@ int globe_grm_apply(globe_ctx* ctx, const double* Z, double* out, int k) {
     GLOBE_RET(check_ready(ctx));
     size_t n = (size_t)ctx->coh.N * k;
     const int rc = host_io(ctx, Z, n, out, n, [&](double* a, double* b) { return grm_apply_dev(ctx, a, k, b); });
-    return with_tc_check(ctx, ctx->prec, rc);
+    return with_tc_check(ctx, rc);
 }
 
 int globe_vx_dev(globe_ctx* ctx, const double* d_x, double* d_out, int k) {
@@ -699,7 +700,7 @@ int globe_vx(globe_ctx* ctx, const double* x, double* out, int k) {
     GLOBE_RET(check_ready(ctx));
     size_t n = (size_t)ctx->coh.Nrec * k;
     const int rc = host_io(ctx, x, n, out, n, [&](double* a, double* b) { return vx_dev(ctx, a, k, b); });
-    return with_tc_check(ctx, ctx->prec, rc);
+    return with_tc_check(ctx, rc);
 }
 
 int globe_precond_apply(globe_ctx* ctx, const double* r, double* z, int k) {
@@ -987,7 +988,8 @@ static int aireml_eval_impl(globe_ctx* ctx, const double* probes, int numMC, uin
 struct PrecScope {
     globe_ctx* ctx;
     int saved;
-    PrecScope(globe_ctx* c, int p) : ctx(c), saved(c->prec) { c->prec = p; }
+    SolveScope solve;
+    PrecScope(globe_ctx* c, int p) : ctx(c), saved(c->prec), solve(c) { c->prec = p; }
     ~PrecScope() { ctx->prec = saved; }
 };
 
@@ -1007,7 +1009,7 @@ int globe_mme(globe_ctx* ctx, const globe_pcg_opts* opts, double* beta, double* 
         PrecScope ps(ctx, opts->precision);
         rc = mme_impl(ctx, opts, beta, uhat, bhat, vinv_r, info);
     }
-    return with_tc_check(ctx, opts->precision, rc);
+    return with_tc_check(ctx, rc);
 }
 
 int globe_aireml_grad(globe_ctx* ctx, const double* probes, int numMC, uint64_t seed, const globe_pcg_opts* opts,
@@ -1020,7 +1022,7 @@ int globe_aireml_grad(globe_ctx* ctx, const double* probes, int numMC, uint64_t 
         PrecScope ps(ctx, opts->precision);
         rc = aireml_grad_impl(ctx, probes, numMC, seed, opts, f_theta, first, trace, grad, info);
     }
-    return with_tc_check(ctx, opts->precision, rc);
+    return with_tc_check(ctx, rc);
 }
 
 int globe_aireml_eval(globe_ctx* ctx, const double* probes, int numMC, uint64_t seed, const globe_pcg_opts* opts,
@@ -1033,7 +1035,7 @@ int globe_aireml_eval(globe_ctx* ctx, const double* probes, int numMC, uint64_t 
         PrecScope ps(ctx, opts->precision);
         rc = aireml_eval_impl(ctx, probes, numMC, seed, opts, first, trace, grad, info);
     }
-    return with_tc_check(ctx, opts->precision, rc);
+    return with_tc_check(ctx, rc);
 }
 
 int globe_aireml_ai(globe_ctx* ctx, const globe_pcg_opts* opts, double* ai, globe_pcg_info* info) {

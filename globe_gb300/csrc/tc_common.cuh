@@ -23,6 +23,7 @@ constexpr int DBITS = 5;          // digit base 32
 constexpr int DHALF = 1 << (DBITS - 1);   // 16: digits in [-16, 16]
 constexpr int NDIG = 9;           // digits per right-hand-side column by default (45 bits)
 constexpr int MIN_DIG = 2;        // fewest digits a context may ask for (globe_set_digits)
+constexpr int ND64 = 12;          // digits per column of the GLOBE_PREC_FP64 products (59 bits: |I| < 2^59)
 
 // The tile-blocked genotype copies hold "tile codes", 2 bits per genotype like the PLINK
 // codes they are made from (re-encoded once, by recode_tile), equal to the genotype:
@@ -116,8 +117,8 @@ __device__ __forceinline__ double absmax_bits(double m, double v) {
 // With YU > 1, YU splits' ND loads issue together: k_combine2 reads 10 splits and waits on
 // them; k_combine1 reads 2, holds more registers, and runs faster one split at a time.
 template <int ND, int YU = 1>
-__device__ __forceinline__ double recombine(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int c,
-                                           int64_t row, double s_hi, double s_lo) {
+__device__ __forceinline__ void recombine_int(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int c,
+                                              int64_t row, long long& hi, long long& lo) {
     constexpr int NH = (ND + 1) / 2;
     long long pj[ND];
     if constexpr (YU == 1) {
@@ -148,11 +149,17 @@ __device__ __forceinline__ double recombine(const float* __restrict__ part, int 
                 }
         }
     }
-    long long hi = 0, lo = 0;
+    hi = lo = 0;
 #pragma unroll
     for (int j = 0; j < NH; ++j) hi = hi * (1 << DBITS) + pj[j];
 #pragma unroll
     for (int j = NH; j < ND; ++j) lo = lo * (1 << DBITS) + pj[j];
+}
+template <int ND, int YU = 1>
+__device__ __forceinline__ double recombine(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int c,
+                                           int64_t row, double s_hi, double s_lo) {
+    long long hi, lo;
+    recombine_int<ND, YU>(part, nsplit, nmma, ldp, c, row, hi, lo);
     return ll_times_pow2(hi, s_hi) + ll_times_pow2(lo, s_lo);
 }
 
@@ -189,13 +196,19 @@ __global__ void k_col_finish(const double* __restrict__ pmax, const double* __re
 // balanced base-32 digits are peeled off from the least significant end in integer
 // arithmetic (d = ((I + 16) mod 32) - 16, in [-16, 15]); the leading digit is what
 // remains, in [-16, 16].  sum_j d_j 32^-j equals x 2^-e rounded to 5 (ND-1) fraction bits.
+// With ND64 digits (the FP64 products) the scaling takes two factors where one would leave the
+// range of a double, and with isum the exact column sum of I is added to isum[2c] 2^30 +
+// isum[2c+1] (integer atomics: the same bits in any order).
 template <int ND, bool GENO>
 __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, int k, const double* __restrict__ colinfo,
-                         uint8_t* __restrict__ D, int64_t kpad) {
+                         uint8_t* __restrict__ D, int64_t kpad, unsigned long long* __restrict__ isum = nullptr) {
     const int c = blockIdx.y;
-    const double sc = ldexp(1.0, DBITS * (ND - 1) - (int)colinfo[2 * c]);   // a power of two: x * sc is exact
+    const int sh = DBITS * (ND - 1) - (int)colinfo[2 * c];
+    const double sc = ldexp(1.0, ND == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
+    const double sc2 = ND == ND64 ? ldexp(1.0, sh - min(sh, 1000)) : 1.0;
     const bool bad = isnan(colinfo[2 * c + 1]);   // non-finite column (k_col_finish): zero digits
     const int64_t nw = kpad >> 2;
+    long long sum_hi = 0, sum_lo = 0;
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
         const int64_t P = w << 2, base = P & ~(int64_t)15;
         const int pl = (int)(P & 15);
@@ -205,7 +218,13 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, in
         for (int q = 0; q < 4; ++q) {
             const int pq = pl + q;
             const int64_t src = base + (GENO ? 4 * q + (pl >> 2) : (pq < 8 ? 2 * pq : 2 * (pq - 8) + 1));
-            I[q] = (src < n && !bad) ? __double2ll_rn(X[src + c * ld] * sc) : 0ll;
+            double x = (src < n && !bad) ? X[src + c * ld] * sc : 0.0;
+            if (ND == ND64) x *= sc2;
+            I[q] = __double2ll_rn(x);
+            if (ND == ND64) {
+                sum_hi += I[q] >> 30;
+                sum_lo += I[q] & ((1ll << 30) - 1);
+            }
         }
         uint32_t word[ND];
 #pragma unroll
@@ -222,6 +241,17 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, in
         }
 #pragma unroll
         for (int j = 0; j < ND; ++j) *reinterpret_cast<uint32_t*>(D + ((int64_t)c * ND + j) * kpad + P) = word[j];
+    }
+    if (ND == ND64 && isum) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, o);
+            sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(isum + 2 * c, (unsigned long long)sum_hi);
+            atomicAdd(isum + 2 * c + 1, (unsigned long long)sum_lo);
+        }
     }
 }
 

@@ -46,7 +46,13 @@ extern "C" {
 #define GLOBE_ERR_UNSUPPORTED (-8) /* option not available for this input */
 
 /* precision of the GRM product and the solve's record arithmetic */
-#define GLOBE_PREC_FP64 0   /* plain FP64 everywhere (the drop-in path) */
+#define GLOBE_PREC_FP64 0   /* FP64 everywhere (the drop-in path).  Genotype GRM products of
+                               some size run as exact integer products on the tensor cores:
+                               each column rounded once to 12 base-32 digits (2^-60 of its
+                               largest entry), sums exact, centring in double-double, one
+                               final FP64 rounding -- closer to the exact product than sums
+                               on the FP64 pipe, which run where the product is small or the
+                               second genotype copy does not fit in device memory */
 #define GLOBE_PREC_MIXED 1  /* genotype GRM product on the FP8 tensor cores with exact
                                base-32 digit slicing of the right-hand sides (9 digits =
                                45 bits by default, matches FP64 to ~1e-13; see
