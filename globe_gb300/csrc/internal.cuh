@@ -67,12 +67,14 @@ struct Genetic {
     int f64_tc = 0;            // FP64 products on the tensor cores: 0 not tried, 1 run, -1 no memory for them
     // dense source
     float* grm = nullptr;    // N(N+1)/2
-    // digit planes of the dense GRM for the tensor-core product (first GLOBE_PREC_MIXED use):
-    // adig_da planes of adig_rows / adig_da rows x adig_np bytes, A ~ 2^adig_e sum_d a_d 32^-d
-    uint8_t* adig = nullptr;
-    int adig_state = 0;      // 0 not built, 1 ready, -1 unusable (memory, non-finite A): double-float kernel
-    int adig_da = 0, adig_e = 0;
-    int64_t adig_np = 0, adig_rows = 0;
+    // digit planes of the dense GRM for the tensor-core products: [0] GLOBE_PREC_MIXED, [1]
+    // GLOBE_PREC_FP64, each built on its first use
+    struct Planes {
+        uint8_t* p = nullptr;    // da planes of rows / da rows x np bytes, A ~ 2^e sum_d a_d 32^-d
+        int state = 0;           // 0 not built, 1 ready, -1 unusable (memory, non-finite A, FP64: row scales)
+        int da = 0, e = 0;
+        int64_t np = 0, rows = 0;
+    } adig[2];
     // both
     double* gdiag = nullptr; // A_ii
     bool gdiag_ok = false;
@@ -336,13 +338,13 @@ int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, d
 int geno_diag(globe_ctx* ctx, double* d);
 
 // k_grm_dense.cu
-int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
+int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
 int dense_apply_df(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
 int dense_diag(globe_ctx* ctx, double* d);
 
 // k_tc_dense.cu
-int dense_digit_planes(globe_ctx* ctx);   // (re)builds the digit planes for the context's digit count
-int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
+int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);    // GLOBE_PREC_MIXED
+int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);   // GLOBE_PREC_FP64
 
 // k_tc_geno.cu
 int ensure_blk1(globe_ctx* ctx);   // SNP-major tile-blocked copy; frees the compacted rows

@@ -1,6 +1,7 @@
-// k_grm_dense.cu -- dense GRM product from the packed lower triangle: FP64
-// (GLOBE_PREC_FP64), and double-float FP32 arithmetic for GLOBE_PREC_MIXED when the
-// tensor-core digit planes of k_tc_dense.cu cannot be held (device memory, non-finite A).
+// k_grm_dense.cu -- dense GRM product from the packed lower triangle, where the tensor-core
+// digit planes of k_tc_dense.cu do not serve: on the FP64 pipe for GLOBE_PREC_FP64 (small
+// products; planes that cannot be held or would not hold every row to FP64), and in
+// double-float FP32 arithmetic for GLOBE_PREC_MIXED (planes that cannot be held).
 //
 //   out (N x k) = scale * A Z,  A(i,j) = lt[max(i,j)(max(i,j)+1)/2 + min(i,j)]
 //   (PCGsolver.cpp:1202-1213, varCompEst.cpp:531-558)
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt,
     }
 }
 
-int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
     const int32_t N = ctx->coh.N;
     const int kcmax = 8;
     for (int c0 = 0; c0 < k; c0 += kcmax) {

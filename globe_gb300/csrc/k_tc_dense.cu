@@ -1,5 +1,5 @@
 // k_tc_dense.cu -- dense GRM product on the 5th-generation tensor cores
-// (GLOBE_PREC_MIXED).
+// (GLOBE_PREC_MIXED, and GLOBE_PREC_FP64 with more digits).
 //
 //   out (N x k) = scale * A Z,  A(i,j) = lt[max(i,j)(max(i,j)+1)/2 + min(i,j)]
 //   (PCGsolver.cpp:1202-1213, varCompEst.cpp:531-558)
@@ -20,6 +20,13 @@
 // tiles of the right-hand sides (kpos), rows padded to a multiple of 256.
 // The planes are full squares (both triangles), 7 N^2 bytes at DA = 7.
 //
+// GLOBE_PREC_FP64 takes DA = 12 planes (A within 2^-59 max|A|: a float32 entry of at least
+// 2^-35 max|A| exactly) and 12 digits of Z (2^-60 of each column's largest entry), and folds
+// the sums in double-double with one rounding at the end.  It holds every row to FP64 as long
+// as no diagonal entry is below 2^-5 max|A| (then the FP64 pipe runs instead).  N = 20k,
+// k = 16 streams 12 N^2 = 4.8 GB in 0.91 ms with its epilogue (5.3 TB/s); 25.1 ms on the FP64
+// pipe, which it was bound by.
+//
 // Kernel (one CTA = 2 x 128 rows x one K range, M=128 x N=NMMA MMAs per row tile):
 //   warp 0     TMA of both operands per stage: two 128 x 128-byte tiles of the
 //              digit planes (HBM) and the NMMA x 128-byte digit tile of Z (L2)
@@ -37,7 +44,8 @@
 namespace globe {
 namespace tc {
 
-constexpr int DA_MAX = 7;        // digit planes of A at most
+constexpr int DA_MAX = 7;        // digit planes of A at most (GLOBE_PREC_MIXED)
+constexpr int DA64 = 12;         // digit planes of A (GLOBE_PREC_FP64)
 constexpr int DMT = 2;           // row tiles per CTA
 constexpr int DROWS = DMT * BM;  // rows per CTA
 constexpr int DK_MAX_CHUNKS = 512;   // K <= 2^16 per CTA: |sum| <= 256 * 2^16 = 2^24, exact in FP32
@@ -159,21 +167,28 @@ __global__ void __launch_bounds__(256, 1)
 }
 
 // max |A| over the packed triangle as float bits (non-negative floats order like their bits),
-// and whether any entry is not finite
-__global__ void k_dense_absmax(const float* __restrict__ lt, int64_t n, unsigned* __restrict__ out) {
-    unsigned mx = 0, bad = 0;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+// whether any entry is not finite, and the smallest diagonal entry (negative ones count as 0)
+__global__ void k_dense_absmax(const float* __restrict__ lt, int64_t n, int32_t N, unsigned* __restrict__ out) {
+    unsigned mx = 0, bad = 0, dmin = 0x7f800000u;
+    const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t e = t0; e < n; e += nt) {
         const float v = lt[e];
         if (!isfinite(v)) bad = 1;
         else mx = max(mx, __float_as_uint(fabsf(v)));
     }
+    for (int64_t i = t0; i < N; i += nt) {
+        const float v = lt[i * (i + 1) / 2 + i];
+        dmin = min(dmin, v > 0.0f ? __float_as_uint(v) : 0u);
+    }
     for (int o = 16; o > 0; o >>= 1) {
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+        dmin = min(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
     }
     if ((threadIdx.x & 31) == 0) {
         atomicMax(out, mx);
         if (bad) atomicOr(out + 1, 1u);
+        atomicMin(out + 2, dmin);
     }
 }
 
@@ -288,64 +303,116 @@ __global__ void k_dense_combine(const float* __restrict__ part, int nsplit, int 
     }
 }
 
+// The FP64 product's epilogue: as k_dense_combine, with DA64 + ND64 - 1 = 23 weights in five
+// exact chunks (|C_q| < 2^31 N), added in double-double, and 2^e_c in two factors.
+__global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict__ part, int nsplit, int nmma,
+                                                         int64_t ldp, int32_t N, int64_t np,
+                                                         const double* __restrict__ colinfo, double sA, double scale,
+                                                         double* __restrict__ out, int64_t ldo) {
+    constexpr int NT = DA64 + ND64 - 1;
+    static_assert(NT <= 25, "five chunks of five weights");
+    const int c = blockIdx.y;
+    const int e = (int)colinfo[2 * c];
+    const double ea = ldexp(1.0, e / 2), eb = ldexp(1.0, e - e / 2), bad = colinfo[2 * c + 1];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        long long T[NT];
+#pragma unroll
+        for (int q = 0; q < NT; ++q) T[q] = 0;
+#pragma unroll
+        for (int d = 0; d < DA64; ++d) {
+            const float* src = part + (int64_t)c * ND64 * ldp + (int64_t)d * np + i;
+            for (int y = 0; y < nsplit; ++y) {
+                float v[ND64];
+#pragma unroll
+                for (int j = 0; j < ND64; ++j) v[j] = src[((int64_t)y * nmma + j) * ldp];
+#pragma unroll
+                for (int j = 0; j < ND64; ++j) T[d + j] += (long long)__float2int_rn(v[j]);
+            }
+        }
+        double h = 0.0, l = 0.0;
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            long long C = 0;
+#pragma unroll
+            for (int m = 0; m < 5; ++m) C = C * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
+            dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : 0x1p-100),
+                   0.0);
+        }
+        out[i + c * ldo] = (h + l) * sA * scale * ea * eb + bad;
+    }
+}
+
 }  // namespace tc
 
 // ---- host side ---------------------------------------------------------------
 
 using namespace tc;
 
-int dense_digit_planes(globe_ctx* ctx) {
+// (Re)builds digit planes: set 0 for the context's digit count, set 1 for the FP64 products
+static int dense_digit_planes(globe_ctx* ctx, int set) {
     auto& g = ctx->gen;
-    const int da = std::min(DA_MAX, ctx->digits);
-    if (g.adig_state != 0 && g.adig_da == da) return GLOBE_OK;
-    dfree(ctx, g.adig);
-    g.adig = nullptr;
-    g.adig_state = -1;   // until the planes are complete
+    auto& a = g.adig[set];
+    const int da = set ? DA64 : std::min(DA_MAX, ctx->digits);
+    if (a.state != 0 && a.da == da) return GLOBE_OK;
+    dfree(ctx, a.p);
+    a.p = nullptr;
+    a.state = -1;   // until the planes are complete
     const int32_t N = ctx->coh.N;
     const int64_t np = ((int64_t)N + BM - 1) / BM * BM;
     const int64_t rows = ((int64_t)da * np + DROWS - 1) / DROWS * DROWS;
     const size_t bytes = (size_t)rows * (size_t)np;
-    // the planes must fit beside what is resident; otherwise the double-float kernel stays in use
+    // the planes must fit beside what is resident, with room for a product's workspaces (set 1:
+    // its split partials are 1 KB a plane row and split); otherwise the other kernels stay in use
     size_t fr = 0, tot = 0;
     GLOBE_CK(ctx, cudaMemGetInfo(&fr, &tot));
-    if (bytes + ((size_t)2 << 30) > fr || rows > INT32_MAX) {
-        g.adig_da = da;
+    const size_t room = ((size_t)2 << 30) + (set ? (size_t)rows * 1024 * 4 : 0);
+    if (set == 0 && bytes + room > fr && g.adig[1].p) {   // the mixed planes come first
+        dfree(ctx, g.adig[1].p);
+        g.adig[1] = Genetic::Planes();
+        GLOBE_CK(ctx, cudaMemGetInfo(&fr, &tot));
+    }
+    if (bytes + room > fr || rows > INT32_MAX) {
+        a.da = da;
         return GLOBE_OK;
     }
-    unsigned* mx;   // words 1-2 of the error-flag slot (word 0 is the kernels' flag): max |A| bits, non-finite
+    unsigned* mx;   // words 1-3 of the error-flag slot (word 0 is the kernels' flag): max |A| bits, non-finite, min A_ii
     GLOBE_RET(tc_err_word(ctx, &mx));
     GLOBE_CK(ctx, cudaMemsetAsync(mx + 1, 0, 2 * sizeof(unsigned), ctx->stream));
+    GLOBE_CK(ctx, cudaMemsetAsync(mx + 3, 0x7f, sizeof(unsigned), ctx->stream));
     const int64_t nelt = (int64_t)N * (N + 1) / 2;
-    k_dense_absmax<<<(unsigned)std::min<int64_t>(div_up(nelt, 256), 152 * 8), 256, 0, ctx->stream>>>(g.grm, nelt,
+    k_dense_absmax<<<(unsigned)std::min<int64_t>(div_up(nelt, 256), 152 * 8), 256, 0, ctx->stream>>>(g.grm, nelt, N,
                                                                                                     mx + 1);
     GLOBE_LAUNCHED(ctx, "k_dense_absmax");
-    unsigned h[2] = {0, 0};
+    unsigned h[3] = {0, 0, 0};
     GLOBE_CK(ctx, cudaMemcpyAsync(h, mx + 1, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    g.adig_da = da;
-    if (h[1]) return GLOBE_OK;   // a non-finite entry: the double-float kernel propagates it
-    float amax;
+    a.da = da;
+    if (h[1]) return GLOBE_OK;   // a non-finite entry: the other kernels propagate it
+    float amax, dmin;
     std::memcpy(&amax, &h[0], sizeof(float));
+    std::memcpy(&dmin, &h[2], sizeof(float));
+    if (set && !(dmin >= amax * 0x1p-5f)) return GLOBE_OK;   // a row too small for the common grid
     int E = 0;
     if (amax > 0.0f) std::frexp((double)amax, &E);
-    g.adig_e = E - (DBITS - 1);   // max|A| 2^-eA in [8, 16)
-    GLOBE_RET(dalloc(ctx, &g.adig, bytes));
+    a.e = E - (DBITS - 1);   // max|A| 2^-eA in [8, 16)
+    GLOBE_RET(dalloc(ctx, &a.p, bytes));
     if (rows > da * np)
-        GLOBE_CK(ctx, cudaMemsetAsync(g.adig + (size_t)da * np * np, 0, (size_t)(rows - da * np) * np, ctx->stream));
+        GLOBE_CK(ctx, cudaMemsetAsync(a.p + (size_t)da * np * np, 0, (size_t)(rows - da * np) * np, ctx->stream));
     const dim3 grid((unsigned)(np / 64), (unsigned)(np / 64));
     switch (da) {
-        case 2: k_dense_digits<2><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
-        case 3: k_dense_digits<3><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
-        case 4: k_dense_digits<4><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
-        case 5: k_dense_digits<5><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
-        case 6: k_dense_digits<6><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
-        default: k_dense_digits<7><<<grid, 256, 0, ctx->stream>>>(g.grm, N, g.adig_e, g.adig, np); break;
+        case 2: k_dense_digits<2><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 3: k_dense_digits<3><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 4: k_dense_digits<4><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 5: k_dense_digits<5><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 6: k_dense_digits<6><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case DA64: k_dense_digits<DA64><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        default: k_dense_digits<7><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
     }
     GLOBE_LAUNCHED(ctx, "k_dense_digits");
     GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    g.adig_np = np;
-    g.adig_rows = rows;
-    g.adig_state = 1;
+    a.np = np;
+    a.rows = rows;
+    a.state = 1;
     return GLOBE_OK;
 }
 
@@ -408,12 +475,13 @@ static int dense_cps(globe_ctx* ctx, int tiles, int nchunks, int nmma) {
 // out (N x kg) = scale * A Z for one group of <= 256 / ND columns
 template <int ND>
 static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out) {
-    auto& g = ctx->gen;
+    constexpr bool F64 = ND == ND64;
+    const auto& a = ctx->gen.adig[F64 ? 1 : 0];
     const int32_t N = ctx->coh.N;
-    const int64_t np = g.adig_np;
+    const int64_t np = a.np;
     const int nch = (int)(np / BK);
     const int nmma = ((kg * ND + 15) / 16) * 16;
-    const int rows = (int)g.adig_rows, tiles = rows / DROWS;
+    const int rows = (int)a.rows, tiles = rows / DROWS;
     const int cps = dense_cps(ctx, tiles, nch, nmma);
     const int splits = (nch + cps - 1) / cps;
     const int64_t ldp = rows;
@@ -424,23 +492,25 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     const int nbr = 304;
     GLOBE_RET(ws(ctx, WS_TC_D1, (size_t)nmma * np, &D));
     GLOBE_RET(ws(ctx, WS_TC_P1, (size_t)splits * nmma * ldp, &P));
-    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(2 * kg + 2 * nbr * kg + 8), &cst));
+    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(4 * kg + 2 * nbr * kg + 8), &cst));
     GLOBE_RET(tc_err_word(ctx, &err));
     double* col = cst;
-    double* pm = cst + 2 * kg;
+    unsigned long long* isum = reinterpret_cast<unsigned long long*>(cst + 2 * kg);   // F64: scratch of k_col_max64
+    double* pm = cst + 4 * kg;
     double* ps = pm + (size_t)nbr * kg;
     CUtensorMap mA, mB;
-    GLOBE_RET(make_map(ctx, &mA, g.adig, (uint64_t)np, (uint64_t)rows, BK, BM, true));
+    GLOBE_RET(make_map(ctx, &mA, a.p, (uint64_t)np, (uint64_t)rows, BK, BM, true));
     GLOBE_RET(make_map(ctx, &mB, D, (uint64_t)np, (uint64_t)nmma, BK, (uint32_t)nmma, true));
     const int nz = col_parts(N);
     unsigned* cnt;
     GLOBE_RET(tc_counters(ctx, kg, &cnt));
-    k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col);
+    if constexpr (F64) k_col_max64<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, cnt, col, isum);
+    else k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col);
     GLOBE_LAUNCHED(ctx, "k_col_maxsum");
     if (nmma > kg * ND)   // digit rows past the kg columns stay zero
         GLOBE_CK(ctx, cudaMemsetAsync(D + (size_t)kg * ND * np, 0, (size_t)(nmma - kg * ND) * np, ctx->stream));
     k_digits<ND, false><<<dim3((unsigned)std::min<int64_t>(div_up(np / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, kg, col, D, np);
+        Z, N, N, kg, col, D, np, nullptr);
     GLOBE_LAUNCHED(ctx, "k_digits");
     {
         ProfScope p(ctx, GLOBE_PROF_GRM_PASS1);
@@ -448,8 +518,13 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
         ctx->stall_next_gemm = 0;
         GLOBE_RET(dense_dispatch(ctx, nmma, mA, mB, rows, nch, cps, P, ldp, err, stall));
     }
-    k_dense_combine<ND><<<dim3(std::min(div_up(N, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        P, splits, nmma, ldp, N, np, g.adig_da, col, std::ldexp(scale, g.adig_e), out, N);
+    const dim3 gc((unsigned)std::min(div_up(N, 256), 1024), kg);
+    if constexpr (F64)
+        k_dense_combine64<<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, col, std::ldexp(1.0, a.e - 20), scale,
+                                                       out, N);
+    else
+        k_dense_combine<ND><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
+                                                         std::ldexp(scale, a.e), out, N);
     GLOBE_LAUNCHED(ctx, "k_dense_combine");
     return GLOBE_OK;
 }
@@ -464,14 +539,13 @@ static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, doubl
         case 7: return dense_group<7>(ctx, Z, kg, scale, out);
         case 8: return dense_group<8>(ctx, Z, kg, scale, out);
         case 9: return dense_group<9>(ctx, Z, kg, scale, out);
+        case ND64: return dense_group<ND64>(ctx, Z, kg, scale, out);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
 
-int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
-    GLOBE_RET(dense_digit_planes(ctx));
-    if (ctx->gen.adig_state != 1) return dense_apply_df(ctx, Z, k, scale, out);
-    const int nd = ctx->digits;
+// out (N x k) = scale * A Z from the planes, nd digits per column
+static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out) {
     const int gmax = 256 / nd;   // MMA width <= 256; near-equal groups
     const int ng = (k + gmax - 1) / gmax;
     for (int gi = 0, c0 = 0; gi < ng; ++gi) {
@@ -480,6 +554,45 @@ int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double*
         c0 += kg;
     }
     return GLOBE_OK;
+}
+
+int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+    GLOBE_RET(dense_digit_planes(ctx, 0));
+    if (ctx->gen.adig[0].state != 1) return dense_apply_df(ctx, Z, k, scale, out);
+    return dense_apply_nd(ctx, ctx->digits, Z, k, scale, out);
+}
+
+// The FP64 product, by its size N N k (FP64 pipe / planes, us a product):
+//  - inside a solve, which repeats the product and so pays for building the planes (0.2 ms at
+//    N = 200, 4.4 ms at 20k), the planes from 1e5 on (2e5: 64 / 34; 1.6e7: 471 / 41;
+//    6.4e9: 25118 / 909);
+//  - a single operator call from 4e6 on, where the first call, with the planes to build, costs
+//    about the same on either (1e6: 191 / 288; 4e6: 352 / 314; 4e8: 8484 / 5179).
+// The choice depends on the sizes only; the FP64 pipe also runs where the planes cannot be held or
+// a row is too small for their common grid.
+// Error against 128-bit sums (N = 2500; normal, constant, count, lognormal, unit and wide-range
+// columns): at most 7.8e-17 of the column, FP64 pipe up to 1.9e-15.
+#ifndef F64_DENSE_SOLVE_MIN
+#define F64_DENSE_SOLVE_MIN 1e5
+#endif
+#ifndef F64_DENSE_CALL_MIN
+#define F64_DENSE_CALL_MIN 4e6
+#endif
+int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+    auto& a = ctx->gen.adig[1];
+    const int32_t N = ctx->coh.N;
+    if (a.state >= 0 && (double)N * N * k >= (ctx->in_solve ? F64_DENSE_SOLVE_MIN : F64_DENSE_CALL_MIN)) {
+        int rc = dense_digit_planes(ctx, 1);
+        if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, ND64, Z, k, scale, out);
+        if (a.state == 1 && rc != GLOBE_ERR_NOMEM) return rc;
+        if (rc != GLOBE_OK && rc != GLOBE_ERR_NOMEM) return rc;
+        if (rc == GLOBE_ERR_NOMEM) {   // give the planes back
+            dfree(ctx, a.p);
+            a.p = nullptr;
+            a.state = -1;
+        }
+    }
+    return dense_apply_fp64_pipe(ctx, Z, k, scale, out);
 }
 
 }  // namespace globe

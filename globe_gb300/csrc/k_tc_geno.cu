@@ -508,26 +508,6 @@ __global__ void k_combine2(const float* __restrict__ part, int nsplit, int nmma,
 // those loads.  N = 20k, M = 20k, k = 5: 148 us a product, 14.5 ms on the FP64 pipe
 // (k_geno_p1 / p2, which it replaces from geno_apply_f64's sizes on).
 
-__device__ __forceinline__ double warp_max_bits(double m) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = absmax_bits(m, __shfl_xor_sync(0xffffffffu, m, o));
-    return m;
-}
-// (h, l) += (a, b): two-sum of the high parts, everything else into l
-__device__ __forceinline__ void dd_add(double& h, double& l, double a, double b) {
-    const double s = __dadd_rn(h, a), bp = __dsub_rn(s, h);
-    l = __dadd_rn(l, __dadd_rn(b, __dadd_rn(__dsub_rn(h, __dsub_rn(s, bp)), __dsub_rn(a, bp))));
-    h = s;
-}
-// colinfo = {scale exponent, 0 or NaN} from max |x| (its bits: NaN and infinity win)
-__device__ __forceinline__ void col_info64(double mx, double* __restrict__ colinfo) {
-    const bool bad = !isfinite(mx);
-    int E = 0;
-    if (!bad && mx > 0) frexp(mx, &E);
-    colinfo[0] = bad ? 0.0 : (double)(E - (DBITS - 1));
-    colinfo[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
-}
-
 // max |x| of each column; the column's last CTA forms colinfo[c] and clears isum for k_digits
 __global__ void k_col_max64(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
                             unsigned* __restrict__ cnt, double* __restrict__ colinfo,

@@ -177,6 +177,33 @@ __host__ __forceinline__ int col_parts(int64_t n) {
     return (int)(p < 1 ? 1 : (p > 304 ? 304 : p));
 }
 
+// ---- the FP64 products (ND64 digits) ----
+__device__ __forceinline__ double warp_max_bits(double m) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = absmax_bits(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
+// (h, l) += (a, b): two-sum of the high parts, everything else into l
+__device__ __forceinline__ void dd_add(double& h, double& l, double a, double b) {
+    const double s = __dadd_rn(h, a), bp = __dsub_rn(s, h);
+    l = __dadd_rn(l, __dadd_rn(b, __dadd_rn(__dsub_rn(h, __dsub_rn(s, bp)), __dsub_rn(a, bp))));
+    h = s;
+}
+// colinfo = {scale exponent, 0 or NaN} from max |x| (its bits: NaN and infinity win)
+__device__ __forceinline__ void col_info64(double mx, double* __restrict__ colinfo) {
+    const bool bad = !isfinite(mx);
+    int E = 0;
+    if (!bad && mx > 0) frexp(mx, &E);
+    colinfo[0] = bad ? 0.0 : (double)(E - (DBITS - 1));
+    colinfo[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+}
+
+// max |x| of each column; the column's last CTA forms colinfo[c] and clears isum[2c], isum[2c+1]
+// for k_digits (k_tc_geno.cu)
+__global__ void k_col_max64(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
+                            unsigned* __restrict__ cnt, double* __restrict__ colinfo,
+                            unsigned long long* __restrict__ isum);
+
 // per-column max |x| and sum over n rows (partials per CTA); colinfo[c] = {exponent e with
 // max |x 2^-e| < 16, column sum} from those partials, or {0, NaN} for a column holding a
 // NaN or an infinity (k_tc_geno.cu).  k_col_maxsum forms colinfo itself when given it and

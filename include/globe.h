@@ -52,7 +52,9 @@ extern "C" {
                                largest entry), sums exact, centring in double-double, one
                                final FP64 rounding -- closer to the exact product than sums
                                on the FP64 pipe, which run where the product is small or the
-                               second genotype copy does not fit in device memory */
+                               second genotype copy does not fit in device memory.  Dense GRM
+                               products the same way, from 12 digit planes of A (12 N^2 bytes;
+                               A within 2^-59 max|A|) */
 #define GLOBE_PREC_MIXED 1  /* genotype GRM product on the FP8 tensor cores with exact
                                base-32 digit slicing of the right-hand sides (9 digits =
                                45 bits by default, matches FP64 to ~1e-13; see

@@ -1,7 +1,8 @@
-"""GLOBE_PREC_FP64 genotype products on the tensor cores (12 base-32 digits, exact sums) against
-the FP64 oracle and against the FP64-pipe kernels, which run the smaller products.
+"""GLOBE_PREC_FP64 products on the tensor cores (12 base-32 digits, exact sums) against the FP64
+oracle and against the FP64-pipe kernels, which run the smaller products.
 
-A single operator call takes the tensor cores from N Mk k = 4e7 on (geno_apply_f64)."""
+A single operator call takes the tensor cores from N Mk k = 4e7 on (geno_apply_f64), N N k = 4e6
+with a dense GRM (dense_apply_f64)."""
 import numpy as np
 import pytest
 
@@ -81,3 +82,61 @@ def test_solve_repeats_and_masks(gctx, orc):
             gctx.set_device_loop(True)
         assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
         assert max(rel(out[0][:, c], ref[:, c]) for c in range(6)) < 1e-9
+
+
+def _dense(gctx, N, seed, shrink=None):
+    rng = np.random.default_rng(seed)
+    W = rng.standard_normal((800, N))
+    A = (W.T @ W / 800).astype(np.float32)
+    if shrink is not None:                                # one individual on a much smaller scale
+        A[shrink] *= np.float32(1e-6)
+        A[:, shrink] *= np.float32(1e-6)
+    lt = A[np.tril_indices(N)]
+    gctx.load_records(np.arange(N, dtype=np.int32), np.ones((N, 1)), np.zeros(N), N)
+    gctx.load_grm(lt, N)
+    gctx.set_vc(VC_F)
+    gctx.set_precision(G.PREC_FP64)
+    low = np.tril(A.astype(np.float64))
+    return low + np.tril(low, -1).T
+
+
+# row tiles of 256 and K chunks of 128, one past them; one to three column groups
+@pytest.mark.parametrize("N,ks", [(2049, (1, 5)), (901, (5, 16)), (640, (10, 21, 22, 43)), (385, (28,))])
+def test_dense_matches_float64(gctx, N, ks):
+    A = _dense(gctx, N, N)
+    rng = np.random.default_rng(1)
+    for k in ks:
+        Z = rng.standard_normal((N, k)) * np.logspace(-200, 200, k)
+        if k > 4:
+            Z[:, 2] = np.exp(2 * rng.standard_normal(N))
+            Z[:, 3] = 0.0
+        got, ref = gctx.grm_apply(Z), VC_F[1] * (A @ Z)
+        # FP64 sums of N terms: sqrt(N) units of 2^-53
+        assert max(rel(got[:, c] / np.abs(Z[:, c]).max(), ref[:, c] / np.abs(Z[:, c]).max())
+                   for c in range(k) if ref[:, c].any()) < 1e-14, k
+        assert k <= 4 or not got[:, 3].any()
+
+
+def test_dense_small_row_keeps_its_digits(gctx):
+    """A row far below max|A| would lose digits on the planes' common grid: the FP64 pipe runs."""
+    N, i = 2049, 77
+    A = _dense(gctx, N, 3, shrink=i)
+    Z = np.random.default_rng(2).standard_normal((N, 2))
+    Z[i] = 0.0
+    got, ref = gctx.grm_apply(Z), VC_F[1] * (A @ Z)
+    assert np.abs(got[i] / ref[i] - 1).max() < 1e-11 and rel(got, ref) < 1e-13
+
+
+def test_dense_precisions_hold_their_own_planes(gctx):
+    """Mixed products between FP64 ones: each precision gives the same bits throughout."""
+    _dense(gctx, 901, 4)
+    Z = np.random.default_rng(3).standard_normal((901, 6))
+    out = {}
+    try:
+        for prec in (G.PREC_MIXED, G.PREC_FP64, G.PREC_MIXED, G.PREC_FP64):
+            gctx.set_precision(prec)
+            out.setdefault(prec, []).append(gctx.grm_apply(Z))
+    finally:
+        gctx.set_precision(G.PREC_FP64)
+    assert all(np.array_equal(a, b) for a, b in out.values())
+    assert 0 < rel(out[G.PREC_MIXED][0], out[G.PREC_FP64][0]) < 1e-9
