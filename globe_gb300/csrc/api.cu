@@ -4,7 +4,7 @@
 #include <cstring>
 #include <vector>
 
-#include "internal.cuh"
+#include "tc_common.cuh"
 
 namespace globe {
 
@@ -137,7 +137,7 @@ static void free_cohort(globe_ctx* ctx) {
 
 static void free_genetic(globe_ctx* ctx) {
     auto& g = ctx->gen;
-    for (void* p : {(void*)g.geno, (void*)g.zs, (void*)g.f, (void*)g.inv, (void*)g.grm, (void*)g.gdiag,
+    for (void* p : {(void*)g.zs, (void*)g.f, (void*)g.inv, (void*)g.grm, (void*)g.gdiag,
                     (void*)g.blk1, (void*)g.blk2, (void*)g.adig[0].p, (void*)g.adig[1].p})
         dfree(ctx, p);
     g = Genetic();
@@ -434,8 +434,7 @@ int globe_set_individuals(globe_ctx* ctx, int32_t N) {
 
 namespace globe {
 
-// statistics, filter and compaction of the kept SNP rows; the tile-blocked layout follows
-// separately (ensure_blk1), after the callers have released their staging copies
+// statistics, filter and the tile-blocked copy of the kept SNP rows
 int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, float min_maf, float max_miss,
                   int64_t* d_alt, int64_t* d_miss, float* d_maf, float* d_mr, uint8_t* d_keep, globe_bed_info* info) {
     if (!ctx) return GLOBE_ERR_ARG;
@@ -449,61 +448,39 @@ int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t strid
     if (!(min_maf >= 0.0f && min_maf <= 0.5f && max_miss >= 0.0f && max_miss <= 1.0f))
         return set_err(ctx, GLOBE_ERR_ARG, "Invalid MAF or missing rate thresholds.");
     free_genetic(ctx);
-    // per-SNP statistics (temporaries where the caller passed NULL)
-    std::vector<void*> tmp;
-    auto need = [&](auto** p, size_t n) -> int {
-        if (*p) return GLOBE_OK;
-        void* q;
-        cudaError_t e = cudaMalloc(&q, n ? n : 16);
-        if (e != cudaSuccess) return cuda_err(ctx, e, "cudaMalloc(stats)");
-        tmp.push_back(q);
-        *p = (std::remove_reference_t<decltype(*p)>)q;
-        return GLOBE_OK;
-    };
-    int rc = GLOBE_OK;
-    if ((rc = need(&d_alt, sizeof(int64_t) * M)) || (rc = need(&d_miss, sizeof(int64_t) * M)) ||
-        (rc = need(&d_keep, (size_t)M))) {
-        for (void* q : tmp) cudaFree(q);
-        return rc;
-    }
-    auto cleanup = [&]() {
-        cudaStreamSynchronize(ctx->stream);
-        for (void* q : tmp) cudaFree(q);
-    };
-    rc = bed_stats(ctx, d_bed, M, stride, N, min_maf, max_miss, d_alt, d_miss, d_maf, d_mr, d_keep);
-    std::vector<uint8_t> keep(M);
-    if (rc == GLOBE_OK && M > 0) {
-        cudaError_t e = cudaMemcpyAsync(keep.data(), d_keep, M, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e != cudaSuccess) rc = cuda_err(ctx, e, "copy keep mask");
-    }
-    if (rc != GLOBE_OK) { cleanup(); return rc; }
-    std::vector<int64_t> idx;
-    idx.reserve(M);
-    for (int64_t s = 0; s < M; ++s)
-        if (keep[s]) idx.push_back(s);
+    // temporaries in one allocation: the statistics the caller passed NULL for, the kept SNPs'
+    // indices and their scan
+    const size_t nb = (size_t)keep_blocks(M) + 1;
+    uint8_t* tmp = nullptr;
+    GLOBE_RET(dalloc(ctx, &tmp, (size_t)M * 24 + nb * 8 + (size_t)M + 16));
+    int64_t* d_idx = reinterpret_cast<int64_t*>(tmp) + 2 * M;
+    int64_t* d_cnt = d_idx + M;
+    if (!d_alt) d_alt = reinterpret_cast<int64_t*>(tmp);
+    if (!d_miss) d_miss = reinterpret_cast<int64_t*>(tmp) + M;
+    if (!d_keep) d_keep = reinterpret_cast<uint8_t*>(d_cnt + nb);
     auto& g = ctx->gen;
-    g.Mk = (int64_t)idx.size();
-    g.stride = (bps + 15) / 16 * 16;
-    int64_t* d_idx = nullptr;
-    if ((rc = dalloc(ctx, &d_idx, idx.size() + 1)) != GLOBE_OK) { cleanup(); return rc; }
-    if (g.Mk > 0) {
-        cudaError_t e = cudaMemcpyAsync(d_idx, idx.data(), sizeof(int64_t) * g.Mk, cudaMemcpyHostToDevice, ctx->stream);
-        if (e != cudaSuccess) { cleanup(); return cuda_err(ctx, e, "copy kept index"); }
-    }
-    if ((rc = dalloc(ctx, &g.geno, (size_t)g.Mk * g.stride)) || (rc = dalloc(ctx, &g.zs, (size_t)g.Mk * 4)) ||
-        (rc = dalloc(ctx, &g.f, (size_t)g.Mk)) || (rc = dalloc(ctx, &g.inv, (size_t)g.Mk)) ||
-        (rc = dalloc(ctx, &g.gdiag, (size_t)N))) {
-        cleanup();
-        return rc;
-    }
-    if ((rc = bed_compact(ctx, d_bed, stride, d_idx, g.Mk, bps, g.geno, g.stride)) ||
-        (rc = snp_coefs(ctx, d_alt, d_miss, d_idx, g.Mk, N, g.f, g.inv, g.zs))) {
-        cleanup();
-        return rc;
-    }
-    cleanup();
-    dfree(ctx, d_idx);
+    auto steps = [&]() -> int {
+        GLOBE_RET(bed_stats(ctx, d_bed, M, stride, N, min_maf, max_miss, d_alt, d_miss, d_maf, d_mr, d_keep));
+        GLOBE_RET(keep_scan(ctx, d_keep, M, d_cnt));
+        GLOBE_CK(ctx, cudaMemcpyAsync(&g.Mk, d_cnt + nb - 1, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+        GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
+        GLOBE_RET(dalloc(ctx, &g.zs, (size_t)g.Mk * 4));
+        GLOBE_RET(dalloc(ctx, &g.f, (size_t)g.Mk));
+        GLOBE_RET(dalloc(ctx, &g.inv, (size_t)g.Mk));
+        GLOBE_RET(dalloc(ctx, &g.gdiag, (size_t)N));
+        if (g.Mk < 1) return GLOBE_OK;
+        GLOBE_RET(keep_scatter(ctx, d_keep, M, d_cnt, d_idx));
+        GLOBE_RET(snp_coefs(ctx, d_alt, d_miss, d_idx, g.Mk, N, g.f, g.inv, g.zs));
+        // the SNP-major tile-blocked copy, whole CTAs of 1 to 4 row tiles (TILE_PAD)
+        g.nch1 = div_up(bps, tc::PKB);
+        g.ntiles1 = div_up(div_up(g.Mk, tc::BM), TILE_PAD) * TILE_PAD;
+        GLOBE_RET(dalloc(ctx, &g.blk1, (size_t)g.ntiles1 * g.nch1 * tc::BM * tc::PKB));
+        return bed_layout(ctx, d_bed, stride, d_idx, g.Mk, bps, g.ntiles1, g.nch1, g.blk1);
+    };
+    const int rc = steps();
+    cudaStreamSynchronize(ctx->stream);
+    dfree(ctx, tmp);
+    if (rc != GLOBE_OK) return rc;
     g.src = GSRC_GENO;
     g.gdiag_ok = false;
     ctx->precond_ok = false;
@@ -522,10 +499,7 @@ extern "C" {
 int globe_load_bed_dev(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, float min_maf,
                        float max_miss, int64_t* d_alt, int64_t* d_miss, float* d_maf, float* d_mr, uint8_t* d_keep,
                        globe_bed_info* info) {
-    int rc = load_bed_rows(ctx, d_bed, M, stride, min_maf, max_miss, d_alt, d_miss, d_maf, d_mr, d_keep, info);
-    // the tile-blocked copy the genotype kernels read; the compacted rows are freed
-    if (rc == GLOBE_OK && ctx->gen.Mk > 0) rc = ensure_blk1(ctx);
-    return rc;
+    return load_bed_rows(ctx, d_bed, M, stride, min_maf, max_miss, d_alt, d_miss, d_maf, d_mr, d_keep, info);
 }
 
 int globe_load_bed(globe_ctx* ctx, const uint8_t* bed, int64_t M, float min_maf, float max_miss,
@@ -566,8 +540,6 @@ int globe_load_bed(globe_ctx* ctx, const uint8_t* bed, int64_t M, float min_maf,
 done:
     cudaStreamSynchronize(ctx->stream);
     for (void* p : {(void*)d_bed, (void*)d_alt, (void*)d_miss, (void*)d_maf, (void*)d_mr, (void*)d_keep}) dfree(ctx, p);
-    // tile-blocked layout once the staging copy of the payload is gone
-    if (rc == GLOBE_OK && ctx->gen.Mk > 0) rc = ensure_blk1(ctx);
     return rc;
 }
 

@@ -107,7 +107,5 @@ done:
         if (host[b]) cudaFreeHost(host[b]);
     }
     for (void* p : {(void*)d_bed, (void*)d_alt, (void*)d_miss, (void*)d_maf, (void*)d_mr, (void*)d_keep}) dfree(ctx, p);
-    // tile-blocked layout once the file's device copy is gone
-    if (rc == GLOBE_OK && ctx->gen.Mk > 0) rc = ensure_blk1(ctx);
     return rc;
 }

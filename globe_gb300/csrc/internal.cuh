@@ -23,8 +23,8 @@ namespace globe {
 //           (individual of block b), rind[Nrec] (individual of record r)
 //   moments per block: n, sum t, sum t^2              (double, N each)
 // Genetic source:
-//   genotype: kept SNP rows, `stride` bytes each (multiple of 16), PLINK
-//             2-bit codes; per-SNP zs table zs[s*4 + code] (double) with
+//   genotype: kept SNPs in tile-blocked copies of 2-bit codes (tc_common.cuh);
+//             per-SNP zs table zs[s*4 + PLINK code] (double) with
 //             zs = (g - 2f) * inv_std, missing -> g = 0
 //   dense:    packed lower triangle float32, N(N+1)/2
 constexpr int SHORT_BLOCK = 48;   // longest record block handled by one thread in the record kernels
@@ -54,12 +54,9 @@ struct Genetic {
     int src = GSRC_NONE;
     // genotype source
     int64_t Mk = 0;          // kept SNPs
-    int64_t stride = 0;      // bytes per SNP row (multiple of 16)
-    uint8_t* geno = nullptr; // Mk x stride compacted rows (PLINK codes), freed once blk1 exists
     double* zs = nullptr;    // Mk x 4
     double* f = nullptr;     // Mk
     double* inv = nullptr;   // Mk
-    int64_t strideT = 0;     // bytes of an individual-major row of blk2 (whole 32-byte chunks)
     // tile-blocked copies (tile codes): block (tile, chunk) = 128 rows x 32 B
     uint8_t* blk1 = nullptr;   // SNP-major: every genotype kernel (built at load)
     uint8_t* blk2 = nullptr;   // individual-major: tensor-core pass 2, GRM build (first use)
@@ -276,8 +273,11 @@ static const int g_bounds_registered = register_bounds_word(&query_bounds_word_t
 int bed_stats(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, int32_t N,
               float min_maf, float max_miss, int64_t* d_alt, int64_t* d_miss, float* d_maf,
               float* d_mr, uint8_t* d_keep);
-int bed_compact(globe_ctx* ctx, const uint8_t* d_bed, int64_t stride_in, const int64_t* d_idx,
-                int64_t Mk, int64_t bps, uint8_t* d_out, int64_t stride_out);
+int keep_blocks(int64_t M);
+int keep_scan(globe_ctx* ctx, const uint8_t* d_keep, int64_t M, int64_t* cnt);
+int keep_scatter(globe_ctx* ctx, const uint8_t* d_keep, int64_t M, const int64_t* cnt, int64_t* idx);
+int bed_layout(globe_ctx* ctx, const uint8_t* d_bed, int64_t stride, const int64_t* d_idx, int64_t Mk, int64_t bps,
+               int ntiles, int nch, uint8_t* dst);
 int snp_coefs(globe_ctx* ctx, const int64_t* d_alt, const int64_t* d_miss, const int64_t* d_idx,
               int64_t Mk, int32_t N, double* d_f, double* d_inv, double* d_zs);
 int synth_bed(globe_ctx* ctx, uint8_t* d_bed, int64_t M, int32_t N, int64_t stride, uint64_t seed,
@@ -347,7 +347,6 @@ int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double*
 int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);   // GLOBE_PREC_FP64
 
 // k_tc_geno.cu
-int ensure_blk1(globe_ctx* ctx);   // SNP-major tile-blocked copy; frees the compacted rows
 int ensure_blk2(globe_ctx* ctx);   // individual-major tile-blocked copy (first tensor-core use)
 int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, float min_maf, float max_miss,
                   int64_t* d_alt, int64_t* d_miss, float* d_maf, float* d_mr, uint8_t* d_keep, globe_bed_info* info);

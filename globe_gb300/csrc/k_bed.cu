@@ -7,15 +7,41 @@
 // missing rate and filter use the same float operations as the reference, so
 // the results are bit-exact.  The FP64 standardisation coefficients are the
 // float->double restatement of getStdGenotype (PCGsolver.cpp:826-842).
-#include "internal.cuh"
+#include <algorithm>
+
+#include "tc_common.cuh"
 
 namespace globe {
 
-// One warp per SNP row; byte-granular so any row alignment works.
-__global__ void k_bed_stats(const uint8_t* __restrict__ bed, int64_t M, int64_t stride, int32_t N,
-                            float min_maf, float max_miss, int64_t* __restrict__ alt_out,
-                            int64_t* __restrict__ miss_out, float* __restrict__ maf_out,
-                            float* __restrict__ mr_out, uint8_t* __restrict__ keep_out) {
+// 16 bytes at p, whatever its alignment: one load, or the aligned words around it (which hold at
+// least one of the 16 bytes each, so they lie in the buffer's allocation)
+__device__ __forceinline__ uint4 load16_any(const uint8_t* __restrict__ p) {
+    const unsigned a = (unsigned)(reinterpret_cast<uintptr_t>(p) & 15u);
+    if (a == 0) return __ldg(reinterpret_cast<const uint4*>(p));
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(p - (a & 3u));
+    if ((a & 3u) == 0) return make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+    const uint32_t w0 = __ldg(q), w1 = __ldg(q + 1), w2 = __ldg(q + 2), w3 = __ldg(q + 3), w4 = __ldg(q + 4);
+    const unsigned sh = 8u * (a & 3u);
+    return make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh), __funnelshift_r(w2, w3, sh),
+                      __funnelshift_r(w3, w4, sh));
+}
+
+// A1 alleles and missing codes of two words' 32 samples: the low and the high bits of their codes
+// packed into one word each, so that three popc (a quarter-rate instruction) serve both
+__device__ __forceinline__ void count_codes(uint32_t x, uint32_t y, int& a, int& ms) {
+    const uint32_t L = (x & 0x55555555u) | ((y & 0x55555555u) << 1);
+    const uint32_t H = ((x >> 1) & 0x55555555u) | (y & 0xAAAAAAAAu);
+    a += 2 * __popc(~(H | L)) + __popc(H & ~L);
+    ms += __popc(L & ~H);
+}
+
+// One warp per SNP row: 16 bytes per lane and step, four steps' loads in flight, the bytes past
+// the last whole 16 (with the last byte's phantom pairs masked) one per lane.  Bound by the
+// payload's read (12.5 GB rows of 25 KB: one byte per lane took 8.7 ms, 1.4 TB/s).
+__global__ void __launch_bounds__(256) k_bed_stats(const uint8_t* __restrict__ bed, int64_t M, int64_t stride, int32_t N,
+                                                   float min_maf, float max_miss, int64_t* __restrict__ alt_out,
+                                                   int64_t* __restrict__ miss_out, float* __restrict__ maf_out,
+                                                   float* __restrict__ mr_out, uint8_t* __restrict__ keep_out) {
     const int lane = threadIdx.x & 31;
     const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= M) return;
@@ -23,14 +49,32 @@ __global__ void k_bed_stats(const uint8_t* __restrict__ bed, int64_t M, int64_t 
     const uint8_t* row = bed + s * stride;
     const int last_pairs = N - (int)((bps - 1) * 4);  // 1..4 real pairs in the last byte
     const unsigned last_mask = 0x55u & ((1u << (2 * last_pairs)) - 1u);
-    long long a = 0, ms = 0;
-    for (int64_t b = lane; b < bps; b += 32) {
+    int ai = 0, mi = 0;   // a lane's share of 2 N < 2^32 alleles
+    const int nfull = (int)((bps - 1) >> 4);
+    int q = lane;
+    for (; q + 96 < nfull; q += 128) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = load16_any(row + (int64_t)(q + 32 * u) * 16);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            count_codes(v[u].x, v[u].y, ai, mi);
+            count_codes(v[u].z, v[u].w, ai, mi);
+        }
+    }
+    for (; q < nfull; q += 32) {
+        const uint4 v = load16_any(row + (int64_t)q * 16);
+        count_codes(v.x, v.y, ai, mi);
+        count_codes(v.z, v.w, ai, mi);
+    }
+    for (int64_t b = (int64_t)nfull * 16 + lane; b < bps; b += 32) {
         unsigned x = row[b];
         unsigned m = (b == bps - 1) ? last_mask : 0x55u;
         unsigned L = x & 0x55u, H = (x >> 1) & 0x55u;
-        a += 2 * __popc(~(H | L) & m) + __popc(H & ~L & m);
-        ms += __popc(L & ~H & m);
+        ai += 2 * __popc(~(H | L) & m) + __popc(H & ~L & m);
+        mi += __popc(L & ~H & m);
     }
+    long long a = ai, ms = mi;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         a += __shfl_xor_sync(0xffffffffu, a, o);
@@ -59,34 +103,111 @@ int bed_stats(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, i
     return GLOBE_OK;
 }
 
-// Copy kept rows into a padded layout.  Phantom pairs of the last byte and
-// the padding bytes become code 11 (genotype 0), so a consumer that runs past
-// N sees zeros.
-__global__ void k_bed_compact(const uint8_t* __restrict__ in, int64_t stride_in,
-                              const int64_t* __restrict__ idx, int64_t Mk, int64_t bps, int32_t N,
-                              uint8_t* __restrict__ out, int64_t stride_out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t k = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (k >= Mk) return;
-    const uint8_t* src = in + idx[k] * stride_in;
-    uint8_t* dst = out + k * stride_out;
-    const int last_pairs = N - (int)((bps - 1) * 4);
-    const unsigned keep_bits = (1u << (2 * last_pairs)) - 1u;
-    for (int64_t b = lane; b < stride_out; b += 32) {
-        unsigned v;
-        if (b < bps - 1) v = src[b];
-        else if (b == bps - 1) v = (src[b] & keep_bits) | (0xFFu & ~keep_bits);
-        else v = 0xFFu;
-        dst[b] = (uint8_t)v;
+// ---- indices of the kept SNPs, in order: per-CTA counts, their scan, the scatter ----
+constexpr int KEEP_T = 1024;
+
+__global__ void __launch_bounds__(KEEP_T) k_keep_count(const uint8_t* __restrict__ keep, int64_t M,
+                                                       int64_t* __restrict__ cnt) {
+    const int64_t s = (int64_t)blockIdx.x * KEEP_T + threadIdx.x;
+    const int n = __syncthreads_count(s < M && keep[s]);
+    if (threadIdx.x == 0) cnt[blockIdx.x] = n;
+}
+// exclusive scan in place, one CTA; cnt[nb] = the total
+__global__ void __launch_bounds__(KEEP_T) k_keep_scan(int64_t* __restrict__ cnt, int nb) {
+    __shared__ int64_t sm[KEEP_T];
+    int64_t base = 0;
+    for (int b0 = 0; b0 < nb; b0 += KEEP_T) {
+        const int b = b0 + threadIdx.x;
+        const int64_t v = b < nb ? cnt[b] : 0;
+        sm[threadIdx.x] = v;
+        __syncthreads();
+        for (int o = 1; o < KEEP_T; o <<= 1) {
+            const int64_t a = threadIdx.x >= o ? sm[threadIdx.x - o] : 0;
+            __syncthreads();
+            sm[threadIdx.x] += a;
+            __syncthreads();
+        }
+        if (b < nb) cnt[b] = base + sm[threadIdx.x] - v;
+        base += sm[KEEP_T - 1];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) cnt[nb] = base;
+}
+__global__ void __launch_bounds__(KEEP_T) k_keep_scatter(const uint8_t* __restrict__ keep, int64_t M,
+                                                         const int64_t* __restrict__ cnt, int64_t* __restrict__ idx) {
+    __shared__ int wsum[KEEP_T / 32];
+    const int64_t s = (int64_t)blockIdx.x * KEEP_T + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool k = s < M && keep[s];
+    const unsigned bal = __ballot_sync(0xffffffffu, k);
+    if (lane == 0) wsum[warp] = __popc(bal);
+    __syncthreads();
+    int64_t at = cnt[blockIdx.x] + __popc(bal & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; ++w) at += wsum[w];
+    if (k) idx[at] = s;
+}
+
+// cnt: keep_blocks(M) + 1 values, left as the offsets and the number of kept SNPs
+int keep_blocks(int64_t M) { return div_up(M, KEEP_T); }
+int keep_scan(globe_ctx* ctx, const uint8_t* d_keep, int64_t M, int64_t* cnt) {
+    if (M > 0) {
+        k_keep_count<<<keep_blocks(M), KEEP_T, 0, ctx->stream>>>(d_keep, M, cnt);
+        GLOBE_LAUNCHED(ctx, "k_keep_count");
+    }
+    k_keep_scan<<<1, KEEP_T, 0, ctx->stream>>>(cnt, keep_blocks(M));
+    GLOBE_LAUNCHED(ctx, "k_keep_scan");
+    return GLOBE_OK;
+}
+int keep_scatter(globe_ctx* ctx, const uint8_t* d_keep, int64_t M, const int64_t* cnt, int64_t* idx) {
+    k_keep_scatter<<<keep_blocks(M), KEEP_T, 0, ctx->stream>>>(d_keep, M, cnt, idx);
+    GLOBE_LAUNCHED(ctx, "k_keep_scatter");
+    return GLOBE_OK;
+}
+
+// Kept rows of the payload -> the SNP-major tile-blocked copy (tile codes), 16 bytes per thread,
+// straight from the payload: rows past Mk, bytes past the row and the phantom pairs of its last
+// byte become genotype 0.  Bound by its one read and one write (12.5 GB each; the former copy
+// of the kept rows moved as much again, a byte per lane, in 10.4 ms).
+__global__ void __launch_bounds__(256) k_bed_layout(const uint8_t* __restrict__ bed, int64_t stride,
+                                                    const int64_t* __restrict__ idx, int64_t Mk, int64_t bps, int32_t N,
+                                                    int64_t ntiles, int64_t nch, uint8_t* __restrict__ dst) {
+    using namespace tc;
+    const int64_t total = ntiles * nch * (BM * PKB / 16);
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t blkid = e / (BM * PKB / 16);
+        const int within = (int)(e % (BM * PKB / 16));
+        const int r = within >> 1, h = within & 1;
+        const int64_t t = blkid / nch, c = blkid % nch;
+        const int64_t row = t * BM + r, byte = c * PKB + h * 16;
+        uint4 v = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        if (row < Mk && byte < bps) {
+            const uint8_t* src = bed + idx[row] * stride + byte;
+            if (byte + 16 < bps) {
+                v = load16_any(src);
+            } else {   // the row's last bytes
+                uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                const int n = (int)(bps - byte), pairs = N - (int)((bps - 1) * 4);
+                const uint32_t real = (1u << (2 * pairs)) - 1u;
+                for (int q = 0; q < n; ++q) {
+                    uint32_t b = src[q];
+                    if (q == n - 1) b = (b & real) | (0xFFu & ~real);
+                    w[q >> 2] = (w[q >> 2] & ~(0xFFu << (8 * (q & 3)))) | (b << (8 * (q & 3)));
+                }
+                v = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        }
+        v = make_uint4(recode_tile(v.x), recode_tile(v.y), recode_tile(v.z), recode_tile(v.w));
+        const int64_t phys = (blkid * BM + r) * 2 + (h ^ ((r >> 2) & 1));   // halves swapped when bit 2 of r is set
+        *reinterpret_cast<uint4*>(dst + phys * 16) = v;
     }
 }
 
-int bed_compact(globe_ctx* ctx, const uint8_t* d_bed, int64_t stride_in, const int64_t* d_idx,
-                int64_t Mk, int64_t bps, uint8_t* d_out, int64_t stride_out) {
-    if (Mk == 0) return GLOBE_OK;
-    k_bed_compact<<<div_up(Mk, 8), 256, 0, ctx->stream>>>(d_bed, stride_in, d_idx, Mk, bps,
-                                                          ctx->coh.N, d_out, stride_out);
-    GLOBE_LAUNCHED(ctx, "k_bed_compact");
+int bed_layout(globe_ctx* ctx, const uint8_t* d_bed, int64_t stride, const int64_t* d_idx, int64_t Mk, int64_t bps,
+               int ntiles, int nch, uint8_t* dst) {
+    const int64_t total = (int64_t)ntiles * nch * (tc::BM * tc::PKB / 16);
+    k_bed_layout<<<(unsigned)std::min<int64_t>((total + 255) / 256, 65535), 256, 0, ctx->stream>>>(
+        d_bed, stride, d_idx, Mk, bps, ctx->coh.N, ntiles, nch, dst);
+    GLOBE_LAUNCHED(ctx, "k_bed_layout");
     return GLOBE_OK;
 }
 

@@ -392,7 +392,6 @@ static int grm_build_f64(globe_ctx* ctx, float* lt) {
     const int64_t nt = (N + 63) / 64;
     const int64_t ntiles = nt * (nt + 1) / 2;
     if (ntiles > 0x7FFFFFFFll) return set_err(ctx, GLOBE_ERR_ARG, "N too large for the FP64 GRM build");
-    GLOBE_RET(ensure_blk1(ctx));
     ProfScope p(ctx, GLOBE_PROF_GRM_BUILD_GEMM);
     k_grm_f64<<<(unsigned)ntiles, 256, 0, ctx->stream>>>(g.blk1, g.Mk, g.nch1, g.zs, N, (double)g.Mk, lt);
     GLOBE_LAUNCHED(ctx, "k_grm_f64");

@@ -66,19 +66,14 @@ __global__ void __launch_bounds__(256) k_geno_p1(const uint8_t* __restrict__ blk
 constexpr int P2_THREADS = 128;  // samples per CTA (32 bytes per SNP row)
 constexpr int P2_TS = 64;        // SNPs per shared-memory tile
 
-// SQUARE: accumulate zs^2 (genetic diagonal) instead of zs * W, as double-float sums of the
-// FP64 squares split into float pairs (GB300's FP64 pipe would bound the 5e10 additions of
-// the full workload at ~0.1 s; on the FP32 pipe they take a few ms).
-template <int KC, bool SQUARE>
+template <int KC>
 __global__ void __launch_bounds__(P2_THREADS) k_geno_p2(const uint8_t* __restrict__ blk, int nch,
                                                         int64_t Mk, int32_t N, const double* __restrict__ zs,
-                                                        const float2* __restrict__ zsq,
                                                         const double* __restrict__ W, int64_t ldw, int kc,
                                                         int64_t s_per, double* __restrict__ part) {
     __shared__ __align__(16) uint8_t gb[P2_TS][32];
     __shared__ double zt[P2_TS][4];
-    __shared__ double wt[P2_TS][KC > 0 ? KC : 1];
-    __shared__ float2 zq[P2_TS][4];   // SQUARE: zs^2 by tile code as (hi, lo) floats
+    __shared__ double wt[P2_TS][KC];
     const int tid = threadIdx.x;
     const int64_t i = (int64_t)blockIdx.x * P2_THREADS + tid;
     const int64_t byte0 = (int64_t)blockIdx.x * 32;   // this CTA's 32-byte chunk of every row
@@ -88,7 +83,6 @@ __global__ void __launch_bounds__(P2_THREADS) k_geno_p2(const uint8_t* __restric
     double acc[KC];
 #pragma unroll
     for (int c = 0; c < KC; ++c) acc[c] = 0.0;
-    float qh = 0.0f, ql = 0.0f;   // SQUARE: double-float sum
     const int sh = 2 * (tid & 3);
     const int bi = tid >> 2;
     for (int64_t s0 = s_beg; s0 < s_end; s0 += P2_TS) {
@@ -102,46 +96,27 @@ __global__ void __launch_bounds__(P2_THREADS) k_geno_p2(const uint8_t* __restric
         }
         for (int e = tid; e < P2_TS * 4; e += P2_THREADS) {
             const int rs = e >> 2;
-            if (SQUARE) zq[rs][e & 3] = rs < ns ? zsq[(s0 + rs) * 4 + (e & 3)] : make_float2(0.0f, 0.0f);
-            else zt[rs][e & 3] = rs < ns ? zs[(s0 + rs) * 4 + (e & 3)] : 0.0;
+            zt[rs][e & 3] = rs < ns ? zs[(s0 + rs) * 4 + (e & 3)] : 0.0;
         }
-        if (!SQUARE) {
-            for (int e = tid; e < P2_TS * KC; e += P2_THREADS) {
-                const int rs = e / KC, c = e % KC;
-                wt[rs][c] = (rs < ns && c < kc) ? W[(s0 + rs) + (size_t)c * ldw] : 0.0;
-            }
+        for (int e = tid; e < P2_TS * KC; e += P2_THREADS) {
+            const int rs = e / KC, c = e % KC;
+            wt[rs][c] = (rs < ns && c < kc) ? W[(s0 + rs) + (size_t)c * ldw] : 0.0;
         }
         __syncthreads();
         for (int rs = 0; rs < ns; ++rs) {
             const unsigned code = (gb[rs][bi] >> sh) & 3u;
-            if (SQUARE) {
-                const float2 q = zq[rs][code];
-                tc::df_add(qh, ql, q.x, q.y);
-            } else {
-                const double z = zsel(code, zt[rs][0], zt[rs][1], zt[rs][2]);
+            const double z = zsel(code, zt[rs][0], zt[rs][1], zt[rs][2]);
 #pragma unroll
-                for (int c = 0; c < KC; ++c) acc[c] += z * wt[rs][c];
-            }
+            for (int c = 0; c < KC; ++c) acc[c] += z * wt[rs][c];
         }
         __syncthreads();
     }
-    if (SQUARE) acc[0] = (double)qh + (double)ql;
     if (i < N) {
-        const size_t base = (size_t)blockIdx.y * (size_t)N * (SQUARE ? 1 : kc);
+        const size_t base = (size_t)blockIdx.y * (size_t)N * kc;
 #pragma unroll
         for (int c = 0; c < KC; ++c)
-            if (c < (SQUARE ? 1 : kc)) part[base + i + (size_t)c * N] = acc[c];
+            if (c < kc) part[base + i + (size_t)c * N] = acc[c];
     }
-}
-
-// zsq[4 s + t] = zs^2 of tile code t as a (hi, lo) float pair (t: 0/3 -> g=0, 1 -> g=1, 2 -> g=2)
-__global__ void k_zs_square(const double* __restrict__ zs, int64_t Mk, float2* __restrict__ zsq) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 4 * Mk) return;
-    const double z = zs[(e & ~3ll) + tc::tile_to_plink((int)(e & 3))];
-    const double q = z * z;
-    const float hi = __double2float_rn(q);
-    zsq[e] = make_float2(hi, __double2float_rn(q - (double)hi));
 }
 
 // out[e] = scale * sum_y part[y * n + e]  (fixed order)
@@ -177,8 +152,7 @@ static int geno_chunk(globe_ctx* ctx, const double* Z, int kc, double scale, dou
     dim3 grid(div_up(N, P2_THREADS), nsplit);
     {
         ProfScope ps(ctx, GLOBE_PROF_GRM_PASS2);
-        k_geno_p2<KC, false><<<grid, P2_THREADS, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, nullptr, W, g.Mk, kc,
-                                                                    s_per, part);
+        k_geno_p2<KC><<<grid, P2_THREADS, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, W, g.Mk, kc, s_per, part);
         GLOBE_LAUNCHED(ctx, "k_geno_p2");
     }
     int64_t n = (int64_t)N * kc;
@@ -196,7 +170,6 @@ int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, d
         GLOBE_CK(ctx, cudaMemsetAsync(out, 0, sizeof(double) * (size_t)N * k, ctx->stream));
         return GLOBE_OK;
     }
-    GLOBE_RET(ensure_blk1(ctx));
     const int kcmax = 8;
     int kc0 = k < kcmax ? k : kcmax;
     double* W;
@@ -221,6 +194,104 @@ int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, d
     return GLOBE_OK;
 }
 
+// ---- A_ii = (1/M) sum_s zs(s,i)^2 (PCGsolver.cpp:924-989) --------------------------
+//
+// zs^2 takes one of three values per SNP, so four SNPs' share of an individual is one entry of a
+// 256-entry table indexed by their four codes (one byte).  Entries are fixed-point int64 on one
+// grid for the whole matrix (2^62 above the largest possible sum), so any split of the SNPs
+// sums to the same bits, within M 2^-63 of the exact sum.
+// A CTA covers 8192 individuals (16 per thread: one word of each of the four SNP rows) and a
+// range of SNPs.  The table is held 16 times over, entry e of copy l at (16 e + l): the 16 lanes
+// of a half warp read 16 different bank pairs whatever their codes.  Two pair tables of 16
+// entries build it (4 stores of two copies per thread).  Bound by the table reads (one 8-byte
+// shared load per 4 genotypes) and the integer work around them.
+constexpr int DG_THREADS = 512;
+
+// the largest zs^2 (non-negative doubles order like their bits)
+__global__ void k_zs_max(const double* __restrict__ zs, int64_t n, unsigned long long* __restrict__ out) {
+    unsigned long long m = 0;
+    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
+        m = max(m, (unsigned long long)__double_as_longlong(zs[e] * zs[e]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+// fraction bits of the fixed-point sums: Mk zs^2 < 2^(62 - bits)
+__device__ __forceinline__ int diag_bits(const unsigned long long* maxq, int64_t Mk) {
+    int E;
+    frexp(__longlong_as_double((long long)*maxq) * (double)Mk, &E);
+    return 62 - E;
+}
+
+__global__ void __launch_bounds__(DG_THREADS, 2) k_geno_diag(const uint8_t* __restrict__ blk, int nch, int64_t Mk,
+                                                             int32_t N, const double* __restrict__ zs,
+                                                             const unsigned long long* __restrict__ maxq, int64_t gper,
+                                                             long long* __restrict__ part) {
+    __shared__ __align__(16) long long lut[256 * 16];
+    __shared__ long long pt[2][16];
+    const int tid = threadIdx.x;
+    const int64_t c = (int64_t)blockIdx.x * (DG_THREADS / 8) + (tid >> 3);   // 128-individual chunk
+    const int w = tid & 7;                                                   // its word of 16 individuals
+    const bool in = c < nch;
+    const int64_t ng = (Mk + 3) / 4, g0 = (int64_t)blockIdx.y * gper, g1 = min(ng, g0 + gper);
+    const double sc = ldexp(1.0, diag_bits(maxq, Mk));
+    const int el = (tid >> 3) & 15, eh = tid >> 7;
+    const long long* mine = lut + (tid & 15);
+    long long acc[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[j] = 0;
+    for (int64_t g = g0; g < g1; ++g) {
+        const int64_t s0 = 4 * g;
+        uint32_t r[4] = {0u, 0u, 0u, 0u};
+        if (in) {
+            const int rr = (int)(s0 & 127);   // a multiple of 4: the four rows share their half swap
+            const uint8_t* p = blk + (((s0 >> 7) * nch + c) * 128 + rr) * 32 + (((w >> 2) ^ ((rr >> 2) & 1)) * 16) + (w & 3) * 4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) r[q] = __ldg(reinterpret_cast<const uint32_t*>(p + 32 * q));
+        }
+        if (tid < 32) {
+            const int64_t sa = s0 + 2 * (tid >> 4);
+            const int ca = tc::tile_to_plink(tid & 3), cb = tc::tile_to_plink((tid >> 2) & 3);
+            long long v = 0;
+            if (sa < Mk) v += __double2ll_rn(zs[4 * sa + ca] * zs[4 * sa + ca] * sc);
+            if (sa + 1 < Mk) v += __double2ll_rn(zs[4 * sa + 4 + cb] * zs[4 * sa + 4 + cb] * sc);
+            pt[tid >> 4][tid & 15] = v;
+        }
+        __syncthreads();
+        const long long vl = pt[0][el];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {   // entry (el, eh + 4 q), copies 2 (tid & 7) and the next
+            const long long v = vl + pt[1][eh + 4 * q];
+            *reinterpret_cast<longlong2*>(lut + (((eh + 4 * q) * 16 + el) * 16 + 2 * (tid & 7))) = make_longlong2(v, v);
+        }
+        __syncthreads();
+        if (in) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                // byte b: the four SNPs' codes of individual 4 b + m
+                const uint32_t t = ((r[0] >> (2 * m)) & 0x03030303u) | (((r[1] >> (2 * m)) & 0x03030303u) << 2) |
+                                   (((r[2] >> (2 * m)) & 0x03030303u) << 4) | (((r[3] >> (2 * m)) & 0x03030303u) << 6);
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[4 * b + m] += mine[((t >> (8 * b)) & 255u) * 16];
+            }
+        }
+    }
+    const int64_t i0 = c * 128 + w * 16;
+    long long* out = part + (int64_t)blockIdx.y * N;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (in && i0 + j < N) out[i0 + j] = acc[j];
+}
+
+__global__ void k_geno_diag_sum(const long long* __restrict__ part, int nsplit, int64_t Mk, int32_t N,
+                                const unsigned long long* __restrict__ maxq, double* __restrict__ d) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    long long a = 0;
+    for (int y = 0; y < nsplit; ++y) a += part[(int64_t)y * N + i];
+    d[i] = ldexp((double)a, -diag_bits(maxq, Mk)) / (double)Mk;
+}
+
 int geno_diag(globe_ctx* ctx, double* d) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
@@ -228,24 +299,23 @@ int geno_diag(globe_ctx* ctx, double* d) {
         GLOBE_CK(ctx, cudaMemsetAsync(d, 0, sizeof(double) * N, ctx->stream));
         return GLOBE_OK;
     }
-    GLOBE_RET(ensure_blk1(ctx));
-    int64_t ctas_x = div_up(N, P2_THREADS);
-    int nsplit = pick_splits(ctas_x, g.Mk);
-    int64_t s_per = ((g.Mk + nsplit - 1) / nsplit + P2_TS - 1) / P2_TS * P2_TS;
-    nsplit = (int)((g.Mk + s_per - 1) / s_per);
-    double* part;
-    GLOBE_RET(ws(ctx, WS_GPART, (size_t)nsplit * N, &part));
-    float2* zsq;
-    GLOBE_RET(ws(ctx, WS_W, (size_t)g.Mk * 4, &zsq));
-    k_zs_square<<<div_up(4 * g.Mk, 256), 256, 0, ctx->stream>>>(g.zs, g.Mk, zsq);
-    GLOBE_LAUNCHED(ctx, "k_zs_square");
-    dim3 grid((unsigned)ctas_x, nsplit);
-    k_geno_p2<1, true><<<grid, P2_THREADS, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, zsq, nullptr, 0, 1,
-                                                              s_per, part);
+    // about four waves of two CTAs an SM (the last one ragged), at least 16 groups of SNPs each
+    const int64_t cx = div_up(div_up(N, 128), DG_THREADS / 8), ng = (g.Mk + 3) / 4;
+    int64_t ns = std::max<int64_t>(1, std::min<int64_t>((8 * 152 + cx - 1) / cx, ng / 16));
+    const int64_t gper = (ng + ns - 1) / ns;
+    ns = (ng + gper - 1) / gper;
+    long long* part;
+    unsigned long long* maxq;
+    GLOBE_RET(ws(ctx, WS_GPART, (size_t)ns * N + 1, &part));
+    maxq = reinterpret_cast<unsigned long long*>(part + ns * N);
+    GLOBE_CK(ctx, cudaMemsetAsync(maxq, 0, sizeof(*maxq), ctx->stream));
+    k_zs_max<<<(unsigned)std::min<int64_t>(div_up(4 * g.Mk, 1024), 304), 256, 0, ctx->stream>>>(g.zs, 4 * g.Mk, maxq);
+    GLOBE_LAUNCHED(ctx, "k_zs_max");
+    k_geno_diag<<<dim3((unsigned)cx, (unsigned)ns), DG_THREADS, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, maxq,
+                                                                                  gper, part);
     GLOBE_LAUNCHED(ctx, "k_geno_diag");
-    // A_ii = (1/M) sum_s zs^2   (PCGsolver.cpp:986-988)
-    k_sum_splits<<<div_up(N, 256), 256, 0, ctx->stream>>>(part, nsplit, N, 1.0 / (double)g.Mk, d, N, N);
-    GLOBE_LAUNCHED(ctx, "k_sum_splits");
+    k_geno_diag_sum<<<div_up(N, 256), 256, 0, ctx->stream>>>(part, (int)ns, g.Mk, N, maxq, d);
+    GLOBE_LAUNCHED(ctx, "k_geno_diag_sum");
     return GLOBE_OK;
 }
 

@@ -682,33 +682,6 @@ __global__ void __launch_bounds__(256) k_blk_transpose(const uint8_t* __restrict
     }
 }
 
-// row-major packed rows (stride bytes) -> tile-blocked layout of tile codes, 16 bytes per
-// thread; rows >= nrows and bytes >= stride become PLINK 0xFF (genotype 0)
-__global__ void k_blockify(const uint8_t* __restrict__ src, int64_t nrows, int64_t stride, int64_t ntiles,
-                           int64_t nch, uint8_t* __restrict__ dst) {
-    const int64_t total = ntiles * nch * (BM * PKB / 16);
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t blkid = e / (BM * PKB / 16);
-        const int within = (int)(e % (BM * PKB / 16));
-        const int r = within >> 1, h = within & 1;
-        const int64_t t = blkid / nch, c = blkid % nch;
-        const int64_t row = t * BM + r, byte = c * PKB + h * 16;
-        uint4 v = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
-        if (row < nrows && byte < stride) {
-            if (byte + 16 <= stride) {
-                v = *reinterpret_cast<const uint4*>(src + row * stride + byte);
-            } else {
-                uint8_t tmp[16];
-                for (int q = 0; q < 16; ++q) tmp[q] = byte + q < stride ? src[row * stride + byte + q] : (uint8_t)0xFF;
-                v = *reinterpret_cast<const uint4*>(tmp);
-            }
-        }
-        v = make_uint4(recode_tile(v.x), recode_tile(v.y), recode_tile(v.z), recode_tile(v.w));
-        const int64_t phys = (blkid * BM + r) * 2 + (h ^ ((r >> 2) & 1));   // halves swapped when bit 2 of r is set
-        *reinterpret_cast<uint4*>(dst + phys * 16) = v;
-    }
-}
-
 }  // namespace tc
 
 // ---- host side ---------------------------------------------------------------
@@ -761,43 +734,13 @@ static int encode_map(globe_ctx* ctx, CUtensorMap* m, const void* base, uint64_t
     return GLOBE_OK;
 }
 
-static int blockify(globe_ctx* ctx, const uint8_t* src, int64_t nrows, int64_t stride, uint8_t** dst, int* nch,
-                    int* ntiles) {
-    *nch = (int)((stride + PKB - 1) / PKB);
-    *ntiles = (int)((nrows + BM - 1) / BM);
-    // whole CTAs: round the tile count up to a multiple of TILE_PAD (a CTA owns 1 to 4 tiles)
-    *ntiles = (*ntiles + TILE_PAD - 1) / TILE_PAD * TILE_PAD;
-    GLOBE_RET(dalloc(ctx, dst, (size_t)(*ntiles) * (*nch) * BM * PKB));
-    const int64_t total = (int64_t)(*ntiles) * (*nch) * (BM * PKB / 16);
-    k_blockify<<<(unsigned)std::min<int64_t>((total + 255) / 256, 65535), 256, 0, ctx->stream>>>(
-        src, nrows, stride, *ntiles, *nch, *dst);
-    GLOBE_LAUNCHED(ctx, "k_blockify");
-    return GLOBE_OK;
-}
-
-// The SNP-major tile-blocked copy (blk1) from the compacted rows, which are freed: every
-// genotype kernel reads the tile-blocked copies.  Called when genotypes are loaded.
-int ensure_blk1(globe_ctx* ctx) {
-    auto& g = ctx->gen;
-    if (g.blk1) return GLOBE_OK;
-    if (!g.geno) return set_err(ctx, GLOBE_ERR_STATE, "no genotype rows to lay out");
-    GLOBE_RET(blockify(ctx, g.geno, g.Mk, g.stride, &g.blk1, &g.nch1, &g.ntiles1));
-    GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    dfree(ctx, g.geno);   // the compacted rows live on as blk1
-    g.geno = nullptr;
-    return GLOBE_OK;
-}
-
 // The individual-major tile-blocked copy (blk2, the tensor-core pass-2 operand) by block
 // transposes of blk1; built on the first tensor-core use, so FP64-only work holds one copy.
 int ensure_blk2(globe_ctx* ctx) {
     auto& g = ctx->gen;
     if (g.blk2) return GLOBE_OK;
-    GLOBE_RET(ensure_blk1(ctx));
     const int32_t N = ctx->coh.N;
-    g.strideT = ((g.Mk + 3) / 4 + PKB - 1) / PKB * PKB;   // individual-major row: SNP bytes, whole chunks
-    if (g.strideT < PKB) g.strideT = PKB;
-    g.nch2 = (int)(g.strideT / PKB);
+    g.nch2 = (int)std::max<int64_t>(1, ((g.Mk + 3) / 4 + PKB - 1) / PKB);   // 32-byte chunks of an individual's SNPs
     g.ntiles2 = (int)((N + BM - 1) / BM);
     g.ntiles2 = (g.ntiles2 + TILE_PAD - 1) / TILE_PAD * TILE_PAD;   // whole CTAs of 1 to 4 tiles
     GLOBE_RET(dalloc(ctx, &g.blk2, (size_t)g.ntiles2 * g.nch2 * BM * PKB));
