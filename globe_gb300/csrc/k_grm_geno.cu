@@ -240,23 +240,31 @@ __global__ void __launch_bounds__(DG_THREADS, 2) k_geno_diag(const uint8_t* __re
     long long acc[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[j] = 0;
-    for (int64_t g = g0; g < g1; ++g) {
+    // a group's four words, and (threads < 32) the two zs of their pair-table entry: loaded one
+    // group ahead of their use
+    uint32_t r[4], rn[4] = {0u, 0u, 0u, 0u};
+    double za = 0.0, zb = 0.0;
+    const int ca = tc::tile_to_plink(tid & 3), cb = tc::tile_to_plink((tid >> 2) & 3);
+    auto fetch = [&](int64_t g) {
         const int64_t s0 = 4 * g;
-        uint32_t r[4] = {0u, 0u, 0u, 0u};
         if (in) {
             const int rr = (int)(s0 & 127);   // a multiple of 4: the four rows share their half swap
             const uint8_t* p = blk + (((s0 >> 7) * nch + c) * 128 + rr) * 32 + (((w >> 2) ^ ((rr >> 2) & 1)) * 16) + (w & 3) * 4;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) r[q] = __ldg(reinterpret_cast<const uint32_t*>(p + 32 * q));
+            for (int q = 0; q < 4; ++q) rn[q] = __ldg(reinterpret_cast<const uint32_t*>(p + 32 * q));
         }
         if (tid < 32) {
             const int64_t sa = s0 + 2 * (tid >> 4);
-            const int ca = tc::tile_to_plink(tid & 3), cb = tc::tile_to_plink((tid >> 2) & 3);
-            long long v = 0;
-            if (sa < Mk) v += __double2ll_rn(zs[4 * sa + ca] * zs[4 * sa + ca] * sc);
-            if (sa + 1 < Mk) v += __double2ll_rn(zs[4 * sa + 4 + cb] * zs[4 * sa + 4 + cb] * sc);
-            pt[tid >> 4][tid & 15] = v;
+            za = sa < Mk ? zs[4 * sa + ca] : 0.0;
+            zb = sa + 1 < Mk ? zs[4 * sa + 4 + cb] : 0.0;
         }
+    };
+    if (g0 < g1) fetch(g0);
+    for (int64_t g = g0; g < g1; ++g) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = rn[q];
+        if (tid < 32) pt[tid >> 4][tid & 15] = __double2ll_rn(za * za * sc) + __double2ll_rn(zb * zb * sc);
+        if (g + 1 < g1) fetch(g + 1);
         __syncthreads();
         const long long vl = pt[0][el];
 #pragma unroll
