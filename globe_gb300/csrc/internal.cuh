@@ -87,7 +87,7 @@ enum SlotId {
     WS_R, WS_Z, WS_P, WS_VP, WS_ZI, WS_GZ, WS_S1, WS_PART, WS_SCAL, WS_COLS, WS_W,
     WS_GPART, WS_B, WS_TMP1, WS_TMP2, WS_TMP3, WS_TMP4, WS_H, WS_HSTAR, WS_PROBE,
     WS_UH, WS_SMALL, WS_IO1, WS_IO2, WS_BHAT, WS_FB, WS_FX,
-    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_S0DF, WS_HDF, WS_TC_CNT, WS_COUNT
+    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_S0DF, WS_HDF, WS_TC_CNT, WS_TC_STAT, WS_COUNT
 };
 
 // Scalars kept on the device during a solve (per column, k entries each).
@@ -114,6 +114,7 @@ struct globe_ctx {
     double vc[5] = {0, 0, 0, 0, 0};
     bool vc_set = false;
     int in_solve = 0;             // inside a call that repeats its products (SolveScope)
+    bool stat_dirty = false;      // a product stopped before it cleared its columns' statistics words
     bool tc_used = false;         // a tensor-core product was launched since the error word was last read
     int prec = GLOBE_PREC_FP64;   // precision of operator calls (globe_set_precision / PCG options)
     int model = GLOBE_MODEL_FULL; // GLOBE_MODEL_NO_TIME: components (sig2e, sig2g) only
@@ -343,15 +344,15 @@ int dense_apply_df(globe_ctx* ctx, const double* Z, int k, double scale, double*
 int dense_diag(globe_ctx* ctx, double* d);
 
 // k_tc_dense.cu
-int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);    // GLOBE_PREC_MIXED
-int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);   // GLOBE_PREC_FP64
+int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready);    // GLOBE_PREC_MIXED
+int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready);   // GLOBE_PREC_FP64
 
 // k_tc_geno.cu
 int ensure_blk2(globe_ctx* ctx);   // individual-major tile-blocked copy (first tensor-core use)
 int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t stride, float min_maf, float max_miss,
                   int64_t* d_alt, int64_t* d_miss, float* d_maf, float* d_mr, uint8_t* d_keep, globe_bed_info* info);
-int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out);    // GLOBE_PREC_MIXED
-int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out);   // GLOBE_PREC_FP64
+int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready);    // GLOBE_PREC_MIXED
+int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready);   // GLOBE_PREC_FP64
 int tc_err_word(globe_ctx* ctx, unsigned** err);   // the kernels' timeout word (cleared when created)
 int tc_check_error(globe_ctx* ctx);                 // reads and clears it: GLOBE_ERR_CUDA if set
 int tc_counters(globe_ctx* ctx, size_t n, unsigned** cnt);   // >= n zeroed per-column arrival counts
@@ -359,7 +360,8 @@ int tc_counters(globe_ctx* ctx, size_t n, unsigned** cnt);   // >= n zeroed per-
 int with_tc_check(globe_ctx* ctx, int rc);
 
 // solver.cu
-int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out);
+// zhi_ready: the kernel that wrote Z raised its columns' statistics words (tc_stat)
+int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out, bool zhi_ready = false);
 int ensure_gdiag(globe_ctx* ctx);
 int ensure_precond(globe_ctx* ctx);
 int vx_dev(globe_ctx* ctx, const double* x, int k, double* out);

@@ -45,8 +45,8 @@ __global__ void k_grm_u4(const double* __restrict__ zs, const double* __restrict
 // the rest: ~48 bits).
 // SNPs >= Mk (padding of the K range) get zero digits and zero.
 __global__ void k_grm_table(const double* __restrict__ U4, const double* __restrict__ f, int64_t Mk, int64_t kpad,
-                            const double* __restrict__ info, uint4* __restrict__ dig, float2* __restrict__ c2v) {
-    const int e = (int)info[0];
+                            const unsigned* __restrict__ hi, uint4* __restrict__ dig, float2* __restrict__ c2v) {
+    const int e = col_exp<NDIG>(*hi);
     const double sc = ldexp(1.0, DBITS * (NDIG - 1) - e), back = ldexp(1.0, e - DBITS * (NDIG - 1));
     for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < 4 * kpad;
          x += (int64_t)gridDim.x * blockDim.x) {
@@ -188,7 +188,7 @@ __global__ void k_grm_c2(const double* __restrict__ part, int nqb, int ncols, do
 // row-contiguous writes of the packed triangle are coalesced.
 __global__ void __launch_bounds__(256) k_grm_combine(const float* __restrict__ part, int nsplit, int64_t ldp,
                                                      int64_t pz, int32_t N, int jb, const double* __restrict__ C2,
-                                                     const double* __restrict__ info, double inv_m,
+                                                     const unsigned* __restrict__ hi, double inv_m,
                                                      float* __restrict__ lt) {
     __shared__ float sv[32][GRM_KG + 1];
     const int z = blockIdx.y;
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(256) k_grm_combine(const float* __restrict__ p
     const int64_t i0 = j0 + (int64_t)blockIdx.x * 32;
     if (j0 >= N || i0 >= N) return;
     double s_hi, s_lo;
-    recombine_scales<NDIG>((int)info[0], s_hi, s_lo);
+    recombine_scales<NDIG>(col_exp<NDIG>(*hi), s_hi, s_lo);
     const float* pzp = part + z * pz;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t i = i0 + lane;
@@ -317,9 +317,9 @@ static int grm_build_tc(globe_ctx* ctx, float* lt) {
     size_t gfit = std::min<size_t>((size_t)ngroups, (size_t)65535);
     gfit = std::min<size_t>(gfit, ((size_t)2 << 30) / per_group);
     const int G = (int)std::max<size_t>(1, gfit);
-    const int nbr = 304;
     BuildBufs B(ctx);
-    double *U4, *C2, *info, *pm, *ps, *c2part;
+    double *U4, *C2, *c2part;
+    unsigned* hi;
     float2* c2v;
     uint4* dig;
     uint8_t* D;
@@ -331,9 +331,8 @@ static int grm_build_tc(globe_ctx* ctx, float* lt) {
     GLOBE_RET(B.get(&C2, (size_t)G * GRM_KG));
     const int nqb = (int)((kpad / 16 + GD_Q - 1) / GD_Q);   // SNP ranges of k_grm_digits
     GLOBE_RET(B.get(&c2part, (size_t)nqb * G * GRM_KG));
-    GLOBE_RET(B.get(&info, (size_t)2));
-    GLOBE_RET(B.get(&pm, (size_t)nbr));
-    GLOBE_RET(B.get(&ps, (size_t)nbr));
+    GLOBE_RET(B.get(&hi, (size_t)1));
+    GLOBE_CK(ctx, cudaMemsetAsync(hi, 0, sizeof(unsigned), ctx->stream));
     GLOBE_RET(B.get(&D, (size_t)G * GRM_NMMA * kpad));
     GLOBE_RET(B.get(&P, (size_t)G * spe * GRM_NMMA * ldp));
     GLOBE_RET(tc_err_word(ctx, &err));
@@ -354,12 +353,10 @@ static int grm_build_tc(globe_ctx* ctx, float* lt) {
     k_grm_u4<<<(unsigned)std::min<int64_t>(div_up(4 * g.Mk, 256), 4096), 256, 0, ctx->stream>>>(g.zs, g.inv, g.Mk,
                                                                                                  U4);
     GLOBE_LAUNCHED(ctx, "k_grm_u4");
-    k_col_maxsum<<<dim3(nbr, 1), 256, 0, ctx->stream>>>(U4, 4 * g.Mk, 4 * g.Mk, pm, ps, nullptr, nullptr);
-    GLOBE_LAUNCHED(ctx, "k_col_maxsum");
-    k_col_finish<<<1, 128, 0, ctx->stream>>>(pm, ps, nbr, 1, info);
-    GLOBE_LAUNCHED(ctx, "k_col_finish");
+    k_col_max<<<dim3(col_parts(4 * g.Mk), 1), 256, 0, ctx->stream>>>(U4, 4 * g.Mk, 4 * g.Mk, hi);
+    GLOBE_LAUNCHED(ctx, "k_col_max");
     k_grm_table<<<(unsigned)std::min<int64_t>(div_up(4 * kpad, 256), 4096), 256, 0, ctx->stream>>>(
-        U4, g.f, g.Mk, kpad, info, dig, c2v);
+        U4, g.f, g.Mk, kpad, hi, dig, c2v);
     GLOBE_LAUNCHED(ctx, "k_grm_table");
     const int64_t pz = (int64_t)spe * GRM_NMMA * ldp;
     for (int jb = 0; jb < N; jb += G * GRM_KG) {
@@ -380,7 +377,7 @@ static int grm_build_tc(globe_ctx* ctx, float* lt) {
             GLOBE_RET(gemm_dispatch(ctx, GRM_NMMA, g.blk2, g.ntiles2, mB, N, nch, splits, P, ldp, err, zg));
         }
         k_grm_combine<<<dim3((unsigned)div_up(N - jb, 32), (unsigned)gb), 256, 0, ctx->stream>>>(
-            P, spe, ldp, pz, N, jb, C2, info, 1.0 / (double)g.Mk, lt);
+            P, spe, ldp, pz, N, jb, C2, hi, 1.0 / (double)g.Mk, lt);
         GLOBE_LAUNCHED(ctx, "k_grm_combine");
     }
     return GLOBE_OK;

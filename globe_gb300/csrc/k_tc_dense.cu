@@ -266,12 +266,13 @@ __global__ void __launch_bounds__(256) k_dense_digits(const float* __restrict__ 
 template <int ND>
 __global__ void k_dense_combine(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int32_t N,
                                 int64_t np, int da, const double* __restrict__ colinfo, double sA,
-                                double* __restrict__ out, int64_t ldo) {
+                                double* __restrict__ out, int64_t ldo, unsigned* __restrict__ zhi) {
     constexpr int NT = DA_MAX + ND - 1;
     static_assert(NT <= 15, "three chunks of five weights");
     const int c = blockIdx.y;
-    const double s0 = sA * ldexp(1.0, (int)colinfo[2 * c] - 20);   // 2^(e_c - 5*4) for chunk 0
-    const bool bad = isnan(colinfo[2 * c + 1]);   // a non-finite column (k_col_finish): NaN out
+    if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;   // cleared for the next product
+    const double s0 = sA * pow2i((int)colinfo[2 * c] - 20);   // 2^(e_c - 5*4) for chunk 0
+    const bool bad = isnan(colinfo[2 * c + 1]);   // a non-finite column: NaN out
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
         long long T[NT];
 #pragma unroll
@@ -308,12 +309,14 @@ __global__ void k_dense_combine(const float* __restrict__ part, int nsplit, int 
 __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict__ part, int nsplit, int nmma,
                                                          int64_t ldp, int32_t N, int64_t np,
                                                          const double* __restrict__ colinfo, double sA, double scale,
-                                                         double* __restrict__ out, int64_t ldo) {
+                                                         double* __restrict__ out, int64_t ldo,
+                                                         unsigned* __restrict__ zhi) {
     constexpr int NT = DA64 + ND64 - 1;
     static_assert(NT <= 25, "five chunks of five weights");
     const int c = blockIdx.y;
+    if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;
     const int e = (int)colinfo[2 * c];
-    const double ea = ldexp(1.0, e / 2), eb = ldexp(1.0, e - e / 2), bad = colinfo[2 * c + 1];
+    const double ea = pow2i(e / 2), eb = pow2i(e - e / 2), bad = colinfo[2 * c + 1];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
         long long T[NT];
 #pragma unroll
@@ -474,7 +477,7 @@ static int dense_cps(globe_ctx* ctx, int tiles, int nchunks, int nmma) {
 
 // out (N x kg) = scale * A Z for one group of <= 256 / ND columns
 template <int ND>
-static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out) {
+static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st) {
     constexpr bool F64 = ND == ND64;
     const auto& a = ctx->gen.adig[F64 ? 1 : 0];
     const int32_t N = ctx->coh.N;
@@ -487,30 +490,19 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     const int64_t ldp = rows;
     uint8_t* D;
     float* P;
-    double* cst;
+    double* col;
     unsigned* err;
-    const int nbr = 304;
     GLOBE_RET(ws(ctx, WS_TC_D1, (size_t)nmma * np, &D));
     GLOBE_RET(ws(ctx, WS_TC_P1, (size_t)splits * nmma * ldp, &P));
-    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(4 * kg + 2 * nbr * kg + 8), &cst));
+    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)2 * kg, &col));
     GLOBE_RET(tc_err_word(ctx, &err));
-    double* col = cst;
-    unsigned long long* isum = reinterpret_cast<unsigned long long*>(cst + 2 * kg);   // F64: scratch of k_col_max64
-    double* pm = cst + 4 * kg;
-    double* ps = pm + (size_t)nbr * kg;
     CUtensorMap mA, mB;
     GLOBE_RET(make_map(ctx, &mA, a.p, (uint64_t)np, (uint64_t)rows, BK, BM, true));
     GLOBE_RET(make_map(ctx, &mB, D, (uint64_t)np, (uint64_t)nmma, BK, (uint32_t)nmma, true));
-    const int nz = col_parts(N);
-    unsigned* cnt;
-    GLOBE_RET(tc_counters(ctx, kg, &cnt));
-    if constexpr (F64) k_col_max64<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, cnt, col, isum);
-    else k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col);
-    GLOBE_LAUNCHED(ctx, "k_col_maxsum");
     if (nmma > kg * ND)   // digit rows past the kg columns stay zero
         GLOBE_CK(ctx, cudaMemsetAsync(D + (size_t)kg * ND * np, 0, (size_t)(nmma - kg * ND) * np, ctx->stream));
     k_digits<ND, false><<<dim3((unsigned)std::min<int64_t>(div_up(np / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, kg, col, D, np, nullptr);
+        Z, N, N, st.zhi, col, D, np, nullptr, nullptr);
     GLOBE_LAUNCHED(ctx, "k_digits");
     {
         ProfScope p(ctx, GLOBE_PROF_GRM_PASS1);
@@ -521,45 +513,49 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     const dim3 gc((unsigned)std::min(div_up(N, 256), 1024), kg);
     if constexpr (F64)
         k_dense_combine64<<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, col, std::ldexp(1.0, a.e - 20), scale,
-                                                       out, N);
+                                                       out, N, st.zhi);
     else
         k_dense_combine<ND><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
-                                                         std::ldexp(scale, a.e), out, N);
+                                                         std::ldexp(scale, a.e), out, N, st.zhi);
     GLOBE_LAUNCHED(ctx, "k_dense_combine");
     return GLOBE_OK;
 }
 
-static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out) {
+static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out, const TcStat& st) {
     switch (nd) {
-        case 2: return dense_group<2>(ctx, Z, kg, scale, out);
-        case 3: return dense_group<3>(ctx, Z, kg, scale, out);
-        case 4: return dense_group<4>(ctx, Z, kg, scale, out);
-        case 5: return dense_group<5>(ctx, Z, kg, scale, out);
-        case 6: return dense_group<6>(ctx, Z, kg, scale, out);
-        case 7: return dense_group<7>(ctx, Z, kg, scale, out);
-        case 8: return dense_group<8>(ctx, Z, kg, scale, out);
-        case 9: return dense_group<9>(ctx, Z, kg, scale, out);
-        case ND64: return dense_group<ND64>(ctx, Z, kg, scale, out);
+        case 2: return dense_group<2>(ctx, Z, kg, scale, out, st);
+        case 3: return dense_group<3>(ctx, Z, kg, scale, out, st);
+        case 4: return dense_group<4>(ctx, Z, kg, scale, out, st);
+        case 5: return dense_group<5>(ctx, Z, kg, scale, out, st);
+        case 6: return dense_group<6>(ctx, Z, kg, scale, out, st);
+        case 7: return dense_group<7>(ctx, Z, kg, scale, out, st);
+        case 8: return dense_group<8>(ctx, Z, kg, scale, out, st);
+        case 9: return dense_group<9>(ctx, Z, kg, scale, out, st);
+        case ND64: return dense_group<ND64>(ctx, Z, kg, scale, out, st);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
 
 // out (N x k) = scale * A Z from the planes, nd digits per column
-static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out) {
+static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out, bool zhi_ready) {
+    TcStat st;
+    GLOBE_RET(tc_stat_fill(ctx, Z, ctx->coh.N, k, &zhi_ready, &st));
     const int gmax = 256 / nd;   // MMA width <= 256; near-equal groups
     const int ng = (k + gmax - 1) / gmax;
     for (int gi = 0, c0 = 0; gi < ng; ++gi) {
         const int kg = k / ng + (gi < k % ng ? 1 : 0);
-        GLOBE_RET(dense_group_nd(ctx, nd, Z + (size_t)c0 * ctx->coh.N, kg, scale, out + (size_t)c0 * ctx->coh.N));
+        GLOBE_RET(dense_group_nd(ctx, nd, Z + (size_t)c0 * ctx->coh.N, kg, scale, out + (size_t)c0 * ctx->coh.N,
+                                 st.from(c0)));
         c0 += kg;
     }
+    ctx->stat_dirty = false;
     return GLOBE_OK;
 }
 
-int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     GLOBE_RET(dense_digit_planes(ctx, 0));
     if (ctx->gen.adig[0].state != 1) return dense_apply_df(ctx, Z, k, scale, out);
-    return dense_apply_nd(ctx, ctx->digits, Z, k, scale, out);
+    return dense_apply_nd(ctx, ctx->digits, Z, k, scale, out, zhi_ready);
 }
 
 // The FP64 product, by its size N N k (FP64 pipe / planes, us a product):
@@ -578,12 +574,12 @@ int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double*
 #ifndef F64_DENSE_CALL_MIN
 #define F64_DENSE_CALL_MIN 4e6
 #endif
-int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& a = ctx->gen.adig[1];
     const int32_t N = ctx->coh.N;
     if (a.state >= 0 && (double)N * N * k >= (ctx->in_solve ? F64_DENSE_SOLVE_MIN : F64_DENSE_CALL_MIN)) {
         int rc = dense_digit_planes(ctx, 1);
-        if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, ND64, Z, k, scale, out);
+        if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, ND64, Z, k, scale, out, zhi_ready);
         if (a.state == 1 && rc != GLOBE_ERR_NOMEM) return rc;
         if (rc != GLOBE_OK && rc != GLOBE_ERR_NOMEM) return rc;
         if (rc == GLOBE_ERR_NOMEM) {   // give the planes back

@@ -353,211 +353,134 @@ __global__ void __launch_bounds__(Geo<NMMA>::NTHREADS, 1)
 
 
 
-// colinfo = {scale exponent e (as double), column sum} of one column from its nparts partials;
-// one warp (the lanes read the partials through L2, so a CTA that did not write them sees
-// them once their writers' fences are past)
-__device__ __forceinline__ void col_finish_warp(const double* __restrict__ pm, const double* __restrict__ ps,
-                                                int nparts, double* __restrict__ colinfo) {
-    const int lane = threadIdx.x & 31;
-    double mx = 0, sm = 0;
-    for (int j = lane; j < nparts; j += 32) {
-        mx = fmax(mx, __ldcg(pm + j));
-        sm += __ldcg(ps + j);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        sm += __shfl_xor_sync(0xffffffffu, sm, o);
-    }
-    if (lane == 0) {
-        // A column holding NaN or +-Inf has a non-finite sum (fmax drops NaN, the sum keeps it).
-        // It is marked by a NaN sum and a zero exponent: k_digits gives it zero digits, and every
-        // epilogue writes NaN for it (through the centring term, or explicitly), as FP64 would.
-        const bool bad = !isfinite(sm) || !isfinite(mx);
-        int E = 0;
-        if (!bad && mx > 0) frexp(mx, &E);
-        colinfo[0] = bad ? 0.0 : (double)(E - (DBITS - 1));  // |x 2^-e| < 16
-        colinfo[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : sm;
-    }
+__global__ void __launch_bounds__(256) k_col_max(const double* __restrict__ X, int64_t n, int64_t ld,
+                                                 unsigned* __restrict__ hi) {
+    const int c = blockIdx.y;
+    unsigned m = 0;
+    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
+        m = max(m, abs_hi(X[r + c * ld]));
+    cta_raise(m, hi + c);
 }
 
-// colinfo[c] = {scale exponent e_c (as double), column sum} from partials; one warp per column
-__global__ void k_col_finish(const double* __restrict__ pmax, const double* __restrict__ psum, int nparts, int k,
-                             double* __restrict__ colinfo) {
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (c >= k) return;
-    col_finish_warp(pmax + (size_t)c * nparts, psum + (size_t)c * nparts, nparts, colinfo + 2 * c);
-}
+// ---- epilogues -------------------------------------------------------------------
+//
+// Pass 1: u[s,c] = inv_s^2 (P1 - 2 f_s S_c), S_c the sum of the column from k_digits; raises
+// the high word of max |u| (pass 2's scale), and the column's last CTA sums the centring term
+// sum_s 2 f_s u over the CTAs' partials.  Pass 2: out[i,c] = scale (P2 - sum_s 2 f u).
+//
+// GLOBE_PREC_FP64 (ND64 = 12 digits, columns held to 2^-60 of their largest entry) carries in
+// double-double what the mixed form rounds around the integer products: the centring terms
+// cancel the uncentred products to a few hundredths or less, so they are subtracted before the
+// one rounding.  Its pass 1 works on z 2^-e (u stays at that scale, and e enters once, in the
+// last multiplication), so no column's magnitude leaves the range of a double on the way.
+// N = 20k, M = 20k, k = 5: 148 us a product, 14.5 ms on the FP64 pipe (k_geno_p1 / p2, which it
+// replaces from geno_apply_f64's sizes on).
+//
+// Both read 4 ND bytes a value and split and do 5 to 30 FP64 operations, of which an SM does two a
+// clock.  So a thread takes ~4 rows (combine_parts) and one sum leaves each CTA: with a fixed
+// 304 CTAs a column, 10k rows spent 28 us a launch on the sums of near-empty CTAs.
 
-// The same inside the kernel that wrote the partials: the last of the column's gridDim.x CTAs
-// to finish (a per-column arrival count, which that CTA resets for the next launch) forms
-// colinfo[c], in the same order as k_col_finish.  Every thread of the CTA calls it, after
-// thread 0 wrote the CTA's partials.
-__device__ __forceinline__ void col_finish_last(const double* __restrict__ pmax, const double* __restrict__ psum,
-                                                int c, unsigned* __restrict__ cnt, double* __restrict__ colinfo) {
+// sum over the CTAs of column c of part[c * nparts ..][NQ] into out[c * NQ ..], by the last of
+// them to arrive (cnt[c], reset); a double-double sum when NQ is 2.  Every thread calls it, thread
+// 0 with its CTA's values.
+template <int NQ>
+__device__ __forceinline__ void col_sum_last(const double (&v)[NQ], double* __restrict__ part, int c,
+                                             unsigned* __restrict__ cnt, double* __restrict__ out) {
     __shared__ bool last;
     const int nparts = (int)gridDim.x;
+    double* pc = part + (size_t)c * nparts * NQ;
     if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) pc[(size_t)blockIdx.x * NQ + q] = v[q];
         __threadfence();   // this CTA's partials, then its arrival
         last = atomicAdd(&cnt[c], 1u) == (unsigned)nparts - 1u;
     }
     __syncthreads();
-    if (last && threadIdx.x < 32) {
-        __threadfence();
-        col_finish_warp(pmax + (size_t)c * nparts, psum + (size_t)c * nparts, nparts, colinfo + 2 * c);
-        if (threadIdx.x == 0) cnt[c] = 0u;
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    double h = 0.0, l = 0.0;
+    for (int j = threadIdx.x; j < nparts; j += 32) {
+        if constexpr (NQ == 2) dd_add(h, l, __ldcg(pc + 2 * j), __ldcg(pc + 2 * j + 1));
+        else h += __ldcg(pc + j);
     }
-}
-
-// per-column max |x| and sum over n rows (partials per CTA); with colinfo, the last CTA of
-// each column also forms colinfo[c] (col_finish_last)
-__global__ void k_col_maxsum(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
-                             double* __restrict__ psum, unsigned* __restrict__ cnt, double* __restrict__ colinfo) {
-    __shared__ double smx[32], ssm[32];
-    const int c = blockIdx.y;
-    double mx = 0, sm = 0;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
-        const double v = X[r + c * ld];
-        mx = absmax_bits(mx, v);
-        sm += v;
-    }
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        sm += __shfl_xor_sync(0xffffffffu, sm, o);
+        const double a = __shfl_down_sync(0xffffffffu, h, o), b = __shfl_down_sync(0xffffffffu, l, o);
+        if constexpr (NQ == 2) dd_add(h, l, a, b);
+        else h += a;
     }
-    if ((threadIdx.x & 31) == 0) {
-        smx[threadIdx.x >> 5] = mx;
-        ssm[threadIdx.x >> 5] = sm;
-    }
-    __syncthreads();
     if (threadIdx.x == 0) {
-        double a = 0, b = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            a = fmax(a, smx[w]);
-            b += ssm[w];
-        }
-        pmax[blockIdx.x + (size_t)c * gridDim.x] = a;
-        psum[blockIdx.x + (size_t)c * gridDim.x] = b;
+        out[(size_t)c * NQ] = h;
+        if constexpr (NQ == 2) out[2 * c + 1] = l;
+        cnt[c] = 0u;
     }
-    if (colinfo) col_finish_last(pmax, psum, c, cnt, colinfo);
 }
 
-// pass-1 epilogue in FP64: u[s,c] = inv_s^2 (2^e_c sum_j 32^-j P1 - 2 f_s S_c); partial max|u|, sum 2 f u,
-// and from the column's last CTA colinfo2[c]
+// zhi[c], no longer needed, is cleared for the next product
 template <int ND>
-__global__ void k_combine1(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int64_t rows, int k,
-                           const double* __restrict__ colinfo, const double* __restrict__ f,
-                           const double* __restrict__ inv, double* __restrict__ U, double* __restrict__ pmax,
-                           double* __restrict__ psum, unsigned* __restrict__ cnt, double* __restrict__ colinfo2) {
-    __shared__ double smx[32], ssm[32];
+__global__ void __launch_bounds__(256) k_combine1(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                                  int64_t rows, const double* __restrict__ colinfo,
+                                                  const long long* __restrict__ isum, const double* __restrict__ f,
+                                                  const double* __restrict__ inv, double* __restrict__ U,
+                                                  double* __restrict__ psum, unsigned* __restrict__ cnt,
+                                                  unsigned* __restrict__ uhi, double* __restrict__ c2,
+                                                  unsigned* __restrict__ zhi) {
+    __shared__ double sm[256], sS2;
     const int c = blockIdx.y;
+    if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;
     double s_hi, s_lo;
     recombine_scales<ND>((int)colinfo[2 * c], s_hi, s_lo);
-    const double Sc = colinfo[2 * c + 1];
-    double mx = 0, sm = 0;
+    // 2 S_c, NaN for a bad column
+    if (threadIdx.x == 0)
+        sS2 = ((double)isum[2 * c] * 0x1p30 + (double)isum[2 * c + 1]) *
+                  pow2i((int)colinfo[2 * c] - DBITS * (ND64 - 1) + 1) + colinfo[2 * c + 1];
+    __syncthreads();
+    const double S2 = sS2;
+    unsigned mx = 0;
+    double acc[1] = {0.0};
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
         const double gv = recombine<ND>(part, nsplit, nmma, ldp, c, s, s_hi, s_lo);
         const double iv = inv[s], fs = f[s];
-        const double u = iv * iv * (gv - 2.0 * fs * Sc);
+        const double u = iv * iv * (gv - fs * S2);
         U[s + c * rows] = u;
-        mx = absmax_bits(mx, u);
-        sm += 2.0 * fs * u;
+        mx = max(mx, abs_hi(u));
+        acc[0] += fs * u;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        sm += __shfl_xor_sync(0xffffffffu, sm, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        smx[threadIdx.x >> 5] = mx;
-        ssm[threadIdx.x >> 5] = sm;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0, b = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            a = fmax(a, smx[w]);
-            b += ssm[w];
-        }
-        pmax[blockIdx.x + (size_t)c * gridDim.x] = a;
-        psum[blockIdx.x + (size_t)c * gridDim.x] = b;
-    }
-    col_finish_last(pmax, psum, c, cnt, colinfo2);   // u's digit scale and centring sum
+    cta_raise(mx, uhi + c);
+    acc[0] = 2.0 * cta_sum_256(acc[0], sm);
+    col_sum_last<1>(acc, psum, c, cnt, c2);
 }
 
-// pass-2 epilogue: out[i,c] = scale (2^e_c sum_j 32^-j P2 - C2_c)
 template <int ND>
-__global__ void k_combine2(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int64_t rows, int k,
-                           const double* __restrict__ colinfo, double scale, double* __restrict__ out, int64_t ldo) {
+__global__ void __launch_bounds__(256) k_combine2(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                                  int64_t rows, const double* __restrict__ colinfo,
+                                                  const double* __restrict__ c2, double scale, double* __restrict__ out,
+                                                  int64_t ldo, unsigned* __restrict__ uhi) {
     const int c = blockIdx.y;
+    if (blockIdx.x == 0 && threadIdx.x == 0) uhi[c] = 0u;
     double s_hi, s_lo;
     recombine_scales<ND>((int)colinfo[2 * c], s_hi, s_lo);
-    const double C2 = colinfo[2 * c + 1];
+    const double C2 = c2[c] + colinfo[2 * c + 1];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
         out[i + c * ldo] = scale * (recombine<ND, 4>(part, nsplit, nmma, ldp, c, i, s_hi, s_lo) - C2);
     }
 }
 
-// ---- the FP64 product's statistics and epilogues ------------------------------
-//
-// GLOBE_PREC_FP64 runs the same two passes with ND64 = 12 digits (columns held to 2^-60 of
-// their largest entry).  What the mixed form rounds around the integer products is carried in
-// double-double here: the centring terms 2 f S and sum 2 f u cancel the uncentred products to
-// a few hundredths or less (S is the exact integer column sum of the digits, isum), so they
-// are subtracted before the one rounding.  Pass 1 works on z 2^-e (u stays at that scale, and
-// e enters once, in the last multiplication), so no column's magnitude leaves the range of a
-// double on the way.  The epilogues read 4 bytes x ND64 x splits per value and are bound by
-// those loads.  N = 20k, M = 20k, k = 5: 148 us a product, 14.5 ms on the FP64 pipe
-// (k_geno_p1 / p2, which it replaces from geno_apply_f64's sizes on).
-
-// max |x| of each column; the column's last CTA forms colinfo[c] and clears isum for k_digits
-__global__ void k_col_max64(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
-                            unsigned* __restrict__ cnt, double* __restrict__ colinfo,
-                            unsigned long long* __restrict__ isum) {
-    __shared__ double smx[8];
-    __shared__ bool last;
-    const int c = blockIdx.y, nparts = (int)gridDim.x;
-    double mx = 0;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-        mx = absmax_bits(mx, X[r + c * ld]);
-    mx = warp_max_bits(mx);
-    if ((threadIdx.x & 31) == 0) smx[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = absmax_bits(mx, smx[w]);
-        pmax[blockIdx.x + (size_t)c * nparts] = mx;
-        __threadfence();
-        last = atomicAdd(&cnt[c], 1u) == (unsigned)nparts - 1u;
-    }
-    __syncthreads();
-    if (last && threadIdx.x < 32) {
-        __threadfence();
-        mx = 0;
-        for (int j = threadIdx.x; j < nparts; j += 32) mx = absmax_bits(mx, __ldcg(pmax + j + (size_t)c * nparts));
-        mx = warp_max_bits(mx);
-        if (threadIdx.x == 0) {
-            col_info64(mx, colinfo + 2 * c);
-            isum[2 * c] = isum[2 * c + 1] = 0ull;
-            cnt[c] = 0u;
-        }
-    }
-}
-
-// pass-1 epilogue: u = inv^2 (P1 - 2 f S) at the scale 2^-e of column c; per CTA max |u| and
-// sum 2 f u (double-double), and from the column's last CTA colinfo2[c] and the centring term
-// c2[2c], c2[2c+1]
 __global__ void __launch_bounds__(256) k_combine1_64(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
                                                      int64_t rows, const double* __restrict__ colinfo,
                                                      const long long* __restrict__ isum, const double* __restrict__ f,
                                                      const double* __restrict__ inv, double* __restrict__ U,
-                                                     double* __restrict__ pmax, double* __restrict__ psum,
-                                                     unsigned* __restrict__ cnt, double* __restrict__ colinfo2,
-                                                     double* __restrict__ c2) {
-    __shared__ double smx[8], ssh[8], ssl[8];
-    __shared__ bool last;
-    const int c = blockIdx.y, nparts = (int)gridDim.x;
+                                                     double* __restrict__ psum, unsigned* __restrict__ cnt,
+                                                     unsigned* __restrict__ uhi, double* __restrict__ c2,
+                                                     unsigned* __restrict__ zhi) {
+    __shared__ double smh[256], sml[256];
+    const int c = blockIdx.y, tid = threadIdx.x;
+    if (blockIdx.x == 0 && tid == 0) zhi[c] = 0u;
     const double bad = colinfo[2 * c + 1];   // 0, or NaN
     const double Sh = ll_times_pow2(isum[2 * c], 0x1p-25), Sl = ll_times_pow2(isum[2 * c + 1], 0x1p-55);
-    double mx = 0, sh = 0, sl = 0;
-    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
+    unsigned mx = 0;
+    double sum[2] = {0.0, 0.0};
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + tid; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
         long long hi, lo;
         recombine_int<ND64>(part, nsplit, nmma, ldp, c, s, hi, lo);
         const double f2 = 2.0 * f[s], iv = inv[s];
@@ -566,68 +489,38 @@ __global__ void __launch_bounds__(256) k_combine1_64(const float* __restrict__ p
         dd_add(d, r, -p, __dsub_rn(ll_times_pow2(lo, 0x1p-55), __fma_rn(f2, Sl, pe)));
         const double u = iv * iv * (d + r) + bad;
         U[s + c * rows] = u;
-        mx = absmax_bits(mx, u);
+        mx = max(mx, abs_hi(u));
         const double t = __dmul_rn(f2, u);
-        dd_add(sh, sl, t, __fma_rn(f2, u, -t));
+        dd_add(sum[0], sum[1], t, __fma_rn(f2, u, -t));
     }
-    mx = warp_max_bits(mx);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double a = __shfl_xor_sync(0xffffffffu, sh, o), b = __shfl_xor_sync(0xffffffffu, sl, o);
-        dd_add(sh, sl, a, b);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        const int w = threadIdx.x >> 5;
-        smx[w] = mx;
-        ssh[w] = sh;
-        ssl[w] = sl;
-    }
+    cta_raise(mx, uhi + c);
+    // the CTA's double-double sum, as cta_sum_256
+    smh[tid] = sum[0];
+    sml[tid] = sum[1];
     __syncthreads();
-    const size_t o0 = (size_t)c * nparts;
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-            mx = absmax_bits(mx, smx[w]);
-            dd_add(sh, sl, ssh[w], ssl[w]);
+    for (int s = 128; s > 0; s >>= 1) {
+        if (tid < s) {
+            dd_add(sum[0], sum[1], smh[tid + s], sml[tid + s]);
+            smh[tid] = sum[0];
+            sml[tid] = sum[1];
         }
-        pmax[o0 + blockIdx.x] = mx;
-        psum[2 * (o0 + blockIdx.x)] = sh;
-        psum[2 * (o0 + blockIdx.x) + 1] = sl;
-        __threadfence();
-        last = atomicAdd(&cnt[c], 1u) == (unsigned)nparts - 1u;
+        __syncthreads();
     }
-    __syncthreads();
-    if (last && threadIdx.x < 32) {
-        __threadfence();
-        mx = sh = sl = 0;
-        for (int j = threadIdx.x; j < nparts; j += 32) {
-            mx = absmax_bits(mx, __ldcg(pmax + o0 + j));
-            dd_add(sh, sl, __ldcg(psum + 2 * (o0 + j)), __ldcg(psum + 2 * (o0 + j) + 1));
-        }
-        mx = warp_max_bits(mx);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const double a = __shfl_xor_sync(0xffffffffu, sh, o), b = __shfl_xor_sync(0xffffffffu, sl, o);
-            dd_add(sh, sl, a, b);
-        }
-        if (threadIdx.x == 0) {
-            col_info64(mx, colinfo2 + 2 * c);
-            c2[2 * c] = sh;
-            c2[2 * c + 1] = sl;
-            cnt[c] = 0u;
-        }
-    }
+    col_sum_last<2>(sum, psum, c, cnt, c2);
 }
 
-// pass-2 epilogue: out[i,c] = scale 2^e (P2 - sum 2 f u), 2^e in two factors
+// 2^e in two factors
 __global__ void __launch_bounds__(256) k_combine2_64(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
                                                      int64_t rows, const double* __restrict__ colinfo1,
                                                      const double* __restrict__ colinfo2, const double* __restrict__ c2,
-                                                     double scale, double* __restrict__ out, int64_t ldo) {
+                                                     double scale, double* __restrict__ out, int64_t ldo,
+                                                     unsigned* __restrict__ uhi) {
     const int c = blockIdx.y;
+    if (blockIdx.x == 0 && threadIdx.x == 0) uhi[c] = 0u;
     double s_hi, s_lo;
     recombine_scales<ND64>((int)colinfo2[2 * c], s_hi, s_lo);
     const int e = (int)colinfo1[2 * c];
-    const double ea = ldexp(1.0, e / 2), eb = ldexp(1.0, e - e / 2);
+    const double ea = pow2i(e / 2), eb = pow2i(e - e / 2);
     const double Ch = c2[2 * c], Cl = c2[2 * c + 1], bad = colinfo2[2 * c + 1];
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
         long long hi, lo;
@@ -939,9 +832,9 @@ static int tune_splits(globe_ctx* ctx, int pass, int nmma, const uint8_t* blk, i
 }
 
 // out (N x k) = scale * Zs'(Zs Z) for one group of <= 256 / ND columns, ND digits per column
-// (ND64: the FP64 product, with its own statistics and epilogues)
+// (ND64: the FP64 product, with its own epilogues); st: the statistics words of its columns
 template <int ND>
-static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out) {
+static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
     const int nmma = ((kg * ND + 15) / 16) * 16;
@@ -963,7 +856,7 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     const int64_t ldp1 = (int64_t)tiles1 * rpc, ldp2 = (int64_t)tiles2 * rpc;
     uint8_t *D1, *D2;
     float *P1, *P2;
-    double *U, *cst, *pm, *ps;
+    double *U, *cst;
     unsigned* err;
     GLOBE_RET(ws(ctx, WS_TC_D1, (size_t)nmma * kpad1, &D1));
     GLOBE_RET(ws(ctx, WS_TC_D2, (size_t)nmma * kpad2, &D2));
@@ -971,31 +864,24 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     GLOBE_RET(ws(ctx, WS_TC_P2, (size_t)(spmax2 + 1) * nmma * ldp2, &P2));
     GLOBE_RET(ws(ctx, WS_TC_U, (size_t)g.Mk * kg + 1, &U));
     constexpr bool F64 = ND == ND64;
-    const int nbr = 304;
-    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(8 * kg + 3 * nbr * kg + 8), &cst));
-    double* col1 = cst;           // 2*kg
-    double* col2 = cst + 2 * kg;  // 2*kg
-    double* c2 = cst + 4 * kg;    // 2*kg, F64: sum 2 f u in double-double
-    unsigned long long* isum = reinterpret_cast<unsigned long long*>(cst + 6 * kg);   // 2*kg, F64: column sums of digits
-    pm = cst + 8 * kg;
-    ps = pm + (size_t)nbr * kg;   // nbr*kg (F64: twice that)
+    GLOBE_RET(ws(ctx, WS_TC_SCAL, (size_t)(6 + 2 * COMBINE_PARTS) * kg, &cst));
+    double* col1 = cst;           // 2*kg: {e, 0 or NaN} of Z's columns
+    double* col2 = cst + 2 * kg;  // 2*kg: of u's
+    double* c2 = cst + 4 * kg;    // kg (F64: 2*kg, double-double): sum 2 f u
+    double* ps = cst + 6 * kg;    // its partials
     GLOBE_RET(tc_err_word(ctx, &err));
     CUtensorMap mB1, mB2;
     GLOBE_RET(make_map(ctx, &mB1, D1, (uint64_t)kpad1, (uint64_t)nmma, BK, (uint32_t)nmma, true));
     GLOBE_RET(make_map(ctx, &mB2, D2, (uint64_t)kpad2, (uint64_t)nmma, BK, (uint32_t)nmma, true));
     // ---- digits of Z
-    const int nz = col_parts(N);
     unsigned* cnt;
-    GLOBE_RET(tc_counters(ctx, 2 * kg, &cnt));
-    if constexpr (F64) k_col_max64<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, cnt, col1, isum);
-    else k_col_maxsum<<<dim3(nz, kg), 256, 0, ctx->stream>>>(Z, N, N, pm, ps, cnt, col1);
-    GLOBE_LAUNCHED(ctx, "k_col_maxsum");
+    GLOBE_RET(tc_counters(ctx, kg, &cnt));
     // digit rows past the kg columns stay zero
     if (nmma > kg * ND)
         GLOBE_CK(ctx, cudaMemsetAsync(D1 + (size_t)kg * ND * kpad1, 0, (size_t)(nmma - kg * ND) * kpad1,
                                       ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad1 / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, kg, col1, D1, kpad1, F64 ? isum : nullptr);
+        Z, N, N, st.zhi, col1, D1, kpad1, st.isum, nullptr);
     GLOBE_LAUNCHED(ctx, "k_digits");
     // ---- pass 1
     int sp1 = 0;
@@ -1008,20 +894,17 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
         GLOBE_RET(gemm_dispatch(ctx, nmma, g.blk1, g.ntiles1, mB1, (int)g.Mk, nch1, sp1, P1, ldp1, err, zg));
     }
     const int sp1e = eff_splits(nch1, sp1);
-    if constexpr (F64)
-        k_combine1_64<<<dim3(std::min(nbr, div_up(g.Mk, 256)), kg), 256, 0, ctx->stream>>>(
-            P1, sp1e, nmma, ldp1, g.Mk, col1, reinterpret_cast<const long long*>(isum), g.f, g.inv, U, pm, ps, cnt + kg,
-            col2, c2);
-    else
-        k_combine1<ND><<<dim3(nbr, kg), 256, 0, ctx->stream>>>(P1, sp1e, nmma, ldp1, g.Mk, kg, col1, g.f, g.inv, U, pm,
-                                                               ps, cnt + kg, col2);
+    const auto combine1 = [] { if constexpr (F64) return k_combine1_64; else return k_combine1<ND>; }();
+    combine1<<<dim3(combine_parts(g.Mk), kg), 256, 0, ctx->stream>>>(
+        P1, sp1e, nmma, ldp1, g.Mk, col1, reinterpret_cast<const long long*>(st.isum), g.f, g.inv, U, ps, cnt, st.uhi, c2,
+        st.zhi);
     GLOBE_LAUNCHED(ctx, "k_combine1");
     // ---- digits of u, pass 2
     if (nmma > kg * ND)
         GLOBE_CK(ctx, cudaMemsetAsync(D2 + (size_t)kg * ND * kpad2, 0, (size_t)(nmma - kg * ND) * kpad2,
                                       ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad2 / 4, 256), 2048), kg), 256, 0, ctx->stream>>>(
-        U, g.Mk, g.Mk, kg, col2, D2, kpad2, nullptr);
+        U, g.Mk, g.Mk, st.uhi, col2, D2, kpad2, nullptr, st.isum);
     GLOBE_LAUNCHED(ctx, "k_digits");
     int sp2 = 0;
     GLOBE_RET(tune_splits(ctx, 2, nmma, g.blk2, g.ntiles2, mB2, N, nch2, cand2, P2, ldp2, err, &sp2));
@@ -1032,30 +915,30 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     const int sp2e = eff_splits(nch2, sp2);
     const dim3 g2((unsigned)std::min(div_up(N, 256), 1024), kg);
     if constexpr (F64)
-        k_combine2_64<<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, col1, col2, c2, scale, out, N);
+        k_combine2_64<<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, col1, col2, c2, scale, out, N, st.uhi);
     else
-        k_combine2<ND><<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, kg, col2, scale, out, N);
+        k_combine2<ND><<<g2, 256, 0, ctx->stream>>>(P2, sp2e, nmma, ldp2, N, col2, c2, scale, out, N, st.uhi);
     GLOBE_LAUNCHED(ctx, "k_combine2");
     return GLOBE_OK;
 }
 
-static int tc_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out) {
+static int tc_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out, const TcStat& st) {
     switch (nd) {
-        case 2: return tc_group<2>(ctx, Z, kg, scale, out);
-        case 3: return tc_group<3>(ctx, Z, kg, scale, out);
-        case 4: return tc_group<4>(ctx, Z, kg, scale, out);
-        case 5: return tc_group<5>(ctx, Z, kg, scale, out);
-        case 6: return tc_group<6>(ctx, Z, kg, scale, out);
-        case 7: return tc_group<7>(ctx, Z, kg, scale, out);
-        case 8: return tc_group<8>(ctx, Z, kg, scale, out);
-        case 9: return tc_group<9>(ctx, Z, kg, scale, out);
-        case ND64: return tc_group<ND64>(ctx, Z, kg, scale, out);
+        case 2: return tc_group<2>(ctx, Z, kg, scale, out, st);
+        case 3: return tc_group<3>(ctx, Z, kg, scale, out, st);
+        case 4: return tc_group<4>(ctx, Z, kg, scale, out, st);
+        case 5: return tc_group<5>(ctx, Z, kg, scale, out, st);
+        case 6: return tc_group<6>(ctx, Z, kg, scale, out, st);
+        case 7: return tc_group<7>(ctx, Z, kg, scale, out, st);
+        case 8: return tc_group<8>(ctx, Z, kg, scale, out, st);
+        case 9: return tc_group<9>(ctx, Z, kg, scale, out, st);
+        case ND64: return tc_group<ND64>(ctx, Z, kg, scale, out, st);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
 
 // out (N x k) = scale * Zs'(Zs Z) with nd digits per column
-static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out) {
+static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
     if (g.Mk == 0) {
@@ -1070,12 +953,15 @@ static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double 
     const int gmax = 256 / nd, gtwo = 192 / nd;
     int ng = (k + gmax - 1) / gmax;
     if (ng > 1) ng = (k + gtwo - 1) / gtwo;
+    TcStat st;
     auto run = [&](int ngroups) -> int {
+        GLOBE_RET(tc_stat_fill(ctx, Z, N, k, &zhi_ready, &st));
         for (int gi = 0, c0 = 0; gi < ngroups; ++gi) {
             const int kg = k / ngroups + (gi < k % ngroups ? 1 : 0);
-            GLOBE_RET(tc_group_nd(ctx, nd, Z + (size_t)c0 * N, kg, scale, out + (size_t)c0 * N));
+            GLOBE_RET(tc_group_nd(ctx, nd, Z + (size_t)c0 * N, kg, scale, out + (size_t)c0 * N, st.from(c0)));
             c0 += kg;
         }
+        ctx->stat_dirty = false;   // every word was cleared on the way
         return GLOBE_OK;
     };
     // Column grouping: the rule above, or -- for 9 or more columns, on first use of (k, digits,
@@ -1103,8 +989,8 @@ static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double 
     return run(cand[best]);
 }
 
-int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
-    return geno_apply_nd(ctx, ctx->digits, Z, k, scale, out);
+int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
+    return geno_apply_nd(ctx, ctx->digits, Z, k, scale, out, zhi_ready);
 }
 
 // The FP64 product.  On the tensor cores (ND64 digits) it needs the individual-major copy and
@@ -1126,7 +1012,7 @@ int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* 
 #ifndef F64_CALL_MIN
 #define F64_CALL_MIN 4e7
 #endif
-int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
+int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
     const double size = (double)N * (double)g.Mk * k;
@@ -1140,7 +1026,7 @@ int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double*
             if (need > (double)fr) g.f64_tc = -1;
         }
         if (g.f64_tc >= 0) {
-            const int rc = geno_apply_nd(ctx, ND64, Z, k, scale, out);
+            const int rc = geno_apply_nd(ctx, ND64, Z, k, scale, out, zhi_ready);
             if (rc != GLOBE_ERR_NOMEM) {
                 if (rc == GLOBE_OK) g.f64_tc = 1;
                 return rc;
@@ -1162,7 +1048,35 @@ int tc_err_word(globe_ctx* ctx, unsigned** err) {
     return GLOBE_OK;
 }
 
-// per-column arrival counts of col_finish_last, zero between launches: (re)created zeroed when
+// The statistics words of k columns (WS_TC_STAT): created zeroed, and cleared by the products that
+// use them; where one stopped half way, cleared here before the next.
+int tc_stat(globe_ctx* ctx, int k, TcStat* st) {
+    const size_t bytes = (size_t)k * (2 * sizeof(unsigned) + 2 * sizeof(unsigned long long));
+    const bool fresh = ctx->ws[WS_TC_STAT].bytes < bytes;
+    unsigned char* p;
+    GLOBE_RET(ws(ctx, WS_TC_STAT, bytes, &p));
+    const int cap = (int)(ctx->ws[WS_TC_STAT].bytes / 24);   // the words' places depend on the slot only
+    if (fresh || ctx->stat_dirty) GLOBE_CK(ctx, cudaMemsetAsync(p, 0, ctx->ws[WS_TC_STAT].bytes, ctx->stream));
+    ctx->stat_dirty = false;
+    st->isum = reinterpret_cast<unsigned long long*>(p);
+    st->zhi = reinterpret_cast<unsigned*>(st->isum + 2 * (size_t)cap);
+    st->uhi = st->zhi + cap;
+    return GLOBE_OK;
+}
+
+int tc_stat_fill(globe_ctx* ctx, const double* Z, int64_t n, int k, bool* ready, TcStat* st) {
+    if (*ready) ctx->stat_dirty = false;   // zhi was filled by the caller's kernel: keep it
+    GLOBE_RET(tc_stat(ctx, k, st));
+    ctx->stat_dirty = true;
+    if (!*ready) {
+        k_col_max<<<dim3(col_parts(n), k), 256, 0, ctx->stream>>>(Z, n, n, st->zhi);
+        GLOBE_LAUNCHED(ctx, "k_col_max");
+    }
+    *ready = false;   // the product consumes it
+    return GLOBE_OK;
+}
+
+// per-column arrival counts of the kernels' last CTAs, zero between launches: (re)created zeroed when
 // more are needed (never inside a capture, where allocation is refused; every shape's first
 // product runs outside one)
 int tc_counters(globe_ctx* ctx, size_t n, unsigned** cnt) {

@@ -19,16 +19,16 @@ int check_ready(globe_ctx* ctx) {
     return GLOBE_OK;
 }
 
-int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out) {
+int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out, bool zhi_ready) {
     ProfScope ps(ctx, GLOBE_PROF_GRM);
+    const bool mixed = ctx->prec == GLOBE_PREC_MIXED;
     if (ctx->gen.src == GSRC_GENO) {
         const double scale = ctx->vc[1] * (ctx->gen.Mk > 0 ? 1.0 / (double)ctx->gen.Mk : 0.0);
-        if (ctx->prec == GLOBE_PREC_MIXED) return geno_apply_tc(ctx, Z, k, scale, out);
-        return geno_apply_f64(ctx, Z, k, scale, out);
+        return mixed ? geno_apply_tc(ctx, Z, k, scale, out, zhi_ready) : geno_apply_f64(ctx, Z, k, scale, out, zhi_ready);
     }
     if (ctx->gen.src == GSRC_DENSE)
-        return ctx->prec == GLOBE_PREC_MIXED ? dense_apply_tc(ctx, Z, k, ctx->vc[1], out)
-                                             : dense_apply_f64(ctx, Z, k, ctx->vc[1], out);
+        return mixed ? dense_apply_tc(ctx, Z, k, ctx->vc[1], out, zhi_ready)
+                     : dense_apply_f64(ctx, Z, k, ctx->vc[1], out, zhi_ready);
     return set_err(ctx, GLOBE_ERR_STATE, "no genetic relationship source loaded");
 }
 

@@ -102,11 +102,9 @@ __device__ __forceinline__ double ll_times_pow2(long long v, double s) {
                                             mant));
 }
 
-// max(m, |v|) for m >= 0 by comparing bits (non-negative doubles order as integers; a NaN v
-// wins, where fmax would drop it -- the column sums carry NaN either way)
-__device__ __forceinline__ double absmax_bits(double m, double v) {
-    const long long a = __double_as_longlong(m), b = __double_as_longlong(v) & 0x7fffffffffffffffll;
-    return __longlong_as_double(a > b ? a : b);
+// 2^e, from its bits where it is a normal double (ldexp runs on the FP64 pipe)
+__device__ __forceinline__ double pow2i(int e) {
+    return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52) : ldexp(1.0, e);
 }
 
 // 2^e sum_j 32^-j P_j of one row of a genotype product, ND digits per column (rows c*ND + j
@@ -166,52 +164,82 @@ __device__ __forceinline__ double recombine(const float* __restrict__ part, int 
 // scale factors of recombine<ND> for exponent e: 2^(e - 5 (ND_HI - 1)) and 2^(e - 5 (ND - 1))
 template <int ND>
 __device__ __forceinline__ void recombine_scales(int e, double& s_hi, double& s_lo) {
-    s_hi = ldexp(1.0, e - DBITS * ((ND + 1) / 2 - 1));
-    s_lo = ldexp(1.0, e - DBITS * (ND - 1));
+    s_hi = pow2i(e - DBITS * ((ND + 1) / 2 - 1));
+    s_lo = pow2i(e - DBITS * (ND - 1));
 }
 
-// CTAs per column of k_col_maxsum for n rows: ~8 values per thread (its FP64 reduction runs
-// on GB300's small FP64 pipe, so surplus CTAs cost more than they hide), at most 304
+// ---- column statistics of a product's inputs ----------------------------------
+//
+// A column x is scaled by the power of two 2^-e with |x 2^-e| < 16.  All that e needs is the
+// largest high word of |x| (sign dropped): its exponent field, or 0x7ff where a NaN or an
+// infinity occurs, which marks the column as bad.  One 32-bit word per column, raised by
+// integer maxima (GB300's FP64 pipe does two operations a clock and SM, so the FP64 maxima and
+// sums of every element that stood here cost more than the data's reads): zeroed between
+// products, filled by k_col_max or by the kernel that writes the column.
+__device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+__device__ __forceinline__ bool col_bad(unsigned hi) { return hi >= 0x7ff00000u; }
+// the exponent e; a zero or subnormal column takes the smallest (ND64, whose 59 bits then reach
+// below the last bit of a double), or the smallest whose scale 2^(5 (ND - 1) - e) is finite
+template <int ND>
+__device__ __forceinline__ int col_exp(unsigned hi) {
+    const int e = (int)(hi >> 20) - 1022 - (DBITS - 1);
+    return col_bad(hi) ? 0 : (ND == ND64 ? e : max(e, -983));
+}
+
+// CTAs per column of k_col_max and the rows each thread of a combine kernel takes: ~8 and ~4
+// values per thread
 __host__ __forceinline__ int col_parts(int64_t n) {
     const int64_t p = (n + 2047) / 2048;
     return (int)(p < 1 ? 1 : (p > 304 ? 304 : p));
 }
-
-// ---- the FP64 products (ND64 digits) ----
-__device__ __forceinline__ double warp_max_bits(double m) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = absmax_bits(m, __shfl_xor_sync(0xffffffffu, m, o));
-    return m;
+constexpr int COMBINE_PARTS = 304;   // CTAs per column of a combine kernel at most (2 per SM)
+__host__ __forceinline__ int combine_parts(int64_t n) {
+    const int64_t p = (n + 1023) / 1024;
+    return (int)(p < 1 ? 1 : (p > COMBINE_PARTS ? COMBINE_PARTS : p));
 }
+
+// sum of v over a CTA of 256 threads, in one order (sm: 256 doubles), valid in thread 0: halves
+// through shared memory, since an FP64 addition costs the same for one lane as for 32
+__device__ __forceinline__ double cta_sum_256(double v, double* sm) {
+    const int t = threadIdx.x;
+    sm[t] = v;
+    __syncthreads();
+#pragma unroll
+    for (int s = 128; s >= 32; s >>= 1) {
+        if (t < s) {
+            v += sm[t + s];
+            sm[t] = v;
+        }
+        __syncthreads();
+    }
+    if (t < 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    }
+    return v;
+}
+// max of m over the CTA, raised in *out
+__device__ __forceinline__ void cta_raise(unsigned m, unsigned* out) {
+    __shared__ unsigned sm[32];
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        m = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0u;
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (threadIdx.x == 0 && m) atomicMax(out, m);
+    }
+}
+
 // (h, l) += (a, b): two-sum of the high parts, everything else into l
 __device__ __forceinline__ void dd_add(double& h, double& l, double a, double b) {
     const double s = __dadd_rn(h, a), bp = __dsub_rn(s, h);
     l = __dadd_rn(l, __dadd_rn(b, __dadd_rn(__dsub_rn(h, __dsub_rn(s, bp)), __dsub_rn(a, bp))));
     h = s;
 }
-// colinfo = {scale exponent, 0 or NaN} from max |x| (its bits: NaN and infinity win)
-__device__ __forceinline__ void col_info64(double mx, double* __restrict__ colinfo) {
-    const bool bad = !isfinite(mx);
-    int E = 0;
-    if (!bad && mx > 0) frexp(mx, &E);
-    colinfo[0] = bad ? 0.0 : (double)(E - (DBITS - 1));
-    colinfo[1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
-}
 
-// max |x| of each column; the column's last CTA forms colinfo[c] and clears isum[2c], isum[2c+1]
-// for k_digits (k_tc_geno.cu)
-__global__ void k_col_max64(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
-                            unsigned* __restrict__ cnt, double* __restrict__ colinfo,
-                            unsigned long long* __restrict__ isum);
-
-// per-column max |x| and sum over n rows (partials per CTA); colinfo[c] = {exponent e with
-// max |x 2^-e| < 16, column sum} from those partials, or {0, NaN} for a column holding a
-// NaN or an infinity (k_tc_geno.cu).  k_col_maxsum forms colinfo itself when given it and
-// zeroed per-column counts cnt (tc_counters), in its last CTA per column; else k_col_finish.
-__global__ void k_col_maxsum(const double* __restrict__ X, int64_t n, int64_t ld, double* __restrict__ pmax,
-                             double* __restrict__ psum, unsigned* __restrict__ cnt, double* __restrict__ colinfo);
-__global__ void k_col_finish(const double* __restrict__ pmax, const double* __restrict__ psum, int nparts, int k,
-                             double* __restrict__ colinfo);
+// hi[c] raised to the largest abs_hi of column c (n rows)
+__global__ void k_col_max(const double* __restrict__ X, int64_t n, int64_t ld, unsigned* __restrict__ hi);
 
 // ND digits of X (n x k, FP64) into D[(c*ND + j) * kpad + pos(r)]  (e4m3); every position
 // in [0, kpad) of the column's digit rows is written (rows >= n give digit 0).  One thread
@@ -223,17 +251,27 @@ __global__ void k_col_finish(const double* __restrict__ pmax, const double* __re
 // balanced base-32 digits are peeled off from the least significant end in integer
 // arithmetic (d = ((I + 16) mod 32) - 16, in [-16, 15]); the leading digit is what
 // remains, in [-16, 16].  sum_j d_j 32^-j equals x 2^-e rounded to 5 (ND-1) fraction bits.
-// With ND64 digits (the FP64 products) the scaling takes two factors where one would leave the
-// range of a double, and with isum the exact column sum of I is added to isum[2c] 2^30 +
-// isum[2c+1] (integer atomics: the same bits in any order).
+// The scale comes from the column's high word hi[c]; CTA 0 of each column leaves {e, 0 or NaN} in
+// colinfo for the epilogues.  With isum the column sum of x, each x rounded to ND64 digits whatever
+// ND, is added to isum[2c] 2^30 + isum[2c+1] in units of 2^(e - 55) (integer atomics: the same
+// bits in any order); clear[2c], clear[2c+1] are set to zero
+// (an isum no longer in use).  With ND64 digits (the FP64 products) the scaling takes two factors
+// where one would leave the range of a double.
 template <int ND, bool GENO>
-__global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, int k, const double* __restrict__ colinfo,
-                         uint8_t* __restrict__ D, int64_t kpad, unsigned long long* __restrict__ isum = nullptr) {
+__global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, const unsigned* __restrict__ hi,
+                         double* __restrict__ colinfo, uint8_t* __restrict__ D, int64_t kpad,
+                         unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear) {
     const int c = blockIdx.y;
-    const int sh = DBITS * (ND - 1) - (int)colinfo[2 * c];
-    const double sc = ldexp(1.0, ND == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
-    const double sc2 = ND == ND64 ? ldexp(1.0, sh - min(sh, 1000)) : 1.0;
-    const bool bad = isnan(colinfo[2 * c + 1]);   // non-finite column (k_col_finish): zero digits
+    const unsigned h = hi[c];
+    const int e = col_exp<ND>(h), sh = DBITS * (ND - 1) - e;
+    const double sc = pow2i(ND == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
+    const double sc2 = ND == ND64 ? pow2i(sh - min(sh, 1000)) : 1.0;
+    const bool bad = col_bad(h);   // non-finite column: zero digits
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        colinfo[2 * c] = (double)e;
+        colinfo[2 * c + 1] = bad ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+        if (clear) clear[2 * c] = clear[2 * c + 1] = 0ull;
+    }
     const int64_t nw = kpad >> 2;
     long long sum_hi = 0, sum_lo = 0;
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
@@ -248,9 +286,10 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, in
             double x = (src < n && !bad) ? X[src + c * ld] * sc : 0.0;
             if (ND == ND64) x *= sc2;
             I[q] = __double2ll_rn(x);
-            if (ND == ND64) {
-                sum_hi += I[q] >> 30;
-                sum_lo += I[q] & ((1ll << 30) - 1);
+            if (isum) {
+                const long long J = ND == ND64 ? I[q] : __double2ll_rn(x * pow2i(DBITS * (ND64 - ND)));
+                sum_hi += J >> 30;
+                sum_lo += J & ((1ll << 30) - 1);
             }
         }
         uint32_t word[ND];
@@ -269,7 +308,7 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, in
 #pragma unroll
         for (int j = 0; j < ND; ++j) *reinterpret_cast<uint32_t*>(D + ((int64_t)c * ND + j) * kpad + P) = word[j];
     }
-    if (ND == ND64 && isum) {
+    if (isum) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             sum_hi += __shfl_xor_sync(0xffffffffu, sum_hi, o);
@@ -294,6 +333,18 @@ struct ZGrid {
     int skip0 = 0, skipz = 0;
     int stall = 0;   // test hook (globe_debug_stall_next_gemm): leave the first digit stage unloaded
 };
+
+// Words of the columns' statistics (tc_common.cuh's top): zhi and uhi, the high words of Z's and
+// u's columns, and isum, the sums of Z's.  Zero between products.
+struct TcStat {
+    unsigned long long* isum = nullptr;
+    unsigned *zhi = nullptr, *uhi = nullptr;
+    TcStat from(int c) const { return TcStat{isum + 2 * (size_t)c, zhi + c, uhi + c}; }
+};
+int tc_stat(globe_ctx* ctx, int k, TcStat* st);
+// the words of Z's k columns (n rows), zhi filled unless *ready (then *ready is reset: the product
+// that follows consumes it)
+int tc_stat_fill(globe_ctx* ctx, const double* Z, int64_t n, int k, bool* ready, TcStat* st);
 
 int make_map(globe_ctx* ctx, CUtensorMap* m, const void* base, uint64_t inner, uint64_t outer, uint32_t box_in,
              uint32_t box_out, bool sw128);
