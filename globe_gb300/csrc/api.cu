@@ -126,7 +126,7 @@ void prof_end(globe_ctx* ctx, int h) {
 static void free_cohort(globe_ctx* ctx) {
     auto& c = ctx->coh;
     for (void* p : {(void*)c.X, (void*)c.y, (void*)c.bstart, (void*)c.bind, (void*)c.rind, (void*)c.bn,
-                    (void*)c.bt, (void*)c.btt, (void*)c.lblk, (void*)c.tdf})
+                    (void*)c.bt, (void*)c.btt, (void*)c.lblk, (void*)c.order, (void*)c.tdf})
         dfree(ctx, p);
     c = Cohort();
     for (void* p : {(void*)ctx->vinv_X, (void*)ctx->vinv_r, (void*)ctx->uhat, (void*)ctx->f_theta}) dfree(ctx, p);
@@ -210,8 +210,7 @@ void globe_destroy(globe_ctx* ctx) {
     for (auto& s : ctx->ws)
         if (s.p) cudaFree(s.p);
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
-    for (auto& g : ctx->pcg_graph)
-        if (g) cudaGraphExecDestroy(g);
+    if (ctx->pcg_graph) cudaGraphExecDestroy(ctx->pcg_graph);
     if (ctx->pcg_loop) cudaGraphExecDestroy(ctx->pcg_loop);
     for (auto& e : ctx->prof_pool) {
         cudaEventDestroy(e.a);
@@ -403,6 +402,17 @@ int globe_load_records(globe_ctx* ctx, int64_t Nrec, int32_t N, int32_t p, const
         GLOBE_CK(ctx, cudaMemcpyAsync(c.lblk, lblk.data(), sizeof(int32_t) * c.nlong, cudaMemcpyHostToDevice,
                                       ctx->stream));
     }
+    // blocks by descending number of records, in file order among equals (a counting sort): the
+    // solve's kernels walk them so, and those with more than SOLVE_HUGE with a CTA each
+    std::vector<int32_t> at((size_t)maxb + 2, 0);
+    std::vector<int4> order(N);
+    for (int32_t b = 0; b < N; ++b) ++at[maxb - (bstart[b + 1] - bstart[b]) + 1];
+    for (int32_t l = 0; l <= maxb; ++l) at[l + 1] += at[l];
+    for (int32_t b = 0; b < N; ++b)
+        order[at[maxb - (bstart[b + 1] - bstart[b])]++] = make_int4(b, bstart[b], bstart[b + 1], bind[b]);
+    while (c.nhuge < N && order[c.nhuge].z - order[c.nhuge].y > SOLVE_HUGE) ++c.nhuge;
+    GLOBE_RET(dalloc(ctx, &c.order, (size_t)N));
+    GLOBE_CK(ctx, cudaMemcpyAsync(c.order, order.data(), sizeof(int4) * N, cudaMemcpyHostToDevice, ctx->stream));
     GLOBE_CK(ctx, cudaMemcpyAsync(c.X, X, sizeof(double) * Nrec * (p + 1), cudaMemcpyHostToDevice, ctx->stream));
     GLOBE_CK(ctx, cudaMemcpyAsync(c.y, y, sizeof(double) * Nrec, cudaMemcpyHostToDevice, ctx->stream));
     GLOBE_CK(ctx, cudaMemcpyAsync(c.bstart, bstart.data(), sizeof(int32_t) * (N + 1), cudaMemcpyHostToDevice,

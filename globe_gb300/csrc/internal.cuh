@@ -28,6 +28,7 @@ namespace globe {
 //             zs = (g - 2f) * inv_std, missing -> g = 0
 //   dense:    packed lower triangle float32, N(N+1)/2
 constexpr int SHORT_BLOCK = 48;   // longest record block handled by one thread in the record kernels
+constexpr int SOLVE_HUGE = 256;   // longest one handled by one thread in a solve's kernels (k_solve.cu)
 
 struct Cohort {
     int64_t Nrec = 0;
@@ -43,6 +44,8 @@ struct Cohort {
     int32_t max_block = 0;
     int32_t* lblk = nullptr;   // blocks with more than SHORT_BLOCK records (device list)
     int32_t nlong = 0;
+    int4* order = nullptr;     // blocks by descending number of records: {block, first, one past last, individual}
+    int32_t nhuge = 0;         // of them, those with more than SOLVE_HUGE
     float2* tdf = nullptr;     // times as double-float pairs (the double-float record kernels)
     double tmax = 0;           // max |t|
     const double* times() const { return X + (size_t)p * Nrec; }
@@ -84,21 +87,10 @@ struct Slot {
 };
 
 enum SlotId {
-    WS_R, WS_Z, WS_P, WS_VP, WS_ZI, WS_GZ, WS_S1, WS_PART, WS_SCAL, WS_COLS, WS_W,
+    WS_R, WS_X, WS_P, WS_VP, WS_ZI, WS_GZ, WS_S1, WS_PART, WS_SCAL, WS_COLS, WS_W,
     WS_GPART, WS_B, WS_TMP1, WS_TMP2, WS_TMP3, WS_TMP4, WS_H, WS_HSTAR, WS_PROBE,
     WS_UH, WS_SMALL, WS_IO1, WS_IO2, WS_BHAT, WS_FB, WS_FX,
-    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_S0DF, WS_HDF, WS_TC_CNT, WS_TC_STAT, WS_COUNT
-};
-
-// Scalars kept on the device during a solve (per column, k entries each).
-struct PcgScalars {
-    double* rz;     // r'z
-    double* rz_new;
-    double* pvp;    // p'Vp
-    double* alpha;
-    double* beta;
-    double* rr;     // |r|^2
-    double* bb;     // |b|^2
+    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_SOLVE, WS_HDF, WS_TC_CNT, WS_TC_STAT, WS_COUNT
 };
 
 }  // namespace globe
@@ -144,10 +136,10 @@ struct globe_ctx {
     std::vector<std::pair<void*, size_t>> allocs;  // persistent allocations (freed on destroy)
     double* hpin = nullptr;       // pinned host scratch for per-iteration scalars
     size_t hpin_n = 0;
-    // CUDA graphs of the block-PCG iteration body (globe_set_graphs), one per parity of the
-    // swapped r'z buffers; updated in place from each call's capture
+    // CUDA graph of the block-PCG iteration body (globe_set_graphs), updated in place from each
+    // call's capture
     int graphs = 1;
-    cudaGraphExec_t pcg_graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t pcg_graph = nullptr;
     // the device-side PCG loop of the last call (one WHILE conditional node), and whether to use it
     cudaGraphExec_t pcg_loop = nullptr;
     int device_loop = 1;
@@ -287,23 +279,14 @@ int synth_bed(globe_ctx* ctx, uint8_t* d_bed, int64_t M, int32_t N, int64_t stri
 // k_records.cu
 int block_moments(globe_ctx* ctx);
 int build_H(globe_ctx* ctx, const double* gdiag, double gconst, double* H, float2* Hdf = nullptr);
-int seg_sums(globe_ctx* ctx, const double* x, const double* z, const double* beta, double* xout,
-             const int32_t* cols, int kact, double* Zi, double* S1);
-// with dot_out and quot: also quot[col] = num[col] / dot_out[col] (the step length, fused)
-int vx_assemble(globe_ctx* ctx, const double* x, const double* GZ, const double* Zi,
-                const double* S1, const int32_t* cols, int kact, double* out, double* dot_out,
-                const double* num = nullptr, double* quot = nullptr);
-int pcg_update(globe_ctx* ctx, const double* H, const double* alpha, double* x, double* r,
-               const double* p, const double* Vp, double* z, const int32_t* cols, int kact,
-               double* rr, double* rz);
-int precond_apply(globe_ctx* ctx, const double* H, const double* r, double* z,
-                  const int32_t* cols, int kact, double* rz);
+int seg_sums(globe_ctx* ctx, const double* x, int k, double* Zi, double* S1);
+int vx_assemble(globe_ctx* ctx, const double* x, const double* GZ, const double* Zi, const double* S1, int k,
+                double* out);
+int precond_apply(globe_ctx* ctx, const double* H, const double* r, double* z, int k);
 int precond_apply_scratch(globe_ctx* ctx, const double* H, const double* r, double* z, int kact, double* part,
                           size_t part_cap, double* rz);
 int col_dots(globe_ctx* ctx, const double* a, const double* b, int64_t n, int64_t lda, int64_t ldb,
              const int32_t* cols, int kact, double* out);
-int scal_alpha(globe_ctx* ctx, const double* num, const double* den, double* out, int kact,
-               float2* out_df = nullptr);
 int xt_mat(globe_ctx* ctx, const double* X, int m1, const double* S, int m2, double* out);
 int sub_mat(globe_ctx* ctx, const double* A, const double* Bm, int m, const double* c, double* out,
             int kout);
@@ -315,24 +298,12 @@ int probes_build(globe_ctx* ctx, const double* draws, int numMC, uint64_t seed, 
 int trace_terms(globe_ctx* ctx, const double* VR, const double* UH, const double* TY, int numMC,
                 double* out);
 
-// k_records_df.cu: the iteration's record kernels on double-float vectors (float2 in the
-// place of each double); Zi, GZ, the partial sums and the scalars stay FP64
+// k_solve.cu
 int to_df(globe_ctx* ctx, const double* in, int64_t n, float2* out);
-struct DfCols {   // up to 4 (source, destination) column blocks; unused destinations null
-    const double* src[4] = {nullptr, nullptr, nullptr, nullptr};
-    double* dst[4] = {nullptr, nullptr, nullptr, nullptr};
-};
-int col_unscales(globe_ctx* ctx, const double* bb, int k, double* unsc);   // unsc[c] = col_unscale(bb[c])
-int cols_to_df(globe_ctx* ctx, const DfCols& v, int64_t n, int k, const double* unsc, double* rz);
-int precond_apply_df(globe_ctx* ctx, const float2* H, const float2* r, float2* z, int k, double* rz);
-int cols_from_df(globe_ctx* ctx, double* v, int64_t n, int k, const double* unsc);
-int seg_sums_df(globe_ctx* ctx, float2* x, const float2* z, const float2* beta, const int32_t* cols, int kact,
-                double* Zi, float2* S0, float2* S1);
-int vx_assemble_df(globe_ctx* ctx, const float2* x, const double* GZ, const float2* S0, const float2* S1,
-                   const int32_t* cols, int kact, float2* out, double* dot_out, const double* num = nullptr,
-                   double* quot = nullptr, float2* quot_df = nullptr);
-int pcg_update_df(globe_ctx* ctx, const float2* H, const float2* alpha, float2* x, float2* r, const float2* p,
-                  const float2* Vp, float2* z, const int32_t* cols, int kact, double* rr, double* rz);
+
+// whether an FP64 product of k columns runs on the tensor cores (known once one has run)
+bool geno_f64_tc(const globe_ctx* ctx, int k);
+bool dense_f64_tc(const globe_ctx* ctx, int k);
 
 // k_grm_geno.cu
 int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
@@ -368,9 +339,4 @@ int vx_dev(globe_ctx* ctx, const double* x, int k, double* out);
 int pcg_dev(globe_ctx* ctx, const double* B, double* X, int k, const globe_pcg_opts* o,
             globe_pcg_info* info);
 int reduce_cols(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out);
-int reduce_cols2(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out0,
-                 double* out1);
-int reduce_cols_div(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out,
-                    const double* num, double* quot, float2* quot_df);
-
 }  // namespace globe

@@ -139,13 +139,12 @@ int build_H(globe_ctx* ctx, const double* gdiag, double gconst, double* H, float
 }
 
 // ---------------------------------------------------------------------------
-// Segment sums (J' x and t-weighted), optionally fused with p = z + beta p.
+// Segment sums (J' x and t-weighted).
 
 __global__ void k_seg_sums(int32_t nblk, int64_t ld, int32_t N, const int32_t* __restrict__ bstart,
                            const int32_t* __restrict__ bind, const double* __restrict__ t,
-                           double* x, const double* __restrict__ z, const double* __restrict__ beta,
-                           const int32_t* __restrict__ cols, int kact, double* __restrict__ Zi,
-                           double* __restrict__ S1, const int32_t* __restrict__ bl) {
+                           const double* __restrict__ x, int k, double* __restrict__ Zi, double* __restrict__ S1,
+                           const int32_t* __restrict__ bl) {
     const int lane = threadIdx.x & 31;
     const int idx = blockIdx.x * RB_WARPS + (threadIdx.x >> 5);
     if (idx >= nblk) return;
@@ -153,25 +152,13 @@ __global__ void k_seg_sums(int32_t nblk, int64_t ld, int32_t N, const int32_t* _
     const int st = bstart[b], en = bstart[b + 1];
     const int i = bind[b];
     if (!GLOBE_BOUNDS(st >= 0 && st <= en && en <= ld && i >= 0 && i < N, 0x0101u)) return;
-    for (int c = 0; c < kact; ++c) {
-        const int col = cols ? cols[c] : c;
-        double* xc = x + (size_t)col * ld;
+    for (int c = 0; c < k; ++c) {
+        const double* xc = x + (size_t)c * ld;
         double s0 = 0, s1 = 0;
-        if (beta) {
-            const double bb = beta[col];
-            const double* zc = z + (size_t)col * ld;
-            for (int r = st + lane; r < en; r += 32) {
-                double v = zc[r] + bb * xc[r];
-                xc[r] = v;
-                s0 += v;
-                s1 += t[r] * v;
-            }
-        } else {
-            for (int r = st + lane; r < en; r += 32) {
-                double v = xc[r];
-                s0 += v;
-                s1 += t[r] * v;
-            }
+        for (int r = st + lane; r < en; r += 32) {
+            double v = xc[r];
+            s0 += v;
+            s1 += t[r] * v;
         }
         s0 = warp_sum(s0);
         s1 = warp_sum(s1);
@@ -184,101 +171,62 @@ __global__ void k_seg_sums(int32_t nblk, int64_t ld, int32_t N, const int32_t* _
 
 // thread-per-block layout: one thread per (block, column)
 __global__ void k_seg_sums_t(int32_t nblk, int64_t ld, int32_t N, const int32_t* __restrict__ bstart,
-                             const int32_t* __restrict__ bind, const double* __restrict__ t, double* x,
-                             const double* __restrict__ z, const double* __restrict__ beta,
-                             const int32_t* __restrict__ cols, double* __restrict__ Zi, double* __restrict__ S1) {
+                             const int32_t* __restrict__ bind, const double* __restrict__ t,
+                             const double* __restrict__ x, double* __restrict__ Zi, double* __restrict__ S1) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nblk) return;
     const int c = blockIdx.y;
-    const int col = cols ? cols[c] : c;
     const int st = bstart[b], en = bstart[b + 1];
     if (!GLOBE_BOUNDS(st >= 0 && st <= en && en <= ld && bind[b] >= 0 && bind[b] < N, 0x0201u)) return;
     if (en - st > SHORT_BLOCK) return;   // a warp per long block handles it
-    double* xc = x + (size_t)col * ld;
+    const double* xc = x + (size_t)c * ld;
     double s0 = 0, s1 = 0;
-    if (beta) {
-        const double bb = beta[col];
-        const double* zc = z + (size_t)col * ld;
 #pragma unroll 4
-        for (int r = st; r < en; ++r) {
-            const double v = zc[r] + bb * xc[r];
-            xc[r] = v;
-            s0 += v;
-            s1 += t[r] * v;
-        }
-    } else {
-#pragma unroll 4
-        for (int r = st; r < en; ++r) {
-            const double v = xc[r];
-            s0 += v;
-            s1 += t[r] * v;
-        }
+    for (int r = st; r < en; ++r) {
+        const double v = xc[r];
+        s0 += v;
+        s1 += t[r] * v;
     }
     const int i = bind[b];
     Zi[i + (size_t)c * N] = s0;
     if (S1) S1[i + (size_t)c * N] = s1;
 }
 
-int seg_sums(globe_ctx* ctx, const double* x, const double* z, const double* beta, double* xout,
-             const int32_t* cols, int kact, double* Zi, double* S1) {
+int seg_sums(globe_ctx* ctx, const double* x, int k, double* Zi, double* S1) {
     auto& c = ctx->coh;
-    // in-place p update: xout must alias x when beta is given
-    double* xx = beta ? xout : const_cast<double*>(x);
     const RecShape rs = rec_shape(ctx);
-    k_seg_sums_t<<<dim3(rs.nbt, kact), TB_THREADS, 0, ctx->stream>>>(c.N, c.Nrec, c.N, c.bstart, c.bind, c.times(),
-                                                                       xx, z, beta, cols, Zi, S1);
+    k_seg_sums_t<<<dim3(rs.nbt, k), TB_THREADS, 0, ctx->stream>>>(c.N, c.Nrec, c.N, c.bstart, c.bind, c.times(), x, Zi,
+                                                                    S1);
     GLOBE_LAUNCHED(ctx, "k_seg_sums_t");
     if (rs.nbl) {
-        k_seg_sums<<<rs.nbl, RB_THREADS, 0, ctx->stream>>>(c.nlong, c.Nrec, c.N, c.bstart, c.bind, c.times(), xx, z,
-                                                            beta, cols, kact, Zi, S1, c.lblk);
+        k_seg_sums<<<rs.nbl, RB_THREADS, 0, ctx->stream>>>(c.nlong, c.Nrec, c.N, c.bstart, c.bind, c.times(), x, k, Zi,
+                                                            S1, c.lblk);
         GLOBE_LAUNCHED(ctx, "k_seg_sums");
     }
     return GLOBE_OK;
 }
 
 // ---------------------------------------------------------------------------
-// out = J GZ + U D U' x + sig2e x  (+ per-column partial dot x'out)
+// out = J GZ + U D U' x + sig2e x
 
 __global__ void k_vx_assemble(int32_t nblk, int64_t ld, int32_t N, const int32_t* __restrict__ bstart,
                               const int32_t* __restrict__ bind, const double* __restrict__ t, VC v,
                               const double* __restrict__ x, const double* __restrict__ GZ,
-                              const double* __restrict__ Zi, const double* __restrict__ S1,
-                              const int32_t* __restrict__ cols, int kact, double* __restrict__ out,
-                              double* __restrict__ part, const int32_t* __restrict__ bl, int slot0, int pstride) {
-    __shared__ double sm[RCH * RB_WARPS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int idx = blockIdx.x * RB_WARPS + warp;
-    const bool live = idx < nblk;
-    const int b = live ? (bl ? bl[idx] : idx) : 0;
-    int st = 0, en = 0, i = 0;
-    if (live) { st = bstart[b]; en = bstart[b + 1]; i = bind[b]; }
-    if (live && !GLOBE_BOUNDS(st >= 0 && st <= en && en <= ld && i >= 0 && i < N, 0x0301u)) st = en = i = 0;
-    for (int c0 = 0; c0 < kact; c0 += RCH) {
-        const int nc = min(RCH, kact - c0);
-        for (int cc = 0; cc < nc; ++cc) {
-            const int c = c0 + cc;
-            const int col = cols ? cols[c] : c;
-            double dot = 0;
-            if (live) {
-                const double s0 = Zi[i + (size_t)c * N], s1 = S1[i + (size_t)c * N];
-                const double g = GZ ? GZ[i + (size_t)c * N] : 0.0;
-                const double a0 = g + v.b0 * s0 + v.b01 * s1;
-                const double a1 = v.b01 * s0 + v.b1 * s1;
-                const double* xc = x + (size_t)col * ld;
-                double* oc = out + (size_t)col * ld;
-                for (int r = st + lane; r < en; r += 32) {
-                    double xv = xc[r];
-                    double o = a0 + t[r] * a1 + v.e * xv;
-                    oc[r] = o;
-                    dot += xv * o;
-                }
-            }
-            if (part) {
-                dot = warp_sum(dot);
-                if (lane == 0) sm[cc * RB_WARPS + warp] = dot;
-            }
-        }
-        if (part) flush_chunk(sm, 1, nc, c0, kact, part, slot0 + blockIdx.x, pstride);
+                              const double* __restrict__ Zi, const double* __restrict__ S1, int k,
+                              double* __restrict__ out, const int32_t* __restrict__ bl) {
+    const int lane = threadIdx.x & 31;
+    const int idx = blockIdx.x * RB_WARPS + (threadIdx.x >> 5);
+    if (idx >= nblk) return;
+    const int b = bl ? bl[idx] : idx;
+    const int st = bstart[b], en = bstart[b + 1], i = bind[b];
+    if (!GLOBE_BOUNDS(st >= 0 && st <= en && en <= ld && i >= 0 && i < N, 0x0301u)) return;
+    for (int c = 0; c < k; ++c) {
+        const double s0 = Zi[i + (size_t)c * N], s1 = S1[i + (size_t)c * N];
+        const double a0 = GZ[i + (size_t)c * N] + v.b0 * s0 + v.b01 * s1;
+        const double a1 = v.b01 * s0 + v.b1 * s1;
+        const double* xc = x + (size_t)c * ld;
+        double* oc = out + (size_t)c * ld;
+        for (int r = st + lane; r < en; r += 32) oc[r] = a0 + t[r] * a1 + v.e * xc[r];
     }
 }
 
@@ -286,186 +234,38 @@ __global__ void k_vx_assemble_t(int32_t nblk, int64_t ld, int32_t N, const int32
                                 const int32_t* __restrict__ bind, const double* __restrict__ t, VC v,
                                 const double* __restrict__ x, const double* __restrict__ GZ,
                                 const double* __restrict__ Zi, const double* __restrict__ S1,
-                                const int32_t* __restrict__ cols, double* __restrict__ out,
-                                double* __restrict__ part, int pstride) {
+                                double* __restrict__ out) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = blockIdx.y;
-    const int col = cols ? cols[c] : c;
-    double dot[1] = {0.0};
-    if (b < nblk && bstart[b + 1] - bstart[b] <= SHORT_BLOCK &&   // long blocks: a warp each
-        GLOBE_BOUNDS(bstart[b] >= 0 && bstart[b + 1] <= ld && bind[b] >= 0 && bind[b] < N, 0x0401u)) {
-        const int st = bstart[b], en = bstart[b + 1], i = bind[b];
-        const double s0 = Zi[i + (size_t)c * N], s1 = S1[i + (size_t)c * N];
-        const double g = GZ ? GZ[i + (size_t)c * N] : 0.0;
-        const double a0 = g + v.b0 * s0 + v.b01 * s1;
-        const double a1 = v.b01 * s0 + v.b1 * s1;
-        const double* xc = x + (size_t)col * ld;
-        double* oc = out + (size_t)col * ld;
+    if (b >= nblk || bstart[b + 1] - bstart[b] > SHORT_BLOCK) return;   // long blocks: a warp each
+    if (!GLOBE_BOUNDS(bstart[b] >= 0 && bstart[b + 1] <= ld && bind[b] >= 0 && bind[b] < N, 0x0401u)) return;
+    const int st = bstart[b], en = bstart[b + 1], i = bind[b];
+    const double s0 = Zi[i + (size_t)c * N], s1 = S1[i + (size_t)c * N];
+    const double a0 = GZ[i + (size_t)c * N] + v.b0 * s0 + v.b01 * s1;
+    const double a1 = v.b01 * s0 + v.b1 * s1;
+    const double* xc = x + (size_t)c * ld;
+    double* oc = out + (size_t)c * ld;
 #pragma unroll 4
-        for (int r = st; r < en; ++r) {
-            const double xv = xc[r];
-            const double o = a0 + t[r] * a1 + v.e * xv;
-            oc[r] = o;
-            dot[0] += xv * o;
-        }
-    }
-    if (part) {
-        const int q[1] = {c};
-        cta_sums<1>(dot, q, part, pstride);
-    }
+    for (int r = st; r < en; ++r) oc[r] = a0 + t[r] * a1 + v.e * xc[r];
 }
 
-int vx_assemble(globe_ctx* ctx, const double* x, const double* GZ, const double* Zi, const double* S1,
-                const int32_t* cols, int kact, double* out, double* dot_out, const double* num, double* quot) {
+int vx_assemble(globe_ctx* ctx, const double* x, const double* GZ, const double* Zi, const double* S1, int k,
+                double* out) {
     auto& c = ctx->coh;
     VC v{ctx->vc[0], ctx->vc[1], ctx->vc[2], ctx->vc[3], ctx->vc[4]};
     const RecShape rs = rec_shape(ctx);
-    double* part = nullptr;
-    if (dot_out) GLOBE_RET(ws(ctx, WS_PART, (size_t)rs.S * kact * 2, &part));
-    k_vx_assemble_t<<<dim3(rs.nbt, kact), TB_THREADS, 0, ctx->stream>>>(c.N, c.Nrec, c.N, c.bstart, c.bind, c.times(),
-                                                                          v, x, GZ, Zi, S1, cols, out, part, rs.S);
+    k_vx_assemble_t<<<dim3(rs.nbt, k), TB_THREADS, 0, ctx->stream>>>(c.N, c.Nrec, c.N, c.bstart, c.bind, c.times(), v, x,
+                                                                       GZ, Zi, S1, out);
     GLOBE_LAUNCHED(ctx, "k_vx_assemble_t");
     if (rs.nbl) {
-        k_vx_assemble<<<rs.nbl, RB_THREADS, 0, ctx->stream>>>(c.nlong, c.Nrec, c.N, c.bstart, c.bind, c.times(), v,
-                                                                x, GZ, Zi, S1, cols, kact, out, part, c.lblk, rs.nbt,
-                                                                rs.S);
+        k_vx_assemble<<<rs.nbl, RB_THREADS, 0, ctx->stream>>>(c.nlong, c.Nrec, c.N, c.bstart, c.bind, c.times(), v, x,
+                                                                GZ, Zi, S1, k, out, c.lblk);
         GLOBE_LAUNCHED(ctx, "k_vx_assemble");
     }
-    if (dot_out) GLOBE_RET(reduce_cols_div(ctx, part, rs.S, kact, cols, dot_out, num, quot, nullptr));
     return GLOBE_OK;
 }
 
 // ---------------------------------------------------------------------------
-// x += a p; r -= a Vp; z = Q^-1 r; partial |r|^2 and r'z.
-
-__global__ void k_pcg_update(int32_t nblk, int64_t ld, const int32_t* __restrict__ bstart,
-                             const double* __restrict__ t, double inv_e, const double* __restrict__ H,
-                             const double* __restrict__ alpha, double* __restrict__ x, double* __restrict__ r,
-                             const double* __restrict__ p, const double* __restrict__ Vp,
-                             double* __restrict__ z, const int32_t* __restrict__ cols, int kact,
-                             double* __restrict__ part, const int32_t* __restrict__ bl, int slot0, int pstride) {
-    __shared__ double sm[2 * RCH * RB_WARPS];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int idx = blockIdx.x * RB_WARPS + warp;
-    const bool live = idx < nblk;
-    const int b = live ? (bl ? bl[idx] : idx) : 0;
-    int st = 0, en = 0;
-    double h00 = 0, h01 = 0, h10 = 0, h11 = 0;
-    if (live) {
-        st = bstart[b];
-        en = bstart[b + 1];
-        h00 = H[4 * b];
-        h01 = H[4 * b + 1];
-        h10 = H[4 * b + 2];
-        h11 = H[4 * b + 3];
-        if (!GLOBE_BOUNDS(st >= 0 && st <= en && en <= ld, 0x0501u)) st = en = 0;
-    }
-    for (int c0 = 0; c0 < kact; c0 += RCH) {
-        const int nc = min(RCH, kact - c0);
-        for (int cc = 0; cc < nc; ++cc) {
-            const int c = c0 + cc;
-            const int col = cols ? cols[c] : c;
-            double rr = 0, rz = 0;
-            if (live) {
-                const double a = alpha[col];
-                double* xc = x + (size_t)col * ld;
-                double* rc = r + (size_t)col * ld;
-                const double* pc = p + (size_t)col * ld;
-                const double* vc = Vp + (size_t)col * ld;
-                double s0 = 0, s1 = 0;
-                for (int q = st + lane; q < en; q += 32) {
-                    xc[q] += a * pc[q];
-                    double rn = rc[q] - a * vc[q];
-                    rc[q] = rn;
-                    rr += rn * rn;
-                    s0 += rn;
-                    s1 += t[q] * rn;
-                }
-                s0 = warp_sum(s0);
-                s1 = warp_sum(s1);
-                const double g0 = h00 * s0 + h01 * s1, g1 = h10 * s0 + h11 * s1;
-                const double g0e = g0 * inv_e, g1e = g1 * inv_e;   // z = r/sig2e - (g0 + g1 t)/sig2e
-                double* zc = z + (size_t)col * ld;
-                for (int q = st + lane; q < en; q += 32) {
-                    double rn = rc[q];
-                    double zv = fma(rn, inv_e, -fma(g1e, t[q], g0e));
-                    zc[q] = zv;
-                    rz += rn * zv;
-                }
-            }
-            rr = warp_sum(rr);
-            rz = warp_sum(rz);
-            if (lane == 0) {
-                sm[cc * RB_WARPS + warp] = rr;
-                sm[(RCH + cc) * RB_WARPS + warp] = rz;
-            }
-        }
-        flush_chunk(sm, 2, nc, c0, kact, part, slot0 + blockIdx.x, pstride);
-    }
-}
-
-__global__ void k_pcg_update_t(int32_t nblk, int64_t ld, const int32_t* __restrict__ bstart,
-                               const double* __restrict__ t, double inv_e, const double* __restrict__ H,
-                               const double* __restrict__ alpha, double* __restrict__ x, double* __restrict__ r,
-                               const double* __restrict__ p, const double* __restrict__ Vp, double* __restrict__ z,
-                               const int32_t* __restrict__ cols, int kact, double* __restrict__ part,
-                               int pstride) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = blockIdx.y;
-    const int col = cols ? cols[c] : c;
-    double acc[2] = {0.0, 0.0};   // |r|^2, r'z
-    if (b < nblk && bstart[b + 1] - bstart[b] <= SHORT_BLOCK &&
-        GLOBE_BOUNDS(bstart[b] >= 0 && bstart[b + 1] <= ld, 0x0601u)) {
-        const int st = bstart[b], en = bstart[b + 1];
-        const double a = alpha[col];
-        double* xc = x + (size_t)col * ld;
-        double* rc = r + (size_t)col * ld;
-        const double* pc = p + (size_t)col * ld;
-        const double* vc = Vp + (size_t)col * ld;
-        double s0 = 0, s1 = 0;
-#pragma unroll 4
-        for (int q = st; q < en; ++q) {
-            xc[q] += a * pc[q];
-            const double rn = rc[q] - a * vc[q];
-            rc[q] = rn;
-            acc[0] += rn * rn;
-            s0 += rn;
-            s1 += t[q] * rn;
-        }
-        const double g0 = H[4 * b] * s0 + H[4 * b + 1] * s1, g1 = H[4 * b + 2] * s0 + H[4 * b + 3] * s1;
-        const double g0e = g0 * inv_e, g1e = g1 * inv_e;   // z = r/sig2e - (g0 + g1 t)/sig2e
-        double* zc = z + (size_t)col * ld;
-#pragma unroll 4
-        for (int q = st; q < en; ++q) {
-            const double rn = rc[q];
-            const double zv = fma(rn, inv_e, -fma(g1e, t[q], g0e));
-            zc[q] = zv;
-            acc[1] += rn * zv;
-        }
-    }
-    const int qi[2] = {c, kact + c};
-    cta_sums<2>(acc, qi, part, pstride);
-}
-
-int pcg_update(globe_ctx* ctx, const double* H, const double* alpha, double* x, double* r, const double* p,
-               const double* Vp, double* z, const int32_t* cols, int kact, double* rr, double* rz) {
-    auto& c = ctx->coh;
-    const RecShape rs = rec_shape(ctx);
-    double* part;
-    GLOBE_RET(ws(ctx, WS_PART, (size_t)rs.S * kact * 2, &part));
-    k_pcg_update_t<<<dim3(rs.nbt, kact), TB_THREADS, 0, ctx->stream>>>(c.N, c.Nrec, c.bstart, c.times(),
-                                                                         1.0 / ctx->vc[0], H, alpha, x, r, p, Vp, z,
-                                                                         cols, kact, part, rs.S);
-    GLOBE_LAUNCHED(ctx, "k_pcg_update_t");
-    if (rs.nbl) {
-        k_pcg_update<<<rs.nbl, RB_THREADS, 0, ctx->stream>>>(c.nlong, c.Nrec, c.bstart, c.times(), 1.0 / ctx->vc[0],
-                                                               H, alpha, x, r, p, Vp, z, cols, kact, part, c.lblk,
-                                                               rs.nbt, rs.S);
-        GLOBE_LAUNCHED(ctx, "k_pcg_update");
-    }
-    return reduce_cols2(ctx, part, rs.S, kact, cols, rr, rz);
-}
-
 // z = Q^-1 r (+ partial r'z)
 __global__ void k_precond_apply(int32_t nblk, int64_t ld, const int32_t* __restrict__ bstart,
                                 const double* __restrict__ t, double inv_e, const double* __restrict__ H,
@@ -570,14 +370,8 @@ static int precond_launch(globe_ctx* ctx, const double* H, const double* r, doub
     return GLOBE_OK;
 }
 
-int precond_apply(globe_ctx* ctx, const double* H, const double* r, double* z, const int32_t* cols, int kact,
-                  double* rz) {
-    const RecShape rs = rec_shape(ctx);
-    double* part = nullptr;
-    if (rz) GLOBE_RET(ws(ctx, WS_PART, (size_t)rs.S * kact * 2, &part));
-    GLOBE_RET(precond_launch(ctx, H, r, z, cols, kact, part, rs));
-    if (rz) GLOBE_RET(reduce_cols(ctx, part, rs.S, kact, cols, rz));
-    return GLOBE_OK;
+int precond_apply(globe_ctx* ctx, const double* H, const double* r, double* z, int k) {
+    return precond_launch(ctx, H, r, z, nullptr, k, nullptr, rec_shape(ctx));
 }
 
 // Same operator with the r'z partials in caller-provided scratch (part, part_cap
@@ -609,62 +403,17 @@ int precond_apply_scratch(globe_ctx* ctx, const double* H, const double* r, doub
 // ---------------------------------------------------------------------------
 // Column reductions
 
-// Quantity y (grid.y) of column c (grid.x): part[y * qstride + j + c*nparts], j < nparts,
-// summed into o.out[y][cols ? cols[c] : c]; with o.quot, also o.quot[col] = o.num[col] / sum
-// (0 where the sum is 0) and its double-float copy o.quot_df -- the step length
-// alpha = r'z / p'Vp fused into the p'Vp reduction.
-struct ReduceOut {
-    double* out[2] = {nullptr, nullptr};
-    const double* num = nullptr;
-    double* quot = nullptr;
-    float2* quot_df = nullptr;
-};
-
-__global__ void k_reduce_cols(const double* __restrict__ part, int nparts, size_t qstride,
-                              const int32_t* __restrict__ cols, ReduceOut o) {
+// out[cols ? cols[c] : c] = sum_j part[j + c*nparts], j < nparts; one CTA per column
+__global__ void k_reduce_cols(const double* __restrict__ part, int nparts, const int32_t* __restrict__ cols,
+                              double* __restrict__ out) {
     __shared__ double sm[256];
     const int c = blockIdx.x;
-    const double v = cta_reduce_256(part + blockIdx.y * qstride + (size_t)c * nparts, nparts, sm);   // 256 threads
-    if (threadIdx.x == 0) {
-        const int col = cols ? cols[c] : c;
-        o.out[blockIdx.y][col] = v;
-        if (o.quot) {
-            const double q = (v != 0.0) ? o.num[col] / v : 0.0;
-            o.quot[col] = q;
-            if (o.quot_df) df::store(o.quot_df + col, df::from_double(q));
-        }
-    }
+    const double v = cta_reduce_256(part + (size_t)c * nparts, nparts, sm);   // 256 threads
+    if (threadIdx.x == 0) out[cols ? cols[c] : c] = v;
 }
 
-// out[cols ? cols[c] : c] = sum_j part[j + c*nparts]
 int reduce_cols(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out) {
-    ReduceOut o;
-    o.out[0] = out;
-    k_reduce_cols<<<kact, 256, 0, ctx->stream>>>(part, nparts, 0, cols, o);
-    GLOBE_LAUNCHED(ctx, "k_reduce_cols");
-    return GLOBE_OK;
-}
-
-// two quantities of kact columns each (the second's partials follow the first's), one launch
-int reduce_cols2(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out0,
-                 double* out1) {
-    ReduceOut o;
-    o.out[0] = out0;
-    o.out[1] = out1;
-    k_reduce_cols<<<dim3(kact, 2), 256, 0, ctx->stream>>>(part, nparts, (size_t)nparts * kact, cols, o);
-    GLOBE_LAUNCHED(ctx, "k_reduce_cols");
-    return GLOBE_OK;
-}
-
-// out as reduce_cols, and quot[col] = num[col] / out[col] (0 where out is 0), quot_df its copy
-int reduce_cols_div(globe_ctx* ctx, const double* part, int nparts, int kact, const int32_t* cols, double* out,
-                    const double* num, double* quot, float2* quot_df) {
-    ReduceOut o;
-    o.out[0] = out;
-    o.num = num;
-    o.quot = quot;
-    o.quot_df = quot_df;
-    k_reduce_cols<<<kact, 256, 0, ctx->stream>>>(part, nparts, 0, cols, o);
+    k_reduce_cols<<<kact, 256, 0, ctx->stream>>>(part, nparts, cols, out);
     GLOBE_LAUNCHED(ctx, "k_reduce_cols");
     return GLOBE_OK;
 }
@@ -700,23 +449,6 @@ int col_dots(globe_ctx* ctx, const double* a, const double* b, int64_t n, int64_
     k_col_dots<<<dim3(nb, kact), 256, 0, ctx->stream>>>(a, b, n, lda, ldb, cols, part);
     GLOBE_LAUNCHED(ctx, "k_col_dots");
     return reduce_cols(ctx, part, nb, kact, cols, out);
-}
-
-// out = num / den (0 where den = 0), and its double-float copy when out_df is given
-__global__ void k_scal_div(const double* __restrict__ num, const double* __restrict__ den, double* out, int k,
-                           float2* __restrict__ out_df) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < k) {
-        const double q = (den[c] != 0.0) ? num[c] / den[c] : 0.0;
-        out[c] = q;
-        if (out_df) df::store(out_df + c, df::from_double(q));
-    }
-}
-
-int scal_alpha(globe_ctx* ctx, const double* num, const double* den, double* out, int k, float2* out_df) {
-    k_scal_div<<<div_up(k, 128), 128, 0, ctx->stream>>>(num, den, out, k, out_df);
-    GLOBE_LAUNCHED(ctx, "k_scal_div");
-    return GLOBE_OK;
 }
 
 // out (m1 x m2) = X' S over Nrec rows; X Nrec x m1, S Nrec x m2.

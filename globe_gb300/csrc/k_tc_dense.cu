@@ -574,10 +574,14 @@ int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double*
 #ifndef F64_DENSE_CALL_MIN
 #define F64_DENSE_CALL_MIN 4e6
 #endif
+static bool f64_dense_size(const globe_ctx* ctx, int k) {
+    return (double)ctx->coh.N * ctx->coh.N * k >= (ctx->in_solve ? F64_DENSE_SOLVE_MIN : F64_DENSE_CALL_MIN);
+}
+bool dense_f64_tc(const globe_ctx* ctx, int k) { return ctx->gen.adig[1].state == 1 && f64_dense_size(ctx, k); }
+
 int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& a = ctx->gen.adig[1];
-    const int32_t N = ctx->coh.N;
-    if (a.state >= 0 && (double)N * N * k >= (ctx->in_solve ? F64_DENSE_SOLVE_MIN : F64_DENSE_CALL_MIN)) {
+    if (a.state >= 0 && f64_dense_size(ctx, k)) {
         int rc = dense_digit_planes(ctx, 1);
         if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, ND64, Z, k, scale, out, zhi_ready);
         if (a.state == 1 && rc != GLOBE_ERR_NOMEM) return rc;

@@ -1012,11 +1012,15 @@ int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* 
 #ifndef F64_CALL_MIN
 #define F64_CALL_MIN 4e7
 #endif
+static bool f64_size(const globe_ctx* ctx, int k) {
+    return (double)ctx->coh.N * (double)ctx->gen.Mk * k >= (ctx->in_solve ? F64_SOLVE_MIN : F64_CALL_MIN);
+}
+bool geno_f64_tc(const globe_ctx* ctx, int k) { return ctx->gen.f64_tc == 1 && f64_size(ctx, k); }
+
 int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
-    const double size = (double)N * (double)g.Mk * k;
-    if (g.f64_tc >= 0 && size >= (ctx->in_solve ? F64_SOLVE_MIN : F64_CALL_MIN)) {
+    if (g.f64_tc >= 0 && f64_size(ctx, k)) {
         if (g.f64_tc == 0 && !g.blk2) {
             // the copy, and at most ~16 split partials of 256 columns beside U, digits and the rest
             const double need = (double)N * (double)g.Mk / 4 * 1.01 + 256.0 * 4 * 16 * (double)N +

@@ -1,4 +1,4 @@
-// records.cuh -- launch shape shared by the record kernels (k_records.cu, k_records_df.cu).
+// records.cuh -- launch shape of the record kernels outside a solve (k_records.cu).
 #pragma once
 
 #include "internal.cuh"
@@ -25,8 +25,7 @@ inline RecShape rec_shape(const globe_ctx* ctx) {
 }
 
 // Sum of one column's nparts partials by a CTA of 256 threads: four strided accumulators per
-// thread, then a tree in sm (256 doubles); every thread returns the sum.  k_reduce_cols and the
-// reductions that the record kernels' last CTAs finish both use it, so the order is one.
+// thread, then a tree in sm (256 doubles); every thread returns the sum.
 __device__ __forceinline__ double cta_reduce_256(const double* __restrict__ pc, int nparts, double* sm) {
     double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
     int j = threadIdx.x;
@@ -46,24 +45,6 @@ __device__ __forceinline__ double cta_reduce_256(const double* __restrict__ pc, 
     const double v = sm[0];
     __syncthreads();   // sm may be reused
     return v;
-}
-
-// The warp-per-block kernels stage per-warp partial sums of RCH columns at a time in static
-// shared memory, sm[(j * RCH + cc) * RB_WARPS + warp] for quantity j < nq and column c0 + cc,
-// so any number of columns fits.  flush_chunk sums them over the CTA's warps, in warp order,
-// into part[slot + (j * kact + c0 + cc) * stride]; every thread of the CTA calls it.
-constexpr int RCH = 32;
-__device__ __forceinline__ void flush_chunk(const double* sm, int nq, int nc, int c0, int kact, double* part, int slot,
-                                            int stride) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < nq * nc; e += blockDim.x) {
-        const int j = e / nc, cc = e - j * nc;
-        double a = 0.0;
-#pragma unroll
-        for (int w = 0; w < RB_WARPS; ++w) a += sm[(j * RCH + cc) * RB_WARPS + w];
-        part[slot + (size_t)(j * kact + c0 + cc) * stride] = a;
-    }
-    __syncthreads();
 }
 
 }  // namespace globe

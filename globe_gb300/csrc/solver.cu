@@ -8,7 +8,8 @@
 #include <vector>
 
 #include "df.cuh"
-#include "internal.cuh"
+#include "solve.cuh"
+#include "tc_common.cuh"
 
 namespace globe {
 
@@ -30,6 +31,15 @@ int grm_apply_dev(globe_ctx* ctx, const double* Z, int k, double* out, bool zhi_
         return mixed ? dense_apply_tc(ctx, Z, k, ctx->vc[1], out, zhi_ready)
                      : dense_apply_f64(ctx, Z, k, ctx->vc[1], out, zhi_ready);
     return set_err(ctx, GLOBE_ERR_STATE, "no genetic relationship source loaded");
+}
+
+// Whether the next product of k columns consumes statistics words that the writer of its input
+// raises: the choice of kernel that grm_apply_dev will make, once it has been made before
+static bool grm_wants_zhi(const globe_ctx* ctx, int k) {
+    const bool mixed = ctx->prec == GLOBE_PREC_MIXED;
+    if (ctx->gen.src == GSRC_GENO) return ctx->gen.Mk > 0 && (mixed || geno_f64_tc(ctx, k));
+    if (ctx->gen.src == GSRC_DENSE) return mixed ? ctx->gen.adig[0].state == 1 : dense_f64_tc(ctx, k);
+    return false;
 }
 
 int ensure_gdiag(globe_ctx* ctx) {
@@ -62,10 +72,9 @@ int vx_dev(globe_ctx* ctx, const double* x, int k, double* out) {
     GLOBE_RET(ws(ctx, WS_ZI, (size_t)N * k, &Zi));
     GLOBE_RET(ws(ctx, WS_S1, (size_t)N * k, &S1));
     GLOBE_RET(ws(ctx, WS_GZ, (size_t)N * k, &GZ));
-    GLOBE_RET(seg_sums(ctx, x, nullptr, nullptr, nullptr, nullptr, k, Zi, S1));
+    GLOBE_RET(seg_sums(ctx, x, k, Zi, S1));
     GLOBE_RET(grm_apply_dev(ctx, Zi, k, GZ));
-    GLOBE_RET(vx_assemble(ctx, x, GZ, Zi, S1, nullptr, k, out, nullptr));
-    return GLOBE_OK;
+    return vx_assemble(ctx, x, GZ, Zi, S1, k, out);
 }
 
 __global__ void k_sub(const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ out, int64_t n) {
@@ -101,12 +110,11 @@ int pcg_dev(globe_ctx* ctx, const double* B, double* X, int k, const globe_pcg_o
     return with_tc_check(ctx, rc);
 }
 
-// Captures `body` (stream work only, nothing run) into a graph and makes ctx->pcg_graph[slot]
-// run it: the cached executable is updated in place when the topology matches, else
+// Captures `body` (stream work only, nothing run) into a graph and makes ctx->pcg_graph run it: the cached executable is updated in place when the topology matches, else
 // instantiated anew.  Allocation is refused while the capture is open.  Returns false, with
 // nothing run and the error message restored, if any step fails.
 template <class F>
-static bool capture_body(globe_ctx* ctx, int slot, F&& body, int64_t* nlaunch) {
+static bool capture_body(globe_ctx* ctx, F&& body, int64_t* nlaunch) {
     const std::string err0 = ctx->err;
     const int64_t l0 = ctx->launches;
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
@@ -122,7 +130,7 @@ static bool capture_body(globe_ctx* ctx, int slot, F&& body, int64_t* nlaunch) {
     ctx->launches = l0;
     bool ok = rc == GLOBE_OK && e == cudaSuccess && g != nullptr;
     if (ok) {
-        cudaGraphExec_t& x = ctx->pcg_graph[slot];
+        cudaGraphExec_t& x = ctx->pcg_graph;
         cudaGraphExecUpdateResultInfo upd;
         if (!(x && cudaGraphExecUpdate(x, g, &upd) == cudaSuccess)) {
             cudaGetLastError();
@@ -145,107 +153,18 @@ static bool capture_body(globe_ctx* ctx, int slot, F&& body, int64_t* nlaunch) {
 // ---- the PCG iterations after the first, as one device-side loop -------------------
 //
 // One graph: a kernel that arms a WHILE conditional node, then the node, whose body is
-// one iteration (the same kernels, in the same order, as a host-driven iteration) followed
-// by k_pcg_check_shift, which applies the stopping rule of the host loop below to the device
-// copies of r'r and p'Vp, sets the node's condition, and shifts beta / r'z.
+// one iteration (the same kernels, in the same order, as a host-driven iteration), whose last
+// kernel also applies the stopping rule of the host loop below to the device copies of r'r and
+// p'Vp and sets the node's condition (PcgLoop, k_solve.cu).
 // So the iterations run without a host synchronisation each, with bit-identical
 // results and iteration counts.  The condition's launch default is 0: only the arming
 // kernel opens the loop, so a condition that could not be set leaves the loop unrun
 // (the host then sees no iteration and carries on itself); inside it every path of the
 // check sets it, and the iteration cap always closes it.
 
-struct PcgLoopState {
-    double last;          // last max ratio (PCGsolver rule, stagnation)
-    long long rhs_iters;  // sum over iterations of active columns
-    int it;               // iterations completed
-    int stag;             // iterations in a row with < 0.5% improvement
-    int status;           // 0 running, 1 converged, 2 stagnated, 3 iteration cap, 4 breakdown
-    int err_col;          // column of a breakdown
-};
-
 __global__ void k_pcg_loop_arm(cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, 1u); }
 
-// the host loop's stopping rule (pcg_run) on the device: one thread, after iteration st->it + 1
-__device__ void pcg_check(const double* __restrict__ rr, const double* __restrict__ pvp,
-                          const double* __restrict__ bb, const int32_t* __restrict__ cols, int kact, int k,
-                          double tol, int rule, int maxit, const double* __restrict__ unsc, PcgLoopState* st,
-                          cudaGraphConditionalHandle h) {
-    const int it = st->it + 1;
-    st->it = it;
-    st->rhs_iters += kact;
-    for (int c = 0; c < kact; ++c) {
-        const int j = cols[c];
-        if (!(pvp[j] > 0.0) || !isfinite(rr[j])) {
-            st->status = 4;
-            st->err_col = j;
-            cudaGraphSetConditional(h, 0u);
-            return;
-        }
-    }
-    bool stop = false;
-    if (rule == GLOBE_RULE_PCGSOLVER) {
-        const double small_b = (double)1e-12f;  // PCGsolver.cpp:1365, :1393
-        double mx = 0.0;
-        for (int j = 0; j < k; ++j) {
-            const double nb = sqrt(bb[j]);
-            const double u = unsc ? unsc[j] : 1.0;
-            const double q = nb > small_b ? sqrt(rr[j]) * u / nb : 0.0;
-            if (q > mx) mx = q;
-        }
-        if (mx < tol) {
-            st->status = 1;
-            stop = true;
-        } else {
-            const double last = st->last;
-            if (last - mx < (double)5e-3f * last) ++st->stag;
-            else st->stag = 0;
-            st->last = mx;
-            if (st->stag >= 10) {
-                st->status = 2;
-                stop = true;
-            }
-        }
-    } else {
-        bool all = true;
-        for (int j = 0; j < k; ++j)
-            if (bb[j] > 0.0 && !(sqrt(rr[j]) * (unsc ? unsc[j] : 1.0) < tol * sqrt(bb[j]))) {
-                all = false;
-                break;
-            }
-        if (all) {
-            st->status = 1;
-            stop = true;
-        }
-    }
-    if (!stop && it >= maxit) {
-        st->status = 3;
-        stop = true;
-    }
-    cudaGraphSetConditional(h, stop ? 0u : 1u);
-}
-
-// The end of a device-loop iteration, one launch: thread 0 applies the stopping rule
-// (pcg_check); every column c < k takes beta = r'z(new) / r'z(old) (0 where r'z(old) = 0, as
-// k_scal_div) and its double-float copy when beta_df is given, then r'z(old) = r'z(new).
-// The check reads r'r and p'Vp only, so the two parts are independent.
-__global__ void k_pcg_check_shift(const double* __restrict__ rr, const double* __restrict__ pvp,
-                                  const double* __restrict__ bb, const int32_t* __restrict__ cols, int kact, int k,
-                                  double tol, int rule, int maxit, const double* __restrict__ unsc, PcgLoopState* st,
-                                  cudaGraphConditionalHandle h, double* __restrict__ rz,
-                                  const double* __restrict__ rz2, double* __restrict__ beta,
-                                  float2* __restrict__ beta_df) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) pcg_check(rr, pvp, bb, cols, kact, k, tol, rule, maxit, unsc, st, h);
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < k) {
-        const double o = rz[c], nw = rz2[c];
-        const double bt = (o != 0.0) ? nw / o : 0.0;
-        beta[c] = bt;
-        if (beta_df) df::store(beta_df + c, df::from_double(bt));
-        rz[c] = nw;
-    }
-}
-
-// Build and run the loop graph; body(h) issues one iteration and its check on the stream.
+// Build and run the loop graph; body(h) issues one iteration with its check on the stream.
 // Returns GLOBE_OK with *ran = false (nothing run) when the graph cannot be built.
 template <class F>
 static int run_device_loop(globe_ctx* ctx, F&& body, int64_t* nlaunch, bool* ran) {
@@ -330,85 +249,74 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
     const int64_t n = c.Nrec;
     const int32_t N = c.N;
     GLOBE_RET(ensure_precond(ctx));
-    double *r, *z, *p, *Vp, *Zi, *GZ, *S1, *scal, *part;
+    double *r, *x, *p, *ind, *Zi, *GZ, *scal;
     int32_t* dcols;
     GLOBE_RET(ws(ctx, WS_R, (size_t)n * k, &r));
-    GLOBE_RET(ws(ctx, WS_Z, (size_t)n * k, &z));
+    GLOBE_RET(ws(ctx, WS_X, (size_t)n * k, &x));
     GLOBE_RET(ws(ctx, WS_P, (size_t)n * k, &p));
-    GLOBE_RET(ws(ctx, WS_VP, (size_t)n * k, &Vp));
+    GLOBE_RET(ws(ctx, WS_SOLVE, (size_t)5 * N * k, &ind));
     GLOBE_RET(ws(ctx, WS_ZI, (size_t)N * k, &Zi));
     GLOBE_RET(ws(ctx, WS_GZ, (size_t)N * k, &GZ));
-    GLOBE_RET(ws(ctx, WS_S1, (size_t)N * k, &S1));
-    GLOBE_RET(ws(ctx, WS_SCAL, (size_t)10 * k, &scal));
+    GLOBE_RET(ws(ctx, WS_SCAL, (size_t)9 * k, &scal));
     GLOBE_RET(ws(ctx, WS_COLS, (size_t)k, &dcols));
-    GLOBE_RET(ws(ctx, WS_PART, (size_t)std::max<int64_t>(div_up(N, 8), 304) * k * 2, &part));
     PcgLoopState* dstate;
     GLOBE_RET(ws(ctx, WS_LOOP, 1, &dstate));
-    const double* H = Hptr(ctx);
-    double* rz = scal;
-    double* rz2 = scal + k;
+    double* bb = scal;
+    double* rr = scal + k;
     double* pvp = scal + 2 * k;
-    double* alpha = scal + 3 * k;
-    double* beta = scal + 4 * k;
-    double* rr = scal + 5 * k;
-    double* bb = scal + 6 * k;
-    double* dunsc = scal + 7 * k;   // per-column unscale factors of a double-float solve
-    float2* alpha_df = reinterpret_cast<float2*>(scal + 8 * k);   // double-float copies of alpha, beta
-    float2* beta_df = reinterpret_cast<float2*>(scal + 9 * k);
+    double* dunsc = scal + 3 * k;   // per-column unscale factors of a double-float solve
     if ((size_t)4 * k > ctx->hpin_n) return set_err(ctx, GLOBE_ERR_ARG, "too many right-hand sides (%d)", k);
     double* h_rr = ctx->hpin;
     double* h_bb = ctx->hpin + k;
     double* h_pvp = ctx->hpin + 2 * k;
 
-    // Under GLOBE_PREC_MIXED the iterations run on double-float vectors (df_records_ok): x, r,
-    // z and p hold pairs, column c scaled by 1/unsc[c] (a power of two, col_unscale), and x is
-    // converted back when the loop ends, however it ends.  From x0 = 0 the set-up itself runs
-    // in double-float (r = b scaled, z = Q^-1 r); from another start point it runs in FP64 and
-    // x, r, z, p are converted in place.  r'z follows the scaling; the host and the device
-    // check unscale r'r exactly (sqrt(rr) unsc = sqrt(rr unsc^2)).
+    // Under GLOBE_PREC_MIXED the iterations run on double-float vectors (df_records_ok), column c
+    // scaled by 1/unsc[c] (a power of two, col_unscale); x is converted back when the loop ends,
+    // however it ends.  From a start point other than x0 = 0, r = b - V x0 is formed in FP64
+    // first.  r'z follows the scaling; the host and the device check unscale r'r exactly
+    // (sqrt(rr) unsc = sqrt(rr unsc^2)).
     const bool df = ctx->prec == GLOBE_PREC_MIXED && ctx->record_df && df_records_ok(ctx);
-    const bool df_setup = df && o->x0mode == GLOBE_X0_ZERO;
-    float2* Hdf = reinterpret_cast<float2*>(ctx->ws[WS_HDF].p);
-    float2* S0df = nullptr;
-    if (df) GLOBE_RET(ws(ctx, WS_S0DF, (size_t)N * k, &S0df));
-    auto F = [](double* v) { return reinterpret_cast<float2*>(v); };
+    SolveVecs sv;
+    sv.df = df;
+    sv.k = k;
+    sv.cols = dcols;
+    sv.x = x;
+    sv.r = r;
+    sv.p = p;
+    sv.ind = ind;
+    sv.alpha = scal + 4 * k;
+    sv.beta = scal + 5 * k;
+    sv.rz = scal + 6 * k;           // and 2 k entries of scratch
+    sv.pvp = pvp;
+    sv.rr = rr;
+    sv.unsc = df ? dunsc : nullptr;
 
     GLOBE_RET(col_dots(ctx, B, B, n, n, n, nullptr, k, bb));
     if (df) GLOBE_RET(col_unscales(ctx, bb, k, dunsc));
-    switch (o->x0mode) {
-        case GLOBE_X0_ZERO:
-            GLOBE_CK(ctx, cudaMemsetAsync(X, 0, sizeof(double) * n * k, ctx->stream));
-            if (df_setup) {
-                DfCols v;
-                v.src[0] = B;
-                v.dst[0] = r;
-                GLOBE_RET(cols_to_df(ctx, v, n, k, dunsc, nullptr));
-            } else {
-                GLOBE_CK(ctx, cudaMemcpyAsync(r, B, sizeof(double) * n * k, cudaMemcpyDeviceToDevice, ctx->stream));
-            }
-            break;
-        case GLOBE_X0_PRECOND:
-            GLOBE_RET(precond_apply(ctx, H, B, X, nullptr, k, nullptr));
-            GLOBE_RET(vx_dev(ctx, X, k, Vp));
-            GLOBE_RET(sub_vec(ctx, B, Vp, r, n * k));
-            break;
-        case GLOBE_X0_GIVEN:
-            GLOBE_RET(vx_dev(ctx, X, k, Vp));
-            GLOBE_RET(sub_vec(ctx, B, Vp, r, n * k));
-            break;
-        default:
-            return set_err(ctx, GLOBE_ERR_ARG, "unknown x0 mode %d", o->x0mode);
+    const bool from_zero = o->x0mode == GLOBE_X0_ZERO;
+    if (o->x0mode == GLOBE_X0_PRECOND) GLOBE_RET(precond_apply(ctx, Hptr(ctx), B, X, k));
+    else if (!from_zero && o->x0mode != GLOBE_X0_GIVEN)
+        return set_err(ctx, GLOBE_ERR_ARG, "unknown x0 mode %d", o->x0mode);
+    if (from_zero) {
+        GLOBE_CK(ctx, cudaMemsetAsync(x, 0, sizeof(double) * n * k, ctx->stream));
+        GLOBE_RET(solve_load(ctx, sv, B, r));
+    } else {
+        double* v0;
+        GLOBE_RET(ws(ctx, WS_VP, (size_t)n * k, &v0));
+        GLOBE_RET(vx_dev(ctx, X, k, v0));
+        GLOBE_RET(sub_vec(ctx, B, v0, v0, n * k));
+        GLOBE_RET(col_dots(ctx, v0, v0, n, n, n, nullptr, k, rr));
+        GLOBE_RET(solve_load(ctx, sv, v0, r));
+        GLOBE_RET(solve_load(ctx, sv, X, x));
     }
-    if (df_setup) GLOBE_RET(precond_apply_df(ctx, Hdf, F(r), F(z), k, rz));
-    else GLOBE_RET(precond_apply(ctx, H, r, z, nullptr, k, rz));
-    GLOBE_CK(ctx, cudaMemcpyAsync(p, z, sizeof(double) * n * k, cudaMemcpyDeviceToDevice, ctx->stream));
+    // columns that never enter the loop keep alpha = 0
+    GLOBE_CK(ctx, cudaMemsetAsync(sv.alpha, 0, sizeof(double) * k, ctx->stream));
+    GLOBE_RET(solve_init(ctx, sv));
     // from x0 = 0, r = b: r'r is b'b (the same kernel on the same values)
-    const bool r_is_b = o->x0mode == GLOBE_X0_ZERO;
-    if (!r_is_b) GLOBE_RET(col_dots(ctx, r, r, n, n, n, nullptr, k, rr));
     GLOBE_CK(ctx, cudaMemcpyAsync(h_bb, bb, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
-    if (!r_is_b) GLOBE_CK(ctx, cudaMemcpyAsync(h_rr, rr, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
+    if (!from_zero) GLOBE_CK(ctx, cudaMemcpyAsync(h_rr, rr, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
     GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    if (r_is_b) std::copy(h_bb, h_bb + k, h_rr);
+    if (from_zero) std::copy(h_bb, h_bb + k, h_rr);
 
     std::vector<double> nb(k), nr(k);
     for (int j = 0; j < k; ++j) {
@@ -429,33 +337,27 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
     std::vector<int32_t> cols;
     for (int j = 0; j < k; ++j)
         if (h_bb[j] > 0.0) cols.push_back(j);
-        else GLOBE_CK(ctx, cudaMemsetAsync(X + (size_t)j * n, 0, sizeof(double) * n, ctx->stream));
 
     std::vector<double> unsc(k, 1.0);
     if (df) {
         for (int j = 0; j < k; ++j) unsc[j] = col_unscale(h_bb[j]);
-        if (!df_setup) {   // x, r, z, p to double-float in place; r'z scaled with them
-            DfCols v;
-            double* vv[4] = {X, r, z, p};
-            for (int j = 0; j < 4; ++j) v.src[j] = v.dst[j] = vv[j];
-            GLOBE_RET(cols_to_df(ctx, v, n, k, dunsc, rz));
-        }
         ctx->record_df_runs += 1;
     }
-    // one iteration on the stream: the operator on p, alpha, and the updates up to r'r and r'z
-    auto iteration = [&](bool first, int kc) -> int {
-        if (df) {
-            GLOBE_RET(seg_sums_df(ctx, F(p), first ? nullptr : F(z), first ? nullptr : beta_df, dcols, kc, Zi, S0df,
-                                  F(S1)));
-            GLOBE_RET(grm_apply_dev(ctx, Zi, kc, GZ));
-            GLOBE_RET(vx_assemble_df(ctx, F(p), GZ, S0df, F(S1), dcols, kc, F(Vp), pvp, rz, alpha, alpha_df));
-            return pcg_update_df(ctx, Hdf, alpha_df, F(X), F(r), F(p), F(Vp), F(z), dcols, kc, rr, rz2);
+    // one iteration on the stream (k_solve.cu); with loop, its last kernel applies the stopping rule
+    bool pending = false;   // x lacks the last iteration's alpha p
+    auto iteration = [&](bool first, int kc, const PcgLoop& loop) -> int {
+        unsigned* zhi = nullptr;
+        if (grm_wants_zhi(ctx, kc)) {
+            TcStat st;
+            GLOBE_RET(tc_stat(ctx, kc, &st));
+            zhi = st.zhi;
+            ctx->stat_dirty = true;   // until the product has cleared the words again
         }
-        if (!first) GLOBE_RET(seg_sums(ctx, p, z, beta, p, dcols, kc, Zi, S1));
-        else GLOBE_RET(seg_sums(ctx, p, nullptr, nullptr, nullptr, dcols, kc, Zi, S1));
-        GLOBE_RET(grm_apply_dev(ctx, Zi, kc, GZ));
-        GLOBE_RET(vx_assemble(ctx, p, GZ, Zi, S1, dcols, kc, Vp, pvp, rz, alpha));   // alpha = r'z / p'Vp
-        return pcg_update(ctx, H, alpha, X, r, p, Vp, z, dcols, kc, rr, rz2);
+        GLOBE_RET(solve_dir(ctx, sv, kc, first, Zi, zhi));
+        GLOBE_RET(grm_apply_dev(ctx, Zi, kc, GZ, zhi != nullptr));
+        GLOBE_RET(solve_step(ctx, sv, kc, GZ));
+        pending = true;
+        return solve_update(ctx, sv, kc, loop);
     };
 
     std::vector<int32_t> uploaded;
@@ -466,8 +368,8 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
     int64_t rhs_iters = 0;
     if (cols.empty()) converged = true;
     bool use_graph = ctx->graphs && !ctx->prof_on;   // profiling times each pass with events
-    std::vector<int32_t> gcols[2];                   // column set each graph was captured for
-    int64_t glaunch[2] = {0, 0};                     // kernels per replay
+    std::vector<int32_t> gcols;                      // column set the graph was captured for
+    int64_t glaunch = 0;                             // kernels per replay
     auto iterate = [&]() -> int {
         for (it = 0; it < o->maxit && !cols.empty(); ++it) {
             const int kact = (int)cols.size();
@@ -479,25 +381,24 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
             }
             // the iteration's stream work, up to the copies of the two k-vectors the host checks
             auto body = [&](bool first) -> int {
-                GLOBE_RET(iteration(first, kact));
+                GLOBE_RET(iteration(first, kact, PcgLoop()));
                 GLOBE_CK(ctx, cudaMemcpyAsync(h_rr, rr, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
                 GLOBE_CK(ctx, cudaMemcpyAsync(h_pvp, pvp, sizeof(double) * k, cudaMemcpyDeviceToHost, ctx->stream));
                 return GLOBE_OK;
             };
             // The first iteration runs directly (it also builds what the products make on first
-            // use).  Later ones replay a graph of the body, captured once per call, parity of the
-            // swapped r'z buffers and column set; a failed capture falls back to direct launches.
+            // use).  Later ones replay a graph of the body, captured once per call and column set; a
+            // failed capture falls back to direct launches.
             bool ran = false;
             if (it > 0 && use_graph) {
-                const int slot = rz == scal ? 0 : 1;
-                if (gcols[slot] != cols) {
-                    gcols[slot].clear();
-                    if (capture_body(ctx, slot, [&]() { return body(false); }, &glaunch[slot])) gcols[slot] = cols;
+                if (gcols != cols) {
+                    gcols.clear();
+                    if (capture_body(ctx, [&]() { return body(false); }, &glaunch)) gcols = cols;
                     else use_graph = false;
                 }
                 if (use_graph) {
-                    GLOBE_CK(ctx, cudaGraphLaunch(ctx->pcg_graph[slot], ctx->stream));
-                    ctx->launches += glaunch[slot];
+                    GLOBE_CK(ctx, cudaGraphLaunch(ctx->pcg_graph, ctx->stream));
+                    ctx->launches += glaunch;
                     ran = true;
                 }
             }
@@ -531,8 +432,6 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
                 if (keep.empty()) { converged = true; ++it; break; }
                 cols.swap(keep);
             }
-            GLOBE_RET(scal_alpha(ctx, rz2, rz, beta, k, df ? beta_df : nullptr));
-            std::swap(rz, rz2);
             // after the first iteration, the rest as one device-side loop (no per-iteration
             // synchronisation) when graphs are on and the column set cannot change
             if (it == 0 && use_graph && ctx->device_loop && !o->mask && o->maxit > 1) {
@@ -540,12 +439,16 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
                 GLOBE_CK(ctx, cudaMemcpyAsync(dstate, &st0, sizeof st0, cudaMemcpyHostToDevice, ctx->stream));
                 const int kc = kact;
                 auto loop_body = [&](cudaGraphConditionalHandle h) -> int {
-                    GLOBE_RET(iteration(false, kc));
-                    k_pcg_check_shift<<<div_up(k, 128), 128, 0, ctx->stream>>>(
-                        rr, pvp, bb, dcols, kc, k, o->tol, o->rule, o->maxit, df ? dunsc : nullptr, dstate, h, rz, rz2,
-                        beta, df ? beta_df : nullptr);
-                    GLOBE_LAUNCHED(ctx, "k_pcg_check_shift");
-                    return GLOBE_OK;
+                    PcgLoop loop;
+                    loop.st = dstate;
+                    loop.h = h;
+                    loop.tol = o->tol;
+                    loop.rule = o->rule;
+                    loop.maxit = o->maxit;
+                    loop.k = k;
+                    loop.bb = bb;
+                    loop.unsc = sv.unsc;
+                    return iteration(false, kc, loop);
                 };
                 int64_t per_it = 0;
                 bool ran = false;
@@ -578,9 +481,12 @@ static int pcg_run(globe_ctx* ctx, const double* B, double* X, int k, const glob
         return GLOBE_OK;
     };
     const int rc = iterate();
-    if (df) {   // x back to FP64, whatever ended the loop (an earlier error's message is kept)
+    {   // x with its last step, to X, whatever ended the loop (an earlier error's message is kept)
         const std::string e0 = ctx->err;
-        const int rc2 = cols_from_df(ctx, X, n, k, dunsc);
+        int rc2 = solve_store(ctx, sv, pending, X);
+        for (int j = 0; j < k && rc2 == GLOBE_OK; ++j)
+            if (!(h_bb[j] > 0.0) && cudaMemsetAsync(X + (size_t)j * n, 0, sizeof(double) * n, ctx->stream) != cudaSuccess)
+                rc2 = set_err(ctx, GLOBE_ERR_CUDA, "clearing a zero column");
         if (rc != GLOBE_OK) ctx->err = e0;
         else if (rc2 != GLOBE_OK) return rc2;
     }
@@ -710,7 +616,7 @@ int globe_precond_apply(globe_ctx* ctx, const double* r, double* z, int k) {
     GLOBE_RET(ensure_precond(ctx));
     size_t n = (size_t)ctx->coh.Nrec * k;
     return host_io(ctx, r, n, z, n, [&](double* a, double* b) {
-        return precond_apply(ctx, (const double*)ctx->ws[WS_H].p, a, b, nullptr, k, nullptr);
+        return precond_apply(ctx, (const double*)ctx->ws[WS_H].p, a, b, k);
     });
 }
 
@@ -803,7 +709,7 @@ static int mme_finish(globe_ctx* ctx, double* beta, double* uhat, double* bhat, 
     GLOBE_RET(ws(ctx, WS_ZI, (size_t)N, &Zi));
     GLOBE_RET(ws(ctx, WS_S1, (size_t)N, &S1));
     if (with_uhat) {
-        GLOBE_RET(seg_sums(ctx, ctx->vinv_r, nullptr, nullptr, nullptr, nullptr, 1, Zi, S1));
+        GLOBE_RET(seg_sums(ctx, ctx->vinv_r, 1, Zi, S1));
         GLOBE_RET(grm_apply_dev(ctx, Zi, 1, ctx->uhat));
     }
     GLOBE_RET(ws(ctx, WS_BHAT, (size_t)2 * N, &dbhat));
@@ -871,7 +777,7 @@ static int grad_probes(globe_ctx* ctx, const double* probes, int numMC, uint64_t
     }
     // V*^-1 Y by the Woodbury block inverse with g = sig2g (varCompEst.cpp:839-862)
     GLOBE_RET(build_H(ctx, nullptr, ctx->vc[1], pb.Hs));
-    GLOBE_RET(precond_apply(ctx, pb.Hs, pb.Y, pb.TY, nullptr, numMC, nullptr));
+    GLOBE_RET(precond_apply(ctx, pb.Hs, pb.Y, pb.TY, numMC));
     return GLOBE_OK;
 }
 
@@ -894,13 +800,13 @@ static int grad_finish(globe_ctx* ctx, int numMC, const double* VY, const ProbeB
     if (with_uhat) {
         GLOBE_CK(ctx, cudaMemcpyAsync(pb.VR0, ctx->vinv_r, sizeof(double) * n, cudaMemcpyDeviceToDevice,
                                       ctx->stream));
-        GLOBE_RET(seg_sums(ctx, pb.VR0, nullptr, nullptr, nullptr, nullptr, numMC + 1, Zi, S1));
+        GLOBE_RET(seg_sums(ctx, pb.VR0, numMC + 1, Zi, S1));
         GLOBE_RET(grm_apply_dev(ctx, Zi, numMC + 1, pb.UH0));
         GLOBE_CK(ctx, cudaMemcpyAsync(ctx->uhat, pb.UH0, sizeof(double) * N, cudaMemcpyDeviceToDevice,
                                       ctx->stream));
         ctx->mme_ok = true;
     } else {
-        GLOBE_RET(seg_sums(ctx, pb.VR, nullptr, nullptr, nullptr, nullptr, numMC, Zi, S1));
+        GLOBE_RET(seg_sums(ctx, pb.VR, numMC, Zi, S1));
         GLOBE_RET(grm_apply_dev(ctx, Zi, numMC, pb.UH));
     }
     GLOBE_RET(ftheta_kernel(ctx, ctx->vinv_r, ctx->uhat, fth));
@@ -971,7 +877,7 @@ static int aireml_eval_impl(globe_ctx* ctx, const double* probes, int numMC, uin
     GLOBE_CK(ctx, cudaMemcpyAsync(FB + (size_t)n * k, pb.Y, sizeof(double) * n * numMC, cudaMemcpyDeviceToDevice,
                                   ctx->stream));
     GLOBE_RET(ensure_precond(ctx));
-    GLOBE_RET(precond_apply(ctx, Hptr(ctx), FB, FX, nullptr, k, nullptr));
+    GLOBE_RET(precond_apply(ctx, Hptr(ctx), FB, FX, k));
     GLOBE_CK(ctx, cudaMemcpyAsync(FX + (size_t)n * k, pb.TY, sizeof(double) * n * numMC, cudaMemcpyDeviceToDevice,
                                   ctx->stream));
     globe_pcg_opts o = *opts;

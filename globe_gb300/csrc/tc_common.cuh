@@ -186,15 +186,17 @@ __device__ __forceinline__ int col_exp(unsigned hi) {
     return col_bad(hi) ? 0 : (ND == ND64 ? e : max(e, -983));
 }
 
-// CTAs per column of k_col_max and the rows each thread of a combine kernel takes: ~8 and ~4
-// values per thread
+// CTAs per column of k_col_max: ~8 values per thread
 __host__ __forceinline__ int col_parts(int64_t n) {
     const int64_t p = (n + 2047) / 2048;
     return (int)(p < 1 ? 1 : (p > 304 ? 304 : p));
 }
-constexpr int COMBINE_PARTS = 304;   // CTAs per column of a combine kernel at most (2 per SM)
+// CTAs per column of a combine kernel: a row per thread up to 32768 rows (a chain of four costs a
+// small product more than the extra sums do), then ~4; at most 2 per SM.  It depends on the rows
+// only, so a column's sums have one order whatever its group.
+constexpr int COMBINE_PARTS = 304;
 __host__ __forceinline__ int combine_parts(int64_t n) {
-    const int64_t p = (n + 1023) / 1024;
+    const int64_t p = n <= 32768 ? (n + 255) / 256 : std::max<int64_t>(128, (n + 1023) / 1024);
     return (int)(p < 1 ? 1 : (p > COMBINE_PARTS ? COMBINE_PARTS : p));
 }
 
