@@ -18,7 +18,9 @@
 // column) pair with the columns of an individual on neighbouring threads: a warp reads whole
 // runs of an individual's records, whatever the number of columns.  Individuals are taken in order
 // of their record counts (Cohort::order), so the threads of a warp walk equally many records; the
-// ones of more than SOLVE_HUGE records (order's first) are walked by a CTA each.  The kernels are
+// ones of more than SOLVE_LONG records (order's first) are walked by all individuals' threads of a
+// CTA together, in CTAs of their own: one thread's walk is a chain of loads and FP64 sums that
+// outlasts the rest (N = 20k with up to 94 records each, FP64: k_update 78 us).  The kernels are
 // bound by the vectors' transfers (in double-float) or by the FP64 pipe (~16 operations a record
 // and column; in FP64).
 //
@@ -41,7 +43,8 @@ constexpr int ST = 288;            // threads per CTA at most
 // k_update: more of either was slower (k_update with 4 records and 3 CTAs: 60 against 53 us at
 // N = 100k, k = 5, 255 against 204 us at N = 50k, k = 65; k_dir with 2 and 4: 153 and 38 against
 // 158 and 36 us), and so was keeping an individual's r and t in registers for k_update's second
-// pass over them (83 us: 2 CTAs).
+// pass over them (83 us: 2 CTAs).  With at most two CTAs an SM to run, where a chain of loads is
+// what counts, k_update takes 4 records at a time.
 constexpr int RU_DIR = 4, RU_UPD = 2, RES_DIR = 3, RES_UPD = 4;
 // CTAs per SM launched at most: k_dir's take two turns, the kernels that end in column sums one
 // (fewer partials)
@@ -87,14 +90,14 @@ struct Args {
     const typename A::S *t, *H;
     const int4* order;               // {block, first record, one past its last, individual} (Cohort::order)
     const int32_t *bind, *cols;
-    int32_t N, nhuge;
+    int32_t N, nlong;
     int64_t Nrec;
     int k, kact, kc, ti;             // columns; active ones; columns per tile, individuals per CTA step
     typename A::V e, inv_e, b0, b01, b1;
     typename A::S *alpha, *beta;     // converted once, where they are formed
     double *rz, *pvp, *rr;
     double* part;
-    int slots;                       // partials per column (CTAs of the huge and of the main launch)
+    int slots, hctas;                // partials per column: CTAs; of them, those that walk the long individuals
     unsigned* cnt;                   // arrival counts, zero between launches: per tile its groups' and
     unsigned* tiles_done;            // the groups' (sum_last); of the tiles
 };
@@ -136,22 +139,20 @@ __device__ __forceinline__ T over_individuals(T v, T* sm, int ti, int kc, int il
 
 // ---- k_dir -----------------------------------------------------------------------
 
+// individuals g0, g0 + gs, ...; returns the largest abs_hi of the thread's sums
 template <class A, bool TEAM>
-__global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first, double* __restrict__ Zi, unsigned* zhi) {
+__device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, const bool first, int64_t g0, int gs,
+                                             typename A::V* sm, double* __restrict__ Zi) {
     using V = typename A::V;
     constexpr int RU = RU_DIR;
-    __shared__ V sm[TEAM ? ST : 1];
-    __shared__ unsigned smu[ST];
-    const Lane l = lane_of(a);
-    const int nidx = TEAM ? a.nhuge : a.N;
-    smu[threadIdx.x] = 0u;
+    const int nidx = TEAM ? a.nlong : a.N;
     const V inv_e = a.inv_e, al = l.on && !first ? A::load(a.alpha + l.col) : A::zero(),
             be = l.on && !first ? A::load(a.beta + l.col) : A::zero();
     const int step = TEAM ? a.ti : 1;
     unsigned m = 0;
-    for (int64_t g = blockIdx.x;; g += gridDim.x) {
-        const int64_t idx = TEAM ? g : a.nhuge + g * a.ti + l.il;
-        if ((TEAM ? g : a.nhuge + g * a.ti) >= nidx) break;   // uniform over the CTA
+    for (int64_t g = g0;; g += gs) {
+        const int64_t idx = TEAM ? g : a.nlong + g * a.ti + l.il;
+        if ((TEAM ? g : a.nlong + g * a.ti) >= nidx) break;   // uniform over the CTA
         V s0 = A::zero(), s1 = A::zero(), pp = A::zero();
         int b = 0, i = 0;
         bool in = l.on && idx < nidx;
@@ -215,6 +216,18 @@ __global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first
             m = max(m, tc::abs_hi(z));
         }
     }
+    return m;
+}
+
+template <class A>
+__global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first, double* __restrict__ Zi, unsigned* zhi) {
+    __shared__ typename A::V sm[ST];
+    __shared__ unsigned smu[ST];
+    const Lane l = lane_of(a);
+    smu[threadIdx.x] = 0u;
+    const int x = blockIdx.x;
+    const unsigned m = x < a.hctas ? dir_walk<A, true>(a, l, first, x, a.hctas, sm, Zi)
+                                   : dir_walk<A, false>(a, l, first, x - a.hctas, (int)gridDim.x - a.hctas, sm, Zi);
     if (zhi) {   // the scale of the product's input (k_col_max's part)
         __syncthreads();
         const int cl = threadIdx.x - l.il * a.kc;
@@ -417,20 +430,19 @@ __device__ void pcg_check(const PcgLoop& p, const double* rr, const double* pvp,
 
 // ---- k_update ---------------------------------------------------------------------
 
-// INIT: r stays (the solve's start): g, r'z only, and no beta
-template <class A, bool TEAM, bool INIT>
-__global__ void __launch_bounds__(ST, RES_UPD) k_update(Args<A> a, int slot0, PcgLoop loop) {
+// individuals g0, g0 + gs, ...: |r|^2 and r'z of the thread's records.  INIT: r stays (the solve's
+// start): g and r'z only
+template <class A, bool TEAM, bool INIT, int RU>
+__device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int64_t g0, int gs, typename A::V* sm,
+                                            typename A::V& rr, typename A::V& rz) {
     using V = typename A::V;
-    constexpr int RU = RU_UPD;
-    __shared__ V sm[TEAM ? ST : 1];
-    const Lane l = lane_of(a);
-    const int nidx = TEAM ? a.nhuge : a.N;
+    const int nidx = TEAM ? a.nlong : a.N;
     const V inv_e = a.inv_e, e = a.e, na = INIT || !l.on ? A::zero() : A::neg(A::load(a.alpha + l.col));
     const int step = TEAM ? a.ti : 1;
-    V rr = A::zero(), rz = A::zero();
-    for (int64_t g = blockIdx.x;; g += gridDim.x) {
-        const int64_t idx = TEAM ? g : a.nhuge + g * a.ti + l.il;
-        if ((TEAM ? g : a.nhuge + g * a.ti) >= nidx) break;   // uniform over the CTA
+    rr = rz = A::zero();
+    for (int64_t g = g0;; g += gs) {
+        const int64_t idx = TEAM ? g : a.nlong + g * a.ti + l.il;
+        if ((TEAM ? g : a.nlong + g * a.ti) >= nidx) break;   // uniform over the CTA
         int b = 0, st = 0, en = 0;
         V s0 = A::zero(), s1 = A::zero(), a0 = A::zero(), a1 = A::zero();
         bool in = l.on && idx < nidx;
@@ -513,10 +525,21 @@ __global__ void __launch_bounds__(ST, RES_UPD) k_update(Args<A> a, int slot0, Pc
             }
         }
     }
+}
+
+template <class A, bool INIT, int RU>
+__global__ void __launch_bounds__(ST, RU == RU_UPD ? RES_UPD : 2) k_update(Args<A> a, PcgLoop loop) {
+    using V = typename A::V;
+    __shared__ V sm[ST];
+    const Lane l = lane_of(a);
+    const int x = blockIdx.x;
+    V rr, rz;
+    if (x < a.hctas) update_walk<A, true, INIT, RU>(a, l, x, a.hctas, sm, rr, rz);
+    else update_walk<A, false, INIT, RU>(a, l, x - a.hctas, (int)gridDim.x - a.hctas, sm, rr, rz);
     const V v[2] = {rz, rr};
     // r'z (new) lands in rz's second half (k entries), |r|^2 in rr
     double* rz2 = a.rz + a.k;
-    if (!sum_last<2>(a, l, v, slot0 + blockIdx.x, rz2, INIT ? rz2 + a.k : a.rr)) return;
+    if (!sum_last<2>(a, l, v, blockIdx.x, rz2, INIT ? rz2 + a.k : a.rr)) return;
     if (threadIdx.x < a.kc) {
         const int c = blockIdx.y * a.kc + threadIdx.x;
         if (c < a.kact) {
@@ -626,7 +649,7 @@ static Shape shape(const globe_ctx* ctx, int kact, int n, int per_sm) {
     s.threads = div_up(s.ti * s.kc, 32) * 32;
     const int most = std::max(1, per_sm * 152 / s.tiles);
     s.ctas = std::max(1, std::min(most, div_up(n, s.ti)));
-    s.huge = std::min(most, (int)ctx->coh.nhuge);
+    s.huge = std::min(std::max(1, 2 * 152 / s.tiles), (int)ctx->coh.nlong_solve);
     return s;
 }
 
@@ -650,7 +673,7 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
     a.order = c.order;
     a.cols = v.cols;
     a.N = c.N;
-    a.nhuge = c.nhuge;
+    a.nlong = c.nlong_solve;
     a.Nrec = c.Nrec;
     a.k = v.k;
     a.kact = kact;
@@ -667,7 +690,8 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
     a.pvp = v.pvp;
     a.rr = v.rr;
     a.slots = s.ctas + s.huge;
-    const size_t most = 2 * PER_SUM * 152 + 1, groups = most / 32 + 1;   // for any number of active columns
+    a.hctas = s.huge;
+    const size_t most = (PER_SUM + 2) * 152 + 2, groups = most / 32 + 1;   // for any number of active columns
     GLOBE_RET(ws(ctx, WS_PART, (most + groups) * 2 * v.k, &a.part));
     GLOBE_RET(tc_counters(ctx, (size_t)div_up(v.k, 128) * (groups + 1) + 1, &a.tiles_done));
     a.cnt = a.tiles_done + 1;
@@ -677,14 +701,10 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
 
 template <class A>
 static int dir(globe_ctx* ctx, const SolveVecs& v, int kact, bool first, double* Zi, unsigned* zhi) {
-    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nhuge, PER_DIR);
+    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nlong_solve, PER_DIR);
     Args<A> a;
     GLOBE_RET(args(ctx, v, kact, s, &a));
-    if (s.huge) {
-        k_dir<A, true><<<dim3(s.huge, s.tiles), s.threads, 0, ctx->stream>>>(a, first, Zi, zhi);
-        GLOBE_LAUNCHED(ctx, "k_dir");
-    }
-    k_dir<A, false><<<dim3(s.ctas, s.tiles), s.threads, 0, ctx->stream>>>(a, first, Zi, zhi);
+    k_dir<A><<<dim3(s.ctas + s.huge, s.tiles), s.threads, 0, ctx->stream>>>(a, first, Zi, zhi);
     GLOBE_LAUNCHED(ctx, "k_dir");
     return GLOBE_OK;
 }
@@ -702,14 +722,12 @@ static int step(globe_ctx* ctx, const SolveVecs& v, int kact, const double* GZ) 
 
 template <class A, bool INIT>
 static int update(globe_ctx* ctx, const SolveVecs& v, int kact, const PcgLoop& loop) {
-    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nhuge, PER_SUM);
+    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nlong_solve, PER_SUM);
     Args<A> a;
     GLOBE_RET(args(ctx, v, kact, s, &a));
-    if (s.huge) {
-        k_update<A, true, INIT><<<dim3(s.huge, s.tiles), s.threads, 0, ctx->stream>>>(a, 0, PcgLoop());
-        GLOBE_LAUNCHED(ctx, "k_update");
-    }
-    k_update<A, false, INIT><<<dim3(s.ctas, s.tiles), s.threads, 0, ctx->stream>>>(a, s.huge, loop);
+    const dim3 grid(s.ctas + s.huge, s.tiles);
+    if (grid.x * grid.y <= 2 * 152) k_update<A, INIT, 4><<<grid, s.threads, 0, ctx->stream>>>(a, loop);
+    else k_update<A, INIT, RU_UPD><<<grid, s.threads, 0, ctx->stream>>>(a, loop);
     GLOBE_LAUNCHED(ctx, "k_update");
     return GLOBE_OK;
 }

@@ -37,6 +37,7 @@
 // Every mbarrier wait is bounded; on timeout the CTA records an error bit, waits
 // (bounded) for its issued copies / MMAs and frees TMEM.
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "tc_ptx.cuh"
@@ -260,28 +261,30 @@ __global__ void __launch_bounds__(256) k_dense_digits(const float* __restrict__ 
 
 // out[i,c] = sA 2^e_c sum_{d,j} 32^-(d+j) P[plane d, digit j](i,c), sA = scale 2^eA.  Each
 // split partial is an exact integer in FP32; they are summed in int64 by total weight
-// s = d + j (T_s, |T_s| <= 7 * 256 N), and the weights folded in three exact int64 chunks of
-// five (C_q = sum_{s=5q}^{5q+4} 32^(5q+4-s) T_s, |C_q| < 2^31 N): three conversions and two
-// FP64 additions per value instead of a recombination per plane.
-template <int ND>
-__global__ void k_dense_combine(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int32_t N,
-                                int64_t np, int da, const double* __restrict__ colinfo, double sA,
-                                double* __restrict__ out, int64_t ldo, unsigned* __restrict__ zhi) {
-    constexpr int NT = DA_MAX + ND - 1;
-    static_assert(NT <= 15, "three chunks of five weights");
-    const int c = blockIdx.y;
-    if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;   // cleared for the next product
-    const double s0 = sA * pow2i((int)colinfo[2 * c] - 20);   // 2^(e_c - 5*4) for chunk 0
-    const bool bad = isnan(colinfo[2 * c + 1]);   // a non-finite column: NaN out
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        long long T[NT];
+// s = d + j (T_s, |T_s| <= 12 * 256 N), and the weights folded in exact int64 chunks of
+// five (C_q = sum_{s=5q}^{5q+4} 32^(5q+4-s) T_s, |C_q| < 2^31 N): a conversion and an FP64 addition
+// per chunk instead of a recombination per plane.  With G = 4, four threads in warps of their own
+// share an output: each sums DG planes, and the first adds the others' weights up through shared
+// memory.  That shortens the chain of loads where few CTAs run (6007 x 5 in FP64: 18.9 -> 13.4
+// us), and costs where many do (20k x 16 mixed: 24.6 -> 36.9 us), so it is taken up to
+// DC_SPLIT_CTAS CTAs of one thread per output.
+constexpr int DC_SPLIT_CTAS = 2 * 152;
+
+// T_0 .. T_{DA + ND - 2} of output i, column c, in the first 256 / G threads; every thread calls it
+template <int DA, int ND, int G>
+__device__ __forceinline__ void dense_weights(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                              int64_t np, int da, int64_t i, bool in, int c, long long (&T)[DA + ND - 1]) {
+    constexpr int DG = (DA + G - 1) / G, NW = DG + ND - 1, DC_I = 256 / G;
+    __shared__ long long sm[G > 1 ? G - 1 : 1][G > 1 ? NW : 1][DC_I];
+    const int pg = threadIdx.x / DC_I, il = threadIdx.x % DC_I;
+    long long w[NW];
 #pragma unroll
-        for (int q = 0; q < NT; ++q) T[q] = 0;
-        // per plane: the ND digit loads of split 0 issued together, further splits after
+    for (int q = 0; q < NW; ++q) w[q] = 0;
+    if (in) {
 #pragma unroll
-        for (int d = 0; d < DA_MAX; ++d) {
-            if (d < da) {
-                const float* src = part + (int64_t)c * ND * ldp + (int64_t)d * np + i;
+        for (int d = 0; d < DG; ++d) {
+            if (pg * DG + d < da) {   // the ND digit loads of split 0 issued together, further splits after
+                const float* src = part + (int64_t)c * ND * ldp + (int64_t)(pg * DG + d) * np + i;
                 long long pj[ND];
 #pragma unroll
                 for (int j = 0; j < ND; ++j) pj[j] = (long long)__float2int_rn(src[(int64_t)j * ldp]);
@@ -291,21 +294,55 @@ __global__ void k_dense_combine(const float* __restrict__ part, int nsplit, int 
                         pj[j] += (long long)__float2int_rn(src[((int64_t)y * nmma + j) * ldp]);
                 }
 #pragma unroll
-                for (int j = 0; j < ND; ++j) T[d + j] += pj[j];
+                for (int j = 0; j < ND; ++j) w[d + j] += pj[j];
             }
         }
-        long long C[3] = {0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-            for (int m = 0; m < 5; ++m) C[q] = C[q] * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
-        const double v = s0 * (ll_times_pow2(C[0], 1.0) + ll_times_pow2(C[1], 0x1p-25) + ll_times_pow2(C[2], 0x1p-50));
-        out[i + c * ldo] = bad ? colinfo[2 * c + 1] : v;
     }
+    if constexpr (G > 1) {
+        if (pg > 0) {
+#pragma unroll
+            for (int q = 0; q < NW; ++q) sm[pg - 1][q][il] = w[q];
+        }
+        __syncthreads();
+        if (pg > 0) return;
+    }
+#pragma unroll
+    for (int q = 0; q < DA + ND - 1; ++q) T[q] = q < NW ? w[q] : 0;
+#pragma unroll
+    for (int g = 1; g < G; ++g)
+#pragma unroll
+        for (int q = 0; q < NW; ++q)
+            if (g * DG + q < DA + ND - 1) T[g * DG + q] += sm[g - 1][q][il];
 }
 
-// The FP64 product's epilogue: as k_dense_combine, with DA64 + ND64 - 1 = 23 weights in five
-// exact chunks (|C_q| < 2^31 N), added in double-double, and 2^e_c in two factors.
+template <int ND, int G>
+__global__ void __launch_bounds__(256) k_dense_combine(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
+                                                       int32_t N, int64_t np, int da, const double* __restrict__ colinfo,
+                                                       double sA, double* __restrict__ out, int64_t ldo,
+                                                       unsigned* __restrict__ zhi) {
+    constexpr int NT = DA_MAX + ND - 1;
+    static_assert(NT <= 15, "three chunks of five weights");
+    const int c = blockIdx.y;
+    constexpr int DC_I = 256 / G;
+    const int64_t i = (int64_t)blockIdx.x * DC_I + threadIdx.x % DC_I;
+    if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;   // cleared for the next product
+    long long T[NT];
+    dense_weights<DA_MAX, ND, G>(part, nsplit, nmma, ldp, np, da, i, i < N, c, T);
+    if (threadIdx.x >= DC_I || i >= N) return;
+    const double s0 = sA * pow2i((int)colinfo[2 * c] - 20);   // 2^(e_c - 5*4) for chunk 0
+    const bool bad = isnan(colinfo[2 * c + 1]);   // a non-finite column: NaN out
+    long long C[3] = {0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+        for (int m = 0; m < 5; ++m) C[q] = C[q] * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
+    const double v = s0 * (ll_times_pow2(C[0], 1.0) + ll_times_pow2(C[1], 0x1p-25) + ll_times_pow2(C[2], 0x1p-50));
+    out[i + c * ldo] = bad ? colinfo[2 * c + 1] : v;
+}
+
+// The FP64 product's epilogue: DA64 + ND64 - 1 = 23 weights in five exact chunks, added in
+// double-double, and 2^e_c in two factors.
+template <int G>
 __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict__ part, int nsplit, int nmma,
                                                          int64_t ldp, int32_t N, int64_t np,
                                                          const double* __restrict__ colinfo, double sA, double scale,
@@ -314,35 +351,23 @@ __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict
     constexpr int NT = DA64 + ND64 - 1;
     static_assert(NT <= 25, "five chunks of five weights");
     const int c = blockIdx.y;
+    constexpr int DC_I = 256 / G;
+    const int64_t i = (int64_t)blockIdx.x * DC_I + threadIdx.x % DC_I;
     if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;
+    long long T[NT];
+    dense_weights<DA64, ND64, G>(part, nsplit, nmma, ldp, np, DA64, i, i < N, c, T);
+    if (threadIdx.x >= DC_I || i >= N) return;
     const int e = (int)colinfo[2 * c];
     const double ea = pow2i(e / 2), eb = pow2i(e - e / 2), bad = colinfo[2 * c + 1];
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        long long T[NT];
+    double h = 0.0, l = 0.0;
 #pragma unroll
-        for (int q = 0; q < NT; ++q) T[q] = 0;
+    for (int q = 0; q < 5; ++q) {
+        long long C = 0;
 #pragma unroll
-        for (int d = 0; d < DA64; ++d) {
-            const float* src = part + (int64_t)c * ND64 * ldp + (int64_t)d * np + i;
-            for (int y = 0; y < nsplit; ++y) {
-                float v[ND64];
-#pragma unroll
-                for (int j = 0; j < ND64; ++j) v[j] = src[((int64_t)y * nmma + j) * ldp];
-#pragma unroll
-                for (int j = 0; j < ND64; ++j) T[d + j] += (long long)__float2int_rn(v[j]);
-            }
-        }
-        double h = 0.0, l = 0.0;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            long long C = 0;
-#pragma unroll
-            for (int m = 0; m < 5; ++m) C = C * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
-            dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : 0x1p-100),
-                   0.0);
-        }
-        out[i + c * ldo] = (h + l) * sA * scale * ea * eb + bad;
+        for (int m = 0; m < 5; ++m) C = C * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
+        dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : 0x1p-100), 0.0);
     }
+    out[i + c * ldo] = (h + l) * sA * scale * ea * eb + bad;
 }
 
 }  // namespace tc
@@ -510,13 +535,18 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
         ctx->stall_next_gemm = 0;
         GLOBE_RET(dense_dispatch(ctx, nmma, mA, mB, rows, nch, cps, P, ldp, err, stall));
     }
-    const dim3 gc((unsigned)std::min(div_up(N, 256), 1024), kg);
-    if constexpr (F64)
-        k_dense_combine64<<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, col, std::ldexp(1.0, a.e - 20), scale,
-                                                       out, N, st.zhi);
-    else
-        k_dense_combine<ND><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
-                                                         std::ldexp(scale, a.e), out, N, st.zhi);
+    const auto combine = [&](auto split) {
+        constexpr int G = decltype(split)::value;
+        const dim3 gc((unsigned)div_up(N, 256 / G), kg);
+        if constexpr (F64)
+            k_dense_combine64<G><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, col, std::ldexp(1.0, a.e - 20),
+                                                              scale, out, N, st.zhi);
+        else
+            k_dense_combine<ND, G><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
+                                                                std::ldexp(scale, a.e), out, N, st.zhi);
+    };
+    if (div_up(N, 256) * kg <= DC_SPLIT_CTAS) combine(std::integral_constant<int, 4>());
+    else combine(std::integral_constant<int, 1>());
     GLOBE_LAUNCHED(ctx, "k_dense_combine");
     return GLOBE_OK;
 }

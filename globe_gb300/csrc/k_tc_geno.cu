@@ -416,8 +416,8 @@ __device__ __forceinline__ void col_sum_last(const double (&v)[NQ], double* __re
     }
 }
 
-// zhi[c], no longer needed, is cleared for the next product
-template <int ND>
+// zhi[c], no longer needed, is cleared for the next product.  YU: splits whose loads issue together
+template <int ND, int YU>
 __global__ void __launch_bounds__(256) k_combine1(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
                                                   int64_t rows, const double* __restrict__ colinfo,
                                                   const long long* __restrict__ isum, const double* __restrict__ f,
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(256) k_combine1(const float* __restrict__ part
     unsigned mx = 0;
     double acc[1] = {0.0};
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
-        const double gv = recombine<ND>(part, nsplit, nmma, ldp, c, s, s_hi, s_lo);
+        const double gv = recombine<ND, YU>(part, nsplit, nmma, ldp, c, s, s_hi, s_lo);
         const double iv = inv[s], fs = f[s];
         const double u = iv * iv * (gv - fs * S2);
         U[s + c * rows] = u;
@@ -466,6 +466,7 @@ __global__ void __launch_bounds__(256) k_combine2(const float* __restrict__ part
     }
 }
 
+template <int YU>
 __global__ void __launch_bounds__(256) k_combine1_64(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp,
                                                      int64_t rows, const double* __restrict__ colinfo,
                                                      const long long* __restrict__ isum, const double* __restrict__ f,
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(256) k_combine1_64(const float* __restrict__ p
     double sum[2] = {0.0, 0.0};
     for (int64_t s = (int64_t)blockIdx.x * blockDim.x + tid; s < rows; s += (int64_t)gridDim.x * blockDim.x) {
         long long hi, lo;
-        recombine_int<ND64>(part, nsplit, nmma, ldp, c, s, hi, lo);
+        recombine_int<ND64, YU>(part, nsplit, nmma, ldp, c, s, hi, lo);
         const double f2 = 2.0 * f[s], iv = inv[s];
         const double p = __dmul_rn(f2, Sh), pe = __fma_rn(f2, Sh, -p);
         double d = ll_times_pow2(hi, 0x1p-25), r = 0.0;
@@ -894,7 +895,10 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
         GLOBE_RET(gemm_dispatch(ctx, nmma, g.blk1, g.ntiles1, mB1, (int)g.Mk, nch1, sp1, P1, ldp1, err, zg));
     }
     const int sp1e = eff_splits(nch1, sp1);
-    const auto combine1 = [] { if constexpr (F64) return k_combine1_64; else return k_combine1<ND>; }();
+    const auto combine1 = [&] {
+        if constexpr (F64) return sp1e <= 2 ? k_combine1_64<1> : k_combine1_64<4>;
+        else return sp1e <= 2 ? k_combine1<ND, 1> : k_combine1<ND, 4>;
+    }();
     combine1<<<dim3(combine_parts(g.Mk), kg), 256, 0, ctx->stream>>>(
         P1, sp1e, nmma, ldp1, g.Mk, col1, reinterpret_cast<const long long*>(st.isum), g.f, g.inv, U, ps, cnt, st.uhi, c2,
         st.zhi);

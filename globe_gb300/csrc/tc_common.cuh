@@ -112,8 +112,8 @@ __device__ __forceinline__ double pow2i(int e) {
 // scaled to an integer, the split partials are summed in int64 and the digits combined in two
 // exact int64 halves (hi = digits 0..ND_HI-1, lo = the rest); the only rounding is the final
 // FP64 addition.
-// With YU > 1, YU splits' ND loads issue together: k_combine2 reads 10 splits and waits on
-// them; k_combine1 reads 2, holds more registers, and runs faster one split at a time.
+// With YU > 1, YU splits' ND loads issue together: the kernels wait on them.  Up to 2 splits (the
+// large shapes' pass 1) run faster one at a time, from fewer registers.
 template <int ND, int YU = 1>
 __device__ __forceinline__ void recombine_int(const float* __restrict__ part, int nsplit, int nmma, int64_t ldp, int c,
                                               int64_t row, long long& hi, long long& lo) {
