@@ -283,23 +283,6 @@ __global__ void __launch_bounds__(256) k_grm_f64(const uint8_t* __restrict__ blk
 
 using namespace tc;
 
-// Temporary device buffers of one build, released on every exit path.
-struct BuildBufs {
-    globe_ctx* ctx;
-    std::vector<void*> ps;
-    explicit BuildBufs(globe_ctx* c) : ctx(c) {}
-    template <class T>
-    int get(T** p, size_t n) {
-        int rc = dalloc(ctx, p, n);
-        if (rc == GLOBE_OK) ps.push_back((void*)*p);
-        return rc;
-    }
-    ~BuildBufs() {
-        cudaStreamSynchronize(ctx->stream);
-        for (void* p : ps) dfree(ctx, p);
-    }
-};
-
 static int grm_build_tc(globe_ctx* ctx, float* lt) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
@@ -312,29 +295,31 @@ static int grm_build_tc(globe_ctx* ctx, float* lt) {
     const int splits = std::max(1, (nch + 4095) / 4096);   // K per CTA <= 2^19 (exact FP32 sums)
     const int spe = eff_splits(nch, splits);
     const int ngroups = (N + GRM_KG - 1) / GRM_KG;
-    // groups per launch: digit operand + partials within ~2 GB
+    // groups per launch: digit operand + partials within ~1.6 GB (the workspace slots, which the
+    // products use too, add a quarter; a build of its own buffers spent 1.7 ms of 11 allocating
+    // and freeing them at N = 10k, M = 30k)
     const size_t per_group = (size_t)GRM_NMMA * kpad + (size_t)spe * GRM_NMMA * ldp * sizeof(float);
     size_t gfit = std::min<size_t>((size_t)ngroups, (size_t)65535);
-    gfit = std::min<size_t>(gfit, ((size_t)2 << 30) / per_group);
+    gfit = std::min<size_t>(gfit, ((size_t)1600 << 20) / per_group);
     const int G = (int)std::max<size_t>(1, gfit);
-    BuildBufs B(ctx);
+    const int nqb = (int)((kpad / 16 + GD_Q - 1) / GD_Q);   // SNP ranges of k_grm_digits
     double *U4, *C2, *c2part;
     unsigned* hi;
     float2* c2v;
     uint4* dig;
-    uint8_t* D;
+    uint8_t *D, *tab;
     float* P;
     unsigned* err;
-    GLOBE_RET(B.get(&U4, (size_t)4 * g.Mk));
-    GLOBE_RET(B.get(&dig, (size_t)4 * kpad));
-    GLOBE_RET(B.get(&c2v, (size_t)4 * kpad));
-    GLOBE_RET(B.get(&C2, (size_t)G * GRM_KG));
-    const int nqb = (int)((kpad / 16 + GD_Q - 1) / GD_Q);   // SNP ranges of k_grm_digits
-    GLOBE_RET(B.get(&c2part, (size_t)nqb * G * GRM_KG));
-    GLOBE_RET(B.get(&hi, (size_t)1));
+    GLOBE_RET(ws(ctx, WS_TC_U, (size_t)4 * g.Mk, &U4));
+    GLOBE_RET(ws(ctx, WS_TC_D2, (size_t)4 * kpad * (sizeof(uint4) + sizeof(float2)), &tab));
+    dig = reinterpret_cast<uint4*>(tab);
+    c2v = reinterpret_cast<float2*>(tab + (size_t)4 * kpad * sizeof(uint4));
+    GLOBE_RET(ws(ctx, WS_TC_P2, (size_t)(nqb + 1) * G * GRM_KG + 1, &C2));
+    c2part = C2 + (size_t)G * GRM_KG;
+    hi = reinterpret_cast<unsigned*>(c2part + (size_t)nqb * G * GRM_KG);
     GLOBE_CK(ctx, cudaMemsetAsync(hi, 0, sizeof(unsigned), ctx->stream));
-    GLOBE_RET(B.get(&D, (size_t)G * GRM_NMMA * kpad));
-    GLOBE_RET(B.get(&P, (size_t)G * spe * GRM_NMMA * ldp));
+    GLOBE_RET(ws(ctx, WS_TC_D1, (size_t)G * GRM_NMMA * kpad, &D));
+    GLOBE_RET(ws(ctx, WS_TC_P1, (size_t)G * spe * GRM_NMMA * ldp, &P));
     GLOBE_RET(tc_err_word(ctx, &err));
     // digit rows GRM_KG * NDIG .. GRM_NMMA - 1 of every group stay zero
     GLOBE_CK(ctx, cudaMemsetAsync(D, 0, (size_t)G * GRM_NMMA * kpad, ctx->stream));

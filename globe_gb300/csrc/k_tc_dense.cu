@@ -524,10 +524,8 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     CUtensorMap mA, mB;
     GLOBE_RET(make_map(ctx, &mA, a.p, (uint64_t)np, (uint64_t)rows, BK, BM, true));
     GLOBE_RET(make_map(ctx, &mB, D, (uint64_t)np, (uint64_t)nmma, BK, (uint32_t)nmma, true));
-    if (nmma > kg * ND)   // digit rows past the kg columns stay zero
-        GLOBE_CK(ctx, cudaMemsetAsync(D + (size_t)kg * ND * np, 0, (size_t)(nmma - kg * ND) * np, ctx->stream));
     k_digits<ND, false><<<dim3((unsigned)std::min<int64_t>(div_up(np / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, st.zhi, col, D, np, nullptr, nullptr);
+        Z, N, N, st.zhi, col, D, np, nullptr, nullptr, nmma - kg * ND);
     GLOBE_LAUNCHED(ctx, "k_digits");
     {
         ProfScope p(ctx, GLOBE_PROF_GRM_PASS1);

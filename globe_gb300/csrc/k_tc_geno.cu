@@ -721,7 +721,23 @@ static std::vector<int> split_candidates_model(globe_ctx* ctx, int tiles, int nc
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess || sms < 1) sms = 152;
     constexpr int CTA_COST = 8;                       // fixed cost of a CTA, in stages
     const int lo = std::max(1, (nchunks + 4095) / 4096);
-    const int hi = std::max(lo, std::min(64, nchunks / 8));
+    int hi = std::max(lo, std::min(64, nchunks / 8));
+    // A shape that leaves SMs idle even so: finer splits, down to 2 stages per CTA, while they run in
+    // one wave, each split costing the combine half a stage (N = 2000, M = 10000: 2 splits of 8
+    // stages took 10 us a pass, 4 of 4 take 8).  The alternative for the tuner is fewer splits: it
+    // times the pass without the combine.
+    if (tiles * hi < sms) {
+        double best = 1e300;
+        int bs = lo;
+        for (int s = lo; s <= std::max(lo, std::min(16, nchunks / 2)) && (s == lo || tiles * s <= sms); ++s) {
+            const double cost = (nchunks + s - 1) / s + CTA_COST + 0.5 * s;
+            if (cost < best) {
+                best = cost;
+                bs = s;
+            }
+        }
+        return bs > lo ? std::vector<int>{bs, std::max(lo, bs / 2)} : std::vector<int>{bs};
+    }
     std::vector<std::pair<double, int>> est;          // (cost, split count) per effective count
     int prev_se = -1;
     for (int s = lo; s <= hi; ++s) {
@@ -877,12 +893,8 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
     // ---- digits of Z
     unsigned* cnt;
     GLOBE_RET(tc_counters(ctx, kg, &cnt));
-    // digit rows past the kg columns stay zero
-    if (nmma > kg * ND)
-        GLOBE_CK(ctx, cudaMemsetAsync(D1 + (size_t)kg * ND * kpad1, 0, (size_t)(nmma - kg * ND) * kpad1,
-                                      ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad1 / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, st.zhi, col1, D1, kpad1, st.isum, nullptr);
+        Z, N, N, st.zhi, col1, D1, kpad1, st.isum, nullptr, nmma - kg * ND);
     GLOBE_LAUNCHED(ctx, "k_digits");
     // ---- pass 1
     int sp1 = 0;
@@ -904,11 +916,8 @@ static int tc_group(globe_ctx* ctx, const double* Z, int kg, double scale, doubl
         st.zhi);
     GLOBE_LAUNCHED(ctx, "k_combine1");
     // ---- digits of u, pass 2
-    if (nmma > kg * ND)
-        GLOBE_CK(ctx, cudaMemsetAsync(D2 + (size_t)kg * ND * kpad2, 0, (size_t)(nmma - kg * ND) * kpad2,
-                                      ctx->stream));
     k_digits<ND, true><<<dim3((unsigned)std::min<int64_t>(div_up(kpad2 / 4, 256), 2048), kg), 256, 0, ctx->stream>>>(
-        U, g.Mk, g.Mk, st.uhi, col2, D2, kpad2, nullptr, st.isum);
+        U, g.Mk, g.Mk, st.uhi, col2, D2, kpad2, nullptr, st.isum, nmma - kg * ND);
     GLOBE_LAUNCHED(ctx, "k_digits");
     int sp2 = 0;
     GLOBE_RET(tune_splits(ctx, 2, nmma, g.blk2, g.ntiles2, mB2, N, nch2, cand2, P2, ldp2, err, &sp2));

@@ -257,14 +257,16 @@ __global__ void k_col_max(const double* __restrict__ X, int64_t n, int64_t ld, u
 // colinfo for the epilogues.  With isum the column sum of x, each x rounded to ND64 digits whatever
 // ND, is added to isum[2c] 2^30 + isum[2c+1] in units of 2^(e - 55) (integer atomics: the same
 // bits in any order); clear[2c], clear[2c+1] are set to zero
-// (an isum no longer in use).  With ND64 digits (the FP64 products) the scaling takes two factors
+// (an isum no longer in use).  The npad digit rows after the last column's are set to zero (the MMA
+// width is a multiple of 16; a memset of them cost a launch of its own).  With ND64 digits (the FP64 products) the scaling takes two factors
 // where one would leave the range of a double.
 template <int ND, bool GENO>
 __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, const unsigned* __restrict__ hi,
                          double* __restrict__ colinfo, uint8_t* __restrict__ D, int64_t kpad,
-                         unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear) {
+                         unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear, int npad) {
     const int c = blockIdx.y;
     const unsigned h = hi[c];
+    const int pad = c == (int)gridDim.y - 1 ? npad : 0;
     const int e = col_exp<ND>(h), sh = DBITS * (ND - 1) - e;
     const double sc = pow2i(ND == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
     const double sc2 = ND == ND64 ? pow2i(sh - min(sh, 1000)) : 1.0;
@@ -309,6 +311,7 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
         }
 #pragma unroll
         for (int j = 0; j < ND; ++j) *reinterpret_cast<uint32_t*>(D + ((int64_t)c * ND + j) * kpad + P) = word[j];
+        for (int j = ND; j < ND + pad; ++j) *reinterpret_cast<uint32_t*>(D + ((int64_t)c * ND + j) * kpad + P) = 0u;
     }
     if (isum) {
 #pragma unroll
