@@ -200,12 +200,16 @@ int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, d
 // 256-entry table indexed by their four codes (one byte).  Entries are fixed-point int64 on one
 // grid for the whole matrix (2^62 above the largest possible sum), so any split of the SNPs
 // sums to the same bits, within M 2^-63 of the exact sum.
-// A CTA covers 8192 individuals (16 per thread: one word of each of the four SNP rows) and a
-// range of SNPs.  The table is held 16 times over, entry e of copy l at (16 e + l): the 16 lanes
-// of a half warp read 16 different bank pairs whatever their codes.  Two pair tables of 16
-// entries build it (4 stores of two copies per thread).  Bound by the table reads (one 8-byte
-// shared load per 4 genotypes) and the integer work around them.
-constexpr int DG_THREADS = 512;
+// A CTA covers 16384 individuals (16 per thread: one word of each SNP row) and a range of SNPs,
+// eight (two tables) a step.  A table is held 16 times over, entry e of copy l at (16 e + l): the
+// 16 lanes of a half warp read 16 different bank pairs whatever their codes.  Two pair tables of
+// 16 entries build it.  One barrier a step: while a step's tables are read, the next step's are
+// written to the other half and the pair tables of the one after it are formed.  Bound by shared
+// memory (N = 100k, M = 200k: 2.8 ms, L1 at 72 %; 8192 individuals a CTA and two barriers per four
+// SNPs, where writing the tables was a third of the traffic: 3.7 ms).
+constexpr int DG_THREADS = 1024;
+constexpr int DG_LUT = 256 * 16 * 8;                  // bytes of a table
+constexpr int DG_SMEM = 4 * DG_LUT + DG_LUT;          // two steps of two tables, aligned to a table's size
 
 // the largest zs^2 (non-negative doubles order like their bits)
 __global__ void k_zs_max(const double* __restrict__ zs, int64_t n, unsigned long long* __restrict__ out) {
@@ -223,66 +227,105 @@ __device__ __forceinline__ int diag_bits(const unsigned long long* maxq, int64_t
     return 62 - E;
 }
 
-__global__ void __launch_bounds__(DG_THREADS, 2) k_geno_diag(const uint8_t* __restrict__ blk, int nch, int64_t Mk,
+// One round of a transpose of the four 2-bit codes of each byte over four words.
+template <int S>
+__device__ __forceinline__ void dg_round(uint32_t (&r)[4], uint32_t m) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if ((k & S) == 0) {
+            const uint32_t t = ((r[k] >> (2 * S)) ^ r[k + S]) & m;
+            r[k + S] ^= t;
+            r[k] ^= t << (2 * S);
+        }
+}
+
+__global__ void __launch_bounds__(DG_THREADS, 1) k_geno_diag(const uint8_t* __restrict__ blk, int nch, int64_t Mk,
                                                              int32_t N, const double* __restrict__ zs,
-                                                             const unsigned long long* __restrict__ maxq, int64_t gper,
+                                                             const unsigned long long* __restrict__ maxq, int64_t sper,
                                                              long long* __restrict__ part) {
-    __shared__ __align__(16) long long lut[256 * 16];
-    __shared__ long long pt[2][16];
+    extern __shared__ __align__(16) char dg_smem[];
+    __shared__ long long pt[2][4][16];   // step parity; pairs of SNPs of a step
     const int tid = threadIdx.x;
+    const uint32_t lut0 = ((uint32_t)__cvta_generic_to_shared(dg_smem) + (DG_LUT - 1)) & ~(uint32_t)(DG_LUT - 1);
     const int64_t c = (int64_t)blockIdx.x * (DG_THREADS / 8) + (tid >> 3);   // 128-individual chunk
     const int w = tid & 7;                                                   // its word of 16 individuals
     const bool in = c < nch;
-    const int64_t ng = (Mk + 3) / 4, g0 = (int64_t)blockIdx.y * gper, g1 = min(ng, g0 + gper);
+    const int64_t nst = (Mk + 7) / 8, st0 = (int64_t)blockIdx.y * sper, st1 = min(nst, st0 + sper);
+    if (st0 >= st1) return;
     const double sc = ldexp(1.0, diag_bits(maxq, Mk));
-    const int el = (tid >> 3) & 15, eh = tid >> 7;
-    const long long* mine = lut + (tid & 15);
     long long acc[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[j] = 0;
-    // a group's four words, and (threads < 32) the two zs of their pair-table entry: loaded one
-    // group ahead of their use
+    // four words of a table's SNPs, loaded one table ahead of their use (a step's rows lie in one block)
     uint32_t r[4], rn[4] = {0u, 0u, 0u, 0u};
-    double za = 0.0, zb = 0.0;
-    const int ca = tc::tile_to_plink(tid & 3), cb = tc::tile_to_plink((tid >> 2) & 3);
-    auto fetch = [&](int64_t g) {
-        const int64_t s0 = 4 * g;
-        if (in) {
-            const int rr = (int)(s0 & 127);   // a multiple of 4: the four rows share their half swap
-            const uint8_t* p = blk + (((s0 >> 7) * nch + c) * 128 + rr) * 32 + (((w >> 2) ^ ((rr >> 2) & 1)) * 16) + (w & 3) * 4;
+    auto fetch = [&](int64_t s0) {
+        if (!in) return;
+        const int rr = (int)(s0 & 127);   // a multiple of 4: the four rows share their half swap
+        const uint8_t* p = blk + (((s0 >> 7) * nch + c) * 128 + rr) * 32 + (((w >> 2) ^ ((rr >> 2) & 1)) * 16) + (w & 3) * 4;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) rn[q] = __ldg(reinterpret_cast<const uint32_t*>(p + 32 * q));
-        }
-        if (tid < 32) {
-            const int64_t sa = s0 + 2 * (tid >> 4);
-            za = sa < Mk ? zs[4 * sa + ca] : 0.0;
-            zb = sa + 1 < Mk ? zs[4 * sa + 4 + cb] : 0.0;
-        }
+        for (int q = 0; q < 4; ++q) rn[q] = __ldg(reinterpret_cast<const uint32_t*>(p + 32 * q));
     };
-    if (g0 < g1) fetch(g0);
-    for (int64_t g = g0; g < g1; ++g) {
+    // threads 0 .. 63: entry tid & 15 of pair table tid >> 4 of step st
+    const int ca = tc::tile_to_plink(tid & 3), cb = tc::tile_to_plink((tid >> 2) & 3);
+    double za = 0.0, zb = 0.0;
+    auto fetch_zs = [&](int64_t st) {
+        if (tid >= 64) return;
+        const int64_t sa = 8 * st + 2 * (tid >> 4);
+        za = st < st1 && sa < Mk ? zs[4 * sa + ca] : 0.0;
+        zb = st < st1 && sa + 1 < Mk ? zs[4 * sa + 4 + cb] : 0.0;
+    };
+    auto put_pairs = [&](int64_t st) {
+        if (tid < 64) pt[st & 1][tid >> 4][tid & 15] = __double2ll_rn(za * za * sc) + __double2ll_rn(zb * zb * sc);
+    };
+    // thread tid writes copies 2 (tid & 7) and the next of entries tid >> 3 and 128 + (tid >> 3)
+    auto put_luts = [&](int64_t st) {
+        const int e = tid >> 3, el = e & 15, eh = e >> 4;
+        const uint32_t base = lut0 + (uint32_t)(st & 1) * (2 * DG_LUT) + (uint32_t)(e * 128 + (tid & 7) * 16);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) r[q] = rn[q];
-        if (tid < 32) pt[tid >> 4][tid & 15] = __double2ll_rn(za * za * sc) + __double2ll_rn(zb * zb * sc);
-        if (g + 1 < g1) fetch(g + 1);
-        __syncthreads();
-        const long long vl = pt[0][el];
+        for (int t = 0; t < 2; ++t) {
+            const long long vl = pt[st & 1][2 * t][el];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {   // entry (el, eh + 4 q), copies 2 (tid & 7) and the next
-            const long long v = vl + pt[1][eh + 4 * q];
-            *reinterpret_cast<longlong2*>(lut + (((eh + 4 * q) * 16 + el) * 16 + 2 * (tid & 7))) = make_longlong2(v, v);
-        }
-        __syncthreads();
-        if (in) {
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                // byte b: the four SNPs' codes of individual 4 b + m
-                const uint32_t t = ((r[0] >> (2 * m)) & 0x03030303u) | (((r[1] >> (2 * m)) & 0x03030303u) << 2) |
-                                   (((r[2] >> (2 * m)) & 0x03030303u) << 4) | (((r[3] >> (2 * m)) & 0x03030303u) << 6);
-#pragma unroll
-                for (int b = 0; b < 4; ++b) acc[4 * b + m] += mine[((t >> (8 * b)) & 255u) * 16];
+            for (int q = 0; q < 2; ++q) {
+                const long long v = vl + pt[st & 1][2 * t + 1][eh + 8 * q];
+                asm volatile("st.shared.v2.b64 [%0], {%1, %1};" ::"r"(base + (uint32_t)(t * DG_LUT + q * (DG_LUT / 2))), "l"(v)
+                             : "memory");
             }
         }
+    };
+    fetch(8 * st0);
+    fetch_zs(st0);
+    put_pairs(st0);
+    fetch_zs(st0 + 1);
+    __syncthreads();
+    put_luts(st0);
+    put_pairs(st0 + 1);
+    fetch_zs(st0 + 2);
+    __syncthreads();
+    for (int64_t st = st0; st < st1; ++st) {
+        if (st + 1 < st1) put_luts(st + 1);
+        put_pairs(st + 2);   // over those of step st, read before the last barrier
+        fetch_zs(st + 3);
+        const uint32_t mine = lut0 + (uint32_t)(st & 1) * (2 * DG_LUT) + (uint32_t)(tid & 15) * 8;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) r[q] = rn[q];
+            if (t == 0 || st + 1 < st1) fetch(8 * st + 4 * (t + 1));
+            if (!in) continue;
+            dg_round<2>(r, 0x0F0F0F0Fu);   // now byte b of r[m]: the four SNPs' codes of individual 4 b + m
+            dg_round<1>(r, 0x33333333u);
+            const uint32_t lut = mine + t * DG_LUT;
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const uint32_t off = (b == 0 ? r[m] << 7 : r[m] >> (8 * b - 7)) & 0x7F80u;   // code x 128 bytes
+                    long long v;
+                    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(off | lut) : "memory");
+                    acc[4 * b + m] += v;
+                }
+        }
+        __syncthreads();
     }
     const int64_t i0 = c * 128 + w * 16;
     long long* out = part + (int64_t)blockIdx.y * N;
@@ -307,11 +350,13 @@ int geno_diag(globe_ctx* ctx, double* d) {
         GLOBE_CK(ctx, cudaMemsetAsync(d, 0, sizeof(double) * N, ctx->stream));
         return GLOBE_OK;
     }
-    // about four waves of two CTAs an SM (the last one ragged), at least 16 groups of SNPs each
-    const int64_t cx = div_up(div_up(N, 128), DG_THREADS / 8), ng = (g.Mk + 3) / 4;
-    int64_t ns = std::max<int64_t>(1, std::min<int64_t>((8 * 152 + cx - 1) / cx, ng / 16));
-    const int64_t gper = (ng + ns - 1) / ns;
-    ns = (ng + gper - 1) / gper;
+    // whole waves of one CTA an SM: four where that leaves a CTA 32 steps of eight SNPs (its first
+    // tables and the partial sums' second pass then cost little), else as few as one; at least 4 steps
+    const int64_t cx = div_up(div_up(N, 128), DG_THREADS / 8), nst = (g.Mk + 7) / 8;
+    const int64_t waves = std::min<int64_t>(4, std::max<int64_t>(1, nst * cx / (32 * 152)));
+    int64_t ns = std::max<int64_t>(1, std::min<int64_t>(waves * 152 / cx, nst / 4));
+    const int64_t sper = (nst + ns - 1) / ns;
+    ns = (nst + sper - 1) / sper;
     long long* part;
     unsigned long long* maxq;
     GLOBE_RET(ws(ctx, WS_GPART, (size_t)ns * N + 1, &part));
@@ -319,8 +364,9 @@ int geno_diag(globe_ctx* ctx, double* d) {
     GLOBE_CK(ctx, cudaMemsetAsync(maxq, 0, sizeof(*maxq), ctx->stream));
     k_zs_max<<<(unsigned)std::min<int64_t>(div_up(4 * g.Mk, 1024), 304), 256, 0, ctx->stream>>>(g.zs, 4 * g.Mk, maxq);
     GLOBE_LAUNCHED(ctx, "k_zs_max");
-    k_geno_diag<<<dim3((unsigned)cx, (unsigned)ns), DG_THREADS, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, maxq,
-                                                                                  gper, part);
+    GLOBE_CK(ctx, cudaFuncSetAttribute(k_geno_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
+    k_geno_diag<<<dim3((unsigned)cx, (unsigned)ns), DG_THREADS, DG_SMEM, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, maxq,
+                                                                                        sper, part);
     GLOBE_LAUNCHED(ctx, "k_geno_diag");
     k_geno_diag_sum<<<div_up(N, 256), 256, 0, ctx->stream>>>(part, (int)ns, g.Mk, N, maxq, d);
     GLOBE_LAUNCHED(ctx, "k_geno_diag_sum");
