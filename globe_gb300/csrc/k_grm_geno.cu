@@ -7,12 +7,13 @@
 //
 // The genotypes are read from the SNP-major tile-blocked copy of the
 // tensor-core path (blk1, tile codes; the only SNP-major copy kept).
-// Pass 1 (w = Zs Z): one warp per SNP row; lanes stream 16-byte pieces of
-// the row (64 samples each).  Pass 2 (Zs' w): a CTA owns 128 consecutive
+// Pass 1 (w = Zs Z): one to eight warps per two SNP rows, a lane per
+// sample.  Pass 2 (Zs' w): a CTA owns 128 consecutive
 // samples (one 32-byte chunk of every SNP row), stages SNP tiles in shared
 // memory and splits the SNP range across CTAs (partials reduced in a fixed
 // order).  zs per SNP is a table indexed by the 2-bit code, so the decode is a
-// select, not arithmetic.  FP64 throughput bounds both passes.
+// select, not arithmetic.  Latency bounds the smallest products, FP64
+// throughput the largest.
 #include "tc_common.cuh"
 
 namespace globe {
@@ -22,45 +23,75 @@ __device__ __forceinline__ double zsel(unsigned code, double t0, double t1, doub
     return code == 1u ? t2 : (code == 2u ? t0 : t1);
 }
 
+// W = Zs Z: wp warps (1, 2, 4 or 8) per two SNPs, a lane per individual, so that the lanes' loads of
+// Z lie side by side and each 16 of them share a word of codes (64 individuals a lane: every load of
+// Z touched 32 lines).  Bound by latency at most sizes that come here, hence wp (p1_warps).
+// N = 601, M = 1503: 15.1 -> 8.5 us; a call of N = 100, M = 100000: 453 -> 148 us.
 template <int KC>
 __global__ void __launch_bounds__(256) k_geno_p1(const uint8_t* __restrict__ blk, int nch, int64_t Mk,
                                                  int32_t N, const double* __restrict__ zs,
                                                  const double* __restrict__ Z, int64_t ldz, int kc,
-                                                 double* __restrict__ W, int64_t ldw) {
-    const int lane = threadIdx.x & 31;
-    const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (s >= Mk) return;
-    const double t0 = zs[4 * s], t1 = zs[4 * s + 1], t2 = zs[4 * s + 2];
-    const int nchunks = (N + 63) >> 6;
-    double acc[KC];
+                                                 double* __restrict__ W, int64_t ldw, int wp) {
+    __shared__ double sm[8][2][KC];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = warp & (wp - 1);
+    const int64_t s = ((int64_t)blockIdx.x * (8 / wp) + warp / wp) * 2;
+    const bool one = s < Mk, two = s + 1 < Mk;   // the copy's rows are padded: the second SNP's codes may be read anyway
+    double t[2][3], acc[2][KC];
 #pragma unroll
-    for (int c = 0; c < KC; ++c) acc[c] = 0.0;
-    for (int q = lane; q < nchunks; q += 32) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(blk + tc::blk_offset(s, (int64_t)q << 4, nch)));
-        const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-        const int i0 = q << 6;
+    for (int u = 0; u < 2; ++u)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint32_t w = w4[j];
+        for (int q = 0; q < 3; ++q) t[u][q] = s + u < Mk ? zs[4 * (s + u) + q] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int c = 0; c < KC; ++c) acc[u][c] = 0.0;
+    const int sh = 2 * (lane & 15);
 #pragma unroll 4
-            for (int e = 0; e < 16; ++e) {
-                const int i = i0 + j * 16 + e;
-                if (i < N) {
-                    const double z = zsel((w >> (2 * e)) & 3u, t0, t1, t2);
+    for (int i = one ? sub * 32 + lane : N; i < N; i += 32 * wp) {
+        double z[2];
 #pragma unroll
-                    for (int c = 0; c < KC; ++c)
-                        if (c < kc) acc[c] += z * __ldg(Z + i + (size_t)c * ldz);
-                }
-            }
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(blk + tc::blk_offset(s + u, (int64_t)(i >> 4) << 2, nch)));
+            z[u] = zsel((w >> sh) & 3u, t[u][0], t[u][1], t[u][2]);
         }
+#pragma unroll
+        for (int c = 0; c < KC; ++c)
+            if (c < kc) {
+                const double x = __ldg(Z + i + (size_t)c * ldz);
+                acc[0][c] += z[0] * x;
+                acc[1][c] += z[1] * x;
+            }
     }
 #pragma unroll
     for (int c = 0; c < KC; ++c) {
-        double a = acc[c];
+        double a = acc[0][c], b = acc[1][c];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0 && c < kc) W[s + (size_t)c * ldw] = a;
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        if (lane == 0) {
+            sm[warp][0][c] = a;
+            sm[warp][1][c] = b;
+        }
     }
+    __syncthreads();
+    if (sub == 0 && lane < 2 * KC) {
+        const int u = lane / KC, c = lane % KC;
+        double a = sm[warp][u][c];
+        for (int q = 1; q < wp; ++q) a += sm[warp + q][u][c];
+        if (c < kc && s + u < Mk) W[s + u + (size_t)c * ldw] = a;
+    }
+}
+
+// Warps per two SNPs: 16 warps an SM where the individuals give each four loads or more; fewer with
+// more columns, which give a warp as many chains and whose sums over its lanes each warp pays for
+// (N = 2000, M = 3000, 6 columns: 329 us a call with 2, 305 with 1; N = 20000, M = 1000, one column:
+// 344 us with 1, 151 with 8).
+static int p1_warps(int64_t Mk, int32_t N, int kc) {
+    int wp = 1;
+    while (wp < 8 && (Mk + 1) / 2 * wp * std::max(1, kc / 2) < 16 * 152 && N > 128 * wp) wp *= 2;
+    return wp;
 }
 
 constexpr int P2_THREADS = 128;  // samples per CTA (32 bytes per SNP row)
@@ -119,12 +150,22 @@ __global__ void __launch_bounds__(P2_THREADS) k_geno_p2(const uint8_t* __restric
     }
 }
 
-// out[e] = scale * sum_y part[y * n + e]  (fixed order)
-__global__ void k_sum_splits(const double* __restrict__ part, int nsplit, int64_t n, double scale,
-                             double* __restrict__ out, int64_t ldo, int64_t rows) {
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-        double a = 0;
-        for (int y = 0; y < nsplit; ++y) a += part[(size_t)y * n + e];
+// out[e] = scale * sum_y part[y * n + e] (fixed order): 32 entries a CTA, eight threads each
+__global__ void __launch_bounds__(256) k_sum_splits(const double* __restrict__ part, int nsplit, int64_t n, double scale,
+                                                    double* __restrict__ out, int64_t ldo, int64_t rows) {
+    __shared__ double sm[8][32];
+    const int x = threadIdx.x & 31, y0 = threadIdx.x >> 5;
+    const int64_t e = (int64_t)blockIdx.x * 32 + x;
+    double a = 0;
+    if (e < n) {
+#pragma unroll 4
+        for (int y = y0; y < nsplit; y += 8) a += __ldg(part + (size_t)y * n + e);
+    }
+    sm[y0][x] = a;
+    __syncthreads();
+    if (y0 == 0 && e < n) {
+#pragma unroll
+        for (int y = 1; y < 8; ++y) a += sm[y][x];
         const int64_t r = e % rows, c = e / rows;
         out[r + c * ldo] = scale * a;
     }
@@ -146,7 +187,8 @@ static int geno_chunk(globe_ctx* ctx, const double* Z, int kc, double scale, dou
     const int32_t N = ctx->coh.N;
     {
         ProfScope ps(ctx, GLOBE_PROF_GRM_PASS1);
-        k_geno_p1<KC><<<div_up(g.Mk, 8), 256, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, Z, N, kc, W, g.Mk);
+        const int wp = p1_warps(g.Mk, N, kc);
+        k_geno_p1<KC><<<div_up(g.Mk, 16 / wp), 256, 0, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, Z, N, kc, W, g.Mk, wp);
         GLOBE_LAUNCHED(ctx, "k_geno_p1");
     }
     dim3 grid(div_up(N, P2_THREADS), nsplit);
@@ -156,9 +198,7 @@ static int geno_chunk(globe_ctx* ctx, const double* Z, int kc, double scale, dou
         GLOBE_LAUNCHED(ctx, "k_geno_p2");
     }
     int64_t n = (int64_t)N * kc;
-    int nb = div_up(n, 256);
-    if (nb > 4096) nb = 4096;
-    k_sum_splits<<<nb, 256, 0, ctx->stream>>>(part, nsplit, n, scale, out, N, N);
+    k_sum_splits<<<(unsigned)div_up(n, 32), 256, 0, ctx->stream>>>(part, nsplit, n, scale, out, N, N);
     GLOBE_LAUNCHED(ctx, "k_sum_splits");
     return GLOBE_OK;
 }
