@@ -1036,20 +1036,22 @@ int geno_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* 
 }
 
 // The FP64 product.  On the tensor cores (ND64 digits) it needs the individual-major copy and
-// ~7 short launches, ~60 us whatever its size while it is small; on the FP64 pipe
-// (k_grm_geno.cu) it needs neither and takes about N Mk k / 1.4e11 seconds above ~25 us (70 us
-// with more than one column).  So, by its size N Mk k (FP64 pipe / tensor cores, us a product):
-//  - inside a solve, which repeats the product, from where the two cross: 8e6 for one column
-//    (3e6: 40 / 62; 8e6: 66 / 68; 2e7: 136 / 72), 1e6 for more (7.5e5: 73 / 59; 4.5e6: 113 / 66;
-//    1e8: 696 / 82; 2e9: 14474 / 148);
+// ~7 short launches, which cost about the same whatever its size while it is small; on the FP64
+// pipe (k_grm_geno.cu) it needs neither, three launches and time that grows with the size.  So, by
+// its size N Mk k:
+//  - inside a solve, which repeats the product, from where the two cross (us an iteration, FP64
+//    pipe / tensor cores): 5e6 for one or two columns (one: 3e6 53 / 60, 8e6 76 / 62, 2e7 129 / 67;
+//    two: 3e6 54 / 59, 9e6 74 / 59), 5e5 for more, whose first pass there waits on more loads
+//    (five: 7.5e5 62 / 56, 4.5e6 88 / 61, 1.2e7 176 / 62; nine: 6e6 96 / 59);
 //  - a single operator call from F64_CALL_MIN on, where the first call, which also lays out the
-//    copy, costs about the same on either (4e7: 351 / 315; 2e7: 166 / 394; 2e8: 1317 / 526).
+//    copy, costs about the same on either (us, one column: 2e7 151 / 199, 4e7 260 / 204; five: 5e6
+//    101 / 131, 2e7 209 / 145, 1e8 901 / 244).
 // The choice depends on the sizes only.  Where the copy and the workspaces do not fit in free
 // device memory, the FP64 pipe runs (decided once per load of genotypes).
 // Error against 128-bit sums (N = 6000, M = 3000; normal, constant, count, lognormal, unit and
 // wide-range columns): 1.3e-16 to 1.9e-16 of the column, FP64 pipe 3.9e-16 to 1.1e-15.
 #ifndef F64_SOLVE_MIN
-#define F64_SOLVE_MIN (k == 1 ? 8e6 : 1e6)
+#define F64_SOLVE_MIN (k <= 2 ? 5e6 : 5e5)
 #endif
 #ifndef F64_CALL_MIN
 #define F64_CALL_MIN 4e7
