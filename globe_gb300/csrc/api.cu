@@ -479,7 +479,7 @@ int load_bed_rows(globe_ctx* ctx, const uint8_t* d_bed, int64_t M, int64_t strid
         // temporaries: the statistics the caller passed NULL for, the kept SNPs' indices and their scan
         const size_t nb = (size_t)keep_blocks(M) + 1;
         int64_t* tmp;
-        GLOBE_RET(ws(ctx, WS_GPART, (size_t)M * 3 + nb + ((size_t)M + 7) / 8, &tmp));
+        GLOBE_RET(ws(ctx, WS_LOAD, (size_t)M * 3 + nb + ((size_t)M + 7) / 8, &tmp));
         int64_t* d_idx = tmp + 2 * M;
         int64_t* d_cnt = d_idx + M;
         if (!have_alt) d_alt = tmp;

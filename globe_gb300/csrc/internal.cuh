@@ -90,7 +90,7 @@ enum SlotId {
     WS_R, WS_X, WS_P, WS_VP, WS_ZI, WS_GZ, WS_S1, WS_PART, WS_SCAL, WS_COLS, WS_W,
     WS_GPART, WS_B, WS_TMP1, WS_TMP2, WS_TMP3, WS_TMP4, WS_H, WS_HSTAR, WS_PROBE,
     WS_UH, WS_SMALL, WS_IO1, WS_IO2, WS_BHAT, WS_FB, WS_FX,
-    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_SOLVE, WS_HDF, WS_TC_CNT, WS_TC_STAT, WS_COUNT
+    WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U, WS_TC_SCAL, WS_TC_ERR, WS_LOOP, WS_SOLVE, WS_HDF, WS_TC_CNT, WS_TC_STAT, WS_LOAD, WS_COUNT
 };
 
 }  // namespace globe
@@ -144,7 +144,7 @@ struct globe_ctx {
     cudaGraphExec_t pcg_loop = nullptr;
     int device_loop = 1;
     int64_t device_loop_runs = 0;
-    // record kernels of GLOBE_PREC_MIXED solves in double-float (k_records_df.cu), and how many
+    // record kernels of GLOBE_PREC_MIXED solves in double-float (k_solve.cu), and how many
     // solves ran them (globe_set_record_df)
     int record_df = 1;
     int64_t record_df_runs = 0;

@@ -232,7 +232,7 @@ int globe_get_digits(const globe_ctx* ctx);
 /* CUDA graphs in the block PCG (on = 1, the default; 0 = direct launches).
  * Each globe_pcg call runs its first iteration directly. It then captures the
  * iteration's stream work (record kernels, GRM product, the copies of the
- * residual norms) once per parity of its swapped r'z buffers and column set,
+ * residual norms) once per column set,
  * and replays it, with the host checking the stopping rule after each
  * iteration (or, by default, once per solve: globe_set_device_loop).
  * Results are identical either way. Graphs are not used while event
@@ -245,7 +245,7 @@ int globe_get_graphs(const globe_ctx* ctx);
 /* Device-side PCG loop (on = 1, the default; needs graphs on).  Without
  * per-column masking the column set of a solve cannot change, so after the
  * first iteration the rest run as one CUDA graph whose WHILE conditional node
- * repeats the iteration; a one-thread kernel at the end of each iteration
+ * repeats the iteration; the last CTA of its last kernel
  * applies the stopping rule of the reference -- max_j |r_j|/|b_j| < tol and the
  * stagnation stop (PCGsolver.cpp:1373-1415), or all_j |r_j| < tol |b_j|
  * (varCompEst.cpp:505-508) -- to the device copies of the residual norms and
@@ -259,10 +259,10 @@ int globe_get_device_loop(const globe_ctx* ctx);
 int64_t globe_device_loop_runs(const globe_ctx* ctx);
 
 /* Double-float record kernels of GLOBE_PREC_MIXED solves (on = 1, the default;
- * 0 = FP64).  The block PCG's record-level vectors (x, r, z, p, Vp) are held
- * as pairs of FP32 numbers (about 48 significant bits) from the end of its
- * FP64 set-up to the end of the solve, and the iteration's segment sums,
- * operator assembly and update run on the FP32 pipe; the GRM product's input
+ * 0 = FP64).  The block PCG's record-level vectors (x, r, p) are held
+ * as pairs of FP32 numbers (about 48 significant bits) from the start point's
+ * residual to the end of the solve, and the iteration's record kernels
+ * run on the FP32 pipe; the GRM product's input
  * and output, the per-column scalars and the dot products past each CTA stay
  * FP64.  Each column runs scaled by a power of two to a unit-size right-hand
  * side (exact), and x is returned in FP64.  A solve keeps the FP64 kernels
