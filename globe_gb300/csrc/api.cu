@@ -415,14 +415,14 @@ int globe_load_records(globe_ctx* ctx, int64_t Nrec, int32_t N, int32_t p, const
                                       ctx->stream));
     }
     // blocks by descending number of records, in file order among equals (a counting sort): the
-    // solve's kernels walk them so, and those with more than SOLVE_LONG by whole CTAs
+    // solve's kernels walk them so, and choose by the lengths above SOLVE_LONG who walks them
     std::vector<int32_t> at((size_t)maxb + 2, 0);
     std::vector<int4> order(N);
     for (int32_t b = 0; b < N; ++b) ++at[maxb - (bstart[b + 1] - bstart[b]) + 1];
     for (int32_t l = 0; l <= maxb; ++l) at[l + 1] += at[l];
     for (int32_t b = 0; b < N; ++b)
         order[at[maxb - (bstart[b + 1] - bstart[b])]++] = make_int4(b, bstart[b], bstart[b + 1], bind[b]);
-    while (c.nlong_solve < N && order[c.nlong_solve].z - order[c.nlong_solve].y > SOLVE_LONG) ++c.nlong_solve;
+    for (int32_t b = 0; b < N && order[b].z - order[b].y > SOLVE_LONG; ++b) c.long_len.push_back(order[b].z - order[b].y);
     GLOBE_RET(dalloc(ctx, &c.order, (size_t)N));
     GLOBE_CK(ctx, cudaMemcpyAsync(c.order, order.data(), sizeof(int4) * N, cudaMemcpyHostToDevice, ctx->stream));
     GLOBE_CK(ctx, cudaMemcpyAsync(c.X, X, sizeof(double) * Nrec * (p + 1), cudaMemcpyHostToDevice, ctx->stream));

@@ -28,7 +28,7 @@ namespace globe {
 //             zs = (g - 2f) * inv_std, missing -> g = 0
 //   dense:    packed lower triangle float32, N(N+1)/2
 constexpr int SHORT_BLOCK = 48;   // longest record block handled by one thread in the record kernels
-constexpr int SOLVE_LONG = 32;    // longest one handled by one thread in a solve's kernels (k_solve.cu)
+constexpr int SOLVE_LONG = 32;    // longest one that a solve's kernels never give to more than one thread (k_solve.cu)
 
 struct Cohort {
     int64_t Nrec = 0;
@@ -45,7 +45,7 @@ struct Cohort {
     int32_t* lblk = nullptr;   // blocks with more than SHORT_BLOCK records (device list)
     int32_t nlong = 0;
     int4* order = nullptr;     // blocks by descending number of records: {block, first, one past last, individual}
-    int32_t nlong_solve = 0;         // of them, those with more than SOLVE_LONG
+    std::vector<int32_t> long_len;   // their numbers of records above SOLVE_LONG
     float2* tdf = nullptr;     // times as double-float pairs (the double-float record kernels)
     double tmax = 0;           // max |t|
     const double* times() const { return X + (size_t)p * Nrec; }

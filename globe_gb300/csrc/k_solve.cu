@@ -17,12 +17,12 @@
 // Layout: the vectors are [record][column], column fastest, and a thread owns an (individual,
 // column) pair with the columns of an individual on neighbouring threads: a warp reads whole
 // runs of an individual's records, whatever the number of columns.  Individuals are taken in order
-// of their record counts (Cohort::order), so the threads of a warp walk equally many records; the
-// ones of more than SOLVE_LONG records (order's first) are walked by all individuals' threads of a
-// CTA together, in CTAs of their own: one thread's walk is a chain of loads and FP64 sums that
-// outlasts the rest (N = 20k with up to 94 records each, FP64: k_update 78 us).  The kernels are
-// bound by the vectors' transfers (in double-float) or by the FP64 pipe (~16 operations a record
-// and column; in FP64).
+// of their record counts (Cohort::order), so the threads of a warp walk equally many records.  One
+// thread's walk is a chain of loads and sums, and outlasts the rest where an individual has many
+// records for the size of the solve: those are walked by teams of a CTA's threads, several
+// individuals at a time, and the longest by a whole CTA each (shape(), which classes them).  The
+// kernels are bound by the vectors' transfers (in double-float) or by the FP64 pipe (~16 operations
+// a record and column; in FP64).
 //
 // Two arithmetics: FP64 (GLOBE_PREC_FP64), and double-float pairs (df.cuh) in the 8 bytes of
 // each double under GLOBE_PREC_MIXED, column c scaled by a power of two (col_unscale) to a
@@ -49,6 +49,8 @@ constexpr int RU_DIR = 4, RU_UPD = 2, RES_DIR = 3, RES_UPD = 4;
 // CTAs per SM launched at most: k_dir's take two turns, the kernels that end in column sums one
 // (fewer partials)
 constexpr int PER_DIR = 2 * RES_DIR, PER_SUM = 4;
+constexpr int PER_LONG = 2;        // and for the individuals that take a whole CTA
+constexpr int TEAM = 8, TEAM_MOST = 32;   // threads of a team
 
 struct ArithF64 {
     using V = double;
@@ -83,6 +85,12 @@ struct ArithDF {
     static __device__ __forceinline__ V madd(V a, V b, V c) { return df::madd(a, b, c); }
 };
 
+// A class of individuals: n of them from order[i0] on, walked by `ctas` CTAs, rt threads of a CTA to
+// each (individual, column)
+struct Part {
+    int32_t i0, n;
+    int ctas, rt;
+};
 // What the kernels take of a solve (SolveVecs, solve.cuh) in their arithmetic's storage type
 template <class A>
 struct Args {
@@ -90,14 +98,15 @@ struct Args {
     const typename A::S *t, *H;
     const int4* order;               // {block, first record, one past its last, individual} (Cohort::order)
     const int32_t *bind, *cols;
-    int32_t N, nlong;
+    int32_t N;
     int64_t Nrec;
     int k, kact, kc, ti;             // columns; active ones; columns per tile, individuals per CTA step
     typename A::V e, inv_e, b0, b01, b1;
     typename A::S *alpha, *beta;     // converted once, where they are formed
     double *rz, *pvp, *rr;
     double* part;
-    int slots, hctas;                // partials per column: CTAs; of them, those that walk the long individuals
+    int slots;                       // partials per column: CTAs
+    Part cls[3];                     // who walks what: whole CTAs, teams, single threads
     unsigned* cnt;                   // arrival counts, zero between launches: per tile its groups' and
     unsigned* tiles_done;            // the groups' (sum_last); of the tiles
 };
@@ -118,52 +127,83 @@ __device__ __forceinline__ Lane lane_of(const Args<A>& a) {
     return l;
 }
 
-// v of the individuals' threads of a column combined into the il = 0 thread's (every thread calls
-// it); sm: ST values
-template <class T, class Op>
-__device__ __forceinline__ T over_individuals(T v, T* sm, int ti, int kc, int il, Op op) {
+// the class of CTA x, and x within it
+template <class A>
+__device__ __forceinline__ int class_of(const Args<A>& a, int& x) {
+    int p = 0;
+    for (; p < 2 && x >= a.cls[p].ctas; ++p) x -= a.cls[p].ctas;
+    return p;
+}
+// A thread's place in its CTA's class: individuals come `per` at a time, this one's slot of them
+// and its place among the slot's rt threads
+struct Team {
+    unsigned i0, n, j0, js;   // individuals i0 + j, j = j0 + slot, in steps of js
+    int rt, per, slot, rl;
+    bool on;
+};
+template <bool MANY, class A>
+__device__ __forceinline__ Team team_of(const Args<A>& a, const Lane& l, const Part& p, int x) {
+    Team w;
+    w.i0 = p.i0;
+    w.n = p.n;
+    w.rt = MANY ? p.rt : 1;
+    w.per = MANY ? a.ti / p.rt : a.ti;
+    w.slot = MANY ? l.il / p.rt : l.il;
+    w.rl = MANY ? l.il - w.slot * p.rt : 0;
+    w.on = l.on && (!MANY || w.slot < w.per);
+    w.j0 = (unsigned)(x * w.per);
+    w.js = (unsigned)(p.ctas * w.per);
+    return w;
+}
+
+// v[q] over the rt threads of each slot and column, in the rl = 0 thread's v and in sm[q ST + its t]
+// (every thread of the CTA calls it)
+template <int Q, class A>
+__device__ __forceinline__ void team_sum(const Args<A>& a, const Team& w, typename A::V (&v)[Q], typename A::V* sm) {
     const int t = threadIdx.x;
-    sm[t] = v;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) sm[q * ST + t] = v[q];
     __syncthreads();
     int s = 1;
-    while (s < ti) s <<= 1;
+    while (s < w.rt) s <<= 1;
     for (s >>= 1; s > 0; s >>= 1) {
-        if (il < s && il + s < ti) {
-            v = op(v, sm[t + s * kc]);
-            sm[t] = v;
+        if (w.on && w.rl < s && w.rl + s < w.rt) {
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
+                v[q] = A::add(v[q], sm[q * ST + t + s * a.kc]);
+                sm[q * ST + t] = v[q];
+            }
         }
         __syncthreads();
     }
-    return v;
 }
 
 // ---- k_dir -----------------------------------------------------------------------
 
-// individuals g0, g0 + gs, ...; returns the largest abs_hi of the thread's sums
-template <class A, bool TEAM>
-__device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, const bool first, int64_t g0, int gs,
+// the CTA's individuals; returns the largest abs_hi of the thread's sums
+template <class A, bool MANY>
+__device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, int c, int x, const bool first,
                                              typename A::V* sm, double* __restrict__ Zi) {
     using V = typename A::V;
     constexpr int RU = RU_DIR;
-    const int nidx = TEAM ? a.nlong : a.N;
+    const Team w = team_of<MANY>(a, l, a.cls[c], x);
     const V inv_e = a.inv_e, al = l.on && !first ? A::load(a.alpha + l.col) : A::zero(),
             be = l.on && !first ? A::load(a.beta + l.col) : A::zero();
-    const int step = TEAM ? a.ti : 1;
+    const int step = MANY ? w.rt : 1;
     unsigned m = 0;
-    for (int64_t g = g0;; g += gs) {
-        const int64_t idx = TEAM ? g : a.nlong + g * a.ti + l.il;
-        if ((TEAM ? g : a.nlong + g * a.ti) >= nidx) break;   // uniform over the CTA
+    for (unsigned j = w.j0; j < w.n; j += w.js) {   // uniform over the CTA
+        const unsigned idx = j + w.slot;
         V s0 = A::zero(), s1 = A::zero(), pp = A::zero();
         int b = 0, i = 0;
-        bool in = l.on && idx < nidx;
+        bool in = w.on && idx < w.n;
         if (in) {
-            const int4 ord = a.order[idx];
+            const int4 ord = a.order[w.i0 + idx];
             const int st = ord.y, en = ord.z;
             b = ord.x;
             i = ord.w;
             in = GLOBE_BOUNDS(b >= 0 && b < a.N && st >= 0 && st <= en && en <= a.Nrec && i >= 0 && i < a.N, 0x1301u);
             const V g0 = A::load(a.G + 2 * ((size_t)b * a.k + l.col)), g1 = A::load(a.G + 2 * ((size_t)b * a.k + l.col) + 1);
-            for (int q0 = st + (TEAM ? l.il : 0); in && q0 < en; q0 += RU * step) {
+            for (int q0 = st + (MANY ? w.rl : 0); in && q0 < en; q0 += RU * step) {
                 V rv[RU], pv[RU], xv[RU], tv[RU];
 #pragma unroll
                 for (int u = 0; u < RU; ++u) {
@@ -196,15 +236,13 @@ __device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, co
                 }
             }
         }
-        if (TEAM) {
-            auto add = [](V u, V w) { return A::add(u, w); };
-            s0 = over_individuals(s0, sm, a.ti, a.kc, l.il, add);
-            __syncthreads();
-            s1 = over_individuals(s1, sm, a.ti, a.kc, l.il, add);
-            __syncthreads();
-            pp = over_individuals(pp, sm, a.ti, a.kc, l.il, add);
-            __syncthreads();
-            in = in && l.il == 0;
+        if (MANY) {
+            V v[3] = {s0, s1, pp};
+            team_sum(a, w, v, sm);
+            s0 = v[0];
+            s1 = v[1];
+            pp = v[2];
+            in = in && w.rl == 0;
         }
         if (in) {
             const size_t o = (size_t)b * a.k + l.col;
@@ -221,13 +259,13 @@ __device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, co
 
 template <class A>
 __global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first, double* __restrict__ Zi, unsigned* zhi) {
-    __shared__ typename A::V sm[ST];
+    __shared__ typename A::V sm[3 * ST];
     __shared__ unsigned smu[ST];
     const Lane l = lane_of(a);
     smu[threadIdx.x] = 0u;
-    const int x = blockIdx.x;
-    const unsigned m = x < a.hctas ? dir_walk<A, true>(a, l, first, x, a.hctas, sm, Zi)
-                                   : dir_walk<A, false>(a, l, first, x - a.hctas, (int)gridDim.x - a.hctas, sm, Zi);
+    int x = blockIdx.x;
+    const int p = class_of(a, x);
+    const unsigned m = p < 2 ? dir_walk<A, true>(a, l, p, x, first, sm, Zi) : dir_walk<A, false>(a, l, 2, x, first, sm, Zi);
     if (zhi) {   // the scale of the product's input (k_col_max's part)
         __syncthreads();
         const int cl = threadIdx.x - l.il * a.kc;
@@ -430,24 +468,23 @@ __device__ void pcg_check(const PcgLoop& p, const double* rr, const double* pvp,
 
 // ---- k_update ---------------------------------------------------------------------
 
-// individuals g0, g0 + gs, ...: |r|^2 and r'z of the thread's records.  INIT: r stays (the solve's
+// the CTA's individuals: |r|^2 and r'z of the thread's records.  INIT: r stays (the solve's
 // start): g and r'z only
-template <class A, bool TEAM, bool INIT, int RU>
-__device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int64_t g0, int gs, typename A::V* sm,
+template <class A, bool MANY, bool INIT, int RU>
+__device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int c, int x, typename A::V* sm,
                                             typename A::V& rr, typename A::V& rz) {
     using V = typename A::V;
-    const int nidx = TEAM ? a.nlong : a.N;
+    const Team w = team_of<MANY>(a, l, a.cls[c], x);
     const V inv_e = a.inv_e, e = a.e, na = INIT || !l.on ? A::zero() : A::neg(A::load(a.alpha + l.col));
-    const int step = TEAM ? a.ti : 1;
+    const int step = MANY ? w.rt : 1;
     rr = rz = A::zero();
-    for (int64_t g = g0;; g += gs) {
-        const int64_t idx = TEAM ? g : a.nlong + g * a.ti + l.il;
-        if ((TEAM ? g : a.nlong + g * a.ti) >= nidx) break;   // uniform over the CTA
+    for (unsigned j = w.j0; j < w.n; j += w.js) {   // uniform over the CTA
+        const unsigned idx = j + w.slot;
         int b = 0, st = 0, en = 0;
         V s0 = A::zero(), s1 = A::zero(), a0 = A::zero(), a1 = A::zero();
-        bool in = l.on && idx < nidx;
+        bool in = w.on && idx < w.n;
         if (in) {
-            const int4 ord = a.order[idx];
+            const int4 ord = a.order[w.i0 + idx];
             b = ord.x;
             st = ord.y;
             en = ord.z;
@@ -464,12 +501,12 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
             const typename A::S* hb = a.H + 4 * (size_t)b;
             g0 = A::mul(A::madd(A::load(hb), s0, A::mul(A::load(hb + 1), s1)), inv_e);
             g1 = A::mul(A::madd(A::load(hb + 2), s0, A::mul(A::load(hb + 3), s1)), inv_e);
-            if (!TEAM || l.il == 0) {
+            if (!MANY || w.rl == 0) {
                 A::store(a.G + 2 * o, g0);
                 A::store(a.G + 2 * o + 1, g1);
             }
         };
-        const int q1 = st + (TEAM ? l.il : 0);
+        const int q1 = st + (MANY ? w.rl : 0);
         for (int q0 = q1; q0 < en; q0 += RU * step) {
             V rv[RU], pv[RU], tv[RU];
 #pragma unroll
@@ -496,13 +533,12 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
                 }
             }
         }
-        if (TEAM) {
-            auto add = [](V u, V w) { return A::add(u, w); };
-            over_individuals(s0, sm, a.ti, a.kc, l.il, add);
-            s0 = sm[threadIdx.x - l.il * a.kc];
-            __syncthreads();
-            over_individuals(s1, sm, a.ti, a.kc, l.il, add);
-            s1 = sm[threadIdx.x - l.il * a.kc];
+        if (MANY) {
+            V v[2] = {s0, s1};
+            team_sum(a, w, v, sm);
+            const int t0 = threadIdx.x - w.rl * a.kc;   // the slot's first thread of this column
+            s0 = sm[t0];
+            s1 = sm[ST + t0];
             __syncthreads();
         }
         if (in) {
@@ -530,12 +566,13 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
 template <class A, bool INIT, int RU>
 __global__ void __launch_bounds__(ST, RU == RU_UPD ? RES_UPD : 2) k_update(Args<A> a, PcgLoop loop) {
     using V = typename A::V;
-    __shared__ V sm[ST];
+    __shared__ V sm[2 * ST];
     const Lane l = lane_of(a);
-    const int x = blockIdx.x;
+    int x = blockIdx.x;
+    const int p = class_of(a, x);
     V rr, rz;
-    if (x < a.hctas) update_walk<A, true, INIT, RU>(a, l, x, a.hctas, sm, rr, rz);
-    else update_walk<A, false, INIT, RU>(a, l, x - a.hctas, (int)gridDim.x - a.hctas, sm, rr, rz);
+    if (p < 2) update_walk<A, true, INIT, RU>(a, l, p, x, sm, rr, rz);
+    else update_walk<A, false, INIT, RU>(a, l, 2, x, sm, rr, rz);
     const V v[2] = {rz, rr};
     // r'z (new) lands in rz's second half (k entries), |r|^2 in rr
     double* rz2 = a.rz + a.k;
@@ -636,20 +673,48 @@ int col_unscales(globe_ctx* ctx, const double* bb, int k, double* unsc) {
 // Column tiles of at most 128, near-equal: whole rows up to 128 columns, since a row's sectors are
 // shared with its neighbours' (two tiles of 33 of 65 columns read 1.6 times the vectors).  As many
 // individuals as leave at most 256 threads, or one more where that wastes fewer.  At most per_sm
-// CTAs per SM over all tiles, each taking every gridDim.x-th group of individuals.
+// CTAs per SM over all tiles for each class, each taking every gridDim.x-th group of individuals.
+//
+// Classes (by_length): one thread walks up to `one` records, ~0.5 us each in a chain: SOLVE_LONG where
+// one CTA's threads an SM suffice for the teams of the rest (N = 20k, records geometric with mean 10,
+// five columns: 6.44 ms a solve, 6.57 with 43), else the more the larger the solve, which takes
+// longer anyway.  Beyond, a team of TEAM threads, and
+// past 32 records for each of those (or half of `one`) the whole CTA.  A team doubles while its
+// threads have more than 16 records and all teams still run at once.  us an iteration with one
+// thread up to 32 and a CTA for each longer individual / with one thread for all / so (mixed; M =
+// 1000): N = 2000, 100-200 records, one column 101 / 248 / 62; N = 20000, 33-48, one 542 / 108 / 114;
+// 100-200, five 788 / 560 / 341; N = 100000, 40-60, one 2756 / 321 / 331, five 2863 / 592 / 598; N =
+// 20000, 3-10 and 600 of 300 records, five 102 / 358 / 98.  (A team from 32 records on whatever the
+// size: N = 20000, 28-36, one column 131, 98 so; a mix of single threads and teams has both tails.)
 struct Shape {
-    int kc, ti, threads, tiles, ctas, huge;
+    int kc, ti, threads, tiles, ctas;
+    Part cls[3];
 };
-static Shape shape(const globe_ctx* ctx, int kact, int n, int per_sm) {
+static Shape shape(const globe_ctx* ctx, int kact, int per_sm, bool by_length) {
+    auto& c = ctx->coh;
     Shape s;
     s.kc = div_up(kact, div_up(kact, 128));
     s.tiles = div_up(kact, s.kc);
     s.ti = 256 / s.kc;
     if (256 - s.ti * s.kc >= 32 && (s.ti + 1) * s.kc <= ST) ++s.ti;
     s.threads = div_up(s.ti * s.kc, 32) * 32;
-    const int most = std::max(1, per_sm * 152 / s.tiles);
-    s.ctas = std::max(1, std::min(most, div_up(n, s.ti)));
-    s.huge = std::min(std::max(1, 2 * 152 / s.tiles), (int)ctx->coh.nlong_solve);
+    auto most = [&](int per) { return std::max(1, per * 152 / s.tiles); };
+    auto longer = [&](int64_t records) {   // individuals of more records
+        return (int)(std::partition_point(c.long_len.begin(), c.long_len.end(), [&](int32_t l) { return l > records; }) -
+                     c.long_len.begin());
+    };
+    int rt = std::min(TEAM, s.ti);
+    const int64_t load = c.Nrec * kact;
+    int64_t one = SOLVE_LONG;
+    if ((int64_t)c.long_len.size() * TEAM * kact > 152 * 256) one += std::min<int64_t>(32, load / 100000) + load / 1000000;
+    const int n1 = by_length ? longer(one) : 0, n0 = by_length ? longer(rt * std::max<int64_t>(32, one / 2)) : 0;
+    while (n1 > n0 && 2 * rt <= std::min(TEAM_MOST, s.ti) && c.long_len[n0] > 16 * rt &&
+           div_up(n1 - n0, s.ti / (2 * rt)) <= most(PER_LONG))
+        rt *= 2;
+    s.cls[0] = Part{0, n0, std::min(n0, most(PER_LONG)), s.ti};
+    s.cls[1] = Part{n0, n1 - n0, std::min(div_up(n1 - n0, s.ti / rt), most(per_sm)), rt};
+    s.cls[2] = Part{n1, c.N - n1, std::min(div_up(c.N - n1, s.ti), most(per_sm)), 1};
+    s.ctas = s.cls[0].ctas + s.cls[1].ctas + s.cls[2].ctas;
     return s;
 }
 
@@ -673,7 +738,6 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
     a.order = c.order;
     a.cols = v.cols;
     a.N = c.N;
-    a.nlong = c.nlong_solve;
     a.Nrec = c.Nrec;
     a.k = v.k;
     a.kact = kact;
@@ -689,9 +753,9 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
     a.rz = v.rz;
     a.pvp = v.pvp;
     a.rr = v.rr;
-    a.slots = s.ctas + s.huge;
-    a.hctas = s.huge;
-    const size_t most = (PER_SUM + 2) * 152 + 2, groups = most / 32 + 1;   // for any number of active columns
+    a.slots = s.ctas;
+    std::copy(s.cls, s.cls + 3, a.cls);
+    const size_t most = (2 * PER_SUM + PER_LONG) * 152 + 3, groups = most / 32 + 1;   // for any number of active columns
     GLOBE_RET(ws(ctx, WS_PART, (most + groups) * 2 * v.k, &a.part));
     GLOBE_RET(tc_counters(ctx, (size_t)div_up(v.k, 128) * (groups + 1) + 1, &a.tiles_done));
     a.cnt = a.tiles_done + 1;
@@ -701,18 +765,17 @@ static int args(globe_ctx* ctx, const SolveVecs& v, int kact, const Shape& s, Ar
 
 template <class A>
 static int dir(globe_ctx* ctx, const SolveVecs& v, int kact, bool first, double* Zi, unsigned* zhi) {
-    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nlong_solve, PER_DIR);
+    const Shape s = shape(ctx, kact, PER_DIR, true);
     Args<A> a;
     GLOBE_RET(args(ctx, v, kact, s, &a));
-    k_dir<A><<<dim3(s.ctas + s.huge, s.tiles), s.threads, 0, ctx->stream>>>(a, first, Zi, zhi);
+    k_dir<A><<<dim3(s.ctas, s.tiles), s.threads, 0, ctx->stream>>>(a, first, Zi, zhi);
     GLOBE_LAUNCHED(ctx, "k_dir");
     return GLOBE_OK;
 }
 
 template <class A>
 static int step(globe_ctx* ctx, const SolveVecs& v, int kact, const double* GZ) {
-    Shape s = shape(ctx, kact, ctx->coh.N, PER_SUM);
-    s.huge = 0;
+    const Shape s = shape(ctx, kact, PER_SUM, false);
     Args<A> a;
     GLOBE_RET(args(ctx, v, kact, s, &a));
     k_step<A><<<dim3(s.ctas, s.tiles), s.threads, 0, ctx->stream>>>(a, GZ);
@@ -722,10 +785,10 @@ static int step(globe_ctx* ctx, const SolveVecs& v, int kact, const double* GZ) 
 
 template <class A, bool INIT>
 static int update(globe_ctx* ctx, const SolveVecs& v, int kact, const PcgLoop& loop) {
-    const Shape s = shape(ctx, kact, ctx->coh.N - ctx->coh.nlong_solve, PER_SUM);
+    const Shape s = shape(ctx, kact, PER_SUM, true);
     Args<A> a;
     GLOBE_RET(args(ctx, v, kact, s, &a));
-    const dim3 grid(s.ctas + s.huge, s.tiles);
+    const dim3 grid(s.ctas, s.tiles);
     if (grid.x * grid.y <= 2 * 152) k_update<A, INIT, 4><<<grid, s.threads, 0, ctx->stream>>>(a, loop);
     else k_update<A, INIT, RU_UPD><<<grid, s.threads, 0, ctx->stream>>>(a, loop);
     GLOBE_LAUNCHED(ctx, "k_update");
