@@ -1007,14 +1007,17 @@ static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double 
         return GLOBE_OK;
     };
     // Column grouping: the rule above, or -- for 9 or more columns, on first use of (k, digits,
-    // N, SNPs), with autotuning on, outside capture and profiling -- the faster of it and one
-    // group more, timed over two rounds (the first also tunes the groups' split counts).  Each column's digits and sums do not depend on its group, so every grouping
-    // gives the same bits and the last run's output stands.
+    // N, SNPs), with autotuning on, outside capture and profiling, and where out does not overlap Z,
+    // which the timed runs read again -- the faster of it and one group more, timed over two rounds
+    // (the first also tunes the groups' split counts).  Each column's digits and sums do not depend
+    // on its group, so every grouping gives the same bits and the last run's output stands.
     const std::vector<int64_t> key = {2, k, nd, N, (int64_t)g.Mk};
     if (!ctx->autotune || ctx->force_splits > 0 || k < 9) return run(ng);
     int chosen = ng;
     if (tuned_lookup(ctx, key, &chosen)) return run(chosen);
-    if (ctx->capturing || ctx->prof_on || ng + 1 > k) return run(ng);
+    const uintptr_t za = (uintptr_t)Z, oa = (uintptr_t)out, len = sizeof(double) * (uintptr_t)N * k;
+    const bool overlap = za < oa + len && oa < za + len;
+    if (ctx->capturing || ctx->prof_on || overlap || ng + 1 > k) return run(ng);
     const std::vector<int> cand = {ng, ng + 1};
     std::vector<float> ms;
     int best = 0;
