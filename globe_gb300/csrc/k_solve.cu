@@ -707,7 +707,8 @@ static Shape shape(const globe_ctx* ctx, int kact, int per_sm, bool by_length) {
     const int64_t load = c.Nrec * kact;
     int64_t one = SOLVE_LONG;
     if ((int64_t)c.long_len.size() * TEAM * kact > 152 * 256) one += std::min<int64_t>(32, load / 100000) + load / 1000000;
-    const int n1 = by_length ? longer(one) : 0, n0 = by_length ? longer(rt * std::max<int64_t>(32, one / 2)) : 0;
+    const int64_t team = std::max(one, rt * std::max<int64_t>(32, one / 2));   // not below `one`, which may be odd
+    const int n1 = by_length ? longer(one) : 0, n0 = by_length ? longer(team) : 0;
     while (n1 > n0 && 2 * rt <= std::min(TEAM_MOST, s.ti) && c.long_len[n0] > 16 * rt &&
            div_up(n1 - n0, s.ti / (2 * rt)) <= most(PER_LONG))
         rt *= 2;

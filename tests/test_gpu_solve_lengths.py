@@ -15,6 +15,8 @@ COHORTS = {
     "all-long": ([33 + (7 * i) % 40 for i in range(700)], (1, 5, 129)),   # teams only, several steps of a CTA
     "all-very-long": ([260 + i for i in range(40)], (1, 5, 129)),           # whole CTAs only
     "none-long": ([1 + (5 * i) % 32 for i in range(900)], (1, 5, 129)),
+    # 390 columns leave teams of two, of which each may take half of an odd limit
+    "two-a-team": ([65, 66, 67, 68] * 20 + [69, 70, 71, 30, 31] * 11, (390,)),
     "mixed": ([300, 290] + [60 + (11 * i) % 50 for i in range(900)] + [2, 9] * 300, (1, 20, 33)),
 }
 
@@ -32,7 +34,7 @@ def _load(ctx, orc, counts):
     ctx.set_vc(VC_F)
     s = orc.Solver(indiv, X, y, N, VC_F, packed=packed)
     s.precond_build()
-    return s, rng.standard_normal((len(indiv), 129))
+    return s, rng.standard_normal((len(indiv), 390))
 
 
 # both sides stop at a relative residual of 1e-11; with up to 513 records an individual V's condition
