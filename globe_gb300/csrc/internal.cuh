@@ -311,6 +311,8 @@ int geno_diag(globe_ctx* ctx, double* d);
 
 // k_grm_dense.cu
 int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
+// the columns c of the k whose words wide[c nw ..] are not all zero
+int dense_redo_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const unsigned* wide, int nw);
 int dense_apply_df(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
 int dense_diag(globe_ctx* ctx, double* d);
 

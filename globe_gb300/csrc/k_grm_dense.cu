@@ -1,7 +1,7 @@
 // k_grm_dense.cu -- dense GRM product from the packed lower triangle, where the tensor-core
 // digit planes of k_tc_dense.cu do not serve: on the FP64 pipe for GLOBE_PREC_FP64 (small
-// products; planes that cannot be held or would not hold every row to FP64), and in
-// double-float FP32 arithmetic for GLOBE_PREC_MIXED (planes that cannot be held).
+// products; planes that cannot be held or would not hold A exactly; columns that the digits do
+// not hold), and in double-float FP32 arithmetic for GLOBE_PREC_MIXED (planes that cannot be held).
 //
 //   out (N x k) = scale * A Z,  A(i,j) = lt[max(i,j)(max(i,j)+1)/2 + min(i,j)]
 //   (PCGsolver.cpp:1202-1213, varCompEst.cpp:531-558)
@@ -14,19 +14,40 @@
 // FP64 the kernel is bound by the FP64 pipe, not by these bytes.
 #include <algorithm>
 
+#include "df.cuh"
 #include "internal.cuh"
 
 namespace globe {
 
 constexpr int DT = 64;
 
-template <int KC>
+// REDO: of column chunk blockIdx.y, only the columns marked in wide (nw words each)
+template <int KC, bool REDO>
 __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt, int32_t N,
                                                    const double* __restrict__ Z, int kc, double scale,
-                                                   double* __restrict__ out) {
+                                                   double* __restrict__ out, const unsigned* __restrict__ wide, int nw) {
     __shared__ float At[DT][DT + 1];
     __shared__ double Zt[DT][KC];
+    __shared__ int redo[KC];
     const int tid = threadIdx.x;
+    if (REDO) {
+        const int c0 = blockIdx.y * KC;
+        kc = min(KC, kc - c0);
+        Z += (size_t)c0 * N;
+        out += (size_t)c0 * N;
+        if (tid < KC) redo[tid] = 0;
+        __syncthreads();
+        bool any = false;
+        for (int e = tid; e < kc * nw; e += 256)
+            if (wide[(size_t)c0 * nw + e]) {
+                redo[e / nw] = 1;
+                any = true;
+            }
+        if (!__syncthreads_or(any)) return;
+    }
+    bool mine = !REDO;   // whether one of the thread's columns is wanted
+    if (REDO)
+        for (int c = tid >> 6; c < kc; c += 4) mine = mine || redo[c];
     const int64_t I0 = (int64_t)blockIdx.x * DT;
     const int row = tid & (DT - 1);
     const int cg = tid >> 6;  // 0..3
@@ -63,12 +84,12 @@ __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt,
         }
         __syncthreads();
 #pragma unroll 4
-        for (int j = 0; j < DT; ++j) {
-            const double a = (double)At[row][j];
+        for (int j = 0; mine && j < DT; ++j) {
+            const double a = REDO ? df::f2d(At[row][j]) : (double)At[row][j];
 #pragma unroll
             for (int q = 0; q < (KC + 3) / 4; ++q) {
                 const int c = cg + 4 * q;
-                if (c < KC) acc[q] += a * Zt[j][c];
+                if (c < KC && (!REDO || redo[c])) acc[q] += a * Zt[j][c];
             }
         }
         __syncthreads();
@@ -78,9 +99,19 @@ __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt,
 #pragma unroll
         for (int q = 0; q < (KC + 3) / 4; ++q) {
             const int c = cg + 4 * q;
-            if (c < kc) out[i + (size_t)c * N] = scale * acc[q];
+            if (c < kc && (!REDO || redo[c])) out[i + (size_t)c * N] = scale * acc[q];
         }
     }
+}
+
+// ~4 us a product where no column is marked; with one marked 4.3 ms at N = 20k, 1.2 ms at 6007 (13.0
+// and 1.5 with the FP64 pipe's conversion instruction and its loop run for unmarked columns too).
+int dense_redo_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const unsigned* wide, int nw) {
+    const int32_t N = ctx->coh.N;
+    k_dense_f64<8, true><<<dim3(div_up(N, DT), div_up(k, 8)), 256, 0, ctx->stream>>>(ctx->gen.grm, N, Z, k, scale, out,
+                                                                                     wide, nw);
+    GLOBE_LAUNCHED(ctx, "k_dense_f64");
+    return GLOBE_OK;
 }
 
 int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out) {
@@ -92,8 +123,8 @@ int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, 
         double* oc = out + (size_t)c0 * N;
         int nb = div_up(N, DT);
         ProfScope ps(ctx, GLOBE_PROF_GRM_PASS1);
-        if (kc <= 4) k_dense_f64<4><<<nb, 256, 0, ctx->stream>>>(ctx->gen.grm, N, Zc, kc, scale, oc);
-        else k_dense_f64<8><<<nb, 256, 0, ctx->stream>>>(ctx->gen.grm, N, Zc, kc, scale, oc);
+        if (kc <= 4) k_dense_f64<4, false><<<nb, 256, 0, ctx->stream>>>(ctx->gen.grm, N, Zc, kc, scale, oc, nullptr, 0);
+        else k_dense_f64<8, false><<<nb, 256, 0, ctx->stream>>>(ctx->gen.grm, N, Zc, kc, scale, oc, nullptr, 0);
         GLOBE_LAUNCHED(ctx, "k_dense_f64");
     }
     return GLOBE_OK;

@@ -20,12 +20,15 @@
 // tiles of the right-hand sides (kpos), rows padded to a multiple of 256.
 // The planes are full squares (both triangles), 7 N^2 bytes at DA = 7.
 //
-// GLOBE_PREC_FP64 takes DA = 12 planes (A within 2^-59 max|A|: a float32 entry of at least
-// 2^-35 max|A| exactly) and 12 digits of Z (2^-60 of each column's largest entry), and folds
-// the sums in double-double with one rounding at the end.  It holds every row to FP64 as long
-// as no diagonal entry is below 2^-5 max|A| (then the FP64 pipe runs instead).  N = 20k,
-// k = 16 streams 12 N^2 = 4.8 GB in 0.91 ms with its epilogue (5.3 TB/s); 25.1 ms on the FP64
-// pipe, which it was bound by.
+// GLOBE_PREC_FP64 takes the 12 to 14 planes that hold every entry of A exactly and 16 digits of Z,
+// which hold an entry exactly or to 2^-53 of itself down to 2^-25 of the column's largest; it folds
+// the exact sums in double-double with one rounding at the end.  So each row is held to FP64 by
+// itself: within 2^-53 (|A| |z|)_i and the rounding, whatever the zeros of A and the magnitudes in z.
+// A column with smaller entries, or a NaN or an infinity, is formed on the FP64 pipe after the
+// others (k_digits marks it; ~1 normal column in 1000 at N = 20k), and a matrix that 14 planes do not hold stays
+// there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its epilogue; 25.1 ms on
+// the FP64 pipe, which it was bound by.  (12 digits of Z and 12 planes whatever A: 0.93 ms, but a row
+// that a column's largest entries do not enter lost up to all of its digits.)
 //
 // Kernel (one CTA = 2 x 128 rows x one K range, M=128 x N=NMMA MMAs per row tile):
 //   warp 0     TMA of both operands per stage: two 128 x 128-byte tiles of the
@@ -46,7 +49,8 @@ namespace globe {
 namespace tc {
 
 constexpr int DA_MAX = 7;        // digit planes of A at most (GLOBE_PREC_MIXED)
-constexpr int DA64 = 12;         // digit planes of A (GLOBE_PREC_FP64)
+constexpr int DA64 = 12;         // digit planes of A at least (GLOBE_PREC_FP64),
+constexpr int DA64_MAX = 14;     // and at most
 constexpr int DMT = 2;           // row tiles per CTA
 constexpr int DROWS = DMT * BM;  // rows per CTA
 constexpr int DK_MAX_CHUNKS = 512;   // K <= 2^16 per CTA: |sum| <= 256 * 2^16 = 2^24, exact in FP32
@@ -168,28 +172,30 @@ __global__ void __launch_bounds__(256, 1)
 }
 
 // max |A| over the packed triangle as float bits (non-negative floats order like their bits),
-// whether any entry is not finite, and the smallest diagonal entry (negative ones count as 0)
-__global__ void k_dense_absmax(const float* __restrict__ lt, int64_t n, int32_t N, unsigned* __restrict__ out) {
-    unsigned mx = 0, bad = 0, dmin = 0x7f800000u;
+// whether any entry is not finite, and LSB0 + the exponent of the lowest bit that any entry holds
+constexpr int LSB0 = 256;
+__global__ void k_dense_scan(const float* __restrict__ lt, int64_t n, unsigned* __restrict__ out) {
+    unsigned mx = 0, bad = 0, lsb = 0x7fffffffu;
     const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
     for (int64_t e = t0; e < n; e += nt) {
         const float v = lt[e];
+        const unsigned b = __float_as_uint(v) & 0x7fffffffu, ex = b >> 23;
         if (!isfinite(v)) bad = 1;
-        else mx = max(mx, __float_as_uint(fabsf(v)));
-    }
-    for (int64_t i = t0; i < N; i += nt) {
-        const float v = lt[i * (i + 1) / 2 + i];
-        dmin = min(dmin, v > 0.0f ? __float_as_uint(v) : 0u);
+        else if (b) {
+            mx = max(mx, b);
+            const unsigned m = ex ? (b & 0x7fffffu) | 0x800000u : b;   // v = m 2^(max(ex, 1) - 150)
+            lsb = min(lsb, LSB0 + max(ex, 1u) - 150u + (unsigned)__ffs((int)m) - 1u);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
         bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-        dmin = min(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
+        lsb = min(lsb, __shfl_xor_sync(0xffffffffu, lsb, o));
     }
     if ((threadIdx.x & 31) == 0) {
         atomicMax(out, mx);
         if (bad) atomicOr(out + 1, 1u);
-        atomicMin(out + 2, dmin);
+        atomicMin(out + 2, lsb);
     }
 }
 
@@ -199,7 +205,8 @@ __global__ void k_dense_absmax(const float* __restrict__ lt, int64_t n, int32_t 
 // plane.  Position P of a group of 16 holds column 2P (P < 8) or 2(P-8)+1 (the inverse of
 // kpos).  x 2^-eA is rounded once to I = round(x 2^-eA 32^(DA-1)); its balanced base-32
 // digits are peeled off from the least significant end (d = ((I + 16) mod 32) - 16); the
-// leading digit is what remains, in [-16, 16].
+// leading digit is what remains, in [-16, 16].  More than DA64 planes: those of the remainder of
+// the first DA64, as k_digits has them.
 template <int DA>
 __global__ void __launch_bounds__(256) k_dense_digits(const float* __restrict__ lt, int32_t N, int eA,
                                                       uint8_t* __restrict__ D, int64_t np) {
@@ -229,24 +236,37 @@ __global__ void __launch_bounds__(256) k_dense_digits(const float* __restrict__ 
         }
     }
     __syncthreads();
-    const double sc = ldexp(1.0, DBITS * (DA - 1) - eA);   // a power of two: x * sc is exact
+    constexpr int DI = DA < DA64 ? DA : DA64;
+    const double sc = ldexp(1.0, DBITS * (DI - 1) - eA);   // a power of two: x * sc is exact
 #pragma unroll 1
     for (int w = tid; w < DT * (DT / 4); w += 256) {
         const int m = w >> 4, pl = (w & 15) * 4;   // row in the block, first K position in the block
         long long I[4];
+        int L[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int p = pl + q, base = p & ~15, pp = p & 15;
             const int jl = base + (pp < 8 ? 2 * pp : 2 * (pp - 8) + 1);
-            I[q] = __double2ll_rn((double)At[m][jl] * sc);
+            const double x = (double)At[m][jl] * sc;
+            I[q] = __double2ll_rn(x);
+            if constexpr (DA > DA64) L[q] = __double2int_rn((x - (double)I[q]) * (double)(1 << (DBITS * (DA - DA64))));
         }
         uint32_t word[DA];
 #pragma unroll
         for (int d = 0; d < DA; ++d) word[d] = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
+            if constexpr (DA > DA64) {
 #pragma unroll
-            for (int d = DA - 1; d > 0; --d) {
+                for (int d = DA - 1; d > DA64; --d) {
+                    const int dg = ((L[q] + DHALF) & (2 * DHALF - 1)) - DHALF;
+                    L[q] = (L[q] - dg) >> DBITS;
+                    word[d] |= e4m3_int(dg) << (8 * q);
+                }
+                word[DA64] |= e4m3_int(L[q]) << (8 * q);
+            }
+#pragma unroll
+            for (int d = DI - 1; d > 0; --d) {
                 const int dg = (int)((I[q] + DHALF) & (2 * DHALF - 1)) - DHALF;
                 I[q] = (I[q] - dg) >> DBITS;   // exact: I - dg is a multiple of 32
                 word[d] |= e4m3_int(dg) << (8 * q);
@@ -340,32 +360,33 @@ __global__ void __launch_bounds__(256) k_dense_combine(const float* __restrict__
     out[i + c * ldo] = bad ? colinfo[2 * c + 1] : v;
 }
 
-// The FP64 product's epilogue: DA64 + ND64 - 1 = 23 weights in five exact chunks, added in
+// The FP64 product's epilogue: up to DA64_MAX + NDZ - 1 = 29 weights in six exact chunks, added in
 // double-double, and 2^e_c in two factors.
 template <int G>
 __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict__ part, int nsplit, int nmma,
-                                                         int64_t ldp, int32_t N, int64_t np,
+                                                         int64_t ldp, int32_t N, int64_t np, int da,
                                                          const double* __restrict__ colinfo, double sA, double scale,
                                                          double* __restrict__ out, int64_t ldo,
                                                          unsigned* __restrict__ zhi) {
-    constexpr int NT = DA64 + ND64 - 1;
-    static_assert(NT <= 25, "five chunks of five weights");
+    constexpr int NT = DA64_MAX + NDZ - 1;
+    static_assert(NT <= 30, "six chunks of five weights");
     const int c = blockIdx.y;
     constexpr int DC_I = 256 / G;
     const int64_t i = (int64_t)blockIdx.x * DC_I + threadIdx.x % DC_I;
     if (blockIdx.x == 0 && threadIdx.x == 0) zhi[c] = 0u;
     long long T[NT];
-    dense_weights<DA64, ND64, G>(part, nsplit, nmma, ldp, np, DA64, i, i < N, c, T);
+    dense_weights<DA64_MAX, NDZ, G>(part, nsplit, nmma, ldp, np, da, i, i < N, c, T);
     if (threadIdx.x >= DC_I || i >= N) return;
     const int e = (int)colinfo[2 * c];
     const double ea = pow2i(e / 2), eb = pow2i(e - e / 2), bad = colinfo[2 * c + 1];
     double h = 0.0, l = 0.0;
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
+    for (int q = 0; q < 6; ++q) {
         long long C = 0;
 #pragma unroll
         for (int m = 0; m < 5; ++m) C = C * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
-        dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : 0x1p-100), 0.0);
+        dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : q == 4 ? 0x1p-100 : 0x1p-125),
+               0.0);
     }
     out[i + c * ldo] = (h + l) * sA * scale * ea * eb + bad;
 }
@@ -376,16 +397,39 @@ __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict
 
 using namespace tc;
 
-// (Re)builds digit planes: set 0 for the context's digit count, set 1 for the FP64 products
+// (Re)builds digit planes: set 0 for the context's digit count, set 1 for the FP64 products, which
+// take the DA64 to DA64_MAX planes that hold every entry of A exactly
 static int dense_digit_planes(globe_ctx* ctx, int set) {
     auto& g = ctx->gen;
     auto& a = g.adig[set];
-    const int da = set ? DA64 : std::min(DA_MAX, ctx->digits);
-    if (a.state != 0 && a.da == da) return GLOBE_OK;
+    int da = set ? DA64 : std::min(DA_MAX, ctx->digits);
+    if (a.state != 0 && (set || a.da == da)) return GLOBE_OK;
     dfree(ctx, a.p);
     a.p = nullptr;
     a.state = -1;   // until the planes are complete
+    a.da = da;
     const int32_t N = ctx->coh.N;
+    unsigned* mx;   // words 1-3 of the error-flag slot (word 0 is the kernels' flag): max |A| bits, non-finite, lowest bit
+    GLOBE_RET(tc_err_word(ctx, &mx));
+    GLOBE_CK(ctx, cudaMemsetAsync(mx + 1, 0, 2 * sizeof(unsigned), ctx->stream));
+    GLOBE_CK(ctx, cudaMemsetAsync(mx + 3, 0x7f, sizeof(unsigned), ctx->stream));
+    const int64_t nelt = (int64_t)N * (N + 1) / 2;
+    k_dense_scan<<<(unsigned)std::min<int64_t>(div_up(nelt, 256), 152 * 8), 256, 0, ctx->stream>>>(g.grm, nelt, mx + 1);
+    GLOBE_LAUNCHED(ctx, "k_dense_scan");
+    unsigned h[3] = {0, 0, 0};
+    GLOBE_CK(ctx, cudaMemcpyAsync(h, mx + 1, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
+    if (h[1]) return GLOBE_OK;   // a non-finite entry: the other kernels propagate it
+    float amax;
+    std::memcpy(&amax, &h[0], sizeof(float));
+    int E = 0;
+    if (amax > 0.0f) std::frexp((double)amax, &E);
+    a.e = E - (DBITS - 1);   // max|A| 2^-eA in [8, 16)
+    if (set && amax > 0.0f) {   // the grid's step 2^(eA - 5 (da - 1)) down to the lowest bit of any entry
+        da = std::max(DA64, 1 + div_up(a.e - ((int)h[2] - LSB0), DBITS));
+        if (da > DA64_MAX) return GLOBE_OK;
+        a.da = da;
+    }
     const int64_t np = ((int64_t)N + BM - 1) / BM * BM;
     const int64_t rows = ((int64_t)da * np + DROWS - 1) / DROWS * DROWS;
     const size_t bytes = (size_t)rows * (size_t)np;
@@ -399,30 +443,7 @@ static int dense_digit_planes(globe_ctx* ctx, int set) {
         g.adig[1] = Genetic::Planes();
         GLOBE_CK(ctx, cudaMemGetInfo(&fr, &tot));
     }
-    if (bytes + room > fr || rows > INT32_MAX) {
-        a.da = da;
-        return GLOBE_OK;
-    }
-    unsigned* mx;   // words 1-3 of the error-flag slot (word 0 is the kernels' flag): max |A| bits, non-finite, min A_ii
-    GLOBE_RET(tc_err_word(ctx, &mx));
-    GLOBE_CK(ctx, cudaMemsetAsync(mx + 1, 0, 2 * sizeof(unsigned), ctx->stream));
-    GLOBE_CK(ctx, cudaMemsetAsync(mx + 3, 0x7f, sizeof(unsigned), ctx->stream));
-    const int64_t nelt = (int64_t)N * (N + 1) / 2;
-    k_dense_absmax<<<(unsigned)std::min<int64_t>(div_up(nelt, 256), 152 * 8), 256, 0, ctx->stream>>>(g.grm, nelt, N,
-                                                                                                    mx + 1);
-    GLOBE_LAUNCHED(ctx, "k_dense_absmax");
-    unsigned h[3] = {0, 0, 0};
-    GLOBE_CK(ctx, cudaMemcpyAsync(h, mx + 1, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    GLOBE_CK(ctx, cudaStreamSynchronize(ctx->stream));
-    a.da = da;
-    if (h[1]) return GLOBE_OK;   // a non-finite entry: the other kernels propagate it
-    float amax, dmin;
-    std::memcpy(&amax, &h[0], sizeof(float));
-    std::memcpy(&dmin, &h[2], sizeof(float));
-    if (set && !(dmin >= amax * 0x1p-5f)) return GLOBE_OK;   // a row too small for the common grid
-    int E = 0;
-    if (amax > 0.0f) std::frexp((double)amax, &E);
-    a.e = E - (DBITS - 1);   // max|A| 2^-eA in [8, 16)
+    if (bytes + room > fr || rows > INT32_MAX) return GLOBE_OK;
     GLOBE_RET(dalloc(ctx, &a.p, bytes));
     if (rows > da * np)
         GLOBE_CK(ctx, cudaMemsetAsync(a.p + (size_t)da * np * np, 0, (size_t)(rows - da * np) * np, ctx->stream));
@@ -433,7 +454,9 @@ static int dense_digit_planes(globe_ctx* ctx, int set) {
         case 4: k_dense_digits<4><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
         case 5: k_dense_digits<5><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
         case 6: k_dense_digits<6><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
-        case DA64: k_dense_digits<DA64><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 12: k_dense_digits<12><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 13: k_dense_digits<13><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
+        case 14: k_dense_digits<14><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
         default: k_dense_digits<7><<<grid, 256, 0, ctx->stream>>>(g.grm, N, a.e, a.p, np); break;
     }
     GLOBE_LAUNCHED(ctx, "k_dense_digits");
@@ -500,10 +523,13 @@ static int dense_cps(globe_ctx* ctx, int tiles, int nchunks, int nmma) {
     return best;
 }
 
-// out (N x kg) = scale * A Z for one group of <= 256 / ND columns
+static int digit_ctas(int64_t np) { return (int)std::min<int64_t>(div_up(np / 4, 256), 1024); }
+
+// out (N x kg) = scale * A Z for one group of <= 256 / ND columns; wide: k_digits' words
 template <int ND>
-static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st) {
-    constexpr bool F64 = ND == ND64;
+static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st,
+                       unsigned* wide) {
+    constexpr bool F64 = ND == NDZ;
     const auto& a = ctx->gen.adig[F64 ? 1 : 0];
     const int32_t N = ctx->coh.N;
     const int64_t np = a.np;
@@ -524,8 +550,8 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     CUtensorMap mA, mB;
     GLOBE_RET(make_map(ctx, &mA, a.p, (uint64_t)np, (uint64_t)rows, BK, BM, true));
     GLOBE_RET(make_map(ctx, &mB, D, (uint64_t)np, (uint64_t)nmma, BK, (uint32_t)nmma, true));
-    k_digits<ND, false><<<dim3((unsigned)std::min<int64_t>(div_up(np / 4, 256), 1024), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, st.zhi, col, D, np, nullptr, nullptr, nmma - kg * ND);
+    k_digits<ND, false><<<dim3((unsigned)digit_ctas(np), kg), 256, 0, ctx->stream>>>(
+        Z, N, N, st.zhi, col, D, np, nullptr, nullptr, nmma - kg * ND, wide);
     GLOBE_LAUNCHED(ctx, "k_digits");
     {
         ProfScope p(ctx, GLOBE_PROF_GRM_PASS1);
@@ -537,8 +563,8 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
         constexpr int G = decltype(split)::value;
         const dim3 gc((unsigned)div_up(N, 256 / G), kg);
         if constexpr (F64)
-            k_dense_combine64<G><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, col, std::ldexp(1.0, a.e - 20),
-                                                              scale, out, N, st.zhi);
+            k_dense_combine64<G><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
+                                                              std::ldexp(1.0, a.e - 20), scale, out, N, st.zhi);
         else
             k_dense_combine<ND, G><<<gc, 256, 0, ctx->stream>>>(P, splits, nmma, ldp, N, np, a.da, col,
                                                                 std::ldexp(scale, a.e), out, N, st.zhi);
@@ -549,23 +575,27 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     return GLOBE_OK;
 }
 
-static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out, const TcStat& st) {
+static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out, const TcStat& st,
+                          unsigned* wide) {
     switch (nd) {
-        case 2: return dense_group<2>(ctx, Z, kg, scale, out, st);
-        case 3: return dense_group<3>(ctx, Z, kg, scale, out, st);
-        case 4: return dense_group<4>(ctx, Z, kg, scale, out, st);
-        case 5: return dense_group<5>(ctx, Z, kg, scale, out, st);
-        case 6: return dense_group<6>(ctx, Z, kg, scale, out, st);
-        case 7: return dense_group<7>(ctx, Z, kg, scale, out, st);
-        case 8: return dense_group<8>(ctx, Z, kg, scale, out, st);
-        case 9: return dense_group<9>(ctx, Z, kg, scale, out, st);
-        case ND64: return dense_group<ND64>(ctx, Z, kg, scale, out, st);
+        case 2: return dense_group<2>(ctx, Z, kg, scale, out, st, wide);
+        case 3: return dense_group<3>(ctx, Z, kg, scale, out, st, wide);
+        case 4: return dense_group<4>(ctx, Z, kg, scale, out, st, wide);
+        case 5: return dense_group<5>(ctx, Z, kg, scale, out, st, wide);
+        case 6: return dense_group<6>(ctx, Z, kg, scale, out, st, wide);
+        case 7: return dense_group<7>(ctx, Z, kg, scale, out, st, wide);
+        case 8: return dense_group<8>(ctx, Z, kg, scale, out, st, wide);
+        case 9: return dense_group<9>(ctx, Z, kg, scale, out, st, wide);
+        case NDZ: return dense_group<NDZ>(ctx, Z, kg, scale, out, st, wide);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
 
 // out (N x k) = scale * A Z from the planes, nd digits per column
 static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out, bool zhi_ready) {
+    const int nw = digit_ctas(ctx->gen.adig[nd == NDZ ? 1 : 0].np);
+    unsigned* wide = nullptr;
+    if (nd == NDZ) GLOBE_RET(ws(ctx, WS_TC_U, (size_t)k * nw, &wide));
     TcStat st;
     GLOBE_RET(tc_stat_fill(ctx, Z, ctx->coh.N, k, &zhi_ready, &st));
     const int gmax = 256 / nd;   // MMA width <= 256; near-equal groups
@@ -573,11 +603,11 @@ static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double
     for (int gi = 0, c0 = 0; gi < ng; ++gi) {
         const int kg = k / ng + (gi < k % ng ? 1 : 0);
         GLOBE_RET(dense_group_nd(ctx, nd, Z + (size_t)c0 * ctx->coh.N, kg, scale, out + (size_t)c0 * ctx->coh.N,
-                                 st.from(c0)));
+                                 st.from(c0), wide ? wide + (size_t)c0 * nw : nullptr));
         c0 += kg;
     }
     ctx->stat_dirty = false;
-    return GLOBE_OK;
+    return wide ? dense_redo_fp64_pipe(ctx, Z, k, scale, out, wide, nw) : GLOBE_OK;
 }
 
 int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
@@ -588,14 +618,15 @@ int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double*
 
 // The FP64 product, by its size N N k (FP64 pipe / planes, us a product):
 //  - inside a solve, which repeats the product and so pays for building the planes (0.2 ms at
-//    N = 200, 4.4 ms at 20k), the planes from 1e5 on (2e5: 64 / 34; 1.6e7: 471 / 41;
-//    6.4e9: 25118 / 909);
+//    N = 200, 4.4 ms at 20k), the planes from 1e5 on (2e5: 64 / 36; 1.6e7: 471 / 44;
+//    6.4e9: 25118 / 1010);
 //  - a single operator call from 4e6 on, where the first call, with the planes to build, costs
 //    about the same on either (1e6: 191 / 288; 4e6: 352 / 314; 4e8: 8484 / 5179).
 // The choice depends on the sizes only; the FP64 pipe also runs where the planes cannot be held or
-// a row is too small for their common grid.
-// Error against 128-bit sums (N = 2500; normal, constant, count, lognormal, unit and wide-range
-// columns): at most 7.8e-17 of the column, FP64 pipe up to 1.9e-15.
+// do not hold A exactly, and for single columns (top of the file).
+// Error against 128-bit sums (N = 2500; normal, constant, count, lognormal and unit columns): at most
+// 1.0e-16 of the column and of (|A| |z|)_i row by row; FP64 pipe (and a column over 12 decades, which
+// it forms) up to 2.4e-15.
 #ifndef F64_DENSE_SOLVE_MIN
 #define F64_DENSE_SOLVE_MIN 1e5
 #endif
@@ -609,9 +640,16 @@ bool dense_f64_tc(const globe_ctx* ctx, int k) { return ctx->gen.adig[1].state =
 
 int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     auto& a = ctx->gen.adig[1];
+    const size_t len = (size_t)ctx->coh.N * k;
+    if (Z < out + len && out < Z + len) {   // every column is read again after out is written
+        double* zc;
+        GLOBE_RET(ws(ctx, WS_W, len, &zc));
+        GLOBE_CK(ctx, cudaMemcpyAsync(zc, Z, sizeof(double) * len, cudaMemcpyDeviceToDevice, ctx->stream));
+        Z = zc;
+    }
     if (a.state >= 0 && f64_dense_size(ctx, k)) {
         int rc = dense_digit_planes(ctx, 1);
-        if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, ND64, Z, k, scale, out, zhi_ready);
+        if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, NDZ, Z, k, scale, out, zhi_ready);
         if (a.state == 1 && rc != GLOBE_ERR_NOMEM) return rc;
         if (rc != GLOBE_OK && rc != GLOBE_ERR_NOMEM) return rc;
         if (rc == GLOBE_ERR_NOMEM) {   // give the planes back

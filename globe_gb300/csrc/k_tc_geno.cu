@@ -1088,8 +1088,8 @@ int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double*
     return geno_apply_fp64_pipe(ctx, Z, k, scale, out);
 }
 
-// The tensor-core kernels' error word: word 0 of the WS_TC_ERR slot (words 1-2 serve
-// k_dense_absmax).  Cleared once, when the slot is created; the kernels only set bits in it
+// The tensor-core kernels' error word: word 0 of the WS_TC_ERR slot (words 1-3 serve
+// k_dense_scan).  Cleared once, when the slot is created; the kernels only set bits in it
 // and tc_check_error reads and clears it, so a timeout in any product of a solve is still
 // reported when the solve ends.
 int tc_err_word(globe_ctx* ctx, unsigned** err) {

@@ -24,6 +24,7 @@ constexpr int DHALF = 1 << (DBITS - 1);   // 16: digits in [-16, 16]
 constexpr int NDIG = 9;           // digits per right-hand-side column by default (45 bits)
 constexpr int MIN_DIG = 2;        // fewest digits a context may ask for (globe_set_digits)
 constexpr int ND64 = 12;          // digits per column of the GLOBE_PREC_FP64 products (59 bits: |I| < 2^59)
+constexpr int NDZ = 16;           // ... of the dense ones: 12 and 4 more, which hold what those leave
 
 // The tile-blocked genotype copies hold "tile codes", 2 bits per genotype like the PLINK
 // codes they are made from (re-encoded once, by recode_tile), equal to the genotype:
@@ -258,18 +259,23 @@ __global__ void k_col_max(const double* __restrict__ X, int64_t n, int64_t ld, u
 // ND, is added to isum[2c] 2^30 + isum[2c+1] in units of 2^(e - 55) (integer atomics: the same
 // bits in any order); clear[2c], clear[2c+1] are set to zero
 // (an isum no longer in use).  The npad digit rows after the last column's are set to zero (the MMA
-// width is a multiple of 16; a memset of them cost a launch of its own).  With ND64 digits (the FP64 products) the scaling takes two factors
-// where one would leave the range of a double.
+// width is a multiple of 16; a memset of them cost a launch of its own).  With ND64 digits and more
+// (the FP64 products) the scaling takes two factors where one would leave the range of a double.
+// NDZ digits: the first ND64 as above, then those of the remainder x 2^-e 32^(ND64-1) - I, which is
+// exact in a double and at most 1/2.  wide[c gridDim.x + CTA] says whether an entry of the CTA has bits
+// below the last digit (it is then more than 2^25 below the column's largest), or the column is bad.
 template <int ND, bool GENO>
 __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, const unsigned* __restrict__ hi,
                          double* __restrict__ colinfo, uint8_t* __restrict__ D, int64_t kpad,
-                         unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear, int npad) {
+                         unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear, int npad,
+                         unsigned* __restrict__ wide = nullptr) {
+    constexpr int NI = ND < ND64 ? ND : ND64;   // digits of I
     const int c = blockIdx.y;
     const unsigned h = hi[c];
     const int pad = c == (int)gridDim.y - 1 ? npad : 0;
-    const int e = col_exp<ND>(h), sh = DBITS * (ND - 1) - e;
-    const double sc = pow2i(ND == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
-    const double sc2 = ND == ND64 ? pow2i(sh - min(sh, 1000)) : 1.0;
+    const int e = col_exp<NI>(h), sh = DBITS * (NI - 1) - e;
+    const double sc = pow2i(NI == ND64 ? min(sh, 1000) : sh);   // a power of two: x * sc is exact
+    const double sc2 = NI == ND64 ? pow2i(sh - min(sh, 1000)) : 1.0;
     const bool bad = col_bad(h);   // non-finite column: zero digits
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         colinfo[2 * c] = (double)e;
@@ -278,20 +284,27 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
     }
     const int64_t nw = kpad >> 2;
     long long sum_hi = 0, sum_lo = 0;
+    bool lost = bad;
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
         const int64_t P = w << 2, base = P & ~(int64_t)15;
         const int pl = (int)(P & 15);
         const int mult = GENO ? geno_digit_mult(pl >> 2) : 1;   // GENO: rows 4 q + pl/4 share its parity
         long long I[4];
+        int L[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int pq = pl + q;
             const int64_t src = base + (GENO ? 4 * q + (pl >> 2) : (pq < 8 ? 2 * pq : 2 * (pq - 8) + 1));
             double x = (src < n && !bad) ? X[src + c * ld] * sc : 0.0;
-            if (ND == ND64) x *= sc2;
+            if (NI == ND64) x *= sc2;
             I[q] = __double2ll_rn(x);
+            if constexpr (ND > ND64) {
+                const double r = (x - (double)I[q]) * (double)(1 << (DBITS * (ND - ND64)));
+                L[q] = __double2int_rn(r);
+                lost = lost || (double)L[q] != r;
+            }
             if (isum) {
-                const long long J = ND == ND64 ? I[q] : __double2ll_rn(x * pow2i(DBITS * (ND64 - ND)));
+                const long long J = NI == ND64 ? I[q] : __double2ll_rn(x * pow2i(DBITS * (ND64 - ND)));
                 sum_hi += J >> 30;
                 sum_lo += J & ((1ll << 30) - 1);
             }
@@ -301,8 +314,17 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
         for (int j = 0; j < ND; ++j) word[j] = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
+            if constexpr (ND > ND64) {
 #pragma unroll
-            for (int j = ND - 1; j > 0; --j) {
+                for (int j = ND - 1; j > ND64; --j) {
+                    const int d = ((L[q] + DHALF) & (2 * DHALF - 1)) - DHALF;
+                    L[q] = (L[q] - d) >> DBITS;
+                    word[j] |= e4m3_int(mult * d) << (8 * q);
+                }
+                word[ND64] |= e4m3_int(mult * L[q]) << (8 * q);   // |L| <= 2^(5 (ND - ND64) - 1): in [-16, 16]
+            }
+#pragma unroll
+            for (int j = NI - 1; j > 0; --j) {
                 const int d = (int)((I[q] + DHALF) & (2 * DHALF - 1)) - DHALF;
                 I[q] = (I[q] - d) >> DBITS;   // exact: I - d is a multiple of 32
                 word[j] |= e4m3_int(mult * d) << (8 * q);
@@ -323,6 +345,10 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
             atomicAdd(isum + 2 * c, (unsigned long long)sum_hi);
             atomicAdd(isum + 2 * c + 1, (unsigned long long)sum_lo);
         }
+    }
+    if constexpr (ND > ND64) {
+        const int any = __syncthreads_or(lost);
+        if (threadIdx.x == 0) wide[(size_t)c * gridDim.x + blockIdx.x] = any ? 1u : 0u;
     }
 }
 

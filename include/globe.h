@@ -53,8 +53,10 @@ extern "C" {
                                final FP64 rounding -- closer to the exact product than sums
                                on the FP64 pipe, which run where the product is small or the
                                second genotype copy does not fit in device memory.  Dense GRM
-                               products the same way, from 12 digit planes of A (12 N^2 bytes;
-                               A within 2^-59 max|A|) */
+                               products from 12 to 14 digit planes that hold A exactly (12 to
+                               14 N^2 bytes) and 16 digits a column, each row within a few
+                               units of 2^-53 (|A| |z|)_i; columns with entries that those
+                               digits do not hold, and the non-finite ones, on the FP64 pipe */
 #define GLOBE_PREC_MIXED 1  /* genotype GRM product on the FP8 tensor cores with exact
                                base-32 digit slicing of the right-hand sides (9 digits =
                                45 bits by default, matches FP64 to ~1e-13; see
