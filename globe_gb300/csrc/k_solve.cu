@@ -27,7 +27,8 @@
 // Two arithmetics: FP64 (GLOBE_PREC_FP64), and double-float pairs (df.cuh) in the 8 bytes of
 // each double under GLOBE_PREC_MIXED, column c scaled by a power of two (col_unscale) to a
 // unit-size right-hand side.  What stays FP64 there: the GRM product's input and output, the
-// per-column scalars, and every sum past a thread's own individuals.
+// per-column scalars, and every sum past FLUSH individuals of a thread (a team's sums over one
+// individual's records are in double-float).
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -83,6 +84,40 @@ struct ArithDF {
     static __device__ __forceinline__ V add(V a, V b) { return df::add(a, b); }
     static __device__ __forceinline__ V mul(V a, V b) { return df::mul(a, b); }
     static __device__ __forceinline__ V madd(V a, V b, V c) { return df::madd(a, b, c); }
+};
+
+// A thread's sums over individuals: in the solve's arithmetic over FLUSH of them, past those in FP64,
+// in the thread's places of tot (shared memory: registers for them spilled).  FP64 sums stay in `part`.
+// (Double-float over all of a CTA's individuals, as many as N asks for: no faster at N = 100k, five
+// columns 88.4 ms a solve either way, 37 226 and 228.)
+constexpr int FLUSH = 8;
+template <class A, int NQ>
+struct Sums {
+    typename A::V part[NQ];
+    double* tot;   // NQ x ST
+    int n = 0;
+    static constexpr bool FLUSHED = !std::is_same_v<typename A::V, double>;
+    __device__ __forceinline__ explicit Sums(double* sm) : tot(sm) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            part[q] = A::zero();
+            if (FLUSHED) tot[q * ST + threadIdx.x] = 0.0;
+        }
+    }
+    // after each individual
+    __device__ __forceinline__ void next() {
+        if (FLUSHED && ++n == FLUSH) {
+            n = 0;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                tot[q * ST + threadIdx.x] += A::to_double(part[q]);
+                part[q] = A::zero();
+            }
+        }
+    }
+    __device__ __forceinline__ double total(int q) const {
+        return A::to_double(part[q]) + (FLUSHED ? tot[q * ST + threadIdx.x] : 0.0);
+    }
 };
 
 // A class of individuals: n of them from order[i0] on, walked by `ctas` CTAs, rt threads of a CTA to
@@ -279,41 +314,37 @@ __global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first
 //
 // An FP64 instruction takes 16 clocks of an SM's FP64 pipe whatever its active lanes, and a
 // dependent one ~40: so every sum keeps columns on the lanes and is two steps of ~sqrt terms.  A
-// CTA adds up its individuals in the solve's arithmetic and leaves one FP64 partial per column and
-// quantity; the last CTA of each group to arrive adds up the group's, and the last group's the
+// CTA adds up its threads' sums and leaves one partial per column and quantity; the last CTA of each group to arrive adds up the group's, and the last group's the
 // groups' (one group where the CTA's threads can take 16 partials each: a second round of
 // arrivals costs ~4 us).  (A warp per column with shuffles, all partials in one last CTA, took 45
 // us at 65 columns.)  The order is one, so the sums' bits are.
 
 // total of the R rows of nw values in sm, valid in threads t < nw; ends without a barrier
-template <class T, class Add>
-__device__ __forceinline__ T two_step(const T* sm, T* sm2, int R, int nw, Add add) {
+__device__ __forceinline__ double two_step(const double* sm, double* sm2, int R, int nw) {
     const int t = threadIdx.x;
     int ns = 1;
     while (ns * ns < R) ++ns;
     ns = max(1, min(ns, (int)blockDim.x / nw));
     const int j0 = t / nw, w = t - j0 * nw;
-    T s = T();
+    double s = 0.0;
     if (j0 < ns && j0 < R) {
         s = sm[j0 * nw + w];
-        for (int j = j0 + ns; j < R; j += ns) s = add(s, sm[j * nw + w]);
+        for (int j = j0 + ns; j < R; j += ns) s += sm[j * nw + w];
     }
     if (ns == 1) return s;
     sm2[t] = s;
     __syncthreads();
     if (t < nw)
-        for (int j = 1; j < min(ns, R); ++j) s = add(s, sm2[j * nw + t]);
+        for (int j = 1; j < min(ns, R); ++j) s += sm2[j * nw + t];
     return s;
 }
 
 // v summed over the tile's CTAs into out0[col] (and out1[col], the second quantity); returns true in
 // every thread of the last CTA, once they are written and visible to it
 template <int NQ, class A>
-__device__ __forceinline__ bool sum_last(const Args<A>& a, const Lane& l, const typename A::V (&v)[NQ], int slot,
+__device__ __forceinline__ bool sum_last(const Args<A>& a, const Lane& l, const double (&v)[NQ], int slot,
                                          double* __restrict__ out0, double* __restrict__ out1) {
-    using V = typename A::V;
-    __shared__ V sm[NQ * ST], sm2[ST];
-    __shared__ double smd[ST], smd2[ST];
+    __shared__ double sm[NQ * ST], sm2[ST], smd[ST], smd2[ST];
     __shared__ bool last;
     const int t = threadIdx.x, kc = a.kc, c0 = blockIdx.y * kc, nc = min(kc, a.kact - c0), nw = NQ * kc;
     // thread t < nw stands for quantity q and column c of the tile
@@ -322,12 +353,12 @@ __device__ __forceinline__ bool sum_last(const Args<A>& a, const Lane& l, const 
     if (l.il < a.ti) {
         const int cl = t - l.il * kc;
 #pragma unroll
-        for (int p = 0; p < NQ; ++p) sm[(l.il * NQ + p) * kc + cl] = l.on ? v[p] : A::zero();
+        for (int p = 0; p < NQ; ++p) sm[(l.il * NQ + p) * kc + cl] = l.on ? v[p] : 0.0;
     }
     __syncthreads();
-    const V s = two_step(sm, sm2, a.ti, nw, [](V x, V y) { return A::add(x, y); });
+    const double s = two_step(sm, sm2, a.ti, nw);
     const size_t row = (size_t)NQ * a.kact;
-    if (mine) a.part[(size_t)slot * row + (size_t)q * a.kact + c0 + c] = A::to_double(s);
+    if (mine) a.part[(size_t)slot * row + (size_t)q * a.kact + c0 + c] = s;
     const int P = (int)blockDim.x / nw;   // threads per column and quantity
     const int gs = min(a.slots, max(32, 16 * P)), ng = (a.slots + gs - 1) / gs, g = slot / gs;
     const int gn = min(gs, a.slots - g * gs);
@@ -357,7 +388,7 @@ __device__ __forceinline__ bool sum_last(const Args<A>& a, const Lane& l, const 
             smd[j0 * nw + w] = x;
         }
         __syncthreads();
-        const double x = two_step(smd, smd2, P, nw, [](double u, double y) { return u + y; });
+        const double x = two_step(smd, smd2, P, nw);
         const bool fin = level == 1 || ng == 1;
         if (mine) {
             if (fin) (q ? out1 : out0)[a.cols ? a.cols[c0 + c] : c0 + c] = x;
@@ -378,7 +409,8 @@ __global__ void __launch_bounds__(ST) k_step(Args<A> a, const double* __restrict
     using V = typename A::V;
     const Lane l = lane_of(a);
     const V e = a.e, b0 = a.b0, b01 = a.b01, b1 = a.b1;
-    V dot = A::zero();
+    __shared__ double tot[ST];
+    Sums<A, 1> dot(tot);
     for (int64_t g = blockIdx.x; g * a.ti < a.N; g += gridDim.x) {
         const int64_t b = g * a.ti + l.il;
         if (!l.on || b >= a.N || !GLOBE_BOUNDS(a.bind[b] >= 0 && a.bind[b] < a.N, 0x1401u)) continue;
@@ -388,9 +420,10 @@ __global__ void __launch_bounds__(ST) k_step(Args<A> a, const double* __restrict
         const V a0 = A::madd(b0, s0, A::madd(b01, s1, gz)), a1 = A::madd(b01, s0, A::mul(b1, s1));
         A::store(a.S0 + o, a0);
         A::store(a.S1 + o, a1);
-        dot = A::madd(e, pp, A::madd(a0, s0, A::madd(a1, s1, dot)));
+        dot.part[0] = A::madd(e, pp, A::madd(a0, s0, A::madd(a1, s1, dot.part[0])));
+        dot.next();
     }
-    const V v[1] = {dot};
+    const double v[1] = {dot.total(0)};
     if (sum_last<1>(a, l, v, blockIdx.x, a.pvp, nullptr) && threadIdx.x < a.kc) {
         const int c = blockIdx.y * a.kc + threadIdx.x;
         if (c < a.kact) {
@@ -472,12 +505,11 @@ __device__ void pcg_check(const PcgLoop& p, const double* rr, const double* pvp,
 // start): g and r'z only
 template <class A, bool MANY, bool INIT, int RU>
 __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int c, int x, typename A::V* sm,
-                                            typename A::V& rr, typename A::V& rz) {
+                                            Sums<A, 2>& sums) {
     using V = typename A::V;
     const Team w = team_of<MANY>(a, l, a.cls[c], x);
     const V inv_e = a.inv_e, e = a.e, na = INIT || !l.on ? A::zero() : A::neg(A::load(a.alpha + l.col));
     const int step = MANY ? w.rt : 1;
-    rr = rz = A::zero();
     for (unsigned j = w.j0; j < w.n; j += w.js) {   // uniform over the CTA
         const unsigned idx = j + w.slot;
         int b = 0, st = 0, en = 0;
@@ -526,7 +558,7 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
                     const V rn = next(rv[u], pv[u], tv[u]);
                     if (!INIT) {
                         A::store(a.r + (size_t)q * a.k + l.col, rn);
-                        rr = A::madd(rn, rn, rr);
+                        sums.part[1] = A::madd(rn, rn, sums.part[1]);
                     }
                     s0 = A::add(s0, rn);
                     s1 = A::madd(tv[u], rn, s1);
@@ -557,9 +589,10 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
 #pragma unroll
                 for (int u = 0; u < RU; ++u)
                     if (q0 + u * step < en)
-                        rz = A::madd(rv[u], A::madd(rv[u], inv_e, A::neg(A::madd(g1, tv[u], g0))), rz);
+                        sums.part[0] = A::madd(rv[u], A::madd(rv[u], inv_e, A::neg(A::madd(g1, tv[u], g0))), sums.part[0]);
             }
         }
+        sums.next();
     }
 }
 
@@ -570,10 +603,11 @@ __global__ void __launch_bounds__(ST, RU == RU_UPD ? RES_UPD : 2) k_update(Args<
     const Lane l = lane_of(a);
     int x = blockIdx.x;
     const int p = class_of(a, x);
-    V rr, rz;
-    if (p < 2) update_walk<A, true, INIT, RU>(a, l, p, x, sm, rr, rz);
-    else update_walk<A, false, INIT, RU>(a, l, 2, x, sm, rr, rz);
-    const V v[2] = {rz, rr};
+    __shared__ double tot[2 * ST];
+    Sums<A, 2> sums(tot);   // r'z, |r|^2
+    if (p < 2) update_walk<A, true, INIT, RU>(a, l, p, x, sm, sums);
+    else update_walk<A, false, INIT, RU>(a, l, 2, x, sm, sums);
+    const double v[2] = {sums.total(0), sums.total(1)};
     // r'z (new) lands in rz's second half (k entries), |r|^2 in rr
     double* rz2 = a.rz + a.k;
     if (!sum_last<2>(a, l, v, blockIdx.x, rz2, INIT ? rz2 + a.k : a.rr)) return;

@@ -49,3 +49,23 @@ def test_lengths_match_oracle(gctx, orc, name):
             X, info = gctx.pcg(B[:, :k], tol=1e-11, rule=G.RULE_AIREML, precision=prec)
             assert info["converged"]
             assert max(rel(X[:, c], ref[:, c]) for c in range(k)) < 1e-8, (name, k, prec)
+
+
+# 1216 pairs of threads at 128 columns: 16 individuals each, so their sums pass from double-float into FP64
+# twice.  Residuals of a few per cent, r recurred in 47 bits from |V p| < 1e3 |p|
+@pytest.mark.parametrize("k", [1, 128])
+def test_sums_over_many_individuals_a_thread(gctx, k):
+    N = 20011
+    rng = np.random.default_rng(N)
+    counts = rng.integers(1, 4, N)
+    indiv = np.repeat(np.arange(N, dtype=np.int32), counts)
+    X = np.column_stack([np.ones(len(indiv)), rng.uniform(0, 2, len(indiv))])
+    gctx.load_records(indiv, X, rng.standard_normal(len(indiv)), N)
+    gctx.load_bed(rng.integers(0, 256, (130, (N + 3) // 4), dtype=np.uint8), min_maf=0.0, max_miss=1.0)
+    gctx.set_vc(VC_F)
+    B = rng.standard_normal((len(indiv), k))
+    for prec in (G.PREC_FP64, G.PREC_MIXED):
+        Y, info = gctx.pcg(B, tol=0.0, maxit=4, rule=G.RULE_AIREML, precision=prec)
+        r = np.linalg.norm(B - gctx.vx(Y), axis=0) / np.linalg.norm(B, axis=0)
+        assert info["iters"] == 4 and 1e-6 < r.max() < 1
+        assert abs(info["max_rel_res"] / r.max() - 1) < 1e-8
