@@ -238,8 +238,11 @@ int geno_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, d
 //
 // zs^2 takes one of three values per SNP, so four SNPs' share of an individual is one entry of a
 // 256-entry table indexed by their four codes (one byte).  Entries are fixed-point int64 on one
-// grid for the whole matrix (2^62 above the largest possible sum), so any split of the SNPs
-// sums to the same bits, within M 2^-63 of the exact sum.
+// grid for the whole matrix, so any split of the SNPs sums to the same bits.  The grid's step is
+// 2^-61 to 2^-62 of S, the sum over the SNPs of the largest zs^2 of any genotype (present or not;
+// rounded up to an integer), and A_ii is within half a step, and the rounding of the zs^2, of the
+// exact one.  (With the largest zs^2 of all times M in S's place one singleton among common SNPs made
+// the step 2000 times wider, at N = 2000.)
 // A CTA covers 16384 individuals (16 per thread: one word of each SNP row) and a range of SNPs,
 // eight (two tables) a step.  A table is held 16 times over, entry e of copy l at (16 e + l): the
 // 16 lanes of a half warp read 16 different bank pairs whatever their codes.  Two pair tables of
@@ -251,21 +254,20 @@ constexpr int DG_THREADS = 1024;
 constexpr int DG_LUT = 256 * 16 * 8;                  // bytes of a table
 constexpr int DG_SMEM = 4 * DG_LUT + DG_LUT;          // two steps of two tables, aligned to a table's size
 
-// the largest zs^2 (non-negative doubles order like their bits)
-__global__ void k_zs_max(const double* __restrict__ zs, int64_t n, unsigned long long* __restrict__ out) {
+// *sum += S (integers: the same whatever the order).  zs^2 < 4 N, so S < 2^63 for 2^30 SNPs
+__global__ void __launch_bounds__(256) k_zs_bound(const double* __restrict__ zs, int64_t Mk,
+                                                  unsigned long long* __restrict__ sum) {
     unsigned long long m = 0;
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-        m = max(m, (unsigned long long)__double_as_longlong(zs[e] * zs[e]));
+    for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < Mk; s += (int64_t)gridDim.x * blockDim.x) {
+        const double a = zs[4 * s], b = zs[4 * s + 1], c = zs[4 * s + 2];
+        m += (unsigned long long)ceil(fmax(a * a, fmax(b * b, c * c)));
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(sum, m);
 }
-// fraction bits of the fixed-point sums: Mk zs^2 < 2^(62 - bits)
-__device__ __forceinline__ int diag_bits(const unsigned long long* maxq, int64_t Mk) {
-    int E;
-    frexp(__longlong_as_double((long long)*maxq) * (double)Mk, &E);
-    return 62 - E;
-}
+// fraction bits of the fixed-point sums: S 2^bits < 2^62
+__device__ __forceinline__ int diag_bits(const unsigned long long* sum) { return __clzll((long long)*sum) - 2; }
 
 // One round of a transpose of the four 2-bit codes of each byte over four words.
 template <int S>
@@ -281,7 +283,7 @@ __device__ __forceinline__ void dg_round(uint32_t (&r)[4], uint32_t m) {
 
 __global__ void __launch_bounds__(DG_THREADS, 1) k_geno_diag(const uint8_t* __restrict__ blk, int nch, int64_t Mk,
                                                              int32_t N, const double* __restrict__ zs,
-                                                             const unsigned long long* __restrict__ maxq, int64_t sper,
+                                                             const unsigned long long* __restrict__ bound, int64_t sper,
                                                              long long* __restrict__ part) {
     extern __shared__ __align__(16) char dg_smem[];
     __shared__ long long pt[2][4][16];   // step parity; pairs of SNPs of a step
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_geno_diag(const uint8_t* __re
     const bool in = c < nch;
     const int64_t nst = (Mk + 7) / 8, st0 = (int64_t)blockIdx.y * sper, st1 = min(nst, st0 + sper);
     if (st0 >= st1) return;
-    const double sc = ldexp(1.0, diag_bits(maxq, Mk));
+    const double sc = ldexp(1.0, diag_bits(bound));
     long long acc[16];
 #pragma unroll
     for (int j = 0; j < 16; ++j) acc[j] = 0;
@@ -375,12 +377,12 @@ __global__ void __launch_bounds__(DG_THREADS, 1) k_geno_diag(const uint8_t* __re
 }
 
 __global__ void k_geno_diag_sum(const long long* __restrict__ part, int nsplit, int64_t Mk, int32_t N,
-                                const unsigned long long* __restrict__ maxq, double* __restrict__ d) {
+                                const unsigned long long* __restrict__ bound, double* __restrict__ d) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     long long a = 0;
     for (int y = 0; y < nsplit; ++y) a += part[(int64_t)y * N + i];
-    d[i] = ldexp((double)a, -diag_bits(maxq, Mk)) / (double)Mk;
+    d[i] = ldexp((double)a, -diag_bits(bound)) / (double)Mk;
 }
 
 int geno_diag(globe_ctx* ctx, double* d) {
@@ -398,17 +400,17 @@ int geno_diag(globe_ctx* ctx, double* d) {
     const int64_t sper = (nst + ns - 1) / ns;
     ns = (nst + sper - 1) / sper;
     long long* part;
-    unsigned long long* maxq;
+    unsigned long long* bound;
     GLOBE_RET(ws(ctx, WS_GPART, (size_t)ns * N + 1, &part));
-    maxq = reinterpret_cast<unsigned long long*>(part + ns * N);
-    GLOBE_CK(ctx, cudaMemsetAsync(maxq, 0, sizeof(*maxq), ctx->stream));
-    k_zs_max<<<(unsigned)std::min<int64_t>(div_up(4 * g.Mk, 1024), 304), 256, 0, ctx->stream>>>(g.zs, 4 * g.Mk, maxq);
-    GLOBE_LAUNCHED(ctx, "k_zs_max");
+    bound = reinterpret_cast<unsigned long long*>(part + ns * N);
+    GLOBE_CK(ctx, cudaMemsetAsync(bound, 0, sizeof(*bound), ctx->stream));
+    k_zs_bound<<<(unsigned)std::min<int64_t>(div_up(g.Mk, 256), 304), 256, 0, ctx->stream>>>(g.zs, g.Mk, bound);
+    GLOBE_LAUNCHED(ctx, "k_zs_bound");
     GLOBE_CK(ctx, cudaFuncSetAttribute(k_geno_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, DG_SMEM));
-    k_geno_diag<<<dim3((unsigned)cx, (unsigned)ns), DG_THREADS, DG_SMEM, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, maxq,
+    k_geno_diag<<<dim3((unsigned)cx, (unsigned)ns), DG_THREADS, DG_SMEM, ctx->stream>>>(g.blk1, g.nch1, g.Mk, N, g.zs, bound,
                                                                                         sper, part);
     GLOBE_LAUNCHED(ctx, "k_geno_diag");
-    k_geno_diag_sum<<<div_up(N, 256), 256, 0, ctx->stream>>>(part, (int)ns, g.Mk, N, maxq, d);
+    k_geno_diag_sum<<<div_up(N, 256), 256, 0, ctx->stream>>>(part, (int)ns, g.Mk, N, bound, d);
     GLOBE_LAUNCHED(ctx, "k_geno_diag_sum");
     return GLOBE_OK;
 }
