@@ -236,7 +236,8 @@ __device__ __forceinline__ unsigned dir_walk(const Args<A>& a, const Lane& l, in
             const int st = ord.y, en = ord.z;
             b = ord.x;
             i = ord.w;
-            in = GLOBE_BOUNDS(b >= 0 && b < a.N && st >= 0 && st <= en && en <= a.Nrec && i >= 0 && i < a.N, 0x1301u);
+            if (!GLOBE_BOUNDS(b >= 0 && b < a.N && st >= 0 && st <= en && en <= a.Nrec && i >= 0 && i < a.N, 0x1601u))
+                in = false, b = 0;
             const V g0 = A::load(a.G + 2 * ((size_t)b * a.k + l.col)), g1 = A::load(a.G + 2 * ((size_t)b * a.k + l.col) + 1);
             for (int q0 = st + (MANY ? w.rl : 0); in && q0 < en; q0 += RU * step) {
                 V rv[RU], pv[RU], xv[RU], tv[RU];
@@ -413,7 +414,7 @@ __global__ void __launch_bounds__(ST) k_step(Args<A> a, const double* __restrict
     Sums<A, 1> dot(tot);
     for (int64_t g = blockIdx.x; g * a.ti < a.N; g += gridDim.x) {
         const int64_t b = g * a.ti + l.il;
-        if (!l.on || b >= a.N || !GLOBE_BOUNDS(a.bind[b] >= 0 && a.bind[b] < a.N, 0x1401u)) continue;
+        if (!l.on || b >= a.N || !GLOBE_BOUNDS(a.bind[b] >= 0 && a.bind[b] < a.N, 0x1701u)) continue;
         const size_t o = (size_t)b * a.k + l.col;
         const V s0 = A::load(a.S0 + o), s1 = A::load(a.S1 + o), pp = A::load(a.PP + o);
         const V gz = A::from(GZ[a.bind[b] + (size_t)l.c * a.N]);
@@ -520,7 +521,7 @@ __device__ __forceinline__ void update_walk(const Args<A>& a, const Lane& l, int
             b = ord.x;
             st = ord.y;
             en = ord.z;
-            if (!GLOBE_BOUNDS(b >= 0 && b < a.N && st >= 0 && st <= en && en <= a.Nrec, 0x1501u)) in = false, st = en = 0;
+            if (!GLOBE_BOUNDS(b >= 0 && b < a.N && st >= 0 && st <= en && en <= a.Nrec, 0x1801u)) in = false, b = st = en = 0;
         }
         const size_t o = (size_t)b * a.k + l.col;
         if (!INIT && in) {
