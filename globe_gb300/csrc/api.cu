@@ -26,13 +26,58 @@ int cuda_err(globe_ctx* ctx, cudaError_t e, const char* what) {
                    cudaGetErrorString(e), cudaGetErrorName(e));
 }
 
+static void free_slot(globe_ctx* ctx, Slot& s) {
+    if (!s.p) return;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(s.p);
+    ctx->dev_bytes -= (int64_t)s.bytes;
+    s = Slot();
+}
+
+bool release_optional(globe_ctx* ctx) {
+    if (ctx->capturing) return false;
+    auto& g = ctx->gen;
+    bool any = false;
+    auto drop = [&](uint8_t*& p) {
+        any = any || p;
+        if (p) cudaStreamSynchronize(ctx->stream);
+        dfree(ctx, p);
+        p = nullptr;
+    };
+    if (!(ctx->pinned & PIN_PLANES64) && g.adig[1].p) {
+        drop(g.adig[1].p);
+        g.adig[1].state = -1;
+    }
+    if (!(ctx->pinned & PIN_TC)) {
+        if (g.blk2_f64) {
+            drop(g.blk2);
+            g.blk2_f64 = false;
+            g.f64_tc = -1;
+        }
+        for (int id : {WS_TC_D1, WS_TC_D2, WS_TC_P1, WS_TC_P2, WS_TC_U}) {
+            any = any || ctx->ws[id].p;
+            free_slot(ctx, ctx->ws[id]);
+        }
+    }
+    return any;
+}
+
+static cudaError_t malloc_or_release(globe_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    if (e == cudaErrorMemoryAllocation && release_optional(ctx)) {
+        e = cudaMalloc(p, bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    return e;
+}
+
 int dalloc_bytes(globe_ctx* ctx, void** p, size_t bytes) {
     *p = nullptr;
     if (ctx->capturing) return set_err(ctx, GLOBE_ERR_STATE, "device allocation during CUDA graph capture");
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMalloc(p, bytes);
+    cudaError_t e = malloc_or_release(ctx, p, bytes);
     if (e != cudaSuccess) {
-        cudaGetLastError();
         return set_err(ctx, GLOBE_ERR_NOMEM, "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
     }
     ctx->dev_bytes += (int64_t)bytes;
@@ -64,17 +109,10 @@ int wslot(globe_ctx* ctx, int id, size_t bytes, void** out) {
         // growth synchronises the stream: not while a capture is open (the caller then runs
         // the same work directly)
         if (ctx->capturing) return set_err(ctx, GLOBE_ERR_STATE, "workspace growth during CUDA graph capture");
-        if (s.p) {
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(s.p);
-            ctx->dev_bytes -= (int64_t)s.bytes;
-            s.p = nullptr;
-            s.bytes = 0;
-        }
+        free_slot(ctx, s);
         size_t want = bytes + bytes / 4 + 256;
-        cudaError_t e = cudaMalloc(&s.p, want);
+        cudaError_t e = malloc_or_release(ctx, &s.p, want);
         if (e != cudaSuccess) {
-            cudaGetLastError();
             s.p = nullptr;
             return set_err(ctx, GLOBE_ERR_NOMEM, "workspace cudaMalloc(%zu bytes) failed: %s", want,
                            cudaGetErrorString(e));

@@ -65,6 +65,7 @@ struct Genetic {
     uint8_t* blk2 = nullptr;   // individual-major: tensor-core pass 2, GRM build (first use)
     int nch1 = 0, ntiles1 = 0, nch2 = 0, ntiles2 = 0;
     int f64_tc = 0;            // FP64 products on the tensor cores: 0 not tried, 1 run, -1 no memory for them
+    bool blk2_f64 = false;     // blk2 was made for those alone: it is given back where memory runs out
     // dense source
     float* grm = nullptr;    // N(N+1)/2
     // digit planes of the dense GRM for the tensor-core products: [0] GLOBE_PREC_MIXED, [1]
@@ -106,6 +107,7 @@ struct globe_ctx {
     double vc[5] = {0, 0, 0, 0, 0};
     bool vc_set = false;
     int in_solve = 0;             // inside a call that repeats its products (SolveScope)
+    unsigned pinned = 0;          // what release_optional must leave (PinScope)
     bool stat_dirty = false;      // a product stopped before it cleared its columns' statistics words
     bool tc_used = false;         // a tensor-core product was launched since the error word was last read
     int prec = GLOBE_PREC_FP64;   // precision of operator calls (globe_set_precision / PCG options)
@@ -173,6 +175,11 @@ int dalloc(globe_ctx* ctx, T** p, size_t n) {
     return dalloc_bytes(ctx, (void**)p, n * sizeof(T));
 }
 void dfree(globe_ctx* ctx, void* p);
+// Frees what only makes later calls faster: the FP64 products' second genotype copy and digit planes
+// (they stay on the FP64 pipe until the next load) and the tensor-core products' workspaces.
+// True if there was any.  An allocation that fails tries again after it.
+bool release_optional(globe_ctx* ctx);
+enum { PIN_TC = 1, PIN_PLANES64 = 2 };   // blk2 and the WS_TC workspaces; adig[1]
 // workspace slot of at least `bytes`
 int wslot(globe_ctx* ctx, int id, size_t bytes, void** out);
 template <class T>
@@ -231,6 +238,16 @@ struct SolveScope {
     ~SolveScope() { --c->in_solve; }
     SolveScope(const SolveScope&) = delete;
     SolveScope& operator=(const SolveScope&) = delete;
+};
+
+// What a product in progress uses of the memory that release_optional frees
+struct PinScope {
+    globe_ctx* c;
+    unsigned saved;
+    PinScope(globe_ctx* ctx, unsigned pins) : c(ctx), saved(ctx->pinned) { c->pinned |= pins; }
+    ~PinScope() { c->pinned = saved; }
+    PinScope(const PinScope&) = delete;
+    PinScope& operator=(const PinScope&) = delete;
 };
 
 // ---- bounds-checked debug build -------------------------------------------------

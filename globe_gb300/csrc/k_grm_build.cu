@@ -286,7 +286,9 @@ using namespace tc;
 static int grm_build_tc(globe_ctx* ctx, float* lt) {
     auto& g = ctx->gen;
     const int32_t N = ctx->coh.N;
+    PinScope pin(ctx, PIN_TC);
     GLOBE_RET(ensure_blk2(ctx));
+    g.blk2_f64 = false;
     const int nch = g.nch2;
     const int64_t kpad = (int64_t)nch * BK;
     const int rpc = rows_per_cta(GRM_NMMA);

@@ -593,6 +593,7 @@ static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, doubl
 
 // out (N x k) = scale * A Z from the planes, nd digits per column
 static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out, bool zhi_ready) {
+    PinScope pin(ctx, nd == NDZ ? PIN_TC | PIN_PLANES64 : PIN_TC);
     const int nw = digit_ctas(ctx->gen.adig[nd == NDZ ? 1 : 0].np);
     unsigned* wide = nullptr;
     if (nd == NDZ) GLOBE_RET(ws(ctx, WS_TC_U, (size_t)k * nw, &wide));
@@ -652,9 +653,8 @@ int dense_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double
         if (rc == GLOBE_OK && a.state == 1) rc = dense_apply_nd(ctx, NDZ, Z, k, scale, out, zhi_ready);
         if (a.state == 1 && rc != GLOBE_ERR_NOMEM) return rc;
         if (rc != GLOBE_OK && rc != GLOBE_ERR_NOMEM) return rc;
-        if (rc == GLOBE_ERR_NOMEM) {   // give the planes back
-            dfree(ctx, a.p);
-            a.p = nullptr;
+        if (rc == GLOBE_ERR_NOMEM) {
+            release_optional(ctx);
             a.state = -1;
         }
     }

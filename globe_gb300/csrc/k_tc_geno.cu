@@ -987,7 +987,10 @@ static int geno_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double 
         GLOBE_CK(ctx, cudaMemsetAsync(out, 0, sizeof(double) * (size_t)N * k, ctx->stream));
         return GLOBE_OK;
     }
+    const bool made = !g.blk2;
+    PinScope pin(ctx, PIN_TC);
     GLOBE_RET(ensure_blk2(ctx));
+    g.blk2_f64 = nd == ND64 && (made || g.blk2_f64);
     // near-equal groups of <= 256 / nd columns (MMA width <= 256).  Groups wider than
     // 192 / nd (MMA width > 192) run one row tile per CTA, which costs more per column than
     // two groups of two tiles once k > 256 / nd: then groups of <= 192 / nd columns
@@ -1083,6 +1086,7 @@ int geno_apply_f64(globe_ctx* ctx, const double* Z, int k, double scale, double*
                 return rc;
             }
             g.f64_tc = -1;
+            release_optional(ctx);
         }
     }
     return geno_apply_fp64_pipe(ctx, Z, k, scale, out);

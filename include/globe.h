@@ -56,7 +56,10 @@ extern "C" {
                                products from 12 to 14 digit planes that hold A exactly (12 to
                                14 N^2 bytes) and 16 digits a column, each row within a few
                                units of 2^-53 (|A| |z|)_i; columns with entries that those
-                               digits do not hold, and the non-finite ones, on the FP64 pipe */
+                               digits do not hold, and the non-finite ones, on the FP64 pipe.
+                               The second copy, the planes and the products' workspaces (a GRM
+                               build's: up to 2 GB) stay with the context; an allocation of
+                               the context that finds no memory takes them */
 #define GLOBE_PREC_MIXED 1  /* genotype GRM product on the FP8 tensor cores with exact
                                base-32 digit slicing of the right-hand sides (9 digits =
                                45 bits by default, matches FP64 to ~1e-13; see
