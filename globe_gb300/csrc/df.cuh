@@ -101,7 +101,6 @@ __device__ __forceinline__ D add(D a, D b) {
     return fast_two_sum(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
 }
 __device__ __forceinline__ D neg(D a) { return make(-a.h, -a.l); }
-__device__ __forceinline__ D sub(D a, D b) { return add(a, neg(b)); }
 // a.h b.h exactly as p + e by one FMA, plus the cross terms
 __device__ __forceinline__ D mul(D a, D b) {
     const float p = __fmul_rn(a.h, b.h);
@@ -112,16 +111,6 @@ __device__ __forceinline__ D mul(D a, D b) {
 }
 // a b + c
 __device__ __forceinline__ D madd(D a, D b, D c) { return add(mul(a, b), c); }
-
-// butterfly sum over the warp (add is commutative, so every lane ends with the same value)
-__device__ __forceinline__ D warp_sum(D v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const D w = make(__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o));
-        v = add(v, w);
-    }
-    return v;
-}
 
 }  // namespace df
 

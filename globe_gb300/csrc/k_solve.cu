@@ -26,9 +26,9 @@
 //
 // Two arithmetics: FP64 (GLOBE_PREC_FP64), and double-float pairs (df.cuh) in the 8 bytes of
 // each double under GLOBE_PREC_MIXED, column c scaled by a power of two (col_unscale) to a
-// unit-size right-hand side.  What stays FP64 there: the GRM product's input and output, the
-// per-column scalars, and every sum past FLUSH individuals of a thread (a team's sums over one
-// individual's records are in double-float).
+// unit-size right-hand side.  What stays FP64 there: the GRM product's input and output, and every
+// sum past FLUSH individuals of a thread (a team's sums over one individual's records are in
+// double-float); alpha and beta are formed from those sums in FP64 and rounded to pairs.
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -315,10 +315,11 @@ __global__ void __launch_bounds__(ST, RES_DIR) k_dir(Args<A> a, const bool first
 //
 // An FP64 instruction takes 16 clocks of an SM's FP64 pipe whatever its active lanes, and a
 // dependent one ~40: so every sum keeps columns on the lanes and is two steps of ~sqrt terms.  A
-// CTA adds up its threads' sums and leaves one partial per column and quantity; the last CTA of each group to arrive adds up the group's, and the last group's the
-// groups' (one group where the CTA's threads can take 16 partials each: a second round of
-// arrivals costs ~4 us).  (A warp per column with shuffles, all partials in one last CTA, took 45
-// us at 65 columns.)  The order is one, so the sums' bits are.
+// CTA adds up its threads' sums and leaves one partial per column and quantity; the last CTA of
+// each group to arrive adds up the group's, and the last group's the groups' (one group where the
+// CTA's threads can take 16 partials each: a second round of arrivals costs ~4 us).  (A warp per
+// column with shuffles, all partials in one last CTA, took 45 us at 65 columns.)  The order is one,
+// so the sums' bits are.
 
 // total of the R rows of nw values in sm, valid in threads t < nw; ends without a barrier
 __device__ __forceinline__ double two_step(const double* sm, double* sm2, int R, int nw) {

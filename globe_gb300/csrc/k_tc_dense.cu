@@ -17,7 +17,7 @@
 //
 // Layout: plane d, row i, K position P at adig[(d*NP + i) * NP + P] with
 // NP = N rounded up to 128 and K permuted within groups of 16 like the digit
-// tiles of the right-hand sides (kpos), rows padded to a multiple of 256.
+// tiles of the right-hand sides (k_digits), rows padded to a multiple of 256.
 // The planes are full squares (both triangles), 7 N^2 bytes at DA = 7.
 //
 // GLOBE_PREC_FP64 takes the 12 to 14 planes that hold every entry of A exactly and 16 digits of Z,
@@ -202,8 +202,7 @@ __global__ void k_dense_scan(const float* __restrict__ lt, int64_t n, unsigned* 
 // The DA digit planes of one 64 x 64 block (I0, J0) of the full square: the block is staged
 // through shared memory (rows of the triangle left of the diagonal, columns of it right of
 // the diagonal: coalesced either way), then each thread writes 4 words of 4 K positions per
-// plane.  Position P of a group of 16 holds column 2P (P < 8) or 2(P-8)+1 (the inverse of
-// kpos).  x 2^-eA is rounded once to I = round(x 2^-eA 32^(DA-1)); its balanced base-32
+// plane.  Position P of a group of 16 holds column 2P (P < 8) or 2(P-8)+1.  x 2^-eA is rounded once to I = round(x 2^-eA 32^(DA-1)); its balanced base-32
 // digits are peeled off from the least significant end (d = ((I + 16) mod 32) - 16); the
 // leading digit is what remains, in [-16, 16].  More than DA64 planes: those of the remainder of
 // the first DA64, as k_digits has them.

@@ -21,9 +21,9 @@
 //   warp 0     bulk copies of the packed 2-bit tiles (tile-blocked layout: each
 //              128-row x 32-byte stage is one contiguous 4 KB block)
 //   warp 1     TMA of the digit tiles [NMMA rows x 128 B, 128B-swizzled]
-//   warp 2     TMEM allocation and the single-thread tcgen05.mma issue
+//   warps 2..  one a row tile: the single-thread tcgen05.mma issue (warp 2: TMEM allocation too)
 //              (kind::f8f6f4, E4M3 x E4M3 -> F32, A from TMEM, B from smem)
-//   warps 3-10 decode 2-bit codes to e4m3 bytes in registers and store them
+//   16 warps   decode 2-bit codes to e4m3 bytes in registers and store them
 //              straight into TMEM (tcgen05.st) as the A operand, then the
 //              epilogue (tcgen05.ld -> FP32 partials)
 // Keeping the decoded operand out of shared memory matters: staged through

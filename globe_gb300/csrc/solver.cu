@@ -110,9 +110,10 @@ int pcg_dev(globe_ctx* ctx, const double* B, double* X, int k, const globe_pcg_o
     return with_tc_check(ctx, rc);
 }
 
-// Captures `body` (stream work only, nothing run) into a graph and makes ctx->pcg_graph run it: the cached executable is updated in place when the topology matches, else
-// instantiated anew.  Allocation is refused while the capture is open.  Returns false, with
-// nothing run and the error message restored, if any step fails.
+// Captures `body` (stream work only, nothing run) into a graph and makes ctx->pcg_graph run it:
+// the cached executable is updated in place when the topology matches, else instantiated anew.
+// Allocation is refused while the capture is open.  Returns false, with nothing run and the error
+// message restored, if any step fails.
 template <class F>
 static bool capture_body(globe_ctx* ctx, F&& body, int64_t* nlaunch) {
     const std::string err0 = ctx->err;

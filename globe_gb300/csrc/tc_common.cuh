@@ -61,12 +61,6 @@ __host__ __device__ __forceinline__ int64_t blk_offset(int64_t row, int64_t b, i
     return (((t * nch + (b >> 5)) * 128 + r) * 32) + h * 16 + (w & 15);
 }
 
-__device__ __forceinline__ int kpos(int64_t i) {
-    // K position of element i within groups of 16 in the dense product's operands (digit planes
-    // of A and digits of Z): evens first, then odds
-    const int q = (int)(i & 15);
-    return (int)(i & ~15ll) + ((q & 1) ? 8 + (q >> 1) : (q >> 1));
-}
 // K position of genotype i of a 16-genotype word after decode_word (k_tc_geno.cu): word r holds
 // the genotypes at field r of the word's four bytes, so position 4 (i % 4) + i / 4.  Its own
 // inverse.  Even genotypes (fields 0 and 2) decode to 2^-9 g, odd ones to 2^-7 g, so the digit
@@ -248,8 +242,8 @@ __global__ void k_col_max(const double* __restrict__ X, int64_t n, int64_t ld, u
 // in [0, kpad) of the column's digit rows is written (rows >= n give digit 0).  One thread
 // fills 4 consecutive positions P..P+3 (a 32-bit word).  GENO: the operand of a genotype
 // product -- pos = kpos_g (position P + q of a group of 16 holds row 4 q + P/4) and digits
-// times geno_digit_mult(row); otherwise the dense product's kpos (position P < 8 holds row
-// 2P, P >= 8 row 2(P-8)+1).
+// times geno_digit_mult(row); otherwise the order of the dense product's planes, evens before odds
+// in each group of 16 (position P < 8 holds row 2P, P >= 8 row 2(P-8)+1).
 // x 2^-e is rounded once to the integer I = round(x 2^-e 32^(ND-1)), |I| <= 2^(5 ND - 1); its
 // balanced base-32 digits are peeled off from the least significant end in integer
 // arithmetic (d = ((I + 16) mod 32) - 16, in [-16, 15]); the leading digit is what
