@@ -45,7 +45,8 @@ constexpr int ST = 288;            // threads per CTA at most
 // N = 100k, k = 5, 255 against 204 us at N = 50k, k = 65; k_dir with 2 and 4: 153 and 38 against
 // 158 and 36 us), and so was keeping an individual's r and t in registers for k_update's second
 // pass over them (83 us: 2 CTAs).  With at most two CTAs an SM to run, where a chain of loads is
-// what counts, k_update takes 4 records at a time.
+// what counts, k_update takes 4 records at a time (mixed, five columns, us an iteration with 2 / 4: 157
+// CTAs 66.4 / 64.5, 295 74.9 / 73.4, 324 76.0 / 76.6, 393 78.6 / 82.0).
 constexpr int RU_DIR = 4, RU_UPD = 2, RES_DIR = 3, RES_UPD = 4;
 // CTAs per SM launched at most: k_dir's take two turns, the kernels that end in column sums one
 // (fewer partials)
