@@ -289,13 +289,14 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
         for (int q = 0; q < 4; ++q) {
             const int pq = pl + q;
             const int64_t src = base + (GENO ? 4 * q + (pl >> 2) : (pq < 8 ? 2 * pq : 2 * (pq - 8) + 1));
-            double x = (src < n && !bad) ? X[src + c * ld] * sc : 0.0;
+            const double raw = (src < n && !bad) ? X[src + c * ld] : 0.0;
+            double x = raw * sc;
             if (NI == ND64) x *= sc2;
             I[q] = __double2ll_rn(x);
             if constexpr (ND > ND64) {
                 const double r = (x - (double)I[q]) * (double)(1 << (DBITS * (ND - ND64)));
                 L[q] = __double2int_rn(r);
-                lost = lost || (double)L[q] != r;
+                lost = lost || (double)L[q] != r || (x == 0.0 && raw != 0.0);   // the scaling may underflow
             }
             if (isum) {
                 const long long J = NI == ND64 ? I[q] : __double2ll_rn(x * pow2i(DBITS * (ND64 - ND)));

@@ -50,6 +50,18 @@ def test_rows_of_families_of_any_magnitude(gctx, N, k, decades):
     assert (np.abs(got - want) <= TOL * size).all()
 
 
+# the smaller families' entries pass below the smallest double when the column is scaled
+@pytest.mark.parametrize("big,small", [(1e300, 1e-60), (1e300, 1e-120), (1e280, 1e-300)])
+def test_rows_across_the_range_of_a_double(gctx, big, small):
+    N = 2049
+    A = _families(gctx, N, 9)
+    Z = np.random.default_rng(6).standard_normal((N, 2))
+    Z[:, 0] *= np.where(np.arange(N) // FAM % 2, big, small)
+    got = gctx.grm_apply(Z)
+    want, size = _want(A, Z)
+    assert (np.abs(got - want) <= TOL * size + 2.0 ** -1074).all()
+
+
 # entries that the least number of planes does not hold exactly; that no number of them does
 @pytest.mark.parametrize("small", [1e-9, 3e-12, 1e-13, 1e-16, 1e-30])
 def test_rows_with_small_entries_of_a(gctx, small):
