@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt,
     }
 }
 
-// ~4 us a product where no column is marked; with one marked 4.3 ms at N = 20k, 1.2 ms at 6007 (13.0
+// 2.8 us a product where no column is marked; with one marked 4.3 ms at N = 20k, 1.2 ms at 6007 (13.0
 // and 1.5 with the FP64 pipe's conversion instruction and its loop run for unmarked columns too).
 int dense_redo_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const unsigned* wide, int nw) {
     const int32_t N = ctx->coh.N;

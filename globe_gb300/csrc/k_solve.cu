@@ -715,9 +715,9 @@ int col_unscales(globe_ctx* ctx, const double* bb, int k, double* unsc) {
 // Classes (by_length): one thread walks up to `one` records, ~0.5 us each in a chain: SOLVE_LONG where
 // one CTA's threads an SM suffice for the teams of the rest (N = 20k, records geometric with mean 10,
 // five columns: 6.44 ms a solve, 6.57 with 43), else the more the larger the solve, which takes
-// longer anyway.  Beyond, a team of TEAM threads, and
-// past 32 records for each of those (or half of `one`) the whole CTA.  A team doubles while its
-// threads have more than 16 records and all teams still run at once.  us an iteration with one
+// longer anyway.  Beyond, a team of TEAM threads, and past 32 records for each of those (or half of
+// `one`) the whole CTA.  A team doubles while its threads have more than 16 records and all teams
+// still run at once.  us an iteration with one
 // thread up to 32 and a CTA for each longer individual / with one thread for all / so (mixed; M =
 // 1000): N = 2000, 100-200 records, one column 101 / 248 / 62; N = 20000, 33-48, one 542 / 108 / 114;
 // 100-200, five 788 / 560 / 341; N = 100000, 40-60, one 2756 / 321 / 331, five 2863 / 592 / 598; N =

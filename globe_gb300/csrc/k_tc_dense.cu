@@ -25,10 +25,12 @@
 // the exact sums in double-double with one rounding at the end.  So each row is held to FP64 by
 // itself: within 2^-53 (|A| |z|)_i and the rounding, whatever the zeros of A and the magnitudes in z.
 // A column with smaller entries, or a NaN or an infinity, is formed on the FP64 pipe after the
-// others (k_digits marks it; ~1 normal column in 1000 at N = 20k), and a matrix that 14 planes do not hold stays
-// there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its epilogue; 25.1 ms on
-// the FP64 pipe, which it was bound by.  (12 digits of Z and 12 planes whatever A: 0.93 ms, but a row
-// that a column's largest entries do not enter lost up to all of its digits.)
+// others (k_digits marks it: one normal column in 700 at N = 20k), and a matrix that 14 planes do
+// not hold stays there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its
+// epilogue; 25.1 ms on the FP64 pipe, which it was bound by.  (12 digits of Z and 12 planes whatever
+// A: 0.93 ms, but a row that a column's largest entries do not enter lost up to all of its digits.
+// Marked columns formed by the combine kernel, a thread a row: 3 us less a product where there are
+// none, 16.5 ms for one at N = 20k.)
 //
 // Kernel (one CTA = 2 x 128 rows x one K range, M=128 x N=NMMA MMAs per row tile):
 //   warp 0     TMA of both operands per stage: two 128 x 128-byte tiles of the
@@ -202,10 +204,10 @@ __global__ void k_dense_scan(const float* __restrict__ lt, int64_t n, unsigned* 
 // The DA digit planes of one 64 x 64 block (I0, J0) of the full square: the block is staged
 // through shared memory (rows of the triangle left of the diagonal, columns of it right of
 // the diagonal: coalesced either way), then each thread writes 4 words of 4 K positions per
-// plane.  Position P of a group of 16 holds column 2P (P < 8) or 2(P-8)+1.  x 2^-eA is rounded once to I = round(x 2^-eA 32^(DA-1)); its balanced base-32
-// digits are peeled off from the least significant end (d = ((I + 16) mod 32) - 16); the
-// leading digit is what remains, in [-16, 16].  More than DA64 planes: those of the remainder of
-// the first DA64, as k_digits has them.
+// plane.  Position P of a group of 16 holds column 2P (P < 8) or 2(P-8)+1.  x 2^-eA is rounded once
+// to I = round(x 2^-eA 32^(DA-1)); its balanced base-32 digits are peeled off from the least
+// significant end (d = ((I + 16) mod 32) - 16); the leading digit is what remains, in [-16, 16].
+// More than DA64 planes: those of the remainder of the first DA64, as k_digits has them.
 template <int DA>
 __global__ void __launch_bounds__(256) k_dense_digits(const float* __restrict__ lt, int32_t N, int eA,
                                                       uint8_t* __restrict__ D, int64_t np) {
@@ -384,8 +386,8 @@ __global__ void __launch_bounds__(256) k_dense_combine64(const float* __restrict
         long long C = 0;
 #pragma unroll
         for (int m = 0; m < 5; ++m) C = C * 32 + (5 * q + m < NT ? T[5 * q + m] : 0);
-        dd_add(h, l, ll_times_pow2(C, q == 0 ? 1.0 : q == 1 ? 0x1p-25 : q == 2 ? 0x1p-50 : q == 3 ? 0x1p-75 : q == 4 ? 0x1p-100 : 0x1p-125),
-               0.0);
+        constexpr double W[6] = {1.0, 0x1p-25, 0x1p-50, 0x1p-75, 0x1p-100, 0x1p-125};
+        dd_add(h, l, ll_times_pow2(C, W[q]), 0.0);
     }
     out[i + c * ldo] = (h + l) * sA * scale * ea * eb + bad;
 }
