@@ -328,8 +328,9 @@ int geno_diag(globe_ctx* ctx, double* d);
 
 // k_grm_dense.cu
 int dense_apply_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
-// the columns c of the k whose words wide[c nw ..] are not all zero
-int dense_redo_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const unsigned* wide, int nw);
+namespace tc { struct Rest; }
+// out += scale A (rest), rest[c nw ..] what the digits left of Z's column c; whole columns where they say so
+int dense_rest_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const tc::Rest* rest, int nw);
 int dense_apply_df(globe_ctx* ctx, const double* Z, int k, double scale, double* out);
 int dense_diag(globe_ctx* ctx, double* d);
 

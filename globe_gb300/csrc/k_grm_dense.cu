@@ -15,42 +15,62 @@
 #include <algorithm>
 
 #include "df.cuh"
-#include "internal.cuh"
+#include "tc_common.cuh"
 
 namespace globe {
 
 constexpr int DT = 64;
 
-// REDO: of column chunk blockIdx.y, only the columns marked in wide (nw words each)
+// REDO, for the columns of chunk blockIdx.y that the digit planes formed: adds what their digits left
+// (rest, nw a column), or forms those anew of which that is not listed
 template <int KC, bool REDO>
 __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt, int32_t N,
                                                    const double* __restrict__ Z, int kc, double scale,
-                                                   double* __restrict__ out, const unsigned* __restrict__ wide, int nw) {
+                                                   double* __restrict__ out, const tc::Rest* __restrict__ rest, int nw) {
     __shared__ float At[DT][DT + 1];
     __shared__ double Zt[DT][KC];
     __shared__ int redo[KC];
     const int tid = threadIdx.x;
+    const int64_t I0 = (int64_t)blockIdx.x * DT;
+    const int row = tid & (DT - 1);
+    const int cg = tid >> 6;  // 0..3
     if (REDO) {
         const int c0 = blockIdx.y * KC;
         kc = min(KC, kc - c0);
         Z += (size_t)c0 * N;
         out += (size_t)c0 * N;
+        rest += (size_t)c0 * nw;
         if (tid < KC) redo[tid] = 0;
         __syncthreads();
         bool any = false;
-        for (int e = tid; e < kc * nw; e += 256)
-            if (wide[(size_t)c0 * nw + e]) {
-                redo[e / nw] = 1;
-                any = true;
-            }
+        for (int e = tid; e < kc * nw; e += 256) {
+            const int n = rest[e].n;
+            if (n > tc::REST_MAX) redo[e / nw] = 1;
+            any = any || n;
+        }
         if (!__syncthreads_or(any)) return;
+        const int64_t i = I0 + row;
+        for (int c = cg; c < kc && i < N; c += 4) {
+            if (redo[c]) continue;
+            double s = 0.0;
+            bool some = false;
+            for (int e = 0; e < nw; ++e) {
+                const tc::Rest& r = rest[(size_t)c * nw + e];
+                for (int t = 0; t < r.n; ++t) {
+                    const int64_t j = r.row[t], hi = max(i, j), lo = min(i, j);
+                    s = __fma_rn((double)lt[hi * (hi + 1) / 2 + lo], r.v[t], s);
+                    some = true;
+                }
+            }
+            if (some) out[i + (size_t)c * N] += scale * s;
+        }
+        any = false;
+        for (int c = 0; c < kc; ++c) any = any || redo[c];
+        if (!any) return;   // the same for every thread
     }
     bool mine = !REDO;   // whether one of the thread's columns is wanted
     if (REDO)
-        for (int c = tid >> 6; c < kc; c += 4) mine = mine || redo[c];
-    const int64_t I0 = (int64_t)blockIdx.x * DT;
-    const int row = tid & (DT - 1);
-    const int cg = tid >> 6;  // 0..3
+        for (int c = cg; c < kc; c += 4) mine = mine || redo[c];
     double acc[(KC + 3) / 4];
 #pragma unroll
     for (int q = 0; q < (KC + 3) / 4; ++q) acc[q] = 0.0;
@@ -104,12 +124,13 @@ __global__ void __launch_bounds__(256) k_dense_f64(const float* __restrict__ lt,
     }
 }
 
-// 2.8 us a product where no column is marked; with one marked 4.3 ms at N = 20k, 1.2 ms at 6007 (13.0
-// and 1.5 with the FP64 pipe's conversion instruction and its loop run for unmarked columns too).
-int dense_redo_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const unsigned* wide, int nw) {
+// 2.8 us a product where nothing is left, 2 to 7 more with an entry in each column; a whole column
+// 4.3 ms at N = 20k, 1.2 ms at 6007 (13.0 and 1.5 with the FP64 pipe's conversion instruction and
+// its loop run for the other columns too).
+int dense_rest_fp64_pipe(globe_ctx* ctx, const double* Z, int k, double scale, double* out, const tc::Rest* rest, int nw) {
     const int32_t N = ctx->coh.N;
     k_dense_f64<8, true><<<dim3(div_up(N, DT), div_up(k, 8)), 256, 0, ctx->stream>>>(ctx->gen.grm, N, Z, k, scale, out,
-                                                                                     wide, nw);
+                                                                                     rest, nw);
     GLOBE_LAUNCHED(ctx, "k_dense_f64");
     return GLOBE_OK;
 }

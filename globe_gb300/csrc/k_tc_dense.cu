@@ -24,13 +24,11 @@
 // which hold an entry exactly or to 2^-53 of itself down to 2^-25 of the column's largest; it folds
 // the exact sums in double-double with one rounding at the end.  So each row is held to FP64 by
 // itself: within 2^-53 (|A| |z|)_i and the rounding, whatever the zeros of A and the magnitudes in z.
-// A column with smaller entries, or a NaN or an infinity, is formed on the FP64 pipe after the
-// others (k_digits marks it: one normal column in 700 at N = 20k), and a matrix that 14 planes do
-// not hold stays there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its
+// What the digits leave of smaller entries (one normal column in 700 has one at N = 20k) is added on
+// the FP64 pipe afterwards; columns with many such entries, or with a NaN or an infinity, are formed
+// there, and a matrix that 14 planes do not hold stays there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its
 // epilogue; 25.1 ms on the FP64 pipe, which it was bound by.  (12 digits of Z and 12 planes whatever
-// A: 0.93 ms, but a row that a column's largest entries do not enter lost up to all of its digits.
-// Marked columns formed by the combine kernel, a thread a row: 3 us less a product where there are
-// none, 16.5 ms for one at N = 20k.)
+// A: 0.93 ms, but a row that a column's largest entries do not enter lost up to all of its digits.)
 //
 // Kernel (one CTA = 2 x 128 rows x one K range, M=128 x N=NMMA MMAs per row tile):
 //   warp 0     TMA of both operands per stage: two 128 x 128-byte tiles of the
@@ -526,10 +524,9 @@ static int dense_cps(globe_ctx* ctx, int tiles, int nchunks, int nmma) {
 
 static int digit_ctas(int64_t np) { return (int)std::min<int64_t>(div_up(np / 4, 256), 1024); }
 
-// out (N x kg) = scale * A Z for one group of <= 256 / ND columns; wide: k_digits' words
+// out (N x kg) = scale * A Z for one group of <= 256 / ND columns; rest: k_digits' (NDZ)
 template <int ND>
-static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st,
-                       unsigned* wide) {
+static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, double* out, const TcStat& st, Rest* rest) {
     constexpr bool F64 = ND == NDZ;
     const auto& a = ctx->gen.adig[F64 ? 1 : 0];
     const int32_t N = ctx->coh.N;
@@ -552,7 +549,7 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
     GLOBE_RET(make_map(ctx, &mA, a.p, (uint64_t)np, (uint64_t)rows, BK, BM, true));
     GLOBE_RET(make_map(ctx, &mB, D, (uint64_t)np, (uint64_t)nmma, BK, (uint32_t)nmma, true));
     k_digits<ND, false><<<dim3((unsigned)digit_ctas(np), kg), 256, 0, ctx->stream>>>(
-        Z, N, N, st.zhi, col, D, np, nullptr, nullptr, nmma - kg * ND, wide);
+        Z, N, N, st.zhi, col, D, np, nullptr, nullptr, nmma - kg * ND, rest);
     GLOBE_LAUNCHED(ctx, "k_digits");
     {
         ProfScope p(ctx, GLOBE_PROF_GRM_PASS1);
@@ -577,17 +574,17 @@ static int dense_group(globe_ctx* ctx, const double* Z, int kg, double scale, do
 }
 
 static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, double scale, double* out, const TcStat& st,
-                          unsigned* wide) {
+                          Rest* rest) {
     switch (nd) {
-        case 2: return dense_group<2>(ctx, Z, kg, scale, out, st, wide);
-        case 3: return dense_group<3>(ctx, Z, kg, scale, out, st, wide);
-        case 4: return dense_group<4>(ctx, Z, kg, scale, out, st, wide);
-        case 5: return dense_group<5>(ctx, Z, kg, scale, out, st, wide);
-        case 6: return dense_group<6>(ctx, Z, kg, scale, out, st, wide);
-        case 7: return dense_group<7>(ctx, Z, kg, scale, out, st, wide);
-        case 8: return dense_group<8>(ctx, Z, kg, scale, out, st, wide);
-        case 9: return dense_group<9>(ctx, Z, kg, scale, out, st, wide);
-        case NDZ: return dense_group<NDZ>(ctx, Z, kg, scale, out, st, wide);
+        case 2: return dense_group<2>(ctx, Z, kg, scale, out, st, rest);
+        case 3: return dense_group<3>(ctx, Z, kg, scale, out, st, rest);
+        case 4: return dense_group<4>(ctx, Z, kg, scale, out, st, rest);
+        case 5: return dense_group<5>(ctx, Z, kg, scale, out, st, rest);
+        case 6: return dense_group<6>(ctx, Z, kg, scale, out, st, rest);
+        case 7: return dense_group<7>(ctx, Z, kg, scale, out, st, rest);
+        case 8: return dense_group<8>(ctx, Z, kg, scale, out, st, rest);
+        case 9: return dense_group<9>(ctx, Z, kg, scale, out, st, rest);
+        case NDZ: return dense_group<NDZ>(ctx, Z, kg, scale, out, st, rest);
     }
     return set_err(ctx, GLOBE_ERR_ARG, "unsupported digit count %d", nd);
 }
@@ -596,8 +593,8 @@ static int dense_group_nd(globe_ctx* ctx, int nd, const double* Z, int kg, doubl
 static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double scale, double* out, bool zhi_ready) {
     PinScope pin(ctx, nd == NDZ ? PIN_TC | PIN_PLANES64 : PIN_TC);
     const int nw = digit_ctas(ctx->gen.adig[nd == NDZ ? 1 : 0].np);
-    unsigned* wide = nullptr;
-    if (nd == NDZ) GLOBE_RET(ws(ctx, WS_TC_U, (size_t)k * nw, &wide));
+    Rest* rest = nullptr;
+    if (nd == NDZ) GLOBE_RET(ws(ctx, WS_TC_U, (size_t)k * nw, &rest));
     TcStat st;
     GLOBE_RET(tc_stat_fill(ctx, Z, ctx->coh.N, k, &zhi_ready, &st));
     const int gmax = 256 / nd;   // MMA width <= 256; near-equal groups
@@ -605,11 +602,11 @@ static int dense_apply_nd(globe_ctx* ctx, int nd, const double* Z, int k, double
     for (int gi = 0, c0 = 0; gi < ng; ++gi) {
         const int kg = k / ng + (gi < k % ng ? 1 : 0);
         GLOBE_RET(dense_group_nd(ctx, nd, Z + (size_t)c0 * ctx->coh.N, kg, scale, out + (size_t)c0 * ctx->coh.N,
-                                 st.from(c0), wide ? wide + (size_t)c0 * nw : nullptr));
+                                 st.from(c0), rest ? rest + (size_t)c0 * nw : nullptr));
         c0 += kg;
     }
     ctx->stat_dirty = false;
-    return wide ? dense_redo_fp64_pipe(ctx, Z, k, scale, out, wide, nw) : GLOBE_OK;
+    return rest ? dense_rest_fp64_pipe(ctx, Z, k, scale, out, rest, nw) : GLOBE_OK;
 }
 
 int dense_apply_tc(globe_ctx* ctx, const double* Z, int k, double scale, double* out, bool zhi_ready) {

@@ -256,13 +256,22 @@ __global__ void k_col_max(const double* __restrict__ X, int64_t n, int64_t ld, u
 // width is a multiple of 16; a memset of them cost a launch of its own).  With ND64 digits and more
 // (the FP64 products) the scaling takes two factors where one would leave the range of a double.
 // NDZ digits: the first ND64 as above, then those of the remainder x 2^-e 32^(ND64-1) - I, which is
-// exact in a double and at most 1/2.  wide[c gridDim.x + CTA] says whether an entry of the CTA has bits
-// below the last digit (it is then more than 2^25 below the column's largest), or the column is bad.
+// exact in a double and at most 1/2.  An entry more than 2^25 below the column's largest may have bits
+// below the last digit still: what the digits leave of such entries goes to rest[c gridDim.x + CTA], by
+// rising row; their number is left_any where they do not fit or cannot be told (a bad column, an
+// entry that the scaling takes to zero).
+constexpr int REST_MAX = 8;       // entries of a Rest
+constexpr int left_any = REST_MAX + 1;
+struct Rest {
+    double v[REST_MAX];           // z = (its digits) + v
+    int row[REST_MAX];
+    int n, pad;
+};
 template <int ND, bool GENO>
 __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, const unsigned* __restrict__ hi,
                          double* __restrict__ colinfo, uint8_t* __restrict__ D, int64_t kpad,
                          unsigned long long* __restrict__ isum, unsigned long long* __restrict__ clear, int npad,
-                         unsigned* __restrict__ wide = nullptr) {
+                         Rest* __restrict__ rest = nullptr) {
     constexpr int NI = ND < ND64 ? ND : ND64;   // digits of I
     const int c = blockIdx.y;
     const unsigned h = hi[c];
@@ -278,7 +287,13 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
     }
     const int64_t nw = kpad >> 2;
     long long sum_hi = 0, sum_lo = 0;
-    bool lost = bad;
+    __shared__ int nrest;
+    Rest* left = nullptr;
+    if constexpr (ND > ND64) {
+        left = rest + (size_t)c * gridDim.x + blockIdx.x;
+        if (threadIdx.x == 0) nrest = bad ? left_any : 0;
+        __syncthreads();
+    }
     for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (int64_t)gridDim.x * blockDim.x) {
         const int64_t P = w << 2, base = P & ~(int64_t)15;
         const int pl = (int)(P & 15);
@@ -296,7 +311,15 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
             if constexpr (ND > ND64) {
                 const double r = (x - (double)I[q]) * (double)(1 << (DBITS * (ND - ND64)));
                 L[q] = __double2int_rn(r);
-                lost = lost || (double)L[q] != r || (x == 0.0 && raw != 0.0);   // the scaling may underflow
+                const double d = r - (double)L[q];   // exact
+                if (x == 0.0 && raw != 0.0) atomicAdd(&nrest, left_any);
+                else if (d != 0.0) {
+                    const int at = atomicAdd(&nrest, 1);
+                    if (at < REST_MAX) {
+                        left->v[at] = ldexp(d, e - DBITS * (ND - 1));
+                        left->row[at] = (int)src;
+                    }
+                }
             }
             if (isum) {
                 const long long J = NI == ND64 ? I[q] : __double2ll_rn(x * pow2i(DBITS * (ND64 - ND)));
@@ -342,8 +365,20 @@ __global__ void k_digits(const double* __restrict__ X, int64_t n, int64_t ld, co
         }
     }
     if constexpr (ND > ND64) {
-        const int any = __syncthreads_or(lost);
-        if (threadIdx.x == 0) wide[(size_t)c * gridDim.x + blockIdx.x] = any ? 1u : 0u;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int m = min(nrest, left_any);
+            left->n = m;
+            for (int a = 1; a < m && m <= REST_MAX; ++a)   // into one order, whatever the threads' was
+                for (int b = a; b > 0 && left->row[b - 1] > left->row[b]; --b) {
+                    const int t = left->row[b];
+                    left->row[b] = left->row[b - 1];
+                    left->row[b - 1] = t;
+                    const double v = left->v[b];
+                    left->v[b] = left->v[b - 1];
+                    left->v[b - 1] = v;
+                }
+        }
     }
 }
 

@@ -55,8 +55,8 @@ extern "C" {
                                second genotype copy does not fit in device memory.  Dense GRM
                                products from 12 to 14 digit planes that hold A exactly (12 to
                                14 N^2 bytes) and 16 digits a column, each row within a few
-                               units of 2^-53 (|A| |z|)_i; columns with entries that those
-                               digits do not hold, and the non-finite ones, on the FP64 pipe.
+                               units of 2^-53 (|A| |z|)_i; what those digits leave of small
+                               entries, and non-finite columns, on the FP64 pipe.
                                The second copy, the planes and the products' workspaces (a GRM
                                build's: up to 2 GB) stay with the context; an allocation of
                                the context that finds no memory takes them */

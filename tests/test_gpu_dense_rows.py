@@ -50,6 +50,27 @@ def test_rows_of_families_of_any_magnitude(gctx, N, k, decades):
     assert (np.abs(got - want) <= TOL * size).all()
 
 
+# what the digits leave of a few entries is added: 1 to 8 in one range of rows, in several, past 8 (then the
+# whole column is formed anew), and of the smallest magnitudes
+@pytest.mark.parametrize("rows", [[3], [40, 41, 42, 43, 44, 45, 46, 47], [80, 81, 82, 83, 84, 85, 86, 87, 88],
+                                  [0, 1023, 1024, 2048], list(range(5, 2049, 130))])
+@pytest.mark.parametrize("small", [1e-9, 1e-40])
+def test_rows_of_a_few_small_entries(gctx, rows, small):
+    N = 2049
+    A = _families(gctx, N, 10)
+    rng = np.random.default_rng(len(rows))
+    Z = rng.standard_normal((N, 9))
+    Z += np.sign(Z) * 0.5                              # the others are within 2^4 of the largest
+    for r in rows:                                     # a family of its own scale each
+        Z[r // FAM * FAM:r // FAM * FAM + FAM, 1::2] = 0.0
+    for r in rows:
+        Z[r, 1::2] = small * rng.standard_normal(4)
+    got = gctx.grm_apply(Z)
+    want, size = _want(A, Z)
+    assert (np.abs(got - want) <= TOL * size).all()
+    assert np.array_equal(got, gctx.grm_apply(Z))
+
+
 # the smaller families' entries pass below the smallest double when the column is scaled
 @pytest.mark.parametrize("big,small", [(1e300, 1e-60), (1e300, 1e-120), (1e280, 1e-300)])
 def test_rows_across_the_range_of_a_double(gctx, big, small):
