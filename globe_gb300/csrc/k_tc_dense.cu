@@ -26,9 +26,10 @@
 // itself: within 2^-53 (|A| |z|)_i and the rounding, whatever the zeros of A and the magnitudes in z.
 // What the digits leave of smaller entries (one normal column in 700 has one at N = 20k) is added on
 // the FP64 pipe afterwards; columns with many such entries, or with a NaN or an infinity, are formed
-// there, and a matrix that 14 planes do not hold stays there altogether.  N = 20k, k = 16 streams 12 N^2 = 4.8 GB in 1.0 ms with its
-// epilogue; 25.1 ms on the FP64 pipe, which it was bound by.  (12 digits of Z and 12 planes whatever
-// A: 0.93 ms, but a row that a column's largest entries do not enter lost up to all of its digits.)
+// there, and a matrix that 14 planes do not hold stays there altogether.  N = 20k, k = 16 streams 12
+// N^2 = 4.8 GB in 1.0 ms with its epilogue; 25.1 ms on the FP64 pipe, which it was bound by.  (12
+// digits of Z and 12 planes whatever A: 0.93 ms, but a row that a column's largest entries do not
+// enter lost up to all of its digits.)
 //
 // Kernel (one CTA = 2 x 128 rows x one K range, M=128 x N=NMMA MMAs per row tile):
 //   warp 0     TMA of both operands per stage: two 128 x 128-byte tiles of the
